@@ -183,10 +183,9 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     double *W = static_cast<double *>(pf->weight);
     double *S = static_cast<double *>(pf->state);
     Scratch scratch(st);
-    uint32_t *err = scratch.get<uint32_t>(1);
+    uint32_t *err = new_err(scratch, st);
     if (err == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
-    VSMC_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
     if (first) {
         // Sampler::initialize: resampling engine key {0, seed}, counter
         // {0, 0, 1, 0}; log-evidence 0

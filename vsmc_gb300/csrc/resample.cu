@@ -887,10 +887,9 @@ int consumed_words(size_t m, size_t n, const int *rep_dev, const int *integ_dev,
 int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
     int *rep, int scheme, Scratch &scratch, cudaStream_t st)
 {
-    uint32_t *err = scratch.get<uint32_t>(1);
+    uint32_t *err = new_err(scratch, st);
     if (err == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
-    VSMC_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
     const bool residual = scheme >= VSMC_CUDA_RESIDUAL;
     const int base = residual ? scheme - VSMC_CUDA_RESIDUAL : scheme;
     const double *wt = w;
@@ -1064,10 +1063,9 @@ int with_err(void *stream, F body)
 {
     cudaStream_t st = as_stream(stream);
     Scratch scratch(st);
-    uint32_t *err = scratch.get<uint32_t>(1);
+    uint32_t *err = new_err(scratch, st);
     if (err == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
-    VSMC_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
     int rc = body(err, scratch, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
