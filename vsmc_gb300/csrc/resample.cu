@@ -13,6 +13,7 @@
 #include "seqsum.cuh"
 #include "resample_internal.cuh"
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -38,10 +39,10 @@ __global__ void k_fill_i32(size_t n, int *p, int v)
     GRID_LOOP(i, n) p[i] = v;
 }
 
-__global__ void k_set_one(int *p, int v)
+// counts without uniforms to compare: v for every particle, plus integ
+__global__ void k_rep_trivial(size_t m, int v, int *rep, const int *integ)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        *p = v;
+    GRID_LOOP(i, m) rep[i] = v + (integ ? integ[i] : 0);
 }
 
 // max-scan key: NaN compares as "above everything", as the reference's
@@ -60,21 +61,6 @@ struct StoreD {
     double *p;
     __device__ void operator()(size_t i, double v) const { p[i] = v; }
 };
-
-// #{j < n : pm_j <= x} (pm non-decreasing)
-__device__ __forceinline__ size_t upper_count(
-    const double *pm, size_t n, double x)
-{
-    size_t lo = 0, hi = n;
-    while (lo < hi) {
-        const size_t mid = lo + (hi - lo) / 2;
-        if (pm[mid] <= x)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
 
 // #{i < m : s_i < x} (s non-decreasing): the first i with s_i >= x
 __device__ __forceinline__ size_t lower_count(
@@ -145,6 +131,10 @@ struct KeysMax {
     {
         return pmk[j];
     }
+    __device__ __forceinline__ const void *at(size_t j) const
+    {
+        return pmk + j;
+    }
 };
 
 struct KeysOwn {
@@ -154,6 +144,7 @@ struct KeysOwn {
         // okey of a non-negative, non-NaN double is its bit pattern
         return __double_as_longlong(u[j]);
     }
+    __device__ __forceinline__ const void *at(size_t j) const { return u + j; }
 };
 
 // The first index j >= lo with pmk_j > x (hi if none), given that every
@@ -229,36 +220,161 @@ __device__ __forceinline__ size_t guess_cn(double c, size_t n)
     return g < n ? static_cast<size_t>(g) : n;
 }
 
-// F[i] = #{j < n : pmk_j <= key(cdf_i)} for i < m - 1, both sequences
-// non-decreasing.  Every scheme spreads its uniforms over [0, 1), so the
-// answer is near n cdf_i: an exponential search from that guess needs a few
-// loads, and consecutive lanes touch neighbouring addresses.  A weight that
-// takes many copies costs a logarithmic number of loads.
-template <class Keys>
-__global__ void __launch_bounds__(kB) k_counts(size_t m, size_t n,
-    const double *cdf, const Keys pmk, uint32_t *F)
+// guess_cn for c >= 0: the high product of c's top 32 significant bits and n
+__device__ __forceinline__ uint32_t guess_below(double c, uint32_t n)
 {
-    GRID_LOOP(i, m - 1)
-    {
-        const double c = cdf[i];
-        F[i] = static_cast<uint32_t>(
-            count_from(pmk, n, okey_cdf(c), guess_cn(c, n)));
-    }
+    const uint32_t h = static_cast<uint32_t>(__double2hiint(c));
+    const uint32_t l = static_cast<uint32_t>(__double2loint(c));
+    const uint32_t ef = h >> 20;
+    const uint32_t m = __funnelshift_l(l, h, 11) | 0x80000000u;
+    return ef < 1023u ? __umulhi(m, n) >> min(1022u - ef, 31u) : n;
 }
 
-__global__ void k_rep_from_counts(size_t m, size_t n, const uint32_t *F,
-    int *rep, const int *integ)
+// The first index j >= lo with pmk_j > x, given that every j < lo has
+// pmk_j <= x: exponential search upwards.
+template <class Keys>
+__device__ __forceinline__ size_t count_ahead(
+    const Keys &pmk, size_t n, long long x, size_t lo)
 {
-    GRID_LOOP(i, m)
-    {
-        const uint32_t hi = i + 1 < m ? F[i] : static_cast<uint32_t>(n);
-        const uint32_t lo = i > 0 ? F[i - 1] : 0u;
-        int r = static_cast<int>(hi - lo);
-        if (integ)
-            r += integ[i];
-        rep[i] = r;
+    size_t hi = n, step = 1;
+    while (lo < n) {
+        const size_t probe = lo + step - 1;
+        if (probe >= n)
+            break;
+        if (pmk[probe] > x) {
+            hi = probe;
+            break;
+        }
+        lo = probe + 1;
+        step <<= 1;
     }
+    return first_above(pmk, lo, hi, x);
 }
+
+// Replication counts straight from the running sums of the weights (an
+// output functor of the sequential sum, so the CDF is never stored): with
+// F_i = #{j < n : pmk_j <= key(cdf_i)} (n for the last particle, whose CDF
+// value the loop never compares), rep_i = F_i - F_{i-1}, plus integ_i where
+// the integer parts are given.
+//   Near: stratified and systematic uniforms, u_j in [j / n, (j + 1) / n] up
+//   to rounding.  The answer is floor(n cdf) or one more: eight guesses of a
+//   thread are loaded together, then the neighbours that confirm them; a
+//   search runs only where one does not.  Striped elements (a warp's lanes
+//   consecutive), so each load touches a few neighbouring lines; blocked
+//   ones touched 16 and the pass took 123 us at 2^24.
+//   else: blocked elements, the thread's first count by exponential search
+//   from n cdf, each next one upwards from the one before (for sorted
+//   uniforms n cdf is off by about sqrt(n), the previous count by a few).
+template <class Keys, bool Near>
+struct SeqCount {
+    Keys pmk;
+    uint32_t m, n;
+    int *rep;
+    const int *integ; // may be null
+    uint32_t *tail;   // the uniforms left to the last particle
+
+    // line l of the uniforms that a tile starting at CDF value c compares
+    __device__ __forceinline__ void prefetch(double c, uint32_t l) const
+    {
+        const uint32_t j = guess_below(c, n) + 16 * l;
+        if (j < n)
+            seq_prefetch(pmk.at(j));
+    }
+
+    __device__ __forceinline__ uint32_t search(double c) const
+    {
+        return static_cast<uint32_t>(
+            count_from(pmk, n, okey_cdf(c), guess_cn(c, n)));
+    }
+
+    __device__ __forceinline__ int one(
+        uint32_t i, uint32_t F, uint32_t &Fl) const
+    {
+        const uint32_t Fk = i + 1 < m ? F : n;
+        int r = static_cast<int>(Fk - Fl);
+        Fl = Fk;
+        if (i + 1 == m)
+            *tail = static_cast<uint32_t>(r);
+        if (integ && i < m)
+            r += integ[i];
+        return r;
+    }
+
+    __device__ __forceinline__ void operator()(uint32_t tile, uint32_t i0,
+        const double (&s)[kSeqItems], double sprev, SeqSmem &sh) const
+    {
+        const uint32_t lane = threadIdx.x & 31;
+        if (Near) {
+            double c[kSeqItems];
+            seq_to_striped(sh.row[threadIdx.x >> 5], s, c);
+            long long x[kSeqItems]; // keys of non-negative sums: their bits
+            uint32_t F[kSeqItems];
+            bool at[kSeqItems];
+#pragma unroll
+            for (int k = 0; k < kSeqItems; ++k) {
+                x[k] = __double_as_longlong(c[k]);
+                F[k] = guess_below(c[k], n);
+            }
+#pragma unroll
+            for (int k = 0; k < kSeqItems; ++k)
+                at[k] = F[k] < n && pmk[F[k]] <= x[k];
+#pragma unroll
+            for (int k = 0; k < kSeqItems; ++k) {
+                // confirms g + 1 (the next uniform is above) or g (the one
+                // before is not)
+                const uint32_t g = F[k];
+                const bool ok = at[k] ? g + 1 == n || pmk[g + 1] > x[k]
+                                      : g == 0 || pmk[g - 1] <= x[k];
+                F[k] = ok ? g + (at[k] ? 1u : 0u)
+                          : static_cast<uint32_t>(count_from(pmk, n, x[k], g));
+            }
+            // the counts before the warp's first element, then row by row
+            uint32_t Fw = i0 == 0 && lane == 0 ? 0u : search(sprev);
+            Fw = __shfl_sync(0xFFFFFFFFu, Fw, 0);
+#pragma unroll
+            for (int k = 0; k < kSeqItems; ++k) {
+                uint32_t Fl = __shfl_up_sync(0xFFFFFFFFu, F[k], 1);
+                if (lane == 0)
+                    Fl = Fw;
+                Fw = __shfl_sync(0xFFFFFFFFu, F[k], 31);
+                const uint32_t i = seq_striped(tile, k);
+                const int r = one(i, F[k], Fl);
+                if (i < m)
+                    rep[i] = r;
+            }
+            return;
+        }
+        uint32_t F[kSeqItems];
+        F[0] = search(s[0]);
+#pragma unroll
+        for (int k = 1; k < kSeqItems; ++k)
+            F[k] = static_cast<uint32_t>(
+                count_ahead(pmk, n, okey_cdf(s[k]), F[k - 1]));
+        uint32_t Fl = __shfl_up_sync(0xFFFFFFFFu, F[kSeqItems - 1], 1);
+        if (lane == 0)
+            Fl = i0 == 0 ? 0u : search(sprev);
+#pragma unroll
+        for (int k = 0; k < kSeqItems; ++k) {
+            const int r = one(i0 + k, F[k], Fl);
+            if (i0 + k < m)
+                rep[i0 + k] = r;
+        }
+    }
+};
+
+// the weights of all particles but the last, whose CDF value is not formed
+struct SeqLoadCdf {
+    const double *w;
+    uint32_t last;
+    __device__ __forceinline__ double operator()(uint32_t i) const
+    {
+        return i < last ? w[i] : 0.0;
+    }
+    __device__ __forceinline__ const double *at(uint32_t i) const
+    {
+        return w + i;
+    }
+};
 
 __global__ void k_index_from_cdf(size_t m, size_t n, const double *cdf,
     const double *pm, int *idx)
@@ -285,36 +401,41 @@ __device__ __forceinline__ uint32_t stream_word(const EngineState &e, size_t k)
     return i == 0 ? b.x : (i == 1 ? b.y : (i == 2 ? b.z : b.w));
 }
 
-// x * 2^-e rounded to the nearest double, ties to even, for 0 <= x < 2^63
-// and a result in the normal range: the rounding of an exact value to 53
-// significant bits done on the integer (IEEE 754 round-to-nearest-even),
-// and the double assembled from its bits, so no FP64 instruction runs.
+// x * 2^-e rounded to the nearest double, ties to even, for a result in the
+// normal range: x normalized to 64 bits, its low 11 bits rounded away and
+// the double assembled from its bits, about 17 integer instructions (the
+// integer conversion takes 16 cycles of an SM per warp, twice as many).
 __device__ __forceinline__ double rne_scaled(uint64_t x, int e)
 {
-    if (x == 0)
-        return 0.0;
-    int b = 64 - __clzll(static_cast<long long>(x)); // significant bits
-    uint64_t m = x;
-    int sh = 0;
-    if (b > 53) {
-        sh = b - 53;
-        const uint64_t rest = x & ((1ull << sh) - 1);
-        const uint64_t half = 1ull << (sh - 1);
-        m = x >> sh;
-        if (rest > half || (rest == half && (m & 1)))
-            ++m;
-        if (m >> 53) { // rounded up to 2^53
-            m >>= 1;
-            ++sh;
-        }
-        b = 53;
-    }
-    // value = m * 2^(sh - e), m < 2^53 with b significant bits
-    const int exp2 = b - 1 + sh - e; // unbiased exponent of the result
-    const uint64_t frac = (m << (53 - b)) & ((1ull << 52) - 1);
-    const uint64_t bits =
-        (static_cast<uint64_t>(exp2 + 1023) << 52) | frac;
-    return __longlong_as_double(static_cast<long long>(bits));
+    const int lz = __clzll(static_cast<long long>(x));
+    const uint64_t y = x << (lz & 63);
+    const uint32_t lo = static_cast<uint32_t>(y);
+    const uint64_t up = (lo & 0x7FFu) + ((lo >> 11) & 1u) > 0x400u ? 1u : 0u;
+    // the leading bit of y >> 11 (and a carry out of the rounding) adds one
+    // to the exponent field
+    const uint64_t field = static_cast<uint64_t>(63 - lz - e + 1022) << 52;
+    return x == 0 ? 0.0
+                  : __longlong_as_double(
+                        static_cast<long long>(field + (y >> 11) + up));
+}
+
+// four consecutive doubles to a 32-byte aligned place in one store (four
+// 8-byte stores of a warp write each 32-byte sector four times over)
+__device__ __forceinline__ void store4(double *p, const double (&v)[4])
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};"
+                 :
+                 : "l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+
+// fl(v delta) for a 32-bit v with one FP64 instruction: 2^52 + v from its
+// bits, times delta, minus 2^52 delta (exact), rounded once.
+__device__ __forceinline__ double mul_u32(
+    uint32_t v, double delta, double minus52delta)
+{
+    return __fma_rn(
+        __hiloint2double(0x43300000, static_cast<int>(v)), delta, minus52delta);
 }
 
 // U01SequenceStratified: u_j = U_j * delta + j * delta.  Word j is at
@@ -322,10 +443,24 @@ __device__ __forceinline__ double rne_scaled(uint64_t x, int e)
 // positions 4b .. 4b + 3.  For n = 2^k (log2n = k, else -1) delta is exact,
 // both products are exact scalings of U_j = w 2^-32 and j, and the one
 // rounding is that of the sum: u_j = RNE(j 2^32 + w) 2^-(32 + k), formed in
-// integers (rne_scaled).  Otherwise the FP64 arithmetic of the reference.
+// integers (rne_scaled).  Otherwise the FP64 arithmetic of the reference in
+// three instructions.
+//
+// What is stored is the running maximum.  For n = 2^k that is u_j itself (a
+// non-decreasing integer sequence rounded to nearest).  Otherwise, with
+// eps = 2^-53, u_i <= (i + 1) delta (1 + 3 eps) and u_j >= j delta (1 - eps),
+// so u_j is below no uniform but possibly u_{j-1}, and below that one only
+// if U_{j-1} - U_j >= 1 - 4 (j + 2) eps, that is word j below 2^34 (n + 2)
+// eps <= 2^12: there word j - 1 is drawn again and the larger uniform kept.
+// u - first is 32-byte aligned, so a block's four uniforms are one store.
 __global__ void k_stratified_seq(EngineState e, size_t n, int log2n, double *u)
 {
     const double delta = 1.0 / static_cast<double>(n);
+    const double d32 = delta * 0x1p-32;
+    const double m52 = -0x1p52 * delta, m20 = -0x1p20 * delta;
+    auto form = [&](uint32_t w, uint32_t j) {
+        return __dadd_rn(mul_u32(w, d32, m20), mul_u32(j, delta, m52));
+    };
     const uint64_t first = e.index;
     const uint64_t nblk = (first + n + 3) / 4;
     GRID_LOOP(b, nblk)
@@ -334,26 +469,36 @@ __global__ void k_stratified_seq(EngineState e, size_t n, int log2n, double *u)
         ctr32_add(c, b);
         const u32x4 w = philox4x32_10(c[0], c[1], c[2], c[3], e.k0, e.k1);
         const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+        double v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint64_t pos = 4 * static_cast<uint64_t>(b) + k;
-            if (pos < first || pos - first >= n)
-                continue;
-            const size_t j = static_cast<size_t>(pos - first);
+            // wraps before the first word, whose values are not stored
+            const uint32_t j =
+                static_cast<uint32_t>(4 * static_cast<uint64_t>(b) + k - first);
             if (log2n >= 0) {
-                u[j] = rne_scaled((static_cast<uint64_t>(j) << 32) | ws[k],
+                v[k] = rne_scaled((static_cast<uint64_t>(j) << 32) | ws[k],
                     32 + log2n);
             } else {
-                const double U = u01_co_d(ws[k]);
-                u[j] = __dadd_rn(__dmul_rn(U, delta),
-                    __dmul_rn(static_cast<double>(j), delta));
+                v[k] = form(ws[k], j);
+                if (ws[k] < (1u << 13) && j > 0 && j < n)
+                    v[k] = fmax(v[k], form(stream_word(e, j - 1), j - 1));
             }
+        }
+        const uint64_t p0 = 4 * static_cast<uint64_t>(b);
+        if (p0 >= first && p0 + 4 - first <= n) {
+            store4(u + (p0 - first), v);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (p0 + k >= first && p0 + k - first < n)
+                    u[p0 + k - first] = v[k];
         }
     }
 }
 
 // U01SequenceSystematic: u0 = U * delta, u_j = u0 + j * delta (for n = 2^k
-// the same integer rounding with one word for every j)
+// the same integer rounding with one word for every j); non-decreasing, as
+// every operation is monotone in j
 __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
 {
     const uint32_t w0 = stream_word(e, 0);
@@ -364,12 +509,20 @@ __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
     }
     const double delta = 1.0 / static_cast<double>(n);
     const double u0 = __dmul_rn(u01_co_d(w0), delta);
+    const double m52 = -0x1p52 * delta;
     GRID_LOOP(j, n)
-    u[j] = __dadd_rn(u0, __dmul_rn(static_cast<double>(j), delta));
+    u[j] = __dadd_rn(u0, mul_u32(static_cast<uint32_t>(j), delta, m52));
 }
 
+// Threads of a block where each element takes many FP64 instructions (19
+// cycles of an SM each): small blocks spread a short vector over all SMs.
+constexpr int kB64 = 64;
+
+int grid64(size_t n) { return grid_for(n ? n : 1, kB64, 1, 32); }
+
 // U01SequenceSorted terms: -log(U_j) / (n - j), summed left to right below
-__global__ void k_sorted_terms(EngineState e, size_t n, double *t)
+__global__ void __launch_bounds__(kB64) k_sorted_terms(
+    EngineState e, size_t n, double *t)
 {
     GRID_LOOP(j, n)
     {
@@ -378,15 +531,47 @@ __global__ void k_sorted_terms(EngineState e, size_t n, double *t)
     }
 }
 
-__global__ void k_sorted_terms_arr(size_t n, const double *u01, double *t)
+__global__ void __launch_bounds__(kB64) k_sorted_terms_arr(
+    size_t n, const double *u01, double *t)
 {
     GRID_LOOP(j, n) t[j] = -(log(u01[j]) / static_cast<double>(n - j));
 }
 
-// u_j = 1 - exp(lmax_j), lmax_j = -prefix_j
-__global__ void k_sorted_finish(size_t n, const double *neg_lmax, double *u)
+// The sorted uniforms u_j = 1 - exp(lmax_j), lmax_j = -s_j, from the running
+// sums s.  They are non-decreasing up to exp's last bit: *unsorted is set
+// where two sums are within 2^-50 (exp is within an ulp, so a larger step
+// cannot be reversed).
+__global__ void __launch_bounds__(kB64) k_sorted_finish(
+    size_t n, const double *s, double *u, uint32_t *unsorted)
 {
-    GRID_LOOP(j, n) u[j] = 1.0 - exp(-neg_lmax[j]);
+    GRID_LOOP(j, n)
+    {
+        const double sj = s[j];
+        if (unsorted && j > 0 && !(sj - s[j - 1] >= 0x1p-50))
+            *unsorted = 1;
+        u[j] = 1.0 - exp(-sj);
+    }
+}
+
+// The running maximum of u in place by one block, if *unsorted (rare, so one
+// block is enough): non-negative doubles order as their bits.
+__global__ void __launch_bounds__(1024) k_running_max(
+    size_t n, double *u, const uint32_t *unsorted)
+{
+    if (*unsorted == 0)
+        return;
+    long long carry = 0;
+    for (size_t base = 0; base < n; base += 1024) {
+        const size_t i = base + threadIdx.x;
+        const long long v = i < n ? __double_as_longlong(u[i]) : 0;
+        long long tot;
+        const long long ex =
+            block_excl_any<long long, OpMaxK, 1024>(v, OpMaxK(), 0, &tot);
+        const long long r = OpMaxK()(carry, OpMaxK()(ex, v));
+        if (i < n)
+            u[i] = __longlong_as_double(r);
+        carry = OpMaxK()(carry, tot);
+    }
 }
 
 __global__ void k_stratified_arr(size_t n, const double *u01, double *out)
@@ -709,59 +894,53 @@ bool size_ok(size_t n) { return n < (size_t(1) << 31); }
 
 // ------------------------------------------------------- internal entries
 
+// the words of new_err past the sums' tickets
+constexpr int kErrUnsorted = 3; // sorted uniforms that step back
+constexpr int kErrTail = 4;     // uniforms left to the last particle
+
 // rep for m weights against n uniforms u (device); integ added if non-null.
-// sorted: the caller knows u is non-decreasing, non-negative and free of
-// NaN (the integer stratified / systematic sequences for N = 2^k), so its
-// running maximum is u itself and is not formed.
+// The uniforms left to the last particle go to err[kErrTail] (m >= 2, n > 0).
 int u01_rep_device(size_t m, size_t n, const double *w, const double *u,
-    int *rep, const int *integ, uint32_t *err, Scratch &scratch,
-    cudaStream_t st, bool sorted)
+    UniformOrder order, int *rep, const int *integ, uint32_t *err,
+    Scratch &scratch, cudaStream_t st)
 {
     if (m == 0)
         return VSMC_CUDA_OK;
     if (m == 1 || n == 0) {
-        if (m == 1) {
-            k_set_one<<<1, 32, 0, st>>>(rep, static_cast<int>(n));
-            VSMC_CUDA_CHECK_LAUNCH();
-            if (integ)
-                k_rep_from_counts<<<1, 32, 0, st>>>(1, n, nullptr, rep, integ);
-        } else {
-            k_fill_i32<<<grid1(m), kB, 0, st>>>(m, rep, 0);
-            VSMC_CUDA_CHECK_LAUNCH();
-            if (integ) {
-                uint32_t *F = scratch.get<uint32_t>(m);
-                if (F == nullptr)
-                    return VSMC_CUDA_ERR_ALLOC;
-                VSMC_CUDA_TRY(cudaMemsetAsync(F, 0, sizeof(uint32_t) * m, st));
-                k_rep_from_counts<<<grid1(m), kB, 0, st>>>(m, 0, F, rep, integ);
-            }
-        }
+        k_rep_trivial<<<grid1(m), kB, 0, st>>>(
+            m, m == 1 ? static_cast<int>(n) : 0, rep, integ);
         VSMC_CUDA_CHECK_LAUNCH();
         return VSMC_CUDA_OK;
     }
-    double *cdf = scratch.get<double>(m - 1);
-    uint32_t *F = scratch.get<uint32_t>(m);
-    if (!cdf || !F)
-        return VSMC_CUDA_ERR_ALLOC;
-    int rc = seqsum_device(m - 1, w, cdf, nullptr, err, scratch, st);
+    SeqArgs a;
+    int rc = seq_args(m, err, false, scratch, &a);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    if (sorted) {
-        k_counts<<<grid1(m), kB, 0, st>>>(m, n, cdf, KeysOwn{u}, F);
-    } else {
-        long long *pmk = scratch.get<long long>(n);
-        long long *pp = scratch.get<long long>(scan_parts(n));
-        if (!pmk || !pp)
-            return VSMC_CUDA_ERR_ALLOC;
-        rc = device_scan(
-            n, LoadOKey{u}, StoreK{pmk}, OpMaxK(), LLONG_MIN, pp, st);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-        k_counts<<<grid1(m), kB, 0, st>>>(m, n, cdf, KeysMax{pmk}, F);
-    }
-    k_rep_from_counts<<<grid1(m), kB, 0, st>>>(m, n, F, rep, integ);
-    VSMC_CUDA_CHECK_LAUNCH();
-    return VSMC_CUDA_OK;
+    const uint32_t m32 = static_cast<uint32_t>(m);
+    const uint32_t n32 = static_cast<uint32_t>(n);
+    const SeqLoadCdf load{w, m32 - 1};
+    a.total = nullptr;
+    a.inv = nullptr;
+    uint32_t *tail = err + kErrTail;
+    if (order == UniformOrder::Near)
+        return seq_scan(a, load,
+            SeqCount<KeysOwn, true>{KeysOwn{u}, m32, n32, rep, integ, tail},
+            st);
+    if (order == UniformOrder::Sorted)
+        return seq_scan(a, load,
+            SeqCount<KeysOwn, false>{KeysOwn{u}, m32, n32, rep, integ, tail},
+            st);
+    long long *pmk = scratch.get<long long>(n);
+    long long *pp = scratch.get<long long>(scan_parts(n));
+    if (!pmk || !pp)
+        return VSMC_CUDA_ERR_ALLOC;
+    rc = device_scan(
+        n, LoadOKey{u}, StoreK{pmk}, OpMaxK(), LLONG_MIN, pp, st);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
+    return seq_scan(a, load,
+        SeqCount<KeysMax, false>{KeysMax{pmk}, m32, n32, rep, integ, tail},
+        st);
 }
 
 int rep_index_device(size_t m, size_t n, const int *rep, int *idx,
@@ -863,27 +1042,6 @@ int residual_device(size_t m, size_t n, const double *w, double *resid,
     return VSMC_CUDA_OK;
 }
 
-// words a lazily read uniform sequence of length n consumed, given the counts
-// (the loop reads up to the first uniform above the second-to-last CDF value)
-int consumed_words(size_t m, size_t n, const int *rep_dev, const int *integ_dev,
-    cudaStream_t st, uint64_t *words)
-{
-    *words = 0;
-    if (m < 2 || n == 0)
-        return VSMC_CUDA_OK;
-    int last = 0, ilast = 0;
-    VSMC_CUDA_TRY(cudaMemcpyAsync(
-        &last, rep_dev + (m - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (integ_dev)
-        VSMC_CUDA_TRY(cudaMemcpyAsync(&ilast, integ_dev + (m - 1),
-            sizeof(int), cudaMemcpyDeviceToHost, st));
-    VSMC_CUDA_TRY(cudaStreamSynchronize(st));
-    const size_t tail = static_cast<size_t>(last - ilast);
-    const size_t jf = n - tail;
-    *words = jf < n ? jf + 1 : n;
-    return VSMC_CUDA_OK;
-}
-
 int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
     int *rep, int scheme, Scratch &scratch, cudaStream_t st)
 {
@@ -907,9 +1065,10 @@ int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
         wt = resid;
     }
     const EngineState es = engine_state(*rng);
-    double *u = scratch.get<double>(N);
+    double *u = scratch.get<double>(N + 4);
     if (u == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
+    u += es.index % 4; // the engine's blocks of four words 32-byte aligned
     // N = 2^k: the uniforms are formed in integers (exact, no FP64)
     int log2n = -1;
     if (N > 0 && (N & (N - 1)) == 0 && N <= (size_t(1) << 31)) {
@@ -917,45 +1076,44 @@ int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
         while ((size_t(1) << log2n) < N)
             ++log2n;
     }
+    UniformOrder order = UniformOrder::Near;
     if (N > 0) {
         if (base == VSMC_CUDA_STRATIFIED) {
             k_stratified_seq<<<grid1(N), kB, 0, st>>>(es, N, log2n, u);
         } else if (base == VSMC_CUDA_SYSTEMATIC) {
             k_systematic_seq<<<grid1(N), kB, 0, st>>>(es, N, log2n, u);
         } else {
+            order = UniformOrder::Sorted;
             double *t = scratch.get<double>(N);
             if (t == nullptr)
                 return VSMC_CUDA_ERR_ALLOC;
-            k_sorted_terms<<<grid1(N), kB, 0, st>>>(es, N, t);
-            VSMC_CUDA_CHECK_LAUNCH();
+            k_sorted_terms<<<grid64(N), kB64, 0, st>>>(es, N, t);
             rc = seqsum_device(N, t, t, nullptr, err, scratch, st, true);
             if (rc != VSMC_CUDA_OK)
                 return rc;
-            k_sorted_finish<<<grid1(N), kB, 0, st>>>(N, t, u);
+            k_sorted_finish<<<grid64(N), kB64, 0, st>>>(
+                N, t, u, err + kErrUnsorted);
+            k_running_max<<<1, 1024, 0, st>>>(N, u, err + kErrUnsorted);
         }
         VSMC_CUDA_CHECK_LAUNCH();
     }
-    // the integer sequences (N = 2^k) round a non-decreasing sequence of
-    // integers to nearest, so they are non-decreasing themselves
-    const bool sorted = log2n >= 0 &&
-        (base == VSMC_CUDA_STRATIFIED || base == VSMC_CUDA_SYSTEMATIC);
-    rc = u01_rep_device(m, N, wt, u, rep, integ, err, scratch, st, sorted);
+    rc = u01_rep_device(m, N, wt, u, order, rep, integ, err, scratch, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    uint64_t words = 0;
-    if (base == VSMC_CUDA_SYSTEMATIC) {
-        words = 1; // the sequence constructor draws once
-    } else if (m >= 1) {
-        rc = consumed_words(m, N, rep, integ, st, &words);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-    }
-    int status = VSMC_CUDA_OK;
-    rc = read_err(err, st, &status);
-    if (rc != VSMC_CUDA_OK)
-        return rc;
+    uint32_t word[kErrWords] = {};
+    VSMC_CUDA_TRY(cudaMemcpyAsync(
+        word, err, sizeof(word), cudaMemcpyDeviceToHost, st));
+    VSMC_CUDA_TRY(cudaStreamSynchronize(st));
+    const int status = err_status(word[0]);
     if (status != VSMC_CUDA_OK)
         return status;
+    // systematic: the sequence constructor draws once; the others draw
+    // lazily, up to the first uniform above the second-to-last CDF value
+    uint64_t words = 0;
+    if (base == VSMC_CUDA_SYSTEMATIC)
+        words = 1;
+    else if (m >= 2 && N > 0)
+        words = std::min<uint64_t>(N - word[kErrTail] + 1, N);
     engine_advance_host(*rng, words);
     return VSMC_CUDA_OK;
 }
@@ -1097,12 +1255,12 @@ int vsmc_cuda_u01_sorted(size_t n, const double *u01, double *u01seq,
         double *t = sc.get<double>(n);
         if (t == nullptr)
             return static_cast<int>(VSMC_CUDA_ERR_ALLOC);
-        k_sorted_terms_arr<<<grid1(n), kB, 0, st>>>(n, u01, t);
+        k_sorted_terms_arr<<<grid64(n), kB64, 0, st>>>(n, u01, t);
         VSMC_CUDA_CHECK_LAUNCH();
         int rc = seqsum_device(n, t, t, nullptr, err, sc, st, true);
         if (rc != VSMC_CUDA_OK)
             return rc;
-        k_sorted_finish<<<grid1(n), kB, 0, st>>>(n, t, u01seq);
+        k_sorted_finish<<<grid64(n), kB64, 0, st>>>(n, t, u01seq, nullptr);
         VSMC_CUDA_CHECK_LAUNCH();
         return static_cast<int>(VSMC_CUDA_OK);
     });
@@ -1150,8 +1308,8 @@ int vsmc_cuda_resample_trans_u01_rep(size_t m, size_t n, const double *weight,
     if (!size_ok(m) || !size_ok(n))
         return VSMC_CUDA_ERR_SIZE;
     return with_err(stream, [&](uint32_t *err, Scratch &sc, cudaStream_t st) -> int {
-        return u01_rep_device(m, n, weight, u01, replication, nullptr, err,
-            sc, st);
+        return u01_rep_device(m, n, weight, u01, UniformOrder::Any,
+            replication, nullptr, err, sc, st);
     });
 }
 

@@ -10,10 +10,11 @@ namespace vsmc_cuda
 
 uint32_t *new_err(Scratch &scratch, cudaStream_t st)
 {
-    uint32_t *err = scratch.get<uint32_t>(4);
+    uint32_t *err = scratch.get<uint32_t>(kErrWords);
     if (err == nullptr)
         return nullptr;
-    const cudaError_t e = cudaMemsetAsync(err, 0, 4 * sizeof(uint32_t), st);
+    const cudaError_t e =
+        cudaMemsetAsync(err, 0, kErrWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) {
         set_last_cuda_error(e);
         return nullptr;
@@ -29,8 +30,8 @@ int seq_args(size_t n, uint32_t *err, bool allow_inf, Scratch &scratch,
     const size_t nt = (n + kSeqTile - 1) / kSeqTile;
     const size_t most = std::min<size_t>(
         static_cast<size_t>(num_sms()) * kSeqOcc, kSeqMaxRanges);
-    const size_t tb = (nt + most - 1) / most;
-    const size_t nb = (nt + tb - 1) / tb;
+    const size_t nb = std::min(nt, most);
+    const size_t tb = (nt + nb - 1) / nb;
     size_t bytes = 0;
     auto place = [&bytes](size_t b) {
         const size_t at = bytes;
@@ -46,9 +47,10 @@ int seq_args(size_t n, uint32_t *err, bool allow_inf, Scratch &scratch,
     const size_t otR = place(sizeof(uint64_t) * ntt);
     const size_t otF = place(sizeof(uint32_t) * ntt);
     const size_t oT = place(2 * sizeof(double));
-    const size_t oA = place(sizeof(uint64_t) * n);
-    const size_t oE = place(sizeof(uint32_t) * n);
-    const size_t oX = place(sizeof(uint16_t) * n);
+    const size_t nl = n <= kSeqSmall ? 0 : n; // the lists
+    const size_t oA = place(sizeof(uint64_t) * nl);
+    const size_t oE = place(sizeof(uint32_t) * nl);
+    const size_t oX = place(sizeof(uint16_t) * nl);
     char *b = scratch.get<char>(bytes);
     if (b == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
@@ -94,10 +96,15 @@ int seqsum_device(size_t n, const double *x, double *prefix, double *total,
     if (total)
         a.total = total;
     a.inv = nullptr;
-    rc = seq_total(a, SeqLoad{x}, SeqLoad{x}, st);
-    if (rc == VSMC_CUDA_OK && prefix)
-        rc = seq_out(a, SeqLoad{x}, SeqStore{prefix, a.n}, st);
-    return rc;
+    return prefix ? seq_scan(a, SeqLoad{x}, SeqStore{prefix, a.n}, st)
+                  : seq_total(a, SeqLoad{x}, st);
+}
+
+int err_status(uint32_t e)
+{
+    if (e & DEV_ERR_NONFINITE)
+        return VSMC_CUDA_ERR_NONFINITE;
+    return e ? VSMC_CUDA_ERR_INTERNAL : VSMC_CUDA_OK;
 }
 
 int read_err(uint32_t *err_dev, cudaStream_t st, int *status)
@@ -106,12 +113,7 @@ int read_err(uint32_t *err_dev, cudaStream_t st, int *status)
     VSMC_CUDA_TRY(cudaMemcpyAsync(
         &e, err_dev, sizeof(e), cudaMemcpyDeviceToHost, st));
     VSMC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (e & DEV_ERR_NONFINITE)
-        *status = VSMC_CUDA_ERR_NONFINITE;
-    else if (e)
-        *status = VSMC_CUDA_ERR_INTERNAL;
-    else
-        *status = VSMC_CUDA_OK;
+    *status = err_status(e);
     return VSMC_CUDA_OK;
 }
 

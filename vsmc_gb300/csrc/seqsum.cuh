@@ -51,6 +51,8 @@
 #include "scan.cuh"
 
 #include <cmath>
+#include <cooperative_groups.h>
+#include <type_traits>
 
 namespace vsmc_cuda
 {
@@ -66,8 +68,8 @@ constexpr int kSeqRowBytes = 32 * 80;
 struct SeqArgs {
     uint32_t n;      // elements
     uint32_t nt;     // tiles
-    uint32_t tb;     // tiles of a block's range
-    uint32_t blocks; // ranges
+    uint32_t tb;     // most tiles of a block's range
+    uint32_t blocks; // ranges: range b is tiles [b nt / blocks, (b + 1) nt / blocks)
     uint64_t flo, fhi; // the margin's bounds on the fraction field
     // per range, blocks + 1 each
     double *P;    // approximate sums, then their exclusive prefixes
@@ -78,7 +80,7 @@ struct SeqArgs {
     double *tP;
     uint64_t *tR;
     uint32_t *tF;
-    // breakpoint k of range b at b * tb * kSeqTile + k: the range's
+    // breakpoint k of range b, from its first element's place on: the range's
     // increments through it, then its sum's bit pattern minus them; its
     // element; its sum's sign and exponent
     uint64_t *adj;
@@ -527,6 +529,14 @@ __device__ __forceinline__ void seq_classify_tile(const SeqArgs &a,
     __syncthreads(); // rR and rF are read above, and change next
 }
 
+// first tile of range b
+__device__ __forceinline__ uint32_t seq_first_tile(
+    const SeqArgs &a, uint32_t b)
+{
+    return static_cast<uint32_t>(
+        static_cast<uint64_t>(b) * a.nt / a.blocks);
+}
+
 // The largest b with F[b] <= g, for exclusive prefixes F[0..m] (F[0] = 0)
 // and g < F[m]: the range that breakpoint g is in.
 __device__ __forceinline__ uint32_t seq_range_of(
@@ -541,6 +551,32 @@ __device__ __forceinline__ uint32_t seq_range_of(
             hi = mid;
     }
     return lo;
+}
+
+// m breakpoints in order by one thread: x their elements, cr the increments
+// through each, replaced by their sums' bit patterns; S the running sum's
+// bit pattern and crprev the increments at the last breakpoint before.
+__device__ __forceinline__ void seq_walk(const double *x, uint64_t *cr,
+    uint32_t m, uint64_t &S, uint64_t &crprev, uint32_t *err)
+{
+    bool off = false;
+    uint64_t c = cr[0];
+    double v = x[0];
+    for (uint32_t j = 0; j < m; ++j) {
+        const uint32_t jn = j + 1 < m ? j + 1 : j;
+        const uint64_t nc = cr[jn];
+        const double nv = x[jn];
+        // the regular elements since the last breakpoint stay in its binade
+        const uint64_t q = S + (c - crprev);
+        off |= (q >> 52) != (S >> 52);
+        S = dbits(__dadd_rn(from_dbits(q), v));
+        cr[j] = S;
+        crprev = c;
+        c = nc;
+        v = nv;
+    }
+    if (off)
+        atomicOr(err, DEV_ERR_BOUND);
 }
 
 // Walks the breakpoints of all ranges in order with real additions, by one
@@ -589,7 +625,9 @@ __device__ __forceinline__ void seq_fixup(const SeqArgs &a, const Load &load)
         s_F[nr] = tot.f;
     }
     __syncthreads();
-    const size_t span = static_cast<size_t>(a.tb) * kSeqTile;
+    auto list = [&](uint32_t b) {
+        return static_cast<size_t>(seq_first_tile(a, b)) * kSeqTile;
+    };
     const uint32_t nbk = tot.f;
     uint64_t S = 0; // the running sum's bit pattern at the last breakpoint
     uint64_t crprev = 0;
@@ -599,34 +637,15 @@ __device__ __forceinline__ void seq_fixup(const SeqArgs &a, const Load &load)
         uint64_t lr = 0;
         if (g < nbk) {
             const uint32_t b = seq_range_of(s_F, nr, g);
-            id = b * span + (g - s_F[b]);
+            id = list(b) + (g - s_F[b]);
             lr = __ldcg(a.adj + id);
             s_cr[threadIdx.x] = s_R[b] + lr;
             s_x[threadIdx.x] = load(__ldcg(a.pos + id));
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const uint32_t m = min(nbk - c0, static_cast<uint32_t>(kB));
-            bool off = false;
-            uint64_t cr = s_cr[0];
-            double x = s_x[0];
-            for (uint32_t j = 0; j < m; ++j) {
-                const uint32_t jn = j + 1 < m ? j + 1 : j;
-                const uint64_t ncr = s_cr[jn];
-                const double nx = s_x[jn];
-                // the regular elements since the last breakpoint stay in
-                // its binade
-                const uint64_t q = S + (cr - crprev);
-                off |= (q >> 52) != (S >> 52);
-                S = dbits(__dadd_rn(from_dbits(q), x));
-                s_cr[j] = S;
-                crprev = cr;
-                cr = ncr;
-                x = nx;
-            }
-            if (off)
-                atomicOr(a.err, DEV_ERR_BOUND);
-        }
+        if (threadIdx.x == 0)
+            seq_walk(s_x, s_cr, min(nbk - c0, static_cast<uint32_t>(kB)), S,
+                crprev, a.err);
         __syncthreads();
         if (g < nbk) {
             const uint64_t s = s_cr[threadIdx.x];
@@ -641,7 +660,7 @@ __device__ __forceinline__ void seq_fixup(const SeqArgs &a, const Load &load)
         uint64_t s = 0;
         if (g > 0) {
             const uint32_t q = seq_range_of(s_F, nr, g - 1);
-            s = a.adj[q * span + (g - 1 - s_F[q])] + (s_R[b] - s_R[q]);
+            s = a.adj[list(q) + (g - 1 - s_F[q])] + (s_R[b] - s_R[q]);
         } else if (s_R[b] != 0) {
             atomicOr(a.err, DEV_ERR_INTERNAL); // a first sum is listed
         }
@@ -782,8 +801,8 @@ constexpr int kSeqOcc = 4;
 __device__ __forceinline__ void seq_range(
     const SeqArgs &a, uint32_t &t0, uint32_t &t1)
 {
-    t0 = blockIdx.x * a.tb;
-    t1 = min(a.nt, t0 + a.tb);
+    t0 = seq_first_tile(a, blockIdx.x);
+    t1 = seq_first_tile(a, blockIdx.x + 1);
 }
 
 template <class Load>
@@ -865,6 +884,11 @@ __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_classify(
         seq_fixup<kSeqBlock>(a, load);
 }
 
+__device__ __forceinline__ void seq_prefetch(const void *p)
+{
+    asm volatile("prefetch.global.L2 [%0];" : : "l"(p));
+}
+
 template <class Load, class Out>
 __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_out(
     const SeqArgs a, const Load load, const Out out)
@@ -884,9 +908,177 @@ __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_out(
         const uint32_t nb = a.tF[tt + (t - t0) + 1] - f0;
         // the last breakpoint before the tile, else the range's start
         const uint64_t start = (f0 ? a.adj[l0 + f0 - 1] : start0) + tR;
+        // half the threads bring the next tile's lines to L2, half what out
+        // reads for this one
+        if (threadIdx.x < kSeqTile / 16) {
+            const uint32_t i = (t + 1) * kSeqTile + threadIdx.x * 16;
+            if (t + 1 < t1 && i < a.n)
+                seq_prefetch(load.at(i));
+        } else {
+            out.prefetch(from_dbits(start), threadIdx.x - kSeqTile / 16);
+        }
         seq_out_tile(a, t, v, start, static_cast<uint32_t>(start >> 52), tR,
             l0 + f0, nb, sh, par, out);
     }
+}
+
+// ------------------------------------------------------- one-cluster sums
+//
+// Up to kSeqSmall elements in one launch: a cluster of at most 8 blocks, a
+// tile each, with the values in registers throughout and the partial results
+// and breakpoint lists in (distributed) shared memory; hardware cluster
+// barriers between the phases.  Three dependent launches with their tickets
+// and lists in L2 made a systematic resampling call at n = 1000 83 us; it
+// takes 41 us with this kernel.  Above 8 tiles (the portable cluster size)
+// the passes above take over.
+
+constexpr uint32_t kSeqSmallTiles = 8; // the portable cluster size
+constexpr size_t kSeqSmall = static_cast<size_t>(kSeqSmallTiles) * kSeqTile;
+
+struct SeqClusterSmem {
+    SeqSmem t;
+    double tsum, total, pa, pb;
+    uint64_t R, start;
+    uint32_t F;
+    uint64_t s_R[kSeqSmallTiles + 1];
+    uint32_t s_F[kSeqSmallTiles + 1];
+    double s_x[kSeqBlock];
+    uint64_t s_cr[kSeqBlock];
+    uint64_t adj[kSeqTile];
+    uint32_t pos[kSeqTile];
+    uint16_t bex[kSeqTile];
+};
+
+// The exact left-to-right sum of the cluster's values (v: the block's tile,
+// striped), in every thread; the tile's starting sum and breakpoints stay in
+// S.  a.adj, a.pos and a.bex point at S's lists.
+__device__ __forceinline__ double seq_cluster_total(
+    const cooperative_groups::cluster_group &cl, const SeqArgs &a,
+    const double (&v)[kSeqItems], SeqClusterSmem &S)
+{
+    const uint32_t tile = cl.block_rank(), nc = cl.num_blocks();
+    const uint32_t lane = threadIdx.x & 31;
+    const double ts = seq_tile_sum(v, a.allow_inf, a.err, S.t, 0);
+    if (threadIdx.x == 0) {
+        S.tsum = ts;
+        S.t.rR = 0;
+        S.t.rF = 0;
+    }
+    cl.sync();
+    if (threadIdx.x < 32) {
+        const double d = lane < nc ? cl.map_shared_rank(&S, lane)->tsum : 0.0;
+        double run = 0;
+        for (uint32_t q = 0; q <= tile; ++q) {
+            if (q == tile && lane == 0)
+                S.pa = run;
+            run += __shfl_sync(0xFFFFFFFFu, d, q);
+        }
+        if (lane == 0)
+            S.pb = run;
+    }
+    __syncthreads();
+    uint64_t R = 0;
+    uint32_t F = 0;
+    seq_classify_tile(a, tile, 0, v, S.pa, S.pb, S.t, 0, R, F);
+    if (threadIdx.x == 0) {
+        S.R = R;
+        S.F = F;
+    }
+    cl.sync();
+    if (tile == 0) { // walk the breakpoints, as seq_fixup does
+        if (threadIdx.x == 0) {
+            uint64_t r = 0;
+            uint32_t f = 0;
+            for (uint32_t q = 0; q < nc; ++q) {
+                S.s_R[q] = r;
+                S.s_F[q] = f;
+                r += cl.map_shared_rank(&S, q)->R;
+                f += cl.map_shared_rank(&S, q)->F;
+            }
+            S.s_R[nc] = r;
+            S.s_F[nc] = f;
+        }
+        __syncthreads();
+        const uint32_t nbk = S.s_F[nc];
+        uint64_t sum = 0, crprev = 0;
+        for (uint32_t c0 = 0; c0 < nbk; c0 += kSeqBlock) {
+            const uint32_t g = c0 + threadIdx.x;
+            SeqClusterSmem *B = &S;
+            uint32_t k = 0;
+            uint64_t lr = 0;
+            if (g < nbk) {
+                const uint32_t b = seq_range_of(S.s_F, nc, g);
+                B = cl.map_shared_rank(&S, b);
+                k = g - S.s_F[b];
+                lr = B->adj[k];
+                S.s_cr[threadIdx.x] = S.s_R[b] + lr;
+                // the element from the staging rows of its block
+                const uint32_t e = B->pos[k] - b * kSeqTile;
+                S.s_x[threadIdx.x] = *reinterpret_cast<const double *>(
+                    B->t.row[e >> 8] + ((e & 255) >> 3) * 80 + (e & 7) * 8);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0)
+                seq_walk(S.s_x, S.s_cr, min(nbk - c0, kSeqBlock + 0u), sum,
+                    crprev, a.err);
+            __syncthreads();
+            if (g < nbk) {
+                const uint64_t s = S.s_cr[threadIdx.x];
+                B->adj[k] = s - lr;
+                B->bex[k] = static_cast<uint16_t>(s >> 52);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x <= nc) {
+            const uint32_t b = threadIdx.x, g = S.s_F[b];
+            uint64_t s = 0;
+            if (g > 0) {
+                const uint32_t q = seq_range_of(S.s_F, nc, g - 1);
+                s = cl.map_shared_rank(&S, q)->adj[g - 1 - S.s_F[q]] +
+                    (S.s_R[b] - S.s_R[q]);
+            } else if (S.s_R[b] != 0) {
+                atomicOr(a.err, DEV_ERR_INTERNAL); // a first sum is listed
+            }
+            if (b < nc)
+                cl.map_shared_rank(&S, b)->start = s;
+            else
+                for (uint32_t q = 0; q < nc; ++q)
+                    cl.map_shared_rank(&S, q)->total = from_dbits(s);
+        }
+    }
+    cl.sync();
+    return S.total;
+}
+
+// sums of up to kSeqSmall elements: a.total and a.inv, and the running sums
+// to out unless it is SeqNoOut
+struct SeqNoOut {
+};
+
+template <class Load, class Out>
+__global__ void __launch_bounds__(kSeqBlock) k_seq_small(
+    SeqArgs a, const Load load, const Out out)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char smem[];
+    SeqClusterSmem &S = *reinterpret_cast<SeqClusterSmem *>(smem);
+    a.adj = S.adj;
+    a.pos = S.pos;
+    a.bex = S.bex;
+    const uint32_t tile = cl.block_rank();
+    double v[kSeqItems];
+    seq_load(load, tile, a.n, v);
+    const double total = seq_cluster_total(cl, a, v, S);
+    if (tile == 0 && threadIdx.x == 0) {
+        if (a.total)
+            *a.total = total;
+        if (a.inv)
+            *a.inv = 1.0 / total;
+    }
+    if constexpr (!std::is_same<Out, SeqNoOut>::value)
+        seq_out_tile(a, tile, v, S.start,
+            static_cast<uint32_t>(S.start >> 52), 0, 0, S.F, S.t, 1, out);
 }
 
 // ------------------------------------------------------------- functors
@@ -897,12 +1089,17 @@ struct SeqLoad {
     {
         return x[i];
     }
+    __device__ __forceinline__ const double *at(uint32_t i) const
+    {
+        return x + i;
+    }
 };
 
 // stores the prefix sums
 struct SeqStore {
     double *p;
     uint32_t n;
+    __device__ __forceinline__ void prefetch(double, uint32_t) const {}
     __device__ __forceinline__ void operator()(uint32_t tile, uint32_t,
         const double (&s)[kSeqItems], double, SeqSmem &sh) const
     {
@@ -920,7 +1117,8 @@ struct SeqStore {
 // ----------------------------------------------------------------- host
 
 // A zeroed error word followed by the sums' two tickets (which every pass
-// leaves zero); null on failure.
+// leaves zero) and words of the caller's, kErrWords in all; null on failure.
+constexpr int kErrWords = 8;
 uint32_t *new_err(Scratch &scratch, cudaStream_t st);
 
 // The buffers for sums of n (1 <= n < 2^31) terms from one scratch
@@ -928,21 +1126,55 @@ uint32_t *new_err(Scratch &scratch, cudaStream_t st);
 int seq_args(size_t n, uint32_t *err, bool allow_inf, Scratch &scratch,
     SeqArgs *a);
 
-// tile sums and classification: after this, a.total / a.inv hold the result
-template <class Load1, class Load2>
-int seq_total(const SeqArgs &a, const Load1 &sums, const Load2 &load,
+template <class Load, class Out>
+int seq_small(const SeqArgs &a, const Load &load, const Out &out,
     cudaStream_t st)
 {
-    k_seq_sums<Load1><<<a.blocks, kSeqBlock, 0, st>>>(a, sums);
-    k_seq_classify<Load2><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
+    // the shared memory limit is a property of the kernel on each device
+    VSMC_CUDA_TRY(cudaFuncSetAttribute(k_seq_small<Load, Out>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize,
+        static_cast<int>(sizeof(SeqClusterSmem))));
+    uint32_t c = 1;
+    while (c < a.nt)
+        c *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(kSeqBlock);
+    cfg.dynamicSmemBytes = sizeof(SeqClusterSmem);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    VSMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_seq_small<Load, Out>, a, load, out));
+    return VSMC_CUDA_OK;
+}
+
+// The sum of load(0 .. n - 1) into a.total / a.inv.
+template <class Load>
+int seq_total(const SeqArgs &a, const Load &load, cudaStream_t st)
+{
+    if (a.n <= kSeqSmall)
+        return seq_small(a, load, SeqNoOut(), st);
+    k_seq_sums<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
+    k_seq_classify<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
 
+// The same, and the running sums to out.
 template <class Load, class Out>
-int seq_out(const SeqArgs &a, const Load &load, const Out &out,
+int seq_scan(const SeqArgs &a, const Load &load, const Out &out,
     cudaStream_t st)
 {
+    if (a.n <= kSeqSmall)
+        return seq_small(a, load, out, st);
+    const int rc = seq_total(a, load, st);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
     k_seq_out<Load, Out><<<a.blocks, kSeqBlock, 0, st>>>(a, load, out);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
@@ -953,6 +1185,9 @@ int seq_out(const SeqArgs &a, const Load &load, const Out &out,
 // Device error bits go to *err (DEV_ERR_NONFINITE for negative / NaN terms).
 int seqsum_device(size_t n, const double *x, double *prefix, double *total,
     uint32_t *err, Scratch &scratch, cudaStream_t st, bool allow_inf = false);
+
+// status of a device error word
+int err_status(uint32_t e);
 
 // copy the device error word to the host (synchronizes) and map it to a
 // status
