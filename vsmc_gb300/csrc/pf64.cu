@@ -6,6 +6,21 @@
 // mean (core/monitor.hpp:242-268).  Only libm (exp / log / sincos / log1p)
 // differs from the reference, so a run tracks the oracle closely.  The step
 // reads the ESS back to decide on resampling, as Particle::resample does.
+//
+// A step is three launches and one host wait:
+//   move   every particle moves, its log-weight log(W) + l is stored in W and
+//          the largest found (an integer atomic);
+//   exp    W = exp(lw - max);
+//   weigh  both left-to-right sums, the normalized weights, ESS, evidence,
+//          the decision and, without a resample, the weighted mean: one
+//          cluster up to 16384 particles, the passes of seqsum.cuh above.
+// The decision and the error word go to mapped host memory.  A resample adds
+// the uniforms, the counts, the slots and one pass that copies particles,
+// sets the weights and takes the mean.  move and exp are bound by the FP64
+// pipe (about 200 and 17 instructions a particle at 19 cycles of an SM per
+// warp), so they run in 64-thread blocks over all SMs: at 2^14 particles a
+// step took 320 us with 256-thread blocks on 16 to 64 SMs, about 60 launches
+// and four waits.
 #include "pf_internal.cuh"
 #include "pf_model.cuh"
 #include "resample_internal.cuh"
@@ -17,33 +32,51 @@
 namespace vsmc_cuda
 {
 
+// What the host reads after a step (mapped pinned memory).
+struct Pf64Host {
+    uint32_t err;
+    uint32_t resample; // ESS < threshold * n
+    uint32_t tail;     // uniforms left to the last particle (a resample's)
+};
+
 struct Pf64State {
-    double *ll = nullptr;   // log-likelihoods of the step
     int *rep = nullptr;
     int *idx = nullptr;
-    double *scal = nullptr; // [0] ess, [1] logz, [2] evidence max, [3] sum
-    double *part = nullptr; // reduction partials
+    double *scal = nullptr; // [0] ess, [1] log-evidence, [2] 1 / n normalized
+                            // and [3] its log, [4], [5] sums
+    double *part = nullptr; // weighted sums of blocks
+    uint32_t *err = nullptr; // kErrWords words (resample_internal.cuh)
+    Pf64Host *host = nullptr, *host_dev = nullptr;
+    Scratch *work = nullptr; // the sums' buffers
+    SeqArgs seq = {};
     vsmc_cuda_rng reng = {};
-    double logz = 0;
+    bool equal = false;   // every weight is 1 / n normalized
+    bool pending = false; // the engine has yet to pass the last resample
+    size_t pending_n = 0; // its uniforms
 };
 
 namespace
 {
 
-constexpr int kB = 256;
+constexpr int kSelB = 128;
 
-__global__ void __launch_bounds__(256) k_move64(uint32_t n, uint32_t ld,
+// Move, log-likelihood and log-weight of every particle; the largest
+// log-weight into *key.  logeq: the logarithm of the common weight when all
+// are equal (null otherwise).
+__global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
     uint32_t t, uint32_t seed, CvConst<double> c, const double *obs,
-    double *s, double *ll)
+    double *s, double *W, const double *logeq, unsigned long long *key)
 {
     const double ox = obs[2 * t + 0], oy = obs[2 * t + 1];
+    unsigned long long m = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         const u32x4 w = particle_block(t, seed, i);
         double X, Y, VX, VY;
+        double z1, z2;
+        normal_pair_d(w.x, w.y, z1, z2);
         if (t == 0) {
-            double z1, z2, z3, z4;
-            normal_pair_d(w.x, w.y, z1, z2);
+            double z3, z4;
             normal_pair_d(w.z, w.w, z3, z4);
             X = __dmul_rn(c.sd_pos0, z1);
             Y = __dmul_rn(c.sd_pos0, z2);
@@ -54,8 +87,6 @@ __global__ void __launch_bounds__(256) k_move64(uint32_t n, uint32_t ld,
             Y = s[ld + i];
             VX = s[2 * ld + i];
             VY = s[3 * ld + i];
-            double z1, z2;
-            normal_pair_d(w.x, w.y, z1, z2);
             cv_move(c, __dmul_rn(c.sigma_a, z1), __dmul_rn(c.sigma_a, z2), X,
                 Y, VX, VY);
         }
@@ -63,83 +94,199 @@ __global__ void __launch_bounds__(256) k_move64(uint32_t n, uint32_t ld,
         s[ld + i] = Y;
         s[2 * ld + i] = VX;
         s[3 * ld + i] = VY;
-        ll[i] = cv_loglik(c, ox, oy, X, Y);
+        double lw = cv_loglik(c, ox, oy, X, Y);
+        if (t != 0)
+            lw = __dadd_rn(logeq ? *logeq : log(W[i]), lw);
+        W[i] = lw;
+        m = max(m, max_key(lw));
     }
+    __shared__ unsigned long long sh[kB64 / 32 + 1];
+    m = block_reduce(m, OpMax(), 0ull, sh);
+    if (threadIdx.x == 0)
+        atomicMax(key, m);
 }
 
-struct OpMaxD {
-    __device__ double operator()(double a, double b) const
-    {
-        return a < b ? b : a;
-    }
+// W = exp(lw - max)
+__global__ void __launch_bounds__(kB64) k_exp64(
+    uint32_t n, double *W, const unsigned long long *key)
+{
+    const double m = from_max_key(*key);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += gridDim.x * blockDim.x)
+        W[i] = exp(W[i] - m);
+}
+
+// where a step's results go
+struct Step64 {
+    uint32_t n, t;
+    double threshold;
+    const double *state;
+    size_t ld;
+    double *W, *scal;
+    double *h_mean, *h_ess, *h_logz;
+    int *h_res;
+    uint32_t *err;
+    unsigned long long *key;
+    Pf64Host *host;
 };
 
-// evidence increment log sum_i W_i exp(ll_i - m) + m (W == null: 1/N each)
-__global__ void __launch_bounds__(256) k_ev_max(uint32_t n, const double *ll,
-    double *part)
+// The step's records, by one thread: the evidence increment is
+// log sum_i W_{t-1,i} exp(l_i) = max + log(sum), the sum being that of the
+// weights before they are normalized (over n equal ones at t = 0).
+__device__ __forceinline__ void step64_record(
+    const Step64 &a, double sum, double ess)
 {
-    double m = -INFINITY;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x)
-        m = fmax(m, ll[i]);
-    __shared__ double sh[kB / 32 + 1];
-    m = block_reduce(m, OpMaxD(), -static_cast<double>(INFINITY), sh);
-    if (threadIdx.x == 0)
-        part[blockIdx.x] = m;
+    const bool res = ess < a.threshold * static_cast<double>(a.n);
+    const double mass = a.t == 0 ? sum / static_cast<double>(a.n) : sum;
+    const double logz = (a.t == 0 ? 0.0 : a.scal[1]) +
+        (from_max_key(*a.key) + log(mass));
+    a.scal[0] = ess;
+    a.scal[1] = logz;
+    a.h_ess[a.t] = ess;
+    a.h_logz[a.t] = logz;
+    a.h_res[a.t] = res ? 1 : 0;
+    *a.key = 0; // for the next step's maximum
+    a.host->err = atomicOr(a.err, 0u);
+    a.host->resample = res ? 1 : 0;
+    __threadfence_system();
 }
 
-__global__ void __launch_bounds__(256) k_ev_sum(uint32_t n, const double *ll,
-    const double *W, const double *part, int nb, double *part2)
+__global__ void k_record64(const Step64 a)
 {
-    __shared__ double sh[kB / 32 + 1];
-    double m = -INFINITY;
-    for (int b = 0; b < nb; ++b)
-        m = fmax(m, part[b]);
-    double s = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x)
-        s += (W ? W[i] : 1.0) * exp(ll[i] - m);
-    s = block_reduce(s, OpAdd(), 0.0, sh);
-    if (threadIdx.x == 0)
-        part2[blockIdx.x] = s;
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        part2[nb] = m;
+    if (threadIdx.x == 0 && blockIdx.x == 0)
+        step64_record(a, a.scal[4], a.scal[5]);
 }
 
-__global__ void k_ev_final(int nb, uint32_t n, bool first,
-    const double *part2, double *scal, double *h_logz, uint32_t t,
-    const double *ess, double *h_ess)
+// Normalization, ESS, records and (without a resample) the weighted mean of
+// up to kSeqSmall particles, by one cluster.
+__global__ void __launch_bounds__(kSeqBlock) k_weigh64(
+    SeqArgs q, const Step64 a)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    SeqClusterSmem &S = seq_cluster_smem(q);
+    __shared__ double s_inv, s_mean[2], sh[kSeqBlock / 32 + 1];
+    __shared__ bool s_res;
+    const uint32_t tile = cl.block_rank();
+    double w[kSeqItems], sq[kSeqItems];
+    seq_load(SeqLoad{a.W}, tile, q.n, w);
+    const double total = seq_cluster_total(cl, q, w, S);
+    if (threadIdx.x == 0)
+        s_inv = 1.0 / total;
+    __syncthreads();
+    const double inv = s_inv;
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k) {
+        const uint32_t i = seq_striped(tile, k);
+        w[k] = __dmul_rn(inv, w[k]);
+        if (i < q.n)
+            a.W[i] = w[k];
+        sq[k] = __dmul_rn(w[k], w[k]);
+    }
+    const double tsq = seq_cluster_total(cl, q, sq, S);
+    if (threadIdx.x == 0) {
+        const double ess = 1.0 / tsq;
+        s_res = ess < a.threshold * static_cast<double>(a.n);
+        if (tile == 0)
+            step64_record(a, total, ess);
+    }
+    __syncthreads();
+    if (s_res) // the same in every block
         return;
-    double s = 0;
-    for (int b = 0; b < nb; ++b)
-        s += part2[b];
-    if (first)
-        s /= static_cast<double>(n);
-    scal[1] += part2[nb] + log(s);
-    h_logz[t] = scal[1];
-    (void)ess;
-    (void)h_ess;
+    double m[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k) {
+        const uint32_t i = seq_striped(tile, k);
+        if (i < q.n) {
+            m[0] += w[k] * a.state[i];
+            m[1] += w[k] * a.state[a.ld + i];
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const double v = block_reduce(m[d], OpAdd(), 0.0, sh);
+        if (threadIdx.x == 0)
+            s_mean[d] = v;
+    }
+    cl.sync();
+    if (tile == 0 && threadIdx.x < 2) {
+        double v = 0;
+        for (uint32_t b = 0; b < cl.num_blocks(); ++b)
+            v += *cl.map_shared_rank(&s_mean[threadIdx.x], b);
+        a.h_mean[2 * a.t + threadIdx.x] = v;
+    }
+    cl.sync(); // the sums are read
 }
 
-__global__ void k_copy1(const double *src, double *dst)
+// After a resample: particles copied to the empty slots (parents keep
+// theirs, so in place), every weight 1 / n normalized, and the mean of the
+// result: block sums, added by the last block (its ticket; nothing waits).
+__global__ void __launch_bounds__(kSelB) k_select64(
+    const Step64 a, double *state, const int *idx, double *part)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        *dst = *src;
+    __shared__ double sh[kSelB / 32 + 1];
+    __shared__ bool last;
+    const double w = a.scal[2];
+    double m[2] = {0.0, 0.0};
+    for (uint32_t i = blockIdx.x * kSelB + threadIdx.x; i < a.n;
+         i += gridDim.x * kSelB) {
+        const uint32_t j = static_cast<uint32_t>(idx[i]);
+        if (j >= a.n) {
+            atomicOr(a.err, DEV_ERR_INTERNAL);
+            continue;
+        }
+        const double x = state[j], y = state[a.ld + j];
+        if (j != i) {
+            const double vx = state[2 * a.ld + j], vy = state[3 * a.ld + j];
+            state[i] = x;
+            state[a.ld + i] = y;
+            state[2 * a.ld + i] = vx;
+            state[3 * a.ld + i] = vy;
+        }
+        a.W[i] = w;
+        m[0] += w * x;
+        m[1] += w * y;
+    }
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const double v = block_reduce(m[d], OpAdd(), 0.0, sh);
+        if (threadIdx.x == 0)
+            part[2 * blockIdx.x + d] = v;
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(a.err + kErrTicket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        double v = 0;
+        for (uint32_t b = threadIdx.x; b < gridDim.x; b += kSelB)
+            v += __ldcg(part + 2 * b + d);
+        v = block_reduce(v, OpAdd(), 0.0, sh);
+        if (threadIdx.x == 0)
+            a.h_mean[2 * a.t + d] = v;
+    }
+    if (threadIdx.x == 0) {
+        a.err[kErrTicket] = 0;
+        a.host->tail = a.err[kErrTail];
+        a.host->err = atomicOr(a.err, 0u);
+        __threadfence_system();
+    }
 }
 
-__global__ void k_set_int(int *p, int v)
+__global__ void k_equal64(const double *W, double *scal)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        *p = v;
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        scal[2] = W[0];
+        scal[3] = log(W[0]);
+    }
 }
 
-__global__ void k_zero_d(double *p)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        *p = 0.0;
-}
+int select_grid(size_t n) { return grid_for(n, kSelB, 1, 4); }
 
 } // namespace
 
@@ -150,13 +297,35 @@ int pf64_create(vsmc_cuda_pf *pf)
         return VSMC_CUDA_ERR_ALLOC;
     pf->p64 = p;
     const size_t n = pf->n;
-    const int nb = grid_for(n, kB, 4, 8);
-    if (cudaMalloc(&p->ll, sizeof(double) * n) != cudaSuccess ||
-        cudaMalloc(&p->rep, sizeof(int) * n) != cudaSuccess ||
+    cudaStream_t st = pf->stream;
+    if (cudaMalloc(&p->rep, sizeof(int) * n) != cudaSuccess ||
         cudaMalloc(&p->idx, sizeof(int) * n) != cudaSuccess ||
         cudaMalloc(&p->scal, sizeof(double) * 8) != cudaSuccess ||
-        cudaMalloc(&p->part, sizeof(double) * (2 * nb + 8)) != cudaSuccess)
+        cudaMalloc(&p->part, sizeof(double) * 2 * select_grid(n)) !=
+            cudaSuccess ||
+        cudaMalloc(&p->err, sizeof(uint32_t) * kErrWords) != cudaSuccess ||
+        cudaHostAlloc(reinterpret_cast<void **>(&p->host), sizeof(Pf64Host),
+            cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void **>(&p->host_dev),
+            p->host, 0) != cudaSuccess)
         return VSMC_CUDA_ERR_ALLOC;
+    p->work = new (std::nothrow) Scratch(st);
+    if (p->work == nullptr)
+        return VSMC_CUDA_ERR_ALLOC;
+    VSMC_CUDA_TRY(cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
+    int rc = seq_args(n, p->err, false, *p->work, &p->seq);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
+    // the weight that Weight::set_equal leaves in every slot, and its log
+    double *W = static_cast<double *>(pf->weight);
+    {
+        Scratch scratch(st);
+        rc = weight_set_equal_device(n, W, nullptr, p->err, scratch, st);
+        if (rc != VSMC_CUDA_OK)
+            return rc;
+    }
+    k_equal64<<<1, 1, 0, st>>>(W, p->scal);
+    VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
 
@@ -165,13 +334,31 @@ void pf64_destroy(vsmc_cuda_pf *pf)
     Pf64State *p = pf->p64;
     if (p == nullptr)
         return;
-    cudaFree(p->ll);
+    delete p->work;
     cudaFree(p->rep);
     cudaFree(p->idx);
     cudaFree(p->scal);
     cudaFree(p->part);
+    cudaFree(p->err);
+    if (p->host)
+        cudaFreeHost(p->host);
     delete p;
     pf->p64 = nullptr;
+}
+
+// both sums and the weights of more than kSeqSmall particles
+static int weigh_large(vsmc_cuda_pf *pf, const Step64 &a)
+{
+    Pf64State *p = pf->p64;
+    cudaStream_t st = pf->stream;
+    SeqArgs q = p->seq;
+    q.total = p->scal + 4;
+    int rc = weight_sums(q, a.W, a.W, p->scal + 5, st);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
+    k_record64<<<1, 32, 0, st>>>(a);
+    VSMC_CUDA_CHECK_LAUNCH();
+    return VSMC_CUDA_OK;
 }
 
 int pf64_step(vsmc_cuda_pf *pf, bool first)
@@ -180,77 +367,81 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     cudaStream_t st = pf->stream;
     const size_t n = pf->n;
     const uint32_t t = static_cast<uint32_t>(pf->t);
-    double *W = static_cast<double *>(pf->weight);
+    const bool small = n <= kSeqSmall;
+    Step64 a = {};
+    a.n = static_cast<uint32_t>(n);
+    a.t = t;
+    a.threshold = pf->threshold;
+    a.state = static_cast<const double *>(pf->state);
+    a.ld = pf->stride;
+    a.W = static_cast<double *>(pf->weight);
+    a.scal = p->scal;
+    a.h_mean = pf->h_mean;
+    a.h_ess = pf->h_ess;
+    a.h_logz = pf->h_logz;
+    a.h_res = pf->h_res;
+    a.err = p->err;
+    a.key = reinterpret_cast<unsigned long long *>(p->err + kErrMax);
+    a.host = p->host_dev;
     double *S = static_cast<double *>(pf->state);
-    Scratch scratch(st);
-    uint32_t *err = new_err(scratch, st);
-    if (err == nullptr)
-        return VSMC_CUDA_ERR_ALLOC;
     if (first) {
         // Sampler::initialize: resampling engine key {0, seed}, counter
-        // {0, 0, 1, 0}; log-evidence 0
+        // {0, 0, 1, 0}
         vsmc_cuda_rng_init(&p->reng, VSMC_CUDA_PHILOX4X32, 0);
         const uint64_t key[2] = {0, pf->seed};
         vsmc_cuda_rng_set_key(&p->reng, 2, key);
         const uint64_t ctr[4] = {0, 0, 1, 0};
         vsmc_cuda_rng_set_ctr(&p->reng, 4, ctr);
-        k_zero_d<<<1, 1, 0, st>>>(p->scal + 1);
+        p->equal = false;
+        p->pending = false;
+        VSMC_CUDA_TRY(
+            cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
     }
     const CvConst<double> c = make_cv_const<double>(pf->model);
-    const int grid = grid_for(n, kB, 1, 8);
-    k_move64<<<grid, kB, 0, st>>>(static_cast<uint32_t>(n),
-        static_cast<uint32_t>(pf->stride), t, pf->seed, c, pf->obs, S, p->ll);
+    k_move64<<<grid64(n), kB64, 0, st>>>(a.n, static_cast<uint32_t>(a.ld), t,
+        pf->seed, c, pf->obs, S, a.W, p->equal ? p->scal + 3 : nullptr, a.key);
+    k_exp64<<<grid64(n), kB64, 0, st>>>(a.n, a.W, a.key);
     VSMC_CUDA_CHECK_LAUNCH();
-    // evidence increment from the weights before they are updated
-    const int nb = grid_for(n, kB, 4, 8);
-    k_ev_max<<<nb, kB, 0, st>>>(static_cast<uint32_t>(n), p->ll, p->part);
-    k_ev_sum<<<nb, kB, 0, st>>>(static_cast<uint32_t>(n), p->ll,
-        first ? nullptr : W, p->part, nb, p->part + nb);
-    k_ev_final<<<1, 32, 0, st>>>(nb, static_cast<uint32_t>(n), first,
-        p->part + nb, p->scal, pf->h_logz, t, nullptr, nullptr);
-    VSMC_CUDA_CHECK_LAUNCH();
-    int rc;
-    if (first) {
-        VSMC_CUDA_TRY(cudaMemcpyAsync(W, p->ll, sizeof(double) * n,
-            cudaMemcpyDeviceToDevice, st));
-        rc = weight_post_set_log_device(n, W, p->scal, err, scratch, st);
-    } else {
-        rc = weight_add_log_device(n, p->ll, W, p->scal, err, scratch, st);
-    }
+    int rc = small ? seq_cluster_launch(k_weigh64, p->seq, st, a)
+                   : weigh_large(pf, a);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    k_copy1<<<1, 1, 0, st>>>(p->scal, pf->h_ess + t);
-    VSMC_CUDA_CHECK_LAUNCH();
-    double ess = 0;
-    VSMC_CUDA_TRY(cudaMemcpyAsync(
-        &ess, p->scal, sizeof(double), cudaMemcpyDeviceToHost, st));
     VSMC_CUDA_TRY(cudaStreamSynchronize(st));
-    const bool resample = ess < pf->threshold * static_cast<double>(n);
-    if (resample) {
-        rc = scheme_device(n, n, &p->reng, W, p->rep, pf->scheme, scratch, st);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-        rc = rep_index_device(n, n, p->rep, p->idx, err, scratch, st);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-        rc = state_copy_device<double>(n, 4, pf->stride, p->idx, S, err, st);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-        rc = weight_set_equal_device(n, W, p->scal, err, scratch, st);
-        if (rc != VSMC_CUDA_OK)
-            return rc;
-    }
-    k_set_int<<<1, 1, 0, st>>>(pf->h_res + t, resample ? 1 : 0);
-    VSMC_CUDA_CHECK_LAUNCH();
-    rc = monitor_mean_device<double>(
-        n, 2, pf->stride, S, W, pf->h_mean + 2 * t, scratch, st);
+    p->equal = false;
+    rc = err_status(p->host->err);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    int status = VSMC_CUDA_OK;
-    rc = read_err(err, st, &status);
-    return rc != VSMC_CUDA_OK ? rc : status;
+    Scratch scratch(st);
+    if (p->host->resample) {
+        if (p->pending) { // the last resample's words are known by now
+            scheme_advance(p->reng, n, p->pending_n, pf->scheme, p->host->tail);
+            p->pending = false;
+        }
+        size_t N = 0;
+        rc = scheme_enqueue(n, n, p->reng, a.W, p->rep, pf->scheme, p->err,
+            &N, scratch, st);
+        if (rc != VSMC_CUDA_OK)
+            return rc;
+        rc = rep_index_device(n, n, p->rep, p->idx, p->err, scratch, st);
+        if (rc != VSMC_CUDA_OK)
+            return rc;
+        k_select64<<<select_grid(n), kSelB, 0, st>>>(a, S, p->idx, p->part);
+        VSMC_CUDA_CHECK_LAUNCH();
+        p->equal = true;
+        p->pending = true;
+        p->pending_n = N;
+    } else if (!small) {
+        rc = monitor_mean_device<double>(
+            n, 2, pf->stride, S, a.W, pf->h_mean + 2 * t, scratch, st);
+    }
+    return rc;
 }
 
-int pf64_final_mean(vsmc_cuda_pf *) { return VSMC_CUDA_OK; }
+// errors of the last step's resample, which its own wait did not see
+int pf64_final_mean(vsmc_cuda_pf *pf)
+{
+    VSMC_CUDA_TRY(cudaStreamSynchronize(pf->stream));
+    return err_status(pf->p64->host->err);
+}
 
 } // namespace vsmc_cuda

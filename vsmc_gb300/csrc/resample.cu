@@ -514,12 +514,6 @@ __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
     u[j] = __dadd_rn(u0, mul_u32(static_cast<uint32_t>(j), delta, m52));
 }
 
-// Threads of a block where each element takes many FP64 instructions (19
-// cycles of an SM each): small blocks spread a short vector over all SMs.
-constexpr int kB64 = 64;
-
-int grid64(size_t n) { return grid_for(n ? n : 1, kB64, 1, 32); }
-
 // U01SequenceSorted terms: -log(U_j) / (n - j), summed left to right below
 __global__ void __launch_bounds__(kB64) k_sorted_terms(
     EngineState e, size_t n, double *t)
@@ -556,7 +550,7 @@ __global__ void __launch_bounds__(kB64) k_sorted_finish(
 // The running maximum of u in place by one block, if *unsorted (rare, so one
 // block is enough): non-negative doubles order as their bits.
 __global__ void __launch_bounds__(1024) k_running_max(
-    size_t n, double *u, const uint32_t *unsorted)
+    size_t n, double *u, uint32_t *unsorted)
 {
     if (*unsorted == 0)
         return;
@@ -572,6 +566,8 @@ __global__ void __launch_bounds__(1024) k_running_max(
             u[i] = __longlong_as_double(r);
         carry = OpMaxK()(carry, tot);
     }
+    if (threadIdx.x == 0)
+        *unsorted = 0;
 }
 
 __global__ void k_stratified_arr(size_t n, const double *u01, double *out)
@@ -612,10 +608,10 @@ __global__ void k_residual_split(size_t m, size_t n, const double *w,
     }
 }
 
-__global__ void k_scale(size_t m, const double *total, double *v)
+__global__ void k_scale(size_t m, const double *inv, double *v)
 {
-    const double inv = 1.0 / *total;
-    GRID_LOOP(i, m) v[i] = __dmul_rn(inv, v[i]);
+    const double c = *inv;
+    GRID_LOOP(i, m) v[i] = __dmul_rn(c, v[i]);
 }
 
 // ------------------------------------------------------------ rep -> index
@@ -638,17 +634,10 @@ struct OpMaxI {
     }
 };
 
-// (empty flag, surplus) for m == n; (rep, 0) for m != n
+// (rep, 0) for m != n
 struct LoadES {
     const int *rep;
-    bool square;
-    __device__ I2 operator()(size_t i) const
-    {
-        const int r = rep[i];
-        if (square)
-            return {r == 0 ? 1 : 0, r > 1 ? r - 1 : 0};
-        return {r, 0};
-    }
+    __device__ I2 operator()(size_t i) const { return {rep[i], 0}; }
 };
 
 struct StoreI2 {
@@ -656,26 +645,15 @@ struct StoreI2 {
     __device__ void operator()(size_t i, I2 v) const { p[i] = v; }
 };
 
-// marks: rank of the first surplus copy of p (m == n), or first output slot
-// of p (m != n), gets p + 1
-__global__ void k_marks(size_t m, bool square, const int *rep, const I2 *incl,
-    int *marks, size_t nmarks, uint32_t *err)
+// marks: the first output slot of p gets p + 1
+__global__ void k_marks(size_t m, const int *rep, const I2 *incl, int *marks,
+    size_t nmarks, uint32_t *err)
 {
     GRID_LOOP(p, m)
     {
         const int r = rep[p];
         if (r < 0) {
             atomicOr(err, DEV_ERR_INTERNAL);
-            continue;
-        }
-        if (square) {
-            if (r > 1) {
-                const int first = incl[p].b - (r - 1); // exclusive surplus
-                if (first >= 0 && static_cast<size_t>(first) < nmarks)
-                    marks[first] = static_cast<int>(p) + 1;
-                else
-                    atomicOr(err, DEV_ERR_INTERNAL);
-            }
         } else if (r > 0) {
             const int first = incl[p].a - r;
             if (first >= 0 && static_cast<size_t>(first) < nmarks)
@@ -713,21 +691,241 @@ struct StoreLastW {
     }
 };
 
-__global__ void k_index_square(size_t n, const int *rep, const I2 *incl,
-    const int *src_of_rank, size_t nrank, int *idx, uint32_t *err)
-{
-    GRID_LOOP(d, n)
+// ---- rep -> index for m == n (resample/transform.hpp:116-133): a parent
+// keeps its slot, the e-th empty slot takes the e-th surplus copy in parent
+// order.  Tiles of 2048 counts (8 consecutive ones per thread), a range of
+// consecutive tiles per block:
+//   count   empty slots and surplus copies of each range; the last block
+//           (its ticket; nothing waits) scans the ranges and checks that the
+//           totals agree;
+//   assign  a block scan gives every slot its ranks: idx = the slot, or
+//           -(rank + 1) for an empty one, and srcs[rank] = the parent of each
+//           surplus copy (a run of more than 8 by its whole warp);
+//   decode  empty slots read their parent.
+// Up to 16384 counts one cluster does all of it in one launch.
+struct SlotArgs {
+    uint32_t n, nt, blocks;
+    const int *rep;
+    int *idx;
+    uint32_t *srcs; // n
+    uint64_t *S;    // blocks + 1: surplus copies of the ranges, then prefixes
+    uint32_t *E;    // blocks + 1: empty slots
+    uint32_t *err;
+};
+
+struct ES {
+    uint64_t s;
+    uint32_t e, pad;
+};
+
+struct OpES {
+    __device__ __forceinline__ ES operator()(const ES &x, const ES &y) const
     {
-        if (rep[d] != 0) {
-            idx[d] = static_cast<int>(d);
-        } else {
-            const int k = incl[d].a - 1; // exclusive empty rank
-            if (k >= 0 && static_cast<size_t>(k) < nrank && src_of_rank[k] > 0)
-                idx[d] = src_of_rank[k] - 1;
-            else
-                atomicOr(err, DEV_ERR_INTERNAL);
-        }
+        return {x.s + y.s, x.e + y.e, 0u};
     }
+};
+
+// the thread's eight counts of a tile (1 past the end: neither empty nor
+// surplus) and their sum; negative ones are reported
+__device__ __forceinline__ ES slot_load(
+    const SlotArgs &a, uint32_t tile, int (&r)[kSeqItems])
+{
+    const uint32_t i0 = tile * kSeqTile + threadIdx.x * kSeqItems;
+    if (i0 + kSeqItems <= a.n &&
+        (reinterpret_cast<uintptr_t>(a.rep) & 15) == 0) {
+        const int4 p = *reinterpret_cast<const int4 *>(a.rep + i0);
+        const int4 q = *reinterpret_cast<const int4 *>(a.rep + i0 + 4);
+        r[0] = p.x;
+        r[1] = p.y;
+        r[2] = p.z;
+        r[3] = p.w;
+        r[4] = q.x;
+        r[5] = q.y;
+        r[6] = q.z;
+        r[7] = q.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSeqItems; ++k)
+            r[k] = i0 + k < a.n ? a.rep[i0 + k] : 1;
+    }
+    ES t = {0, 0, 0};
+    bool neg = false;
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k) {
+        t.e += r[k] == 0 ? 1u : 0u;
+        t.s += r[k] > 1 ? static_cast<uint32_t>(r[k]) - 1u : 0u;
+        neg |= r[k] < 0;
+    }
+    if (neg)
+        atomicOr(a.err, DEV_ERR_INTERNAL);
+    return t;
+}
+
+// Places the thread's slots from the ranks before it.  out: what an empty
+// slot of rank e gets until its source is known.
+__device__ __forceinline__ void slot_place(const SlotArgs &a, uint32_t tile,
+    const int (&r)[kSeqItems], ES at)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t i0 = tile * kSeqTile + threadIdx.x * kSeqItems;
+    uint32_t s = static_cast<uint32_t>(at.s);
+    uint32_t e = at.e;
+    int o[kSeqItems];
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k) {
+        const uint32_t i = i0 + k;
+        o[k] = r[k] == 0 ? -static_cast<int>(e) - 1 : static_cast<int>(i);
+        e += r[k] == 0 ? 1u : 0u;
+        const uint32_t len = r[k] > 1 ? static_cast<uint32_t>(r[k]) - 1u : 0u;
+        if (len <= 8)
+            for (uint32_t q = 0; q < len; ++q)
+                a.srcs[s + q] = i;
+        unsigned big = __ballot_sync(0xFFFFFFFFu, len > 8);
+        while (big) {
+            const int who = __ffs(big) - 1;
+            big &= big - 1;
+            const uint32_t s1 = __shfl_sync(0xFFFFFFFFu, s, who);
+            const uint32_t n1 = __shfl_sync(0xFFFFFFFFu, len, who);
+            const uint32_t p1 = __shfl_sync(0xFFFFFFFFu, i, who);
+            for (uint32_t q = lane; q < n1; q += 32)
+                a.srcs[s1 + q] = p1;
+        }
+        s += len;
+    }
+    if (i0 + kSeqItems <= a.n &&
+        (reinterpret_cast<uintptr_t>(a.idx) & 15) == 0) {
+        int4 *q = reinterpret_cast<int4 *>(a.idx + i0);
+        q[0] = make_int4(o[0], o[1], o[2], o[3]);
+        q[1] = make_int4(o[4], o[5], o[6], o[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSeqItems; ++k)
+            if (i0 + k < a.n)
+                a.idx[i0 + k] = o[k];
+    }
+}
+
+__device__ __forceinline__ void slot_range(
+    const SlotArgs &a, uint32_t &t0, uint32_t &t1)
+{
+    const uint64_t b = blockIdx.x;
+    t0 = static_cast<uint32_t>(b * a.nt / a.blocks);
+    t1 = static_cast<uint32_t>((b + 1) * a.nt / a.blocks);
+}
+
+__global__ void __launch_bounds__(kSeqBlock) k_slots_count(const SlotArgs a)
+{
+    uint32_t t0, t1;
+    slot_range(a, t0, t1);
+    ES acc = {0, 0, 0};
+    for (uint32_t t = t0; t < t1; ++t) {
+        int r[kSeqItems];
+        acc = OpES()(acc, slot_load(a, t, r));
+    }
+    ES tot;
+    block_excl_any<ES, OpES, kSeqBlock>(acc, OpES(), ES{0, 0, 0}, &tot);
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        a.S[blockIdx.x] = tot.s;
+        a.E[blockIdx.x] = tot.e;
+        __threadfence();
+        last = atomicAdd(a.err + kErrTicket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+    const uint32_t per = (a.blocks + kSeqBlock - 1) / kSeqBlock;
+    const uint32_t b0 = min(a.blocks, threadIdx.x * per);
+    const uint32_t b1 = min(a.blocks, b0 + per);
+    ES sum = {0, 0, 0};
+    for (uint32_t i = b0; i < b1; ++i) {
+        sum.s += __ldcg(a.S + i);
+        sum.e += __ldcg(a.E + i);
+    }
+    ES run = block_excl_any<ES, OpES, kSeqBlock>(
+        sum, OpES(), ES{0, 0, 0}, &tot);
+    for (uint32_t i = b0; i < b1; ++i) {
+        const uint64_t s = __ldcg(a.S + i);
+        const uint32_t e = __ldcg(a.E + i);
+        a.S[i] = run.s;
+        a.E[i] = run.e;
+        run.s += s;
+        run.e += e;
+    }
+    if (threadIdx.x == 0) {
+        a.err[kErrTicket] = 0;
+        if (tot.s != tot.e)
+            atomicOr(a.err, DEV_ERR_COUNTS);
+    }
+}
+
+__global__ void __launch_bounds__(kSeqBlock) k_slots_assign(const SlotArgs a)
+{
+    if (*a.err & DEV_ERR_COUNTS)
+        return;
+    uint32_t t0, t1;
+    slot_range(a, t0, t1);
+    ES before = {a.S[blockIdx.x], a.E[blockIdx.x], 0u};
+    for (uint32_t t = t0; t < t1; ++t) {
+        int r[kSeqItems];
+        const ES mine = slot_load(a, t, r);
+        ES tot;
+        const ES ex = block_excl_any<ES, OpES, kSeqBlock>(
+            mine, OpES(), ES{0, 0, 0}, &tot);
+        slot_place(a, t, r, OpES()(before, ex));
+        before = OpES()(before, tot);
+    }
+}
+
+__global__ void __launch_bounds__(kB) k_slots_decode(const SlotArgs a)
+{
+    if (*a.err & DEV_ERR_COUNTS)
+        return;
+    GRID_LOOP(i, a.n)
+    {
+        const int v = a.idx[i];
+        if (v < 0)
+            a.idx[i] = static_cast<int>(a.srcs[-v - 1]);
+    }
+}
+
+// all of it by one cluster (a.n <= kSeqSmall)
+__global__ void __launch_bounds__(kSeqBlock) k_slots_small(
+    SeqArgs, const SlotArgs a)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    __shared__ ES s_tot;
+    const uint32_t tile = cl.block_rank(), nc = cl.num_blocks();
+    int r[kSeqItems];
+    const ES mine = slot_load(a, tile, r);
+    ES tot;
+    ES at = block_excl_any<ES, OpES, kSeqBlock>(
+        mine, OpES(), ES{0, 0, 0}, &tot);
+    if (threadIdx.x == 0)
+        s_tot = tot;
+    cl.sync();
+    ES all = {0, 0, 0};
+    for (uint32_t q = 0; q < nc; ++q) {
+        const ES o = *cl.map_shared_rank(&s_tot, q);
+        if (q < tile)
+            at = OpES()(at, o);
+        all = OpES()(all, o);
+    }
+    if (all.s == all.e)
+        slot_place(a, tile, r, at);
+    else if (threadIdx.x == 0)
+        atomicOr(a.err, DEV_ERR_COUNTS);
+    cl.sync(); // srcs written; no block's totals are read any more
+    if (all.s != all.e)
+        return;
+    const uint32_t i0 = tile * kSeqTile + threadIdx.x * kSeqItems;
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k)
+        if (r[k] == 0 && i0 + k < a.n)
+            a.idx[i0 + k] = static_cast<int>(
+                __ldcg(a.srcs + (-a.idx[i0 + k] - 1)));
 }
 
 __global__ void k_index_flat(size_t total, const int *src, int *idx)
@@ -769,9 +967,21 @@ __global__ void k_copy_state(size_t n, size_t dim, size_t ld, const int *idx,
     GRID_LOOP(d, n)
     {
         const size_t s = static_cast<size_t>(idx[d]);
-        if (s != d)
-            for (size_t r = 0; r < dim; ++r)
-                state[r * ld + d] = state[r * ld + s];
+        if (s == d)
+            continue;
+        // four rows' loads in flight together
+        size_t r = 0;
+        for (; r + 4 <= dim; r += 4) {
+            T *p = state + r * ld;
+            const T v0 = p[s], v1 = p[ld + s], v2 = p[2 * ld + s],
+                    v3 = p[3 * ld + s];
+            p[d] = v0;
+            p[ld + d] = v1;
+            p[2 * ld + d] = v2;
+            p[3 * ld + d] = v3;
+        }
+        for (; r < dim; ++r)
+            state[r * ld + d] = state[r * ld + s];
     }
 }
 
@@ -784,50 +994,86 @@ struct OpMaxD {
     }
 };
 
-__global__ void k_reduce_max(size_t n, const double *v, double *part)
+// The largest log-weight into *key (zero before).  Add: the log-weights are
+// log(W) + l first (add_log, weight.hpp:168-173), stored in W.  FP64 log is
+// the cost: 64-thread blocks, one integer atomic each.
+template <bool Add>
+__global__ void __launch_bounds__(kB64) k_lw_max(
+    size_t n, const double *l, double *W, unsigned long long *key)
 {
-    double m = -INFINITY;
-    GRID_LOOP(i, n) m = fmax(m, v[i]);
-    __shared__ double sh[kB / 32 + 1];
-    m = block_reduce(m, OpMaxD(), -static_cast<double>(INFINITY), sh);
+    unsigned long long m = 0;
+    GRID_LOOP(i, n)
+    {
+        double v = l[i];
+        if (Add) {
+            v = __dadd_rn(log(W[i]), v);
+            W[i] = v;
+        }
+        m = max(m, max_key(v));
+    }
+    __shared__ unsigned long long sh[kB64 / 32 + 1];
+    m = block_reduce(m, OpMax(), 0ull, sh);
     if (threadIdx.x == 0)
-        part[blockIdx.x] = m;
-}
-
-__global__ void k_max_parts(int nb, double *part)
-{
-    double m = -INFINITY;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-        m = fmax(m, part[b]);
-    __shared__ double sh[kB / 32 + 1];
-    m = block_reduce(m, OpMaxD(), -static_cast<double>(INFINITY), sh);
-    if (threadIdx.x == 0)
-        part[0] = m;
+        atomicMax(key, m);
 }
 
 // W = exp(lw - max)  (post_set_log -> normalize(true), weight.hpp:202-229)
-__global__ void k_exp_shift(size_t n, const double *lw, const double *mx,
-    double *W)
+__global__ void __launch_bounds__(kB64) k_exp_shift(
+    size_t n, const double *lw, const unsigned long long *key, double *W)
 {
-    const double m = *mx;
+    const double m = from_max_key(*key);
     GRID_LOOP(i, n) W[i] = exp(lw[i] - m);
 }
 
-// W = log(W) + l  (add_log, weight.hpp:168-173)
-__global__ void k_log_add(size_t n, const double *l, double *W)
-{
-    GRID_LOOP(i, n) W[i] = __dadd_rn(log(W[i]), l[i]);
-}
+// the normalized weights, stored, and their squares as the terms to sum
+struct ScaleSquare {
+    const double *v;
+    const double *inv;
+    double *W;
+    __device__ __forceinline__ double operator()(uint32_t i) const
+    {
+        const double w = __dmul_rn(*inv, v[i]);
+        W[i] = w;
+        return __dmul_rn(w, w);
+    }
+};
 
-__global__ void k_square(size_t n, const double *W, double *sq)
-{
-    GRID_LOOP(i, n) sq[i] = __dmul_rn(W[i], W[i]);
-}
+struct SquareLoad {
+    const double *W;
+    __device__ __forceinline__ double operator()(uint32_t i) const
+    {
+        return __dmul_rn(W[i], W[i]);
+    }
+};
 
-__global__ void k_inv_total(const double *total, double *ess)
+// Weight::normalize (weight.hpp:208-229) of up to kSeqSmall weights by one
+// cluster: both left-to-right sums with the weights in registers.
+__global__ void __launch_bounds__(kSeqBlock) k_normalize_small(
+    SeqArgs a, const double *v, double *W, double *ess)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        *ess = 1.0 / *total;
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    SeqClusterSmem &S = seq_cluster_smem(a);
+    __shared__ double s_inv;
+    const uint32_t tile = cl.block_rank();
+    double w[kSeqItems];
+    seq_load(SeqLoad{v}, tile, a.n, w);
+    const double total = seq_cluster_total(cl, a, w, S);
+    if (threadIdx.x == 0)
+        s_inv = 1.0 / total;
+    __syncthreads();
+    const double inv = s_inv;
+#pragma unroll
+    for (int k = 0; k < kSeqItems; ++k) {
+        const uint32_t i = seq_striped(tile, k);
+        w[k] = __dmul_rn(inv, w[k]);
+        if (i < a.n)
+            W[i] = w[k];
+        w[k] = __dmul_rn(w[k], w[k]);
+    }
+    const double sq = seq_cluster_total(cl, a, w, S);
+    if (ess && tile == 0 && threadIdx.x == 0)
+        *ess = 1.0 / sq;
 }
 
 __global__ void k_fill_d(size_t n, double *p, double v)
@@ -837,29 +1083,46 @@ __global__ void k_fill_d(size_t n, double *p, double v)
 
 // ---------------------------------------------------------------- monitor
 
+// Weighted sums of dim rows: per-block partials, four rows to a pass over
+// the weights, then a block for each row's partials (one thread adding 304
+// partials at 64 cycles of FP64 latency each took 21 us).
 template <typename T>
-__global__ void k_wsum(size_t n, size_t dim, size_t ld, const T *state,
-    const double *W, double *part)
+__global__ void __launch_bounds__(kB) k_wsum(size_t n, size_t dim, size_t ld,
+    const T *state, const double *W, double *part)
 {
+    constexpr int kD = 4;
     __shared__ double sh[kB / 32 + 1];
-    for (size_t d = 0; d < dim; ++d) {
-        double s = 0;
-        GRID_LOOP(i, n) s += W[i] * static_cast<double>(state[d * ld + i]);
-        s = block_reduce(s, OpAdd(), 0.0, sh);
-        if (threadIdx.x == 0)
-            part[d * gridDim.x + blockIdx.x] = s;
+    for (size_t d0 = 0; d0 < dim; d0 += kD) {
+        const int nd = dim - d0 < kD ? static_cast<int>(dim - d0) : kD;
+        double s[kD] = {};
+        GRID_LOOP(i, n)
+        {
+            const double w = W[i];
+#pragma unroll
+            for (int d = 0; d < kD; ++d)
+                if (d < nd)
+                    s[d] += w * static_cast<double>(state[(d0 + d) * ld + i]);
+        }
+#pragma unroll
+        for (int d = 0; d < kD; ++d)
+            if (d < nd) {
+                const double t = block_reduce(s[d], OpAdd(), 0.0, sh);
+                if (threadIdx.x == 0)
+                    part[(d0 + d) * gridDim.x + blockIdx.x] = t;
+            }
     }
 }
 
-__global__ void k_wsum_final(size_t dim, int nb, const double *part,
-    double *out)
+__global__ void __launch_bounds__(kB) k_wsum_final(
+    int nb, const double *part, double *out)
 {
-    if (threadIdx.x < dim && blockIdx.x == 0) {
-        double s = 0;
-        for (int b = 0; b < nb; ++b)
-            s += part[threadIdx.x * nb + b];
-        out[threadIdx.x] = s;
-    }
+    __shared__ double sh[kB / 32 + 1];
+    double s = 0;
+    for (int b = threadIdx.x; b < nb; b += kB)
+        s += part[static_cast<size_t>(blockIdx.x) * nb + b];
+    s = block_reduce(s, OpAdd(), 0.0, sh);
+    if (threadIdx.x == 0)
+        out[blockIdx.x] = s;
 }
 
 EngineState engine_state(const vsmc_cuda_rng &r)
@@ -893,10 +1156,6 @@ bool size_ok(size_t n) { return n < (size_t(1) << 31); }
 } // namespace
 
 // ------------------------------------------------------- internal entries
-
-// the words of new_err past the sums' tickets
-constexpr int kErrUnsorted = 3; // sorted uniforms that step back
-constexpr int kErrTail = 4;     // uniforms left to the last particle
 
 // rep for m weights against n uniforms u (device); integ added if non-null.
 // The uniforms left to the last particle go to err[kErrTail] (m >= 2, n > 0).
@@ -943,58 +1202,73 @@ int u01_rep_device(size_t m, size_t n, const double *w, const double *u,
         st);
 }
 
+static int rep_index_square(size_t n, const int *rep, int *idx, uint32_t *err,
+    Scratch &scratch, cudaStream_t st)
+{
+    SlotArgs a = {};
+    a.n = static_cast<uint32_t>(n);
+    a.nt = static_cast<uint32_t>((n + kSeqTile - 1) / kSeqTile);
+    a.rep = rep;
+    a.idx = idx;
+    a.err = err;
+    a.srcs = scratch.get<uint32_t>(n);
+    if (a.srcs == nullptr)
+        return VSMC_CUDA_ERR_ALLOC;
+    if (n <= kSeqSmall) {
+        SeqArgs q = {};
+        q.n = a.n;
+        q.nt = a.nt;
+        return seq_cluster_launch(k_slots_small, q, st, a);
+    }
+    a.blocks = static_cast<uint32_t>(grid_for(a.nt, 1, 1, kSeqOcc));
+    a.S = scratch.get<uint64_t>(a.blocks + 1);
+    a.E = scratch.get<uint32_t>(a.blocks + 1);
+    if (!a.S || !a.E)
+        return VSMC_CUDA_ERR_ALLOC;
+    k_slots_count<<<a.blocks, kSeqBlock, 0, st>>>(a);
+    k_slots_assign<<<a.blocks, kSeqBlock, 0, st>>>(a);
+    k_slots_decode<<<grid1(n), kB, 0, st>>>(a);
+    VSMC_CUDA_CHECK_LAUNCH();
+    return VSMC_CUDA_OK;
+}
+
 int rep_index_device(size_t m, size_t n, const int *rep, int *idx,
     uint32_t *err, Scratch &scratch, cudaStream_t st)
 {
     if (m == 0 || n == 0)
         return VSMC_CUDA_OK;
-    const bool square = m == n;
+    if (m == n)
+        return rep_index_square(n, rep, idx, err, scratch, st);
     I2 *incl = scratch.get<I2>(m);
     I2 *pp = scratch.get<I2>(scan_parts(m));
     if (!incl || !pp)
         return VSMC_CUDA_ERR_ALLOC;
-    int rc = device_scan(m, LoadES{rep, square}, StoreI2{incl}, OpI2(),
-        I2{0, 0}, pp, st);
+    int rc = device_scan(
+        m, LoadES{rep}, StoreI2{incl}, OpI2(), I2{0, 0}, pp, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    // the number of ranks / slots is needed on the host to size the scan
+    // the number of slots is needed on the host to size the scan
     I2 tot;
     VSMC_CUDA_TRY(cudaMemcpyAsync(
         &tot, incl + (m - 1), sizeof(I2), cudaMemcpyDeviceToHost, st));
     VSMC_CUDA_TRY(cudaStreamSynchronize(st));
-    size_t nmarks;
-    if (square) {
-        if (tot.a != tot.b || tot.a < 0)
-            return VSMC_CUDA_ERR_ARG; // counts do not sum to n
-        nmarks = static_cast<size_t>(tot.a);
-    } else {
-        if (tot.a < 0 || static_cast<size_t>(tot.a) > n)
-            return VSMC_CUDA_ERR_ARG;
-        nmarks = static_cast<size_t>(tot.a);
-    }
-    if (nmarks == 0) {
-        if (square)
-            k_index_square<<<grid1(n), kB, 0, st>>>(
-                n, rep, incl, nullptr, 0, idx, err);
-        VSMC_CUDA_CHECK_LAUNCH();
+    if (tot.a < 0 || static_cast<size_t>(tot.a) > n)
+        return VSMC_CUDA_ERR_ARG;
+    const size_t nmarks = static_cast<size_t>(tot.a);
+    if (nmarks == 0)
         return VSMC_CUDA_OK;
-    }
     int *marks = scratch.get<int>(nmarks);
     int *srcs = scratch.get<int>(nmarks);
     int *pm = scratch.get<int>(scan_parts(nmarks));
     if (!marks || !srcs || !pm)
         return VSMC_CUDA_ERR_ALLOC;
     VSMC_CUDA_TRY(cudaMemsetAsync(marks, 0, sizeof(int) * nmarks, st));
-    k_marks<<<grid1(m), kB, 0, st>>>(m, square, rep, incl, marks, nmarks, err);
+    k_marks<<<grid1(m), kB, 0, st>>>(m, rep, incl, marks, nmarks, err);
     VSMC_CUDA_CHECK_LAUNCH();
     rc = device_scan(nmarks, LoadI{marks}, StoreI{srcs}, OpMaxI(), 0, pm, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    if (square)
-        k_index_square<<<grid1(n), kB, 0, st>>>(
-            n, rep, incl, srcs, nmarks, idx, err);
-    else
-        k_index_flat<<<grid1(nmarks), kB, 0, st>>>(nmarks, srcs, idx);
+    k_index_flat<<<grid1(nmarks), kB, 0, st>>>(nmarks, srcs, idx);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1010,15 +1284,18 @@ int residual_device(size_t m, size_t n, const double *w, double *resid,
     }
     k_residual_split<<<grid1(m), kB, 0, st>>>(m, n, w, resid, integ, err);
     VSMC_CUDA_CHECK_LAUNCH();
-    double *total = scratch.get<double>(1);
     long long *isum = scratch.get<long long>(1);
     long long *pp = scratch.get<long long>(scan_parts(m));
-    if (!total || !isum || !pp)
+    if (!isum || !pp)
         return VSMC_CUDA_ERR_ALLOC;
-    int rc = seqsum_device(m, resid, nullptr, total, err, scratch, st);
+    SeqArgs a;
+    int rc = seq_args(m, err, false, scratch, &a);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    k_scale<<<grid1(m), kB, 0, st>>>(m, total, resid);
+    rc = seq_total(a, SeqLoad{resid}, st);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
+    k_scale<<<grid1(m), kB, 0, st>>>(m, a.inv, resid);
     VSMC_CUDA_CHECK_LAUNCH();
     // the integer parts summed in 64 bits: unnormalized weights can push
     // the sum past 2^31, and a wrapped 32-bit sum could land back in [0, n]
@@ -1042,12 +1319,10 @@ int residual_device(size_t m, size_t n, const double *w, double *resid,
     return VSMC_CUDA_OK;
 }
 
-int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
-    int *rep, int scheme, Scratch &scratch, cudaStream_t st)
+int scheme_enqueue(size_t m, size_t n, const vsmc_cuda_rng &rng,
+    const double *w, int *rep, int scheme, uint32_t *err, size_t *N_out,
+    Scratch &scratch, cudaStream_t st)
 {
-    uint32_t *err = new_err(scratch, st);
-    if (err == nullptr)
-        return VSMC_CUDA_ERR_ALLOC;
     const bool residual = scheme >= VSMC_CUDA_RESIDUAL;
     const int base = residual ? scheme - VSMC_CUDA_RESIDUAL : scheme;
     const double *wt = w;
@@ -1064,7 +1339,8 @@ int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
             return rc;
         wt = resid;
     }
-    const EngineState es = engine_state(*rng);
+    *N_out = N;
+    const EngineState es = engine_state(rng);
     double *u = scratch.get<double>(N + 4);
     if (u == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
@@ -1097,7 +1373,32 @@ int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
         }
         VSMC_CUDA_CHECK_LAUNCH();
     }
-    rc = u01_rep_device(m, N, wt, u, order, rep, integ, err, scratch, st);
+    return u01_rep_device(m, N, wt, u, order, rep, integ, err, scratch, st);
+}
+
+void scheme_advance(
+    vsmc_cuda_rng &rng, size_t m, size_t N, int scheme, uint32_t tail)
+{
+    // systematic: the sequence constructor draws once; the others draw
+    // lazily, up to the first uniform above the second-to-last CDF value
+    uint64_t words = 0;
+    if (scheme == VSMC_CUDA_SYSTEMATIC ||
+        scheme == VSMC_CUDA_RESIDUAL_SYSTEMATIC)
+        words = 1;
+    else if (m >= 2 && N > 0)
+        words = std::min<uint64_t>(N - tail + 1, N);
+    engine_advance_host(rng, words);
+}
+
+int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
+    int *rep, int scheme, Scratch &scratch, cudaStream_t st)
+{
+    uint32_t *err = new_err(scratch, st);
+    if (err == nullptr)
+        return VSMC_CUDA_ERR_ALLOC;
+    size_t N = 0;
+    const int rc =
+        scheme_enqueue(m, n, *rng, w, rep, scheme, err, &N, scratch, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
     uint32_t word[kErrWords] = {};
@@ -1107,55 +1408,50 @@ int scheme_device(size_t m, size_t n, vsmc_cuda_rng *rng, const double *w,
     const int status = err_status(word[0]);
     if (status != VSMC_CUDA_OK)
         return status;
-    // systematic: the sequence constructor draws once; the others draw
-    // lazily, up to the first uniform above the second-to-last CDF value
-    uint64_t words = 0;
-    if (base == VSMC_CUDA_SYSTEMATIC)
-        words = 1;
-    else if (m >= 2 && N > 0)
-        words = std::min<uint64_t>(N - word[kErrTail] + 1, N);
-    engine_advance_host(*rng, words);
+    scheme_advance(*rng, m, N, scheme, word[kErrTail]);
     return VSMC_CUDA_OK;
 }
 
-// Weight::normalize(use_log) on W in place: sum, scale, ESS (weight.hpp:208-229)
-int weight_normalize_device(size_t n, double *W, double *ess_dev,
-    uint32_t *err, Scratch &scratch, cudaStream_t st)
+// Both sums of more than kSeqSmall weights: W = v / sum(v), *ess (may be
+// null); a.total gets the first.
+int weight_sums(SeqArgs a, const double *v, double *W, double *ess,
+    cudaStream_t st)
 {
-    double *total = scratch.get<double>(1);
-    double *sq = scratch.get<double>(n);
-    double *tsq = scratch.get<double>(1);
-    if (!total || !sq || !tsq)
-        return VSMC_CUDA_ERR_ALLOC;
-    int rc = seqsum_device(n, W, nullptr, total, err, scratch, st);
+    const int rc = seq_total(a, SeqLoad{v}, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    k_scale<<<grid1(n), kB, 0, st>>>(n, total, W);
-    k_square<<<grid1(n), kB, 0, st>>>(n, W, sq);
-    VSMC_CUDA_CHECK_LAUNCH();
-    rc = seqsum_device(n, sq, nullptr, tsq, err, scratch, st);
-    if (rc != VSMC_CUDA_OK)
-        return rc;
-    if (ess_dev) {
-        k_inv_total<<<1, 32, 0, st>>>(tsq, ess_dev);
-        VSMC_CUDA_CHECK_LAUNCH();
-    }
-    return VSMC_CUDA_OK;
+    const ScaleSquare scale{v, a.inv, W};
+    a.total = nullptr;
+    a.inv = ess;
+    return seq_total_large(a, scale, SquareLoad{W}, st);
 }
 
-// post_set_log: subtract the max, exponentiate, normalize
-int weight_post_set_log_device(size_t n, double *W, double *ess_dev,
-    uint32_t *err, Scratch &scratch, cudaStream_t st)
+// Weight::normalize: W = v / sum(v), ESS (weight.hpp:208-229); v may be W
+int weight_normalize_device(size_t n, const double *v, double *W,
+    double *ess_dev, uint32_t *err, Scratch &scratch, cudaStream_t st)
 {
-    const int nb = grid1(n);
-    double *part = scratch.get<double>(nb);
-    if (part == nullptr)
-        return VSMC_CUDA_ERR_ALLOC;
-    k_reduce_max<<<nb, kB, 0, st>>>(n, W, part);
-    k_max_parts<<<1, kB, 0, st>>>(nb, part);
-    k_exp_shift<<<grid1(n), kB, 0, st>>>(n, W, part, W);
+    SeqArgs a;
+    int rc = seq_args(n, err, false, scratch, &a);
+    if (rc != VSMC_CUDA_OK)
+        return rc;
+    if (n <= kSeqSmall)
+        return seq_cluster_launch(k_normalize_small, a, st, v, W, ess_dev);
+    return weight_sums(a, v, W, ess_dev, st);
+}
+
+// the running maximum's key, two words of new_err's
+unsigned long long *max_word(uint32_t *err)
+{
+    return reinterpret_cast<unsigned long long *>(err + kErrMax);
+}
+
+int weight_set_log_device(size_t n, const double *lw, double *W,
+    double *ess_dev, uint32_t *err, Scratch &scratch, cudaStream_t st)
+{
+    k_lw_max<false><<<grid64(n), kB64, 0, st>>>(n, lw, nullptr, max_word(err));
+    k_exp_shift<<<grid64(n), kB64, 0, st>>>(n, lw, max_word(err), W);
     VSMC_CUDA_CHECK_LAUNCH();
-    return weight_normalize_device(n, W, ess_dev, err, scratch, st);
+    return weight_normalize_device(n, W, W, ess_dev, err, scratch, st);
 }
 
 int weight_set_equal_device(size_t n, double *W, double *ess_dev,
@@ -1163,27 +1459,30 @@ int weight_set_equal_device(size_t n, double *W, double *ess_dev,
 {
     k_fill_d<<<grid1(n), kB, 0, st>>>(n, W, 1.0 / static_cast<double>(n));
     VSMC_CUDA_CHECK_LAUNCH();
-    return weight_normalize_device(n, W, ess_dev, err, scratch, st);
+    return weight_normalize_device(n, W, W, ess_dev, err, scratch, st);
 }
 
 int weight_add_log_device(size_t n, const double *l, double *W,
     double *ess_dev, uint32_t *err, Scratch &scratch, cudaStream_t st)
 {
-    k_log_add<<<grid1(n), kB, 0, st>>>(n, l, W);
+    k_lw_max<true><<<grid64(n), kB64, 0, st>>>(n, l, W, max_word(err));
+    k_exp_shift<<<grid64(n), kB64, 0, st>>>(n, W, max_word(err), W);
     VSMC_CUDA_CHECK_LAUNCH();
-    return weight_post_set_log_device(n, W, ess_dev, err, scratch, st);
+    return weight_normalize_device(n, W, W, ess_dev, err, scratch, st);
 }
 
 template <typename T>
 int monitor_mean_device(size_t n, size_t dim, size_t ld, const T *state,
     const double *W, double *out, Scratch &scratch, cudaStream_t st)
 {
-    const int nb = grid_for(n, kB, 8, 2);
+    const int nb = grid_for(n, kB, 2, 2);
     double *part = scratch.get<double>(dim * nb);
     if (part == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
     k_wsum<T><<<nb, kB, 0, st>>>(n, dim, ld, state, W, part);
-    k_wsum_final<<<1, 32, 0, st>>>(dim, nb, part, out);
+    if (dim)
+        k_wsum_final<<<static_cast<unsigned>(dim), kB, 0, st>>>(
+            nb, part, out);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1460,10 +1759,7 @@ int vsmc_cuda_weight_set(size_t n, const double *w, double *W,
     if (!size_ok(n))
         return VSMC_CUDA_ERR_SIZE;
     return with_err(stream, [&](uint32_t *err, Scratch &sc, cudaStream_t st) -> int {
-        if (W != w)
-            VSMC_CUDA_TRY(cudaMemcpyAsync(W, w, sizeof(double) * n,
-                cudaMemcpyDeviceToDevice, st));
-        return weight_normalize_device(n, W, ess_dev, err, sc, st);
+        return weight_normalize_device(n, w, W, ess_dev, err, sc, st);
     });
 }
 
@@ -1477,10 +1773,7 @@ int vsmc_cuda_weight_set_log(size_t n, const double *lw, double *W,
     if (!size_ok(n))
         return VSMC_CUDA_ERR_SIZE;
     return with_err(stream, [&](uint32_t *err, Scratch &sc, cudaStream_t st) -> int {
-        if (W != lw)
-            VSMC_CUDA_TRY(cudaMemcpyAsync(W, lw, sizeof(double) * n,
-                cudaMemcpyDeviceToDevice, st));
-        return weight_post_set_log_device(n, W, ess_dev, err, sc, st);
+        return weight_set_log_device(n, lw, W, ess_dev, err, sc, st);
     });
 }
 

@@ -104,6 +104,8 @@ int err_status(uint32_t e)
 {
     if (e & DEV_ERR_NONFINITE)
         return VSMC_CUDA_ERR_NONFINITE;
+    if (e & DEV_ERR_COUNTS)
+        return VSMC_CUDA_ERR_ARG;
     return e ? VSMC_CUDA_ERR_INTERNAL : VSMC_CUDA_OK;
 }
 

@@ -949,6 +949,17 @@ struct SeqClusterSmem {
     uint16_t bex[kSeqTile];
 };
 
+// the block's dynamic shared memory, with a's lists in it
+__device__ __forceinline__ SeqClusterSmem &seq_cluster_smem(SeqArgs &a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SeqClusterSmem &S = *reinterpret_cast<SeqClusterSmem *>(smem);
+    a.adj = S.adj;
+    a.pos = S.pos;
+    a.bex = S.bex;
+    return S;
+}
+
 // The exact left-to-right sum of the cluster's values (v: the block's tile,
 // striped), in every thread; the tile's starting sum and breakpoints stay in
 // S.  a.adj, a.pos and a.bex point at S's lists.
@@ -1061,11 +1072,7 @@ __global__ void __launch_bounds__(kSeqBlock) k_seq_small(
 {
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
-    extern __shared__ __align__(16) unsigned char smem[];
-    SeqClusterSmem &S = *reinterpret_cast<SeqClusterSmem *>(smem);
-    a.adj = S.adj;
-    a.pos = S.pos;
-    a.bex = S.bex;
+    SeqClusterSmem &S = seq_cluster_smem(a);
     const uint32_t tile = cl.block_rank();
     double v[kSeqItems];
     seq_load(load, tile, a.n, v);
@@ -1126,12 +1133,13 @@ uint32_t *new_err(Scratch &scratch, cudaStream_t st);
 int seq_args(size_t n, uint32_t *err, bool allow_inf, Scratch &scratch,
     SeqArgs *a);
 
-template <class Load, class Out>
-int seq_small(const SeqArgs &a, const Load &load, const Out &out,
-    cudaStream_t st)
+// A kernel of one cluster with a tile per block (a.n <= kSeqSmall).
+template <class... Params, class... Args>
+int seq_cluster_launch(void (*kernel)(SeqArgs, Params...), const SeqArgs &a,
+    cudaStream_t st, const Args &...args)
 {
     // the shared memory limit is a property of the kernel on each device
-    VSMC_CUDA_TRY(cudaFuncSetAttribute(k_seq_small<Load, Out>,
+    VSMC_CUDA_TRY(cudaFuncSetAttribute(kernel,
         cudaFuncAttributeMaxDynamicSharedMemorySize,
         static_cast<int>(sizeof(SeqClusterSmem))));
     uint32_t c = 1;
@@ -1149,7 +1157,28 @@ int seq_small(const SeqArgs &a, const Load &load, const Out &out,
     at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    VSMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_seq_small<Load, Out>, a, load, out));
+    VSMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a,
+        static_cast<std::remove_cv_t<std::remove_reference_t<Params>>>(
+            args)...));
+    return VSMC_CUDA_OK;
+}
+
+template <class Load, class Out>
+int seq_small(const SeqArgs &a, const Load &load, const Out &out,
+    cudaStream_t st)
+{
+    return seq_cluster_launch(k_seq_small<Load, Out>, a, st, load, out);
+}
+
+// The sum by the large passes: sums sees every element once (it may compute
+// and store them), load gives the same values afterwards.
+template <class Sums, class Load>
+int seq_total_large(const SeqArgs &a, const Sums &sums, const Load &load,
+    cudaStream_t st)
+{
+    k_seq_sums<Sums><<<a.blocks, kSeqBlock, 0, st>>>(a, sums);
+    k_seq_classify<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
+    VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
 
@@ -1159,10 +1188,7 @@ int seq_total(const SeqArgs &a, const Load &load, cudaStream_t st)
 {
     if (a.n <= kSeqSmall)
         return seq_small(a, load, SeqNoOut(), st);
-    k_seq_sums<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
-    k_seq_classify<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
-    VSMC_CUDA_CHECK_LAUNCH();
-    return VSMC_CUDA_OK;
+    return seq_total_large(a, load, load, st);
 }
 
 // The same, and the running sums to out.
@@ -1185,6 +1211,10 @@ int seq_scan(const SeqArgs &a, const Load &load, const Out &out,
 // Device error bits go to *err (DEV_ERR_NONFINITE for negative / NaN terms).
 int seqsum_device(size_t n, const double *x, double *prefix, double *total,
     uint32_t *err, Scratch &scratch, cudaStream_t st, bool allow_inf = false);
+
+// error bit: replication counts that do not sum to the slots
+// (VSMC_CUDA_ERR_ARG)
+enum : unsigned { DEV_ERR_COUNTS = 8u };
 
 // status of a device error word
 int err_status(uint32_t e);
