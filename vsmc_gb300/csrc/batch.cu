@@ -1279,7 +1279,7 @@ template <typename T>
 static int balloc(T **p, size_t count)
 {
     void *q = nullptr;
-    VSMC_CUDA_TRY(cudaMalloc(&q, sizeof(T) * (count ? count : 1)));
+    VSMC_CUDA_TRY(device_malloc(&q, sizeof(T) * (count ? count : 1)));
     *p = static_cast<T *>(q);
     return VSMC_CUDA_OK;
 }

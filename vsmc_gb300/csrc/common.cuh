@@ -236,8 +236,13 @@ int num_sms();
 int grid_for(size_t work_items, int block, int items_per_thread,
     int blocks_per_sm = 4);
 
-// Stream-ordered scratch allocation (cudaMallocAsync on the caller's
-// stream).  RAII: freed on the same stream when it goes out of scope.
+// cudaMalloc; out of memory, it is tried again after the scratch pools gave
+// back what no call uses.
+cudaError_t device_malloc(void **p, size_t bytes);
+
+// Stream-ordered scratch allocation on the caller's stream, from the
+// library's pool of its device.  RAII: freed on the same stream when it goes
+// out of scope.
 class Scratch
 {
     public:

@@ -425,7 +425,7 @@ template <typename T>
 static int dalloc(T **p, size_t count)
 {
     void *q = nullptr;
-    VSMC_CUDA_TRY(cudaMalloc(&q, sizeof(T) * (count ? count : 1)));
+    VSMC_CUDA_TRY(device_malloc(&q, sizeof(T) * (count ? count : 1)));
     *p = static_cast<T *>(q);
     return VSMC_CUDA_OK;
 }
@@ -964,7 +964,7 @@ int vsmc_cuda_pf_record_genealogy(vsmc_cuda_pf *pf, int on)
         return VSMC_CUDA_ERR_ARG;
     if (on && pf->gen == nullptr) {
         void *p = nullptr;
-        VSMC_CUDA_TRY(cudaMalloc(&p, sizeof(int32_t) * pf->n * pf->max_steps));
+        VSMC_CUDA_TRY(device_malloc(&p, sizeof(int32_t) * pf->n * pf->max_steps));
         pf->gen = static_cast<int32_t *>(p);
     }
     if ((on != 0) != pf->record_gen)
@@ -982,7 +982,7 @@ int vsmc_cuda_pf_set_mcmc(vsmc_cuda_pf *pf, size_t sweeps, double scale)
         return VSMC_CUDA_ERR_SIZE;
     if (sweeps > 0 && pf->h_acc == nullptr) {
         void *p = nullptr;
-        VSMC_CUDA_TRY(cudaMalloc(&p, sizeof(uint32_t) * pf->max_steps));
+        VSMC_CUDA_TRY(device_malloc(&p, sizeof(uint32_t) * pf->max_steps));
         pf->h_acc = static_cast<uint32_t *>(p);
         VSMC_CUDA_TRY(cudaMemset(pf->h_acc, 0, sizeof(uint32_t) * pf->max_steps));
     }

@@ -298,12 +298,16 @@ int pf64_create(vsmc_cuda_pf *pf)
     pf->p64 = p;
     const size_t n = pf->n;
     cudaStream_t st = pf->stream;
-    if (cudaMalloc(&p->rep, sizeof(int) * n) != cudaSuccess ||
-        cudaMalloc(&p->idx, sizeof(int) * n) != cudaSuccess ||
-        cudaMalloc(&p->scal, sizeof(double) * 8) != cudaSuccess ||
-        cudaMalloc(&p->part, sizeof(double) * 2 * select_grid(n)) !=
-            cudaSuccess ||
-        cudaMalloc(&p->err, sizeof(uint32_t) * kErrWords) != cudaSuccess ||
+    auto get = [](auto **q, size_t bytes) {
+        void *v = nullptr;
+        const cudaError_t e = device_malloc(&v, bytes);
+        *q = static_cast<std::remove_pointer_t<decltype(q)>>(v);
+        return e == cudaSuccess;
+    };
+    if (!get(&p->rep, sizeof(int) * n) || !get(&p->idx, sizeof(int) * n) ||
+        !get(&p->scal, sizeof(double) * 8) ||
+        !get(&p->part, sizeof(double) * 2 * select_grid(n)) ||
+        !get(&p->err, sizeof(uint32_t) * kErrWords) ||
         cudaHostAlloc(reinterpret_cast<void **>(&p->host), sizeof(Pf64Host),
             cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(reinterpret_cast<void **>(&p->host_dev),

@@ -295,6 +295,20 @@ __device__ __forceinline__ bool seq_last_block(uint32_t *ticket, SeqSmem &sh)
 
 // ------------------------------------------------------------- tile sums
 
+// t 2^(E - 1075) as a double (E = 0xFFFF: infinite), by the exponent field
+// where the result is a normal number
+__device__ __forceinline__ double seq_scaled(uint64_t t, uint32_t E)
+{
+    if (E == 0xFFFFu)
+        return from_dbits(kInfBits);
+    const double d = __ull2double_rn(t);
+    const int e = static_cast<int>(E) - 1075;
+    if (t != 0 && E > 64 && E < 1983)
+        return __hiloint2double(
+            __double2hiint(d) + (e << 20), __double2loint(d));
+    return ldexp(d, e);
+}
+
 // Approximate sum of the tile's values (v striped, 0 past the end), valid
 // in thread 0.  Negative, NaN and (unless allowed) infinite values are
 // reported and count as 0.
@@ -364,9 +378,7 @@ __device__ __forceinline__ double seq_tile_sum(const double (&v)[kSeqItems],
         for (int o = kSeqWarps / 2; o > 0; o >>= 1)
             t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
         if (lane == 0)
-            s = Em == 0xFFFFu
-                ? from_dbits(kInfBits)
-                : ldexp(__ull2double_rn(t), static_cast<int>(Em) - 1075);
+            s = seq_scaled(t, Em);
     }
     return s;
 }
@@ -997,17 +1009,18 @@ __device__ __forceinline__ double seq_cluster_total(
     }
     cl.sync();
     if (tile == 0) { // walk the breakpoints, as seq_fixup does
-        if (threadIdx.x == 0) {
-            uint64_t r = 0;
-            uint32_t f = 0;
-            for (uint32_t q = 0; q < nc; ++q) {
-                S.s_R[q] = r;
-                S.s_F[q] = f;
-                r += cl.map_shared_rank(&S, q)->R;
-                f += cl.map_shared_rank(&S, q)->F;
+        if (threadIdx.x < 32) {
+            const SeqClusterSmem *B = cl.map_shared_rank(&S, min(lane, nc - 1));
+            const uint64_t r = warp_incl_any(lane < nc ? B->R : 0ull, OpAdd());
+            const uint32_t f = warp_incl_any(lane < nc ? B->F : 0u, OpAdd());
+            if (lane < nc) {
+                S.s_R[lane + 1] = r;
+                S.s_F[lane + 1] = f;
             }
-            S.s_R[nc] = r;
-            S.s_F[nc] = f;
+            if (lane == 0) {
+                S.s_R[0] = 0;
+                S.s_F[0] = 0;
+            }
         }
         __syncthreads();
         const uint32_t nbk = S.s_F[nc];
