@@ -332,6 +332,69 @@ __device__ __forceinline__ void pf_particle(const Model &model,
     acc.push(lw, x);
 }
 
+// ------------------------------------------------- FP64 block reductions
+//
+// An FP64 instruction of a warp takes 19 cycles of its SM, so the sums below
+// split the values over the lanes as they go: NV values over 32 lanes in
+// about NV + 4 additions, not 5 NV.  Every addition is the same pair as in a
+// plain butterfly, so the results are the same bits.
+
+// v[0..NV) summed over the warp; value k ends in lane warp_sum_lane<NV>(k)
+// (in v[0] there).
+template <int NV>
+__device__ __forceinline__ void warp_sum_split(double (&v)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    int n = NV;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        if (n > 1) {
+            const int h = (n + 1) / 2;
+            const bool up = (lane & d) != 0;
+#pragma unroll
+            for (int i = 0; i < (NV + 1) / 2; ++i)
+                if (i < h) {
+                    const double hi = i + h < n ? v[i + h] : 0.0;
+                    const double keep = up ? hi : v[i];
+                    const double send = up ? v[i] : hi;
+                    v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, d);
+                }
+            n = h;
+        } else {
+            v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], d);
+        }
+    }
+}
+
+template <int NV>
+__host__ __device__ constexpr int warp_sum_lane(int k)
+{
+    int lane = 0, n = NV;
+    for (int d = 16; d > 0; d >>= 1)
+        if (n > 1) {
+            const int h = (n + 1) / 2;
+            if (k >= h) {
+                lane |= d;
+                k -= h;
+            }
+            n = h;
+        }
+    return lane;
+}
+
+// the value warp_sum_split leaves in the calling lane (NV and more: none)
+template <int NV>
+__device__ __forceinline__ int warp_sum_value()
+{
+    const int lane = threadIdx.x & 31;
+    int v = NV;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (lane == warp_sum_lane<NV>(k))
+            v = k;
+    return v;
+}
+
 // ------------------------------------------------------------ fused step
 
 template <class Model, bool First, PfMon Mon>
@@ -437,7 +500,7 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
     constexpr int kW = kPfBlock / 32;
     __shared__ LseMon<AMD> shw[kW];
     __shared__ float shp[kMaxMonitorDim + 1][kW];
-    __shared__ double shd[3 + 2 * kMaxMonitorDim + 1][kW];
+    __shared__ double shd[2 + 2 * kMaxMonitorDim + 1][kW];
     __shared__ float shmax[kW];
     __shared__ bool is_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -458,29 +521,30 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
 #pragma unroll
         for (int d = kW / 2; d > 0; d >>= 1)
             w.merge(w.shfl_xor(d));
-        if (lane == 0) {
-            PfPartial p;
-            p.m = w.m;
-            p.s = w.s;
-            p.s2 = w.s2;
-#pragma unroll
-            for (int d = 0; d < kMaxMonitorDim; ++d) {
-                p.mon[d] = d < AMD ? w.mon[d < AMD ? d : 0] : 0.0;
-                double pv = 0;
-                if (prev_on && d < MD)
-                    for (int k = 0; k < kW; ++k)
-                        pv += shp[d < MD ? d : 0][k];
-                p.prev[d] = pv;
-            }
-            double pw = 0;
-            if (prev_on)
+        // the warps' monitor sums in FP64, a component per lane (its last
+        // one, the weights)
+        double pv = 0;
+        if (prev_on && lane <= kMaxMonitorDim)
+            if (lane < MD || lane == kMaxMonitorDim)
                 for (int k = 0; k < kW; ++k)
-                    pw += shp[kMaxMonitorDim][k];
-            p.prev_w = pw;
-            a.part[blockIdx.x] = p;
-            __threadfence();
-            is_last = atomicAdd(&a.sc->done, 1u) == gridDim.x - 1;
+                    pv += shp[lane][k];
+        PfPartial *p = a.part + blockIdx.x;
+        if (lane == 0) {
+            p->m = w.m;
+            p->s = w.s;
+            p->s2 = w.s2;
+#pragma unroll
+            for (int d = 0; d < kMaxMonitorDim; ++d)
+                p->mon[d] = d < AMD ? w.mon[d < AMD ? d : 0] : 0.0;
         }
+        if (lane < kMaxMonitorDim)
+            p->prev[lane] = pv;
+        else if (lane == kMaxMonitorDim)
+            p->prev_w = pv;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0)
+            is_last = atomicAdd(&a.sc->done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!is_last)
@@ -501,69 +565,69 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
 #pragma unroll
     for (int w = 1; w < kW; ++w)
         M = fmaxf(M, shmax[w]);
-    double v[3 + 2 * kMaxMonitorDim + 1] = {};
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        const double pm = __ldcg(&a.part[b].m);
-        if (pm > -INFINITY) {
-            const double f = __expf(static_cast<float>(pm) - M);
-            v[0] += __ldcg(&a.part[b].s) * f;
-            v[1] += __ldcg(&a.part[b].s2) * f * f;
+    // S, S2, then the sums this mode has: the step's own monitor, or the
+    // previous step's and its weights
+    constexpr int NV = 2 + AMD + (prev_on ? MD + 1 : 0);
+    double v[NV] = {};
+    if (wid * 32 < static_cast<int>(gridDim.x)) { // records for this warp
+        for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+            const double pm = __ldcg(&a.part[b].m);
+            if (pm > -INFINITY) {
+                const double f = __expf(static_cast<float>(pm) - M);
+                v[0] += __ldcg(&a.part[b].s) * f;
+                v[1] += __ldcg(&a.part[b].s2) * f * f;
 #pragma unroll
-            for (int d = 0; d < AMD; ++d)
-                v[3 + d] += __ldcg(&a.part[b].mon[d]) * f;
-        }
-        if (prev_on) {
-#pragma unroll
-            for (int d = 0; d < MD; ++d)
-                v[3 + kMaxMonitorDim + d] += __ldcg(&a.part[b].prev[d]);
-            v[3 + 2 * kMaxMonitorDim] += __ldcg(&a.part[b].prev_w);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3 + 2 * kMaxMonitorDim + 1; ++k) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1)
-            v[k] += __shfl_xor_sync(0xFFFFFFFFu, v[k], d);
-        if (lane == 0)
-            shd[k][wid] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double S = 0, S2 = 0, MON[kMaxMonitorDim] = {},
-               PREV[kMaxMonitorDim] = {}, PW = 0;
-        for (int w = 0; w < kW; ++w) {
-            S += shd[0][w];
-            S2 += shd[1][w];
-#pragma unroll
-            for (int d = 0; d < MD; ++d) {
-                MON[d] += shd[3 + d][w];
-                PREV[d] += shd[3 + kMaxMonitorDim + d][w];
+                for (int d = 0; d < AMD; ++d)
+                    v[2 + d] += __ldcg(&a.part[b].mon[d]) * f;
             }
-            PW += shd[3 + 2 * kMaxMonitorDim][w];
-        }
-        if (prev_on && t >= 1 && t - 1 < a.max_steps) {
+            if (prev_on) {
 #pragma unroll
-            for (int d = 0; d < MD; ++d)
-                a.h_mean[static_cast<size_t>(t - 1) * MD + d] = PREV[d] / PW;
+                for (int d = 0; d < MD; ++d)
+                    v[2 + AMD + d] += __ldcg(&a.part[b].prev[d]);
+                v[NV - 1] += __ldcg(&a.part[b].prev_w);
+            }
         }
-        PfScalars &sc = *a.sc;
-        const double prev_mass = resampled ? static_cast<double>(n) : sc.S;
-        const bool rec = t < a.max_steps;
-        const double ess = S * S / S2;
+        warp_sum_split(v);
+    }
+    const int mine = warp_sum_value<NV>();
+    if (mine < NV)
+        shd[mine][wid] = v[0];
+    __syncthreads();
+    if (wid != 0)
+        return;
+    // one warp finishes: lane k sums value k over the warps, then the
+    // quotients and the two logarithms are taken in different lanes at once
+    double tot = 0;
+    if (lane < NV)
+        for (int w = 0; w < kW; ++w)
+            tot += shd[lane][w];
+    PfScalars &sc = *a.sc;
+    const double S = __shfl_sync(0xFFFFFFFFu, tot, 0);
+    const double S2 = __shfl_sync(0xFFFFFFFFu, tot, 1);
+    const double PW = __shfl_sync(0xFFFFFFFFu, tot, NV - 1);
+    const double prev_mass = resampled ? static_cast<double>(n) : sc.S;
+    // lane 1: ESS; a monitor component in its own lane: its mean
+    const double quot = (lane == 1 ? S * S : tot) /
+        (lane == 1 ? S2 : (prev_on && lane >= 2 + AMD ? PW : S));
+    const double lg = log(lane == 1 ? prev_mass : S);
+    const double ess = __shfl_sync(0xFFFFFFFFu, quot, 1);
+    const double lg_prev = __shfl_sync(0xFFFFFFFFu, lg, 1);
+    const bool rec = t < a.max_steps;
+    if (prev_on && t >= 1 && t - 1 < a.max_steps && lane >= 2 + AMD &&
+        lane < 2 + AMD + MD)
+        a.h_mean[static_cast<size_t>(t - 1) * MD + (lane - 2 - AMD)] = quot;
+    if (Mon == PfMon::Current && lane >= 2 && lane < 2 + MD) {
+        sc.mean[lane - 2] = quot;
+        if (rec)
+            a.h_mean[static_cast<size_t>(t) * MD + (lane - 2)] = quot;
+    }
+    if (lane == 0) {
         const double M1 = static_cast<double>(M);
-        sc.logz += M1 + log(S) - log(prev_mass);
+        sc.logz += M1 + lg - lg_prev;
         if (!(S > 0) || !(ess > 0))
             sc.err |= DEV_ERR_NONFINITE;
         const int flag =
             ess < a.threshold * static_cast<double>(n) ? 1 : 0;
-        if (Mon == PfMon::Current) {
-#pragma unroll
-            for (int d = 0; d < MD; ++d) {
-                sc.mean[d] = MON[d] / S;
-                if (rec)
-                    a.h_mean[static_cast<size_t>(t) * MD + d] = MON[d] / S;
-            }
-        }
         if (rec) {
             a.h_ess[t] = ess;
             a.h_logz[t] = sc.logz;
