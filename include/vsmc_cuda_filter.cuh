@@ -70,6 +70,7 @@ enum : unsigned {
     DEV_ERR_NONFINITE = 1u, // NaN / inf / negative weight where forbidden
     DEV_ERR_BOUND = 2u,     // an exactness or iteration bound was exceeded
     DEV_ERR_INTERNAL = 4u,  // an index left its range
+    DEV_ERR_TIMEOUT = 16u,  // a bounded wait gave up
 };
 
 // Device-resident filter scalars (one per filter; the library allocates
@@ -139,53 +140,37 @@ struct LseMon {
     float m, s, s2;
     float mon[MD > 0 ? MD : 1];
 
+    // Both without branches: the side with the larger max keeps its sums,
+    // the other's are scaled by e = exp(its max - the larger one).  A weight
+    // that is -inf or NaN, and an empty side, add nothing (e = 0).
     template <int D>
     __device__ __forceinline__ void push(float v, const float (&x)[D])
     {
-        if (!(v > -INFINITY)) // -inf and NaN carry no weight
-            return;
-        if (v > m) {
-            const float e = __expf(m - v);
-            s = s * e + 1.0f;
-            s2 = s2 * e * e + 1.0f;
+        const bool up = v > m;
+        const bool ok = v > -INFINITY; // -inf and NaN carry no weight
+        const float e = ok ? __expf(up ? m - v : v - m) : 0.0f;
+        s = fmaf(up ? s : 1.0f, e, up ? 1.0f : s);
+        s2 = fmaf((up ? s2 : 1.0f) * e, e, up ? 1.0f : s2);
 #pragma unroll
-            for (int d = 0; d < MD; ++d)
-                mon[d] = mon[d] * e + x[d];
-            m = v;
-        } else {
-            const float e = __expf(v - m);
-            s += e;
-            s2 = fmaf(e, e, s2);
-#pragma unroll
-            for (int d = 0; d < MD; ++d)
-                mon[d] = fmaf(e, x[d], mon[d]);
+        for (int d = 0; d < MD; ++d) {
+            const float y = fmaf(up ? mon[d] : e, up ? e : x[d],
+                up ? x[d] : mon[d]);
+            mon[d] = ok ? y : mon[d];
         }
+        m = up ? v : m;
     }
 
     __device__ __forceinline__ void merge(const LseMon &o)
     {
-        if (!(o.m > -INFINITY))
-            return;
-        if (!(m > -INFINITY)) {
-            *this = o;
-            return;
-        }
-        if (o.m > m) {
-            const float e = __expf(m - o.m);
-            s = s * e + o.s;
-            s2 = s2 * e * e + o.s2;
+        const bool up = o.m > m;
+        const float lo = up ? m : o.m, hi = up ? o.m : m;
+        const float e = lo > -INFINITY ? __expf(lo - hi) : 0.0f;
+        s = fmaf(up ? s : o.s, e, up ? o.s : s);
+        s2 = fmaf((up ? s2 : o.s2) * e, e, up ? o.s2 : s2);
 #pragma unroll
-            for (int d = 0; d < MD; ++d)
-                mon[d] = mon[d] * e + o.mon[d];
-            m = o.m;
-        } else {
-            const float e = __expf(o.m - m);
-            s += o.s * e;
-            s2 += o.s2 * e * e;
-#pragma unroll
-            for (int d = 0; d < MD; ++d)
-                mon[d] += o.mon[d] * e;
-        }
+        for (int d = 0; d < MD; ++d)
+            mon[d] = fmaf(up ? mon[d] : o.mon[d], e, up ? o.mon[d] : mon[d]);
+        m = hi;
     }
 
     __device__ __forceinline__ LseMon shfl_xor(int lanes) const
@@ -397,18 +382,28 @@ __device__ __forceinline__ int warp_sum_value()
 
 // ------------------------------------------------------------ fused step
 
+// Shared memory of a step's reductions.
+template <class Model, PfMon Mon>
+struct PfStepSmem {
+    static constexpr int kW = kPfBlock / 32;
+    static constexpr int AMD = Mon == PfMon::Current ? Model::monitor_dim : 0;
+    LseMon<AMD> shw[kW];
+    float shp[kMaxMonitorDim + 1][kW];
+    double shd[2 + 2 * kMaxMonitorDim + 1][kW];
+    float shmax[kW];
+};
+
+// One block's share of step t: its tiles of particles moved and weighted, and
+// their sums left in *p (by warp 0; the caller orders the write).
 template <class Model, bool First, PfMon Mon>
-__global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
-    const PfStepArgs a, const Model model)
+__device__ __forceinline__ void pf_step_record(const PfStepArgs &a,
+    const Model &model, uint32_t t, int resampled, bool gather, float Mprev,
+    PfPartial *p, PfStepSmem<Model, Mon> &sh)
 {
     constexpr int D = Model::dim;
     constexpr int MD = Model::monitor_dim;
     // the evidence sums carry the monitor only for the current-step mode
     constexpr int AMD = Mon == PfMon::Current ? MD : 0;
-    const uint32_t t = a.sc->step;
-    const int resampled = First ? 1 : a.sc->resampled;
-    const bool gather = First ? false : (a.sc->gather != 0);
-    const float Mprev = First ? 0.0f : static_cast<float>(a.sc->M);
     const typename Model::step_type ctx = model.step(t);
     const uint32_t n = a.n;
     LseMon<AMD> acc = lse_empty<AMD>();
@@ -498,37 +493,24 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
     // ---- block level in FP32 (warp 0 merges the warps' records), then one
     // FP64 record per block
     constexpr int kW = kPfBlock / 32;
-    __shared__ LseMon<AMD> shw[kW];
-    __shared__ float shp[kMaxMonitorDim + 1][kW];
-    __shared__ double shd[2 + 2 * kMaxMonitorDim + 1][kW];
-    __shared__ float shmax[kW];
-    __shared__ bool is_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) {
-        shw[wid] = acc;
+        sh.shw[wid] = acc;
         if (prev_on) {
 #pragma unroll
             for (int d = 0; d < MD; ++d)
-                shp[d][wid] = prev.x[d];
-            shp[kMaxMonitorDim][wid] = prev.w;
+                sh.shp[d][wid] = prev.x[d];
+            sh.shp[kMaxMonitorDim][wid] = prev.w;
         }
     }
     __syncthreads();
     if (wid == 0) {
         LseMon<AMD> w = lse_empty<AMD>();
         if (lane < kW)
-            w = shw[lane];
+            w = sh.shw[lane];
 #pragma unroll
         for (int d = kW / 2; d > 0; d >>= 1)
             w.merge(w.shfl_xor(d));
-        // the warps' monitor sums in FP64, a component per lane (its last
-        // one, the weights)
-        double pv = 0;
-        if (prev_on && lane <= kMaxMonitorDim)
-            if (lane < MD || lane == kMaxMonitorDim)
-                for (int k = 0; k < kW; ++k)
-                    pv += shp[lane][k];
-        PfPartial *p = a.part + blockIdx.x;
         if (lane == 0) {
             p->m = w.m;
             p->s = w.s;
@@ -537,83 +519,133 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
             for (int d = 0; d < kMaxMonitorDim; ++d)
                 p->mon[d] = d < AMD ? w.mon[d < AMD ? d : 0] : 0.0;
         }
-        if (lane < kMaxMonitorDim)
-            p->prev[lane] = pv;
-        else if (lane == kMaxMonitorDim)
-            p->prev_w = pv;
-        __threadfence();
-        __syncwarp();
-        if (lane == 0)
-            is_last = atomicAdd(&a.sc->done, 1u) == gridDim.x - 1;
+    } else if (wid == 1) {
+        // the warps' monitor sums in FP64: eight lanes a component (the
+        // last one, the weights), summed pairwise
+        static_assert(kW == 8, "eight lanes a component");
+        constexpr int kC = MD + 1;
+#pragma unroll
+        for (int c0 = 0; c0 <= kMaxMonitorDim; c0 += 4) {
+            const int c = c0 + lane / 8;
+            double x = prev_on && c < kC
+                ? static_cast<double>(
+                      sh.shp[c < MD ? c : kMaxMonitorDim][lane % 8])
+                : 0.0;
+            if (prev_on && c0 < kC)
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+                    x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+            if (lane % 8 == 0 && c <= kMaxMonitorDim) {
+                // component MD is the weights; unused ones are zero
+                if (c == MD)
+                    p->prev_w = x;
+                else if (c < MD)
+                    p->prev[c] = x;
+                else
+                    p->prev[c - 1] = 0.0;
+            }
+        }
     }
-    __syncthreads();
-    if (!is_last)
-        return;
+}
 
-    // ---- last block: combine every block's record in FP64
-    __threadfence();
-    float M = -INFINITY;
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x)
-        M = fmaxf(M, static_cast<float>(__ldcg(&a.part[b].m)));
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-        M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, d));
-    if (lane == 0)
-        shmax[wid] = M;
-    __syncthreads();
-    M = shmax[0];
-#pragma unroll
-    for (int w = 1; w < kW; ++w)
-        M = fmaxf(M, shmax[w]);
+// The step's result from every block's record, in FP64, into sc (the
+// filter's scalars) and, if write, the histories; by one whole block, whose
+// warps 0 and 1 finish.  Every block that runs it gets the same bits.  Local:
+// the records are this block's own (plain loads, shared memory allowed).
+template <class Model, bool First, PfMon Mon, bool Local = false>
+__device__ __forceinline__ void pf_step_combine(const PfStepArgs &a,
+    const PfPartial *part, uint32_t nblk, PfScalars &sc, bool write,
+    uint32_t t, int resampled, PfStepSmem<Model, Mon> &sh)
+{
+    constexpr int MD = Model::monitor_dim;
+    constexpr int AMD = Mon == PfMon::Current ? MD : 0;
+    constexpr bool prev_on = !First && Mon == PfMon::Previous;
+    constexpr int kW = kPfBlock / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t n = a.n;
+    auto ld = [](const double *p) { return Local ? *p : __ldcg(p); };
     // S, S2, then the sums this mode has: the step's own monitor, or the
     // previous step's and its weights
     constexpr int NV = 2 + AMD + (prev_on ? MD + 1 : 0);
-    double v[NV] = {};
-    if (wid * 32 < static_cast<int>(gridDim.x)) { // records for this warp
-        for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-            const double pm = __ldcg(&a.part[b].m);
-            if (pm > -INFINITY) {
-                const double f = __expf(static_cast<float>(pm) - M);
-                v[0] += __ldcg(&a.part[b].s) * f;
-                v[1] += __ldcg(&a.part[b].s2) * f * f;
+    const double prev_mass = resampled ? static_cast<double>(n) : sc.S;
+    float M = -INFINITY;
+    double tot = 0; // lane k of the finishing warps: value k
+    if (nblk == 1) {
+        // one record: the sums are its own (every factor is exp(0) = 1)
+        M = static_cast<float>(ld(&part->m));
+        if (lane < NV)
+            tot = lane == 0 ? ld(&part->s)
+                : lane == 1 ? ld(&part->s2)
+                : lane < 2 + AMD ? ld(&part->mon[lane - 2])
+                : lane < NV - 1  ? ld(&part->prev[lane - 2 - AMD])
+                                 : ld(&part->prev_w);
+        __syncthreads(); // sc.S is read
+    } else {
+        for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x)
+            M = fmaxf(M, static_cast<float>(ld(&part[b].m)));
 #pragma unroll
-                for (int d = 0; d < AMD; ++d)
-                    v[2 + d] += __ldcg(&a.part[b].mon[d]) * f;
-            }
-            if (prev_on) {
+        for (int d = 16; d > 0; d >>= 1)
+            M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, d));
+        if (lane == 0)
+            sh.shmax[wid] = M;
+        __syncthreads();
+        M = sh.shmax[0];
 #pragma unroll
-                for (int d = 0; d < MD; ++d)
-                    v[2 + AMD + d] += __ldcg(&a.part[b].prev[d]);
-                v[NV - 1] += __ldcg(&a.part[b].prev_w);
+        for (int w = 1; w < kW; ++w)
+            M = fmaxf(M, sh.shmax[w]);
+        double v[NV] = {};
+        if (wid * 32 < static_cast<int>(nblk)) { // records for this warp
+            for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x) {
+                const double pm = ld(&part[b].m);
+                if (pm > -INFINITY) {
+                    const double f = __expf(static_cast<float>(pm) - M);
+                    v[0] += ld(&part[b].s) * f;
+                    v[1] += ld(&part[b].s2) * f * f;
+#pragma unroll
+                    for (int d = 0; d < AMD; ++d)
+                        v[2 + d] += ld(&part[b].mon[d]) * f;
+                }
+                if (prev_on) {
+#pragma unroll
+                    for (int d = 0; d < MD; ++d)
+                        v[2 + AMD + d] += ld(&part[b].prev[d]);
+                    v[NV - 1] += ld(&part[b].prev_w);
+                }
             }
+            warp_sum_split(v);
         }
-        warp_sum_split(v);
+        const int mine = warp_sum_value<NV>();
+        if (mine < NV)
+            sh.shd[mine][wid] = v[0];
+        __syncthreads();
+        if (lane < NV)
+            for (int w = 0; w < kW && w * 32 < static_cast<int>(nblk); ++w)
+                tot += sh.shd[lane][w];
     }
-    const int mine = warp_sum_value<NV>();
-    if (mine < NV)
-        shd[mine][wid] = v[0];
-    __syncthreads();
-    if (wid != 0)
+    // two warps finish, each with the totals: the quotients in the lanes of
+    // warp 0, the logarithms in two lanes of warp 1
+    if (wid > 1)
         return;
-    // one warp finishes: lane k sums value k over the warps, then the
-    // quotients and the two logarithms are taken in different lanes at once
-    double tot = 0;
-    if (lane < NV)
-        for (int w = 0; w < kW; ++w)
-            tot += shd[lane][w];
-    PfScalars &sc = *a.sc;
     const double S = __shfl_sync(0xFFFFFFFFu, tot, 0);
+    const double M1 = static_cast<double>(M);
+    const bool rec = write && t < a.max_steps;
+    if (wid == 1) {
+        const double lg = log(lane == 1 ? prev_mass : S);
+        const double lg_prev = __shfl_sync(0xFFFFFFFFu, lg, 1);
+        if (lane == 0) {
+            sc.logz += M1 + lg - lg_prev;
+            if (rec)
+                a.h_logz[t] = sc.logz;
+        }
+        return;
+    }
     const double S2 = __shfl_sync(0xFFFFFFFFu, tot, 1);
     const double PW = __shfl_sync(0xFFFFFFFFu, tot, NV - 1);
-    const double prev_mass = resampled ? static_cast<double>(n) : sc.S;
     // lane 1: ESS; a monitor component in its own lane: its mean
     const double quot = (lane == 1 ? S * S : tot) /
         (lane == 1 ? S2 : (prev_on && lane >= 2 + AMD ? PW : S));
-    const double lg = log(lane == 1 ? prev_mass : S);
     const double ess = __shfl_sync(0xFFFFFFFFu, quot, 1);
-    const double lg_prev = __shfl_sync(0xFFFFFFFFu, lg, 1);
-    const bool rec = t < a.max_steps;
-    if (prev_on && t >= 1 && t - 1 < a.max_steps && lane >= 2 + AMD &&
+    if (prev_on && write && t >= 1 && t - 1 < a.max_steps && lane >= 2 + AMD &&
         lane < 2 + AMD + MD)
         a.h_mean[static_cast<size_t>(t - 1) * MD + (lane - 2 - AMD)] = quot;
     if (Mon == PfMon::Current && lane >= 2 && lane < 2 + MD) {
@@ -622,15 +654,12 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
             a.h_mean[static_cast<size_t>(t) * MD + (lane - 2)] = quot;
     }
     if (lane == 0) {
-        const double M1 = static_cast<double>(M);
-        sc.logz += M1 + lg - lg_prev;
         if (!(S > 0) || !(ess > 0))
             sc.err |= DEV_ERR_NONFINITE;
         const int flag =
             ess < a.threshold * static_cast<double>(n) ? 1 : 0;
         if (rec) {
             a.h_ess[t] = ess;
-            a.h_logz[t] = sc.logz;
             a.h_res[t] = flag;
         }
         sc.M = M1;
@@ -642,6 +671,31 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
         sc.step = t + 1;
         sc.done = 0;
     }
+}
+
+template <class Model, bool First, PfMon Mon>
+__global__ void __launch_bounds__(kPfBlock, 4) k_pf_step(
+    const PfStepArgs a, const Model model)
+{
+    __shared__ PfStepSmem<Model, Mon> sh;
+    __shared__ bool is_last;
+    const uint32_t t = a.sc->step;
+    const int resampled = First ? 1 : a.sc->resampled;
+    const bool gather = First ? false : (a.sc->gather != 0);
+    const float Mprev = First ? 0.0f : static_cast<float>(a.sc->M);
+    pf_step_record<Model, First, Mon>(a, model, t, resampled, gather, Mprev,
+        a.part + blockIdx.x, sh);
+    if (threadIdx.x < 64)
+        __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        is_last = atomicAdd(&a.sc->done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last)
+        return;
+    __threadfence();
+    pf_step_combine<Model, First, Mon>(
+        a, a.part, gridDim.x, *a.sc, true, t, resampled, sh);
 }
 
 // ------------------------------------------------------------ host launch

@@ -754,24 +754,35 @@ __global__ void __launch_bounds__(kPfBlock) k_brs_qsum(const BatchArgs a)
         }
         acc = block_reduce(acc, OpAdd(), uint64_t(0), sh);
         // the filter's last chunk to finish (a thread-fenced ticket on
-        // done3; nothing waits) sets the filter's counting constants
-        if (threadIdx.x == 0) {
-            a.rs_q[v] = acc;
-            __threadfence();
+        // done3; nothing waits) sets the filter's counting constants, by
+        // the block's first warp
+        if (threadIdx.x < 32) {
             PfScalars &S = a.st[c.f];
-            if (atomicAdd(&S.done3, 1u) == c.nc - 1) {
-                S.done3 = 0;
+            int last = 0;
+            if (threadIdx.x == 0) {
+                a.rs_q[v] = acc;
                 __threadfence();
-                uint64_t Q = 0;
-                for (uint32_t k = 0; k < c.nc; ++k)
+                last = atomicAdd(&S.done3, 1u) == c.nc - 1 ? 1 : 0;
+                if (last)
+                    S.done3 = 0;
+                __threadfence();
+            }
+            last = __shfl_sync(0xFFFFFFFFu, last, 0);
+            if (last) {
+                uint64_t Q = 0; // at most 32 chunks
+                for (uint32_t k = threadIdx.x; k < c.nc; k += 32)
                     Q += __ldcg(a.rs_q + c.base + k);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    Q += __shfl_xor_sync(0xFFFFFFFFu, Q, o);
                 uint32_t err = 0;
                 cdf_constants(S, Q, c.n, a.scheme == VSMC_CUDA_SYSTEMATIC, err);
-                if (err & ~DEV_ERR_NONFINITE) // a zero total: pass 2 says so
+                // a zero total: pass 2 says so
+                if (threadIdx.x == 0 && (err & ~DEV_ERR_NONFINITE))
                     atomicOr(&S.err, err & ~DEV_ERR_NONFINITE);
             }
         }
-        __syncthreads(); // thread 0 done before the next chunk
+        __syncthreads(); // the ticket is done before the next chunk
     }
 }
 

@@ -8,7 +8,9 @@
 // log sum_i W_{t-1,i} exp(l_{t,i}) (user_guide/tex/smc.tex:176-182).
 #include "pf_internal.cuh"
 #include "pf32.cuh"
+#include "pf32_run.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -222,6 +224,118 @@ static int step32(vsmc_cuda_pf *pf)
     return VSMC_CUDA_OK;
 }
 
+// the whole-run kernel of a filter
+static const void *run_kernel(int scheme, RunKind kind)
+{
+    const bool sys = scheme == VSMC_CUDA_SYSTEMATIC;
+    switch (kind) {
+        case RunKind::Block:
+            return sys ? reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, true, RunKind::Block>)
+                       : reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, false, RunKind::Block>);
+        case RunKind::Cluster:
+            return sys ? reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, true, RunKind::Cluster>)
+                       : reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, false, RunKind::Cluster>);
+        default:
+            return sys ? reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, true, RunKind::Grid>)
+                       : reinterpret_cast<const void *>(
+                             k_pf32_run<CvModel, false, RunKind::Grid>);
+    }
+}
+
+constexpr size_t kRunCluster = 8; // the portable cluster size
+
+static RunKind run_kind(size_t tiles)
+{
+    return tiles == 1 ? RunKind::Block
+        : tiles <= kRunCluster ? RunKind::Cluster
+                               : RunKind::Grid;
+}
+
+// Tiles of a filter that the whole-run kernel takes: a tile per block, all
+// blocks resident.
+static size_t run_tiles_most(int scheme)
+{
+    int dev = 0, coop = 0, occ = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ,
+            run_kernel(scheme, RunKind::Grid), kPfBlock, 0) != cudaSuccess)
+        return 0;
+    if (!coop)
+        return kRunCluster;
+    return std::max(kRunCluster,
+        static_cast<size_t>(num_sms()) *
+            static_cast<size_t>(std::min(occ, kRunOcc)));
+}
+
+// Whether a run of this filter is one kernel: the plain step
+// (its kernels follow nothing else), a tile per block, all blocks resident.
+static bool run_is_one_kernel(const vsmc_cuda_pf *pf)
+{
+    return pf->precision == 32 && !pf->custom && pf->use_graph &&
+        pf->run_blocks > 0 && !pf->record_gen && pf->mcmc_sweeps == 0;
+}
+
+// Steps of one launch: a bound on a kernel's time, not on the run.
+constexpr size_t kRunSteps = 1024;
+
+static int run32(vsmc_cuda_pf *pf, size_t T)
+{
+    for (size_t t0 = 0; t0 < T; t0 += kRunSteps) {
+        VSMC_CUDA_TRY(
+            cudaMemsetAsync(pf->run_bar, 0, sizeof(uint32_t), pf->stream));
+        PfStepArgs a = step_args(pf, nullptr, nullptr);
+        a.mon_prev = 1;
+        Rs32Args r = make_rs_args32(pf, nullptr, 0, false);
+        CvModel m = cv_model(pf);
+        RunArgs run = {};
+        run.buf[0] = buf32(pf, 0);
+        run.buf[1] = buf32(pf, 1);
+        run.cur = pf->cur;
+        run.t0 = static_cast<uint32_t>(t0);
+        run.steps = static_cast<uint32_t>(T - t0 < kRunSteps ? T - t0
+                                                             : kRunSteps);
+        run.sc = pf->sc;
+        run.bar = pf->run_bar;
+        run.tiles = static_cast<uint32_t>(pf->run_blocks);
+        void *args[] = {&a, &r, &m, &run};
+        const RunKind kind = run_kind(pf->run_blocks);
+        const void *f = run_kernel(pf->scheme, kind);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(pf->run_blocks));
+        cfg.blockDim = dim3(kPfBlock);
+        cfg.stream = pf->stream;
+        cudaLaunchAttribute at = {};
+        if (kind == RunKind::Cluster) {
+            unsigned c = 2; // blocks past the tiles have no particles
+            while (c < pf->run_blocks)
+                c *= 2;
+            cfg.gridDim = dim3(c);
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = c;
+            at.val.clusterDim.y = 1;
+            at.val.clusterDim.z = 1;
+        } else {
+            at.id = cudaLaunchAttributeCooperative;
+            at.val.cooperative = kind == RunKind::Grid ? 1 : 0;
+        }
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        VSMC_CUDA_TRY(cudaLaunchKernelExC(&cfg, f, args));
+        if (run.steps % 2)
+            pf->cur = 1 - pf->cur;
+        pf->t = t0 + run.steps;
+    }
+    pf->mean_pending = true;
+    return VSMC_CUDA_OK;
+}
+
 // apply a pending resampling gather to the stored state (host-side views)
 static int materialize32(vsmc_cuda_pf *pf)
 {
@@ -408,7 +522,7 @@ static void free_all(vsmc_cuda_pf *pf)
         pf->obs,
         pf->h_mean,
         pf->h_ess, pf->h_logz, pf->h_res, pf->sc, pf->part, pf->qpart,
-        pf->epart, pf->cpart, pf->rep, pf->idx, pf->empties};
+        pf->epart, pf->cpart, pf->rep, pf->idx, pf->empties, pf->run_bar};
     for (void *p : ptrs)
         if (p)
             cudaFree(p);
@@ -436,6 +550,8 @@ static int sync_and_check(vsmc_cuda_pf *pf)
     uint32_t err = 0;
     VSMC_CUDA_TRY(cudaMemcpy(&err, &pf->sc->err, sizeof(err),
         cudaMemcpyDeviceToHost));
+    if (err & DEV_ERR_TIMEOUT)
+        return VSMC_CUDA_ERR_TIMEOUT;
     if (err & DEV_ERR_NONFINITE)
         return VSMC_CUDA_ERR_NONFINITE;
     if (err)
@@ -532,8 +648,19 @@ static int pf_create(vsmc_cuda_pf **out, size_t n, size_t dim,
         while ((size_t(1) << lg) < n)
             ++lg;
         pf->shift = static_cast<uint32_t>(63 - lg);
+        if (model) {
+            const size_t tiles = (n + kPfTile - 1) / kPfTile;
+            const size_t step = sms *
+                static_cast<size_t>(
+                    pf_step_occupancy<CvModel, false, PfMon::Previous>());
+            if (chunk == static_cast<size_t>(kPfTile) && tiles <= step &&
+                tiles <= run_tiles_most(scheme))
+                pf->run_blocks = tiles;
+            PF_TRY(dalloc(&pf->run_bar, 1));
+        }
         PF_TRY(dalloc(&pf->part, pf->max_grid));
-        PF_TRY(dalloc(&pf->qpart, pf->grid_rs * (kRsWarps + 1)));
+        PF_TRY(dalloc(&pf->qpart,
+            std::max<size_t>(pf->grid_rs * (kRsWarps + 1), 2 * kRunCluster)));
         PF_TRY(dalloc(&pf->epart, pf->grid_rs * (kRsWarps + 1)));
         PF_TRY(dalloc(&pf->cpart, pf->grid_rs * (kRsWarps + 1)));
         PF_TRY(dalloc(reinterpret_cast<char **>(&pf->state2),
@@ -912,9 +1039,18 @@ int vsmc_cuda_pf_run_device(vsmc_cuda_pf *pf, size_t T, const double *obs_dev)
     if (obs_dev != pf->obs)
         VSMC_CUDA_TRY(cudaMemcpyAsync(pf->obs, obs_dev, 2 * T * sizeof(double),
             cudaMemcpyDeviceToDevice, pf->stream));
-    int rc = pf_begin(pf);
-    for (size_t t = 1; rc == VSMC_CUDA_OK && t < T; ++t)
-        rc = pf_next(pf);
+    int rc;
+    if (run_is_one_kernel(pf)) {
+        rc = reset_scalars(pf);
+        pf->t = 0;
+        pf->mean_pending = false;
+        if (rc == VSMC_CUDA_OK)
+            rc = run32(pf, T);
+    } else {
+        rc = pf_begin(pf);
+        for (size_t t = 1; rc == VSMC_CUDA_OK && t < T; ++t)
+            rc = pf_next(pf);
+    }
     if (rc == VSMC_CUDA_OK)
         rc = pf_flush_mean(pf);
     return rc;

