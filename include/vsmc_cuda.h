@@ -626,8 +626,8 @@ int vsmc_cuda_batch_autotune(vsmc_cuda_batch *batch, const double *obs_dev,
     int steps, float *ms_host);
 /* Scan schedule of the batched resampling: a filter's particles are
  * resampled in chunks of min_chunk (4096, 8192, 16384 or 32768), doubled
- * until the filter has at most 32 chunks; each chunk is one entry of the
- * step's resampling list.  Results do not depend on it (the counts are
+ * until the filter has at most 32 chunks; each chunk is eight entries of the
+ * step's resampling list, one warp's work each.  Results do not depend on it (the counts are
  * exact integers).  autotune_schedule times the first `steps` steps for each
  * of the four and keeps the fastest; ms_host (4 floats, may be NULL) gets
  * the times.  No reference counterpart. */

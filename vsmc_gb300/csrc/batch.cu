@@ -4,7 +4,7 @@
 // horizon, model constants and seed, advance together: per global step one
 // persistent kernel moves, weights and reduces the particles of every filter
 // still running, and three kernels resample the filters whose ESS fell below
-// the threshold, in equal chunks listed by the step kernel.  A whole run
+// the threshold, in equal units listed by the step kernel.  A whole run
 // (every step of the longest horizon) is one CUDA graph.
 //
 // Filter f behaves exactly as a single precision-32 filter (pf.cu) with seed
@@ -32,6 +32,8 @@
 #include "pf32_dev.cuh"
 #include "pf_model.cuh"
 
+#include <cuda_pipeline.h>
+
 #include <algorithm>
 #include <type_traits>
 #include <cmath>
@@ -55,7 +57,7 @@ struct BFilter {
     uint32_t hist_off; // first history entry (caller's filter order)
     uint32_t seed;
     uint32_t shift;    // fixed-point K = 63 - ceil(log2 n)
-    uint32_t rs_chunk; // resampling chunk: a multiple of 4096 particles
+    uint32_t rs_unit;  // particles of a resampling unit (a warp's)
     union {
         CvConst<float> c;   // position / Student-t model
         BearingsConst bc;   // bearings-only model
@@ -77,8 +79,8 @@ constexpr int kKindLearned = 2;  // bearings-only, learned proposal
 struct BatchArgs {
     const BFilter *flt;
     PfScalars *st;               // dynamic state, one per filter
-    const uint32_t *tile_filter; // filter of each tile
-    const uint32_t *active;      // [tmax + 1] tiles of the filters with T >= t
+    const uint4 *segs;      // {first tile, tiles, filter, 0} of each segment
+    const uint32_t *active; // [tmax + 1] segments of the filters with T >= t
     const float *ax, *ay, *avx, *avy; // state in
     float *bx, *by, *bvx, *bvy;       // state out
     float *lw;
@@ -91,12 +93,13 @@ struct BatchArgs {
     int *h_res;
     uint32_t *step; // global step counter
     // resampling list of the step: rs_list[rpar * rs_cap + v] = {filter,
-    // chunk}, rs_count[rpar] entries; per-entry totals of the passes
+    // unit}, rs_count[rpar] entries; per-entry totals of the passes, turned
+    // into prefixes by the filter's last unit
     uint2 *rs_list;
     uint32_t *rs_count;
-    uint32_t *work; // step kernel's tile counters, by step parity
-    uint64_t *rs_q;
-    uint32_t *rs_e, *rs_c;
+    uint32_t *work; // step kernel's segment counters, by step parity
+    uint64_t *rs_q;  // CDF
+    uint64_t *rs_ec; // copies (high half) and empty slots
     uint32_t rs_cap, rpar;
     const uint32_t *packed; // proposal network (learned kind)
     uint32_t nfilters, tmax;
@@ -136,6 +139,27 @@ __device__ __forceinline__ void batch_one(const CvConst<float> &c,
     lse_push(lw, m, s, s2);
 }
 
+__device__ __forceinline__ void load_run(const int32_t *p, int32_t (&v)[4])
+{
+    const int4 q = __ldcs(reinterpret_cast<const int4 *>(p));
+    v[0] = q.x;
+    v[1] = q.y;
+    v[2] = q.z;
+    v[3] = q.w;
+}
+
+__device__ __forceinline__ void load_run(const int32_t *p, int32_t (&v)[2])
+{
+    const int2 q = __ldcs(reinterpret_cast<const int2 *>(p));
+    v[0] = q.x;
+    v[1] = q.y;
+}
+
+__device__ __forceinline__ void load_run(const int32_t *p, int32_t (&v)[1])
+{
+    v[0] = __ldcs(p);
+}
+
 template <int kPPT>
 __device__ __forceinline__ void load_run(const float *p, float (&v)[kPPT])
 {
@@ -167,19 +191,58 @@ __device__ __forceinline__ void store_run(float *p, const float (&v)[kPPT])
     }
 }
 
-// The record of `count` consecutive tiles of one filter done by this block
-// (FP32 within a warp, FP64 across warps), written at the first of them
-// (the others get empty records) and, in the block that completes the
-// filter's last tile, the filter's FP64 combination: ESS, log-evidence
-// increment, resampling decision and histories (or, at t == T, the last
-// weighted mean).  All threads of the block call it.
-template <int kBlock, bool First>
-__device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
-    uint32_t count, uint32_t f, const BFilter &F, PfScalars &S, uint32_t t,
-    bool mon, float m, float s, float s2, float sx, float sy, float sw,
-    float *shm, float (*shw)[kBlock / 32], bool &is_last)
+// What a block needs to know of a segment (consecutive tiles of one filter),
+// in shared memory: loaded while the block works on the segment before.
+struct SegMeta {
+    BFilter F;
+    uint32_t tile, count, f; // count 0: no more segments
+    int32_t resampled, gather;
+    float Mf;
+};
+
+// The segment with number idx (>= nseg: none), by one warp, without waiting
+// for it (cp.async; the caller waits and synchronizes).
+__device__ __forceinline__ void seg_fetch(
+    const BatchArgs &a, uint32_t idx, uint32_t nseg, SegMeta &m)
 {
-    constexpr int kW = kBlock / 32;
+    const uint32_t lane = threadIdx.x & 31;
+    if (idx >= nseg) {
+        if (lane == 0)
+            m.count = 0;
+        return;
+    }
+    const uint4 seg = a.segs[idx];
+    if (lane == 0) {
+        m.tile = seg.x;
+        m.count = seg.y;
+        m.f = seg.z;
+    }
+    static_assert(sizeof(BFilter) % 4 == 0, "whole words");
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(a.flt + seg.z);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(&m.F);
+    for (uint32_t w = lane; w < sizeof(BFilter) / 4; w += 32)
+        __pipeline_memcpy_async(dst + w, src + w, 4);
+    const PfScalars &S = a.st[seg.z];
+    if (lane == 0)
+        __pipeline_memcpy_async(&m.resampled, &S.resampled, 4);
+    else if (lane == 1)
+        __pipeline_memcpy_async(&m.gather, &S.gather, 4);
+    else if (lane == 2)
+        __pipeline_memcpy_async(&m.Mf, &S.Mf, 4);
+    __pipeline_commit();
+}
+
+// a segment's sums of each warp
+template <int kW>
+struct SegSums {
+    float v[6][kW]; // m, s, s2, sx, sy, sw
+};
+
+// the warp's sums over its lanes, left in sums
+template <int kW>
+__device__ __forceinline__ void seg_record_warp(SegSums<kW> &sums, float m,
+    float s, float s2, float sx, float sy, float sw)
+{
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -192,21 +255,38 @@ __device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
         lse_merge_f(m, s, s2, om, os, os2);
     }
     if (lane == 0) {
-        shm[wid] = m;
-        shw[0][wid] = s;
-        shw[1][wid] = s2;
-        shw[2][wid] = sx;
-        shw[3][wid] = sy;
-        shw[4][wid] = sw;
+        sums.v[0][wid] = m;
+        sums.v[1][wid] = s;
+        sums.v[2][wid] = s2;
+        sums.v[3][wid] = sx;
+        sums.v[4][wid] = sy;
+        sums.v[5][wid] = sw;
     }
-    __syncthreads();
-    if (wid == 0) {
-        // warp 0 merges the warps' records in FP32
+}
+
+// The record of a segment from its warps' sums (FP32 within the segment,
+// FP64 across), written at its first tile (its other tiles get empty
+// records) and, when it completes the filter's last tile, the filter's FP64
+// combination: ESS, log-evidence increment, resampling decision and
+// histories (or, at t == T, the last weighted mean).  By one warp; the other
+// warps of the block go on with the next segment.
+template <int kW, bool First>
+__device__ __forceinline__ void seg_finish(const BatchArgs &a,
+    const SegMeta &meta, uint32_t t, bool mon, const SegSums<kW> &sums)
+{
+    const int lane = threadIdx.x & 31;
+    const BFilter &F = meta.F;
+    const uint32_t tile = meta.tile, count = meta.count, f = meta.f;
+    PfScalars &S = a.st[f];
+    {
+        // merges the warps' records in FP32
         const bool in = lane < kW;
-        float wm = in ? shm[lane] : -INFINITY;
-        float ws = in ? shw[0][lane] : 0.0f, ws2 = in ? shw[1][lane] : 0.0f;
-        float wx = in ? shw[2][lane] : 0.0f, wy = in ? shw[3][lane] : 0.0f;
-        float ww = in ? shw[4][lane] : 0.0f;
+        float wm = in ? sums.v[0][lane] : -INFINITY;
+        float ws = in ? sums.v[1][lane] : 0.0f;
+        float ws2 = in ? sums.v[2][lane] : 0.0f;
+        float wx = in ? sums.v[3][lane] : 0.0f;
+        float wy = in ? sums.v[4][lane] : 0.0f;
+        float ww = in ? sums.v[5][lane] : 0.0f;
 #pragma unroll
         for (int d = kW / 2; d > 0; d >>= 1) {
             const float om = __shfl_xor_sync(0xFFFFFFFFu, wm, d);
@@ -217,6 +297,7 @@ __device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
             ww += __shfl_xor_sync(0xFFFFFFFFu, ww, d);
             lse_merge_f(wm, ws, ws2, om, os, os2);
         }
+        int last = 0;
         if (lane == 0) {
             const TileRecord p = {wx, wy, ww, wm, ws, ws2};
             a.part[tile] = p;
@@ -224,56 +305,67 @@ __device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
             for (uint32_t k = 1; k < count; ++k)
                 a.part[tile + k] = empty;
             __threadfence();
-            is_last = atomicAdd(&S.done, count) == F.ntiles - count;
+            last = atomicAdd(&S.done, count) == F.ntiles - count ? 1 : 0;
         }
+        if (!__shfl_sync(0xFFFFFFFFu, last, 0))
+            return;
     }
-    __syncthreads();
-    if (!is_last)
-        return;
-    // ---- the filter's last tile: warp 0 combines its tile records in FP64
     __threadfence();
-    if (wid != 0)
-        return;
+    // ---- the filter's last tile: its tile records in FP64
     float M = -INFINITY;
     for (uint32_t b = lane; b < F.ntiles; b += 32)
         M = fmaxf(M, __ldcg(&a.part[F.tile0 + b].m));
     M = warp_reduce(M, OpMax());
-    double T1 = 0, T2 = 0, TX = 0, TY = 0, TW = 0;
+    // T1, T2, TX, TY, TW; the values are split over the lanes as they are
+    // summed, and the quotients and logarithms taken in different lanes (an
+    // FP64 instruction takes 19 cycles of the SM and 64 of latency)
+    double v[5] = {};
     for (uint32_t b = lane; b < F.ntiles; b += 32) {
-        const TileRecord p = a.part[F.tile0 + b];
-        TX += p.sx;
-        TY += p.sy;
-        TW += p.sw;
+        const float2 *q =
+            reinterpret_cast<const float2 *>(a.part + F.tile0 + b);
+        const float2 q0 = __ldcg(q), q1 = __ldcg(q + 1), q2 = __ldcg(q + 2);
+        const TileRecord p = {q0.x, q0.y, q1.x, q1.y, q2.x, q2.y};
+        v[2] += p.sx;
+        v[3] += p.sy;
+        v[4] += p.sw;
         if (p.m > -INFINITY) {
             const double fct = __expf(p.m - M);
-            T1 += p.s * fct;
-            T2 += p.s2 * fct * fct;
+            v[0] += p.s * fct;
+            v[1] += p.s2 * fct * fct;
         }
     }
-    T1 = warp_reduce(T1, OpAdd());
-    T2 = warp_reduce(T2, OpAdd());
-    TX = warp_reduce(TX, OpAdd());
-    TY = warp_reduce(TY, OpAdd());
-    TW = warp_reduce(TW, OpAdd());
-    uint32_t rs_first = ~0u; // first list entry of the filter's chunks
+    warp_sum_split(v);
+    const double T1 = __shfl_sync(0xFFFFFFFFu, v[0], warp_sum_lane<5>(0));
+    const double T2 = __shfl_sync(0xFFFFFFFFu, v[0], warp_sum_lane<5>(1));
+    const double TX = __shfl_sync(0xFFFFFFFFu, v[0], warp_sum_lane<5>(2));
+    const double TY = __shfl_sync(0xFFFFFFFFu, v[0], warp_sum_lane<5>(3));
+    const double TW = __shfl_sync(0xFFFFFFFFu, v[0], warp_sum_lane<5>(4));
+    // the previous weights' mass: their own normalizer (the single filter's
+    // step kernel uses the same one)
+    const double prev_mass =
+        First || S.resampled ? static_cast<double>(F.n) : S.S;
+    const double quot = (lane == 0 ? T1 * T1 : lane == 1 ? TX : TY) /
+        (lane == 0 ? T2 : TW);
+    const double lg = mon ? 0.0 : log(lane == 1 ? prev_mass : T1);
+    const double mx = __shfl_sync(0xFFFFFFFFu, quot, 1);
+    const double my = __shfl_sync(0xFFFFFFFFu, quot, 2);
+    const double lg_prev = __shfl_sync(0xFFFFFFFFu, lg, 1);
+    uint32_t rs_first = ~0u; // first list entry of the filter's units
+    const uint32_t nu = (F.n + F.rs_unit - 1) / F.rs_unit;
     if (lane == 0) {
         if (mon) {
-            a.h_mean[2 * (F.hist_off + F.T - 1) + 0] = TX / TW;
-            a.h_mean[2 * (F.hist_off + F.T - 1) + 1] = TY / TW;
+            a.h_mean[2 * (F.hist_off + F.T - 1) + 0] = mx;
+            a.h_mean[2 * (F.hist_off + F.T - 1) + 1] = my;
             S.resampled = 0; // finished: nothing left to resample
             S.gather = 0;
         } else {
-            // the previous weights' mass: their own normalizer (the
-            // single filter's step kernel uses the same one)
-            const double prev_mass =
-                First || S.resampled ? static_cast<double>(F.n) : S.S;
             if (!First) {
-                a.h_mean[2 * (F.hist_off + t - 1) + 0] = TX / TW;
-                a.h_mean[2 * (F.hist_off + t - 1) + 1] = TY / TW;
+                a.h_mean[2 * (F.hist_off + t - 1) + 0] = mx;
+                a.h_mean[2 * (F.hist_off + t - 1) + 1] = my;
             }
-            const double ess = T1 * T1 / T2;
+            const double ess = quot;
             const double M1 = static_cast<double>(M);
-            S.logz += M1 + log(T1) - log(prev_mass);
+            S.logz += M1 + lg - lg_prev;
             if (!(T1 > 0) || !(ess > 0))
                 S.err |= DEV_ERR_NONFINITE;
             const int flag =
@@ -289,9 +381,8 @@ __device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
             S.gather = 0;
             S.step = t + 1;
             if (flag) {
-                const uint32_t nc = (F.n + F.rs_chunk - 1) / F.rs_chunk;
-                const uint32_t v = atomicAdd(a.rs_count + a.rpar, nc);
-                if (v + nc <= a.rs_cap)
+                const uint32_t v = atomicAdd(a.rs_count + a.rpar, nu);
+                if (v + nu <= a.rs_cap)
                     rs_first = v;
                 else
                     S.err |= DEV_ERR_INTERNAL;
@@ -301,27 +392,36 @@ __device__ __forceinline__ void tile_finish(const BatchArgs &a, uint32_t tile,
     }
     rs_first = __shfl_sync(0xFFFFFFFFu, rs_first, 0);
     if (rs_first != ~0u) {
-        // list the filter's resampling chunks
+        // list the filter's resampling units
         uint2 *list = a.rs_list + static_cast<size_t>(a.rpar) * a.rs_cap;
-        const uint32_t nc = (F.n + F.rs_chunk - 1) / F.rs_chunk;
-        for (uint32_t j = lane; j < nc; j += 32)
+        for (uint32_t j = lane; j < nu; j += 32)
             list[rs_first + j] = make_uint2(f, j);
     }
 }
 
-// slot i's source inside the filter after a resample (bounds-checked)
-__device__ __forceinline__ uint32_t batch_source(
-    const BatchArgs &a, const BFilter &F, PfScalars &S, uint32_t i)
+// the sources, inside the filter, of kN slots with index entries I after a
+// resample (bounds-checked); their loads are in flight together
+template <int kN>
+__device__ __forceinline__ void batch_sources(const BatchArgs &a,
+    const BFilter &F, PfScalars &S, const int32_t (&I)[kN],
+    uint32_t (&src)[kN])
 {
-    const int32_t v = a.idx[F.off + i];
-    const uint32_t e = static_cast<uint32_t>(-(v + 1));
-    uint32_t src = v >= 0 ? static_cast<uint32_t>(v)
-                          : (e < F.n ? __ldcg(a.srcs + F.off + e) : F.n);
-    if (src >= F.n) {
-        atomicOr(&S.err, DEV_ERR_INTERNAL);
-        src = 0;
+    uint32_t most = 0;
+#pragma unroll
+    for (int k = 0; k < kN; ++k) {
+        const uint32_t e = static_cast<uint32_t>(-(I[k] + 1));
+        src[k] = I[k] >= 0 ? static_cast<uint32_t>(I[k])
+                           : (e < F.n ? __ldcg(a.srcs + F.off + e) : F.n);
     }
-    return src;
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+        most = max(most, src[k]);
+    if (most >= F.n) {
+        atomicOr(&S.err, DEV_ERR_INTERNAL);
+#pragma unroll
+        for (int k = 0; k < kN; ++k)
+            src[k] = src[k] < F.n ? src[k] : 0;
+    }
 }
 
 // bootstrap body of the bearings-only model (prior at t == 0)
@@ -348,54 +448,63 @@ __device__ __forceinline__ void bearings_one(const BearingsConst &c,
     lse_push(lw, m, s, s2);
 }
 
+// Tiles of a segment at most: one at the default 4 x 256 shape (1024
+// particles, whose FP32 records then group the particles as the single
+// filter's blocks do), 2048 particles' worth for smaller tiles (fewer
+// records; 1024 took 231 ms per 4096-filter run, 2048 225 ms, 4096 227 ms).
+constexpr uint32_t seg_tiles(uint32_t tile)
+{
+    return tile >= 1024 ? 1u : 2048u / tile;
+}
+
 // One global step of every running filter (bootstrap kinds).  A filter at
 // t < T moves and weights its particles; at t == T it only records the
-// weighted mean of its final particles.  Each block takes a contiguous run
-// of tiles and records one reduction per filter it touches.
+// weighted mean of its final particles.  A persistent block takes segments
+// from a counter until none is left, so one whose segments are slower
+// (gathered reads after a resample, many small filters) takes fewer.  The
+// next segment's number and description are fetched while the current one
+// is computed, and one warp (in turn) records a finished segment while the
+// others start on the next: with three barriers and the chain counter, tile,
+// filter, state in front of every segment's loads, a tile of 1024 particles
+// took 10 us.  The registers bound the blocks of an SM: 512
+// filters, 100 steps, took 10.62 ms with 64 registers (4 blocks of 256),
+// 12.02 with 48 (5 blocks) and 10.91 with 80 (3 blocks).
 template <int kBlock, int kPPT, bool First, int Kind>
-__global__ void __launch_bounds__(kBlock, 1280 / kBlock) k_batch_step(
+__global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_batch_step(
     const BatchArgs a)
 {
     constexpr uint32_t kTile = kBlock * kPPT;
     constexpr int kW = kBlock / 32;
-    // tiles a block takes at a time: one tile at the default 4 x 256 shape
-    // (1024 particles, whose per-tile FP32 records then group the particles
-    // as the single filter's blocks do), 2048 particles for smaller tiles
-    // (fewer segment records; 1024 took 231 ms per 4096-filter run, 2048
-    // 225 ms, 4096 227 ms)
-    constexpr uint32_t kGrab = kTile >= 1024 ? 1u : 2048u / kTile;
     const uint32_t t = *a.step;
-    const uint32_t ntiles = t <= a.tmax ? a.active[t] : 0u;
-    __shared__ float shm[kW];
-    __shared__ float shw[5][kW];
-    __shared__ bool is_last;
-    __shared__ uint32_t grab;
+    const uint32_t nseg = t <= a.tmax ? a.active[t] : 0u;
+    // a block's slots: a description is read by its segment's recorder until
+    // the next segment's barrier, so three of them
+    __shared__ SegMeta metas[3];
+    __shared__ SegSums<kW> sums[2];
+    const uint32_t lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5;
     // the next step's counter was last used by the previous step's launch
     if (blockIdx.x == 0 && threadIdx.x == 0)
         a.work[(t + 1) & 1u] = 0;
-    // Blocks take runs of kGrab tiles from a counter until none is left, so
-    // a block whose tiles are slower (gathered reads after a resample, many
-    // small filters) takes fewer of them.
-    for (;;) {
-    if (threadIdx.x == 0)
-        grab = atomicAdd(a.work + (t & 1u), kGrab);
+    if (wid == kW - 1) {
+        seg_fetch(a, blockIdx.x, nseg, metas[0]);
+        __pipeline_wait_prior(0);
+    }
     __syncthreads();
-    const uint32_t lo = grab;
-    __syncthreads();
-    if (lo >= ntiles)
-        break;
-    const uint32_t hi = min(ntiles, lo + kGrab);
-    // the run is cut into segments of one filter each; a segment reads its
-    // filter's description and state once, then streams its tiles
-    uint32_t tile = lo;
-    while (tile < hi) {
-        const uint32_t f = a.tile_filter[tile];
-        const BFilter F = a.flt[f];
-        PfScalars &S = a.st[f];
+    uint32_t slot = 0;
+    for (uint32_t it = 0;; ++it) {
+        const SegMeta &meta = metas[slot];
+        slot = slot == 2 ? 0 : slot + 1;
+        if (meta.count == 0)
+            break;
+        uint32_t next = 0;
+        if (wid == kW - 1 && lane == 0)
+            next = gridDim.x + atomicAdd(a.work + (t & 1u), 1u);
+        const BFilter &F = meta.F;
         const bool mon = !First && t == F.T;
-        const int resampled = First ? 1 : S.resampled;
-        const bool gather = First ? false : (S.gather != 0);
-        const float Mprev = First ? 0.0f : S.Mf;
+        const int resampled = First ? 1 : meta.resampled;
+        const bool gather = First ? false : (meta.gather != 0);
+        const float Mprev = First ? 0.0f : meta.Mf;
         float ox = 0.0f, oy = 0.0f;
         if (!mon) {
             if (Kind == kKindCv) {
@@ -405,113 +514,127 @@ __global__ void __launch_bounds__(kBlock, 1280 / kBlock) k_batch_step(
                 ox = a.obs[F.obs_off + t];
             }
         }
-        const uint32_t seg = tile;
-        uint32_t end = min(hi, F.tile0 + F.ntiles);
-        if (end <= tile) { // a tile table that disagrees with the filters
-            if (threadIdx.x == 0)
-                atomicOr(&S.err, DEV_ERR_INTERNAL);
-            end = tile + 1;
-        }
         float m = -INFINITY, s = 0, s2 = 0, sx = 0, sy = 0, sw = 0;
-        for (; tile < end; ++tile) {
+        const uint32_t end = meta.tile + meta.count;
+        for (uint32_t tile = meta.tile; tile < end; ++tile) {
             const uint32_t i0 = (tile - F.tile0) * kTile + threadIdx.x * kPPT;
-            const bool full = i0 + kPPT <= F.n;
-            float X[kPPT], Y[kPPT], VX[kPPT], VY[kPPT], LW[kPPT];
-#pragma unroll
-            for (int k = 0; k < kPPT; ++k)
-                X[k] = Y[k] = VX[k] = VY[k] = LW[k] = 0.0f;
-            if (!First) {
-                const uint32_t g0 = F.off + i0;
-                // after a resample, a group whose slots all keep their own
-                // particle reads like an unresampled one
-                bool own = !gather;
-                if (gather && full && kPPT == 4) {
-                    const int4 I = __ldcs(reinterpret_cast<const int4 *>(a.idx + g0));
-                    const int b = static_cast<int>(i0);
-                    own = I.x == b && I.y == b + 1 && I.z == b + 2 && I.w == b + 3;
-                }
-                if (own && full) {
-                    load_run<kPPT>(a.ax + g0, X);
-                    load_run<kPPT>(a.ay + g0, Y);
-                    load_run<kPPT>(a.avx + g0, VX);
-                    load_run<kPPT>(a.avy + g0, VY);
+            const uint32_t g0 = F.off + i0;
+            // one particle: weight its sums, move it and weight it, or (at
+            // t == T) weight its sums alone
+            auto body = [&](uint32_t i, float &x, float &y, float &vx,
+                            float &vy, float &lw) {
+                if (mon) {
+                    const float wo = resampled ? 1.0f : __expf(lw - Mprev);
+                    sx += wo * x;
+                    sy += wo * y;
+                    sw += wo;
+                } else if (Kind == kKindCv) {
+                    batch_one<First>(F.c, F.seed, i, t, ox, oy, resampled,
+                        Mprev, x, y, vx, vy, lw, m, s, s2, sx, sy, sw);
                 } else {
+                    bearings_one<First>(F.bc, F.seed, i, t, ox, resampled,
+                        Mprev, x, y, vx, vy, lw, m, s, s2, sx, sy, sw);
+                }
+            };
+            const bool fetch = wid == kW - 1 && tile == meta.tile;
+            if (i0 + kPPT <= F.n) {
+                // a whole group: no test per particle, so its particles'
+                // chains interleave
+                float X[kPPT], Y[kPPT], VX[kPPT], VY[kPPT], LW[kPPT];
+                if (First) {
 #pragma unroll
-                    for (int k = 0; k < kPPT; ++k) {
-                        const uint32_t i = i0 + k;
-                        if (i < F.n) {
-                            const uint32_t src =
-                                gather ? batch_source(a, F, S, i) : i;
-                            X[k] = a.ax[F.off + src];
-                            Y[k] = a.ay[F.off + src];
-                            VX[k] = a.avx[F.off + src];
-                            VY[k] = a.avy[F.off + src];
+                    for (int k = 0; k < kPPT; ++k)
+                        X[k] = Y[k] = VX[k] = VY[k] = LW[k] = 0.0f;
+                } else {
+                    int32_t I[kPPT];
+                    // after a resample, a group whose slots all keep their
+                    // own particle reads like an unresampled one
+                    bool own = true;
+                    if (gather) {
+                        load_run(a.idx + g0, I);
+#pragma unroll
+                        for (int k = 0; k < kPPT; ++k)
+                            own = own && I[k] == static_cast<int>(i0) + k;
+                    }
+                    if (own) {
+                        load_run<kPPT>(a.ax + g0, X);
+                        load_run<kPPT>(a.ay + g0, Y);
+                        load_run<kPPT>(a.avx + g0, VX);
+                        load_run<kPPT>(a.avy + g0, VY);
+                    } else {
+                        uint32_t src[kPPT];
+                        batch_sources<kPPT>(a, F, a.st[meta.f], I, src);
+#pragma unroll
+                        for (int k = 0; k < kPPT; ++k) {
+                            X[k] = a.ax[F.off + src[k]];
+                            Y[k] = a.ay[F.off + src[k]];
+                            VX[k] = a.avx[F.off + src[k]];
+                            VY[k] = a.avy[F.off + src[k]];
                         }
                     }
-                }
-                if (!resampled) {
-                    if (full) {
+                    if (!resampled) {
                         load_run<kPPT>(a.lw + g0, LW);
                     } else {
 #pragma unroll
                         for (int k = 0; k < kPPT; ++k)
-                            if (i0 + k < F.n)
-                                LW[k] = a.lw[g0 + k];
+                            LW[k] = 0.0f;
                     }
                 }
-            }
-            if (mon) {
 #pragma unroll
                 for (int k = 0; k < kPPT; ++k)
-                    if (i0 + k < F.n) {
-                        const float wo = resampled ? 1.0f : __expf(LW[k] - Mprev);
-                        sx += wo * X[k];
-                        sy += wo * Y[k];
-                        sw += wo;
-                    }
-            } else {
-#pragma unroll
-                for (int k = 0; k < kPPT; ++k)
-                    if (i0 + k < F.n) {
-                        if (Kind == kKindCv)
-                            batch_one<First>(F.c, F.seed, i0 + k, t, ox, oy,
-                                resampled, Mprev, X[k], Y[k], VX[k], VY[k], LW[k],
-                                m, s, s2, sx, sy, sw);
-                        else
-                            bearings_one<First>(F.bc, F.seed, i0 + k, t, ox,
-                                resampled, Mprev, X[k], Y[k], VX[k], VY[k], LW[k],
-                                m, s, s2, sx, sy, sw);
-                    }
-                const uint32_t g0 = F.off + i0;
-                if (full) {
+                    body(i0 + k, X[k], Y[k], VX[k], VY[k], LW[k]);
+                if (!mon) {
                     store_run<kPPT>(a.bx + g0, X);
                     store_run<kPPT>(a.by + g0, Y);
                     store_run<kPPT>(a.bvx + g0, VX);
                     store_run<kPPT>(a.bvy + g0, VY);
                     store_run<kPPT>(a.lw + g0, LW);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < kPPT; ++k)
-                        if (i0 + k < F.n) {
-                            a.bx[g0 + k] = X[k];
-                            a.by[g0 + k] = Y[k];
-                            a.bvx[g0 + k] = VX[k];
-                            a.bvy[g0 + k] = VY[k];
-                            a.lw[g0 + k] = LW[k];
+                }
+            } else {
+#pragma unroll 1
+                for (uint32_t i = i0; i < F.n && i < i0 + kPPT; ++i) {
+                    const uint32_t g = F.off + i;
+                    float x = 0, y = 0, vx = 0, vy = 0, lw = 0;
+                    if (!First) {
+                        uint32_t src[1] = {i};
+                        if (gather) {
+                            const int32_t I[1] = {a.idx[g]};
+                            batch_sources<1>(a, F, a.st[meta.f], I, src);
                         }
+                        x = a.ax[F.off + src[0]];
+                        y = a.ay[F.off + src[0]];
+                        vx = a.avx[F.off + src[0]];
+                        vy = a.avy[F.off + src[0]];
+                        if (!resampled)
+                            lw = a.lw[g];
+                    }
+                    body(i, x, y, vx, vy, lw);
+                    if (!mon) {
+                        a.bx[g] = x;
+                        a.by[g] = y;
+                        a.bvx[g] = vx;
+                        a.bvy[g] = vy;
+                        a.lw[g] = lw;
+                    }
                 }
             }
+            __syncwarp();
+            if (fetch)
+                seg_fetch(a, __shfl_sync(0xFFFFFFFFu, next, 0), nseg,
+                    metas[slot]);
         }
-        // the filter's segment ends here: record it
-        tile_finish<kBlock, First>(a, seg, end - seg, f, F, S, t, mon, m, s,
-            s2, sx, sy, sw, shm, shw, is_last);
+        seg_record_warp(sums[it & 1], m, s, s2, sx, sy, sw);
+        if (wid == kW - 1)
+            __pipeline_wait_prior(0);
         __syncthreads();
-    }
+        if (static_cast<uint32_t>(wid) == it % kW)
+            seg_finish<kW, First>(a, meta, t, mon, sums[it & 1]);
     }
 }
 
 constexpr int kLearnBlock = 128;                // 4 warps
 constexpr uint32_t kLearnTile = kLearnBlock;     // 32 particles a warp
+constexpr uint32_t kLearnSeg = 1024u / kLearnTile; // tiles of a segment
 
 // One global step of the learned-proposal filters.  Each warp evaluates the
 // proposal network for 32 particles on the tensor cores (two 16-row tiles
@@ -523,61 +646,59 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
 {
     constexpr int kW = kLearnBlock / 32;
     __shared__ __align__(16) uint32_t sp[kPackedWords];
-    __shared__ float shm[kW];
-    __shared__ float shw[5][kW];
-    __shared__ bool is_last;
     const uint32_t t = *a.step;
-    const uint32_t ntiles = t <= a.tmax ? a.active[t] : 0u;
+    const uint32_t nseg = t <= a.tmax ? a.active[t] : 0u;
     if (!First)
         load_packed(sp, a.packed);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = lane >> 2, q = lane & 3;
-    // tiles a block takes at a time (1024 particles), from a per-step
-    // counter; the next step's counter was last used by the previous step
-    constexpr uint32_t kGrab = 1024u / kLearnTile;
-    __shared__ uint32_t grab;
+    __shared__ SegMeta metas[3];
+    __shared__ SegSums<kW> sums[2];
+    // the next step's counter was last used by the previous step's launch
     if (blockIdx.x == 0 && threadIdx.x == 0)
         a.work[(t + 1) & 1u] = 0;
-    for (;;) {
-    if (threadIdx.x == 0)
-        grab = atomicAdd(a.work + (t & 1u), kGrab);
+    if (wid == kW - 1) {
+        seg_fetch(a, blockIdx.x, nseg, metas[0]);
+        __pipeline_wait_prior(0);
+    }
     __syncthreads();
-    const uint32_t lo = grab;
-    __syncthreads();
-    if (lo >= ntiles)
-        break;
-    const uint32_t hi = min(ntiles, lo + kGrab);
-    // one segment per filter: its description and state are read once
-    uint32_t tile = lo;
-    while (tile < hi) {
-        const uint32_t f = a.tile_filter[tile];
-        const BFilter F = a.flt[f];
-        const BearingsConst &c = F.bc;
-        PfScalars &S = a.st[f];
-        const bool mon = !First && t == F.T;
-        const int resampled = First ? 1 : S.resampled;
-        const bool gather = First ? false : (S.gather != 0);
-        const float Mprev = First ? 0.0f : S.Mf;
-        const float z = mon ? 0.0f : a.obs[F.obs_off + t];
-        const uint32_t seg = tile;
-        uint32_t end = min(hi, F.tile0 + F.ntiles);
-        if (end <= tile) { // a tile table that disagrees with the filters
-            if (threadIdx.x == 0)
-                atomicOr(&S.err, DEV_ERR_INTERNAL);
-            end = tile + 1;
+    uint32_t slot = 0;
+    for (uint32_t it = 0;; ++it) {
+        const SegMeta &meta = metas[slot];
+        slot = slot == 2 ? 0 : slot + 1;
+        if (meta.count == 0)
+            break;
+        if (wid == kW - 1) { // the next segment
+            uint32_t next = 0;
+            if (lane == 0)
+                next = gridDim.x + atomicAdd(a.work + (t & 1u), 1u);
+            seg_fetch(
+                a, __shfl_sync(0xFFFFFFFFu, next, 0), nseg, metas[slot]);
         }
+        const BFilter F = meta.F; // in registers
+        const BearingsConst &c = F.bc;
+        const bool mon = !First && t == F.T;
+        const int resampled = First ? 1 : meta.resampled;
+        const bool gather = First ? false : (meta.gather != 0);
+        const float Mprev = First ? 0.0f : meta.Mf;
+        const float z = mon ? 0.0f : a.obs[F.obs_off + t];
+        const uint32_t end = meta.tile + meta.count;
         float m = -INFINITY, s = 0, s2 = 0, sx = 0, sy = 0, sw = 0;
-        for (; tile < end; ++tile) {
+        for (uint32_t tile = meta.tile; tile < end; ++tile) {
             const uint32_t i =
                 (tile - F.tile0) * kLearnTile + 32 * wid + g + 8 * q;
             const bool mine = i < F.n;
             float x = 0, y = 0, vx = 0, vy = 0, lw = 0;
             if (!First && mine) {
-                const uint32_t src = gather ? batch_source(a, F, S, i) : i;
-                x = a.ax[F.off + src];
-                y = a.ay[F.off + src];
-                vx = a.avx[F.off + src];
-                vy = a.avy[F.off + src];
+                uint32_t src[1] = {i};
+                if (gather) {
+                    const int32_t I[1] = {a.idx[F.off + i]};
+                    batch_sources<1>(a, F, a.st[meta.f], I, src);
+                }
+                x = a.ax[F.off + src[0]];
+                y = a.ay[F.off + src[0]];
+                vx = a.avx[F.off + src[0]];
+                vy = a.avy[F.off + src[0]];
                 lw = resampled ? 0.0f : a.lw[F.off + i];
             }
             if (mon) {
@@ -652,414 +773,205 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
                 a.lw[gi] = lw;
             }
         }
-        tile_finish<kLearnBlock, First>(a, seg, end - seg, f, F, S, t, mon, m,
-            s, s2, sx, sy, sw, shm, shw, is_last);
+        seg_record_warp(sums[it & 1], m, s, s2, sx, sy, sw);
+        if (wid == kW - 1)
+            __pipeline_wait_prior(0);
         __syncthreads();
-    }
+        if (static_cast<uint32_t>(wid) == it % kW)
+            seg_finish<kW, First>(a, meta, t, mon, sums[it & 1]);
     }
 }
 
 // ---------------------------------------------------------------- resampling
 //
 // The filters that resample at a step are resampled together by three
-// kernels over the step's list of equal chunks: entry v of the list is chunk
-// k of filter f (its particles [k c, (k + 1) c) with c = F.rs_chunk), and
-// the chunks of a filter are consecutive entries, listed by the block that
-// finished the filter's step (tile_finish).  The three passes are the single
-// filter's k_rs32_qsum / count / assign: a fixed-point total per chunk,
-// replication counts, and slot assignment with the sources of the empty
-// slots.  A chunk
-// takes its offsets from the per-chunk totals of the earlier chunks of its
-// filter (at most kMaxRsChunks, summed by every warp on its own).  Blocks
-// walk the list with a grid stride: the grids are fixed when a run is
-// captured, and filters that do not resample cost nothing.
+// kernels over the step's list of units: entry v of the list is unit k of
+// filter f (its particles [k u, (k + 1) u) with u = F.rs_unit), and the units
+// of a filter are consecutive entries, listed by the block that finished the
+// filter's step (tile_finish).  A unit is one warp's work, and the passes are
+// the single filter's over one warp range (qsum_range, count_range,
+// assign_range), without a block barrier: a block per chunk of 4096 particles
+// with block-wide scans took 34, 22 and 11 us a step at 512 filters, mostly
+// barriers and, in filters below 4096 particles, idle warps; it is 37, 20
+// and 15 us now with 6 million particles resampled in a step (early steps).
+// Eight units a chunk took 10.62 ms for 100 steps, sixteen 11.21, four 11.57.
+// The
+// last unit of a filter to finish a pass (a ticket per filter, nothing
+// waits) turns the units' totals into prefixes and records what the next
+// pass needs.  Warps walk the list with a grid stride: the grids are fixed
+// when a run is captured, and filters that do not resample cost nothing.
 
 // one list entry, with its filter's sizes
-struct RsChunk {
-    uint32_t f, k;    // filter, chunk of the filter
-    uint32_t base;    // list entry of the filter's chunk 0
-    uint32_t nc;      // chunks of the filter
-    uint32_t n, off, shift;
-    uint32_t lo, hi;  // particles (or surplus ranks) of the chunk
+struct RsUnit {
+    uint32_t f, k;   // filter, unit of the filter
+    uint32_t base;   // list entry of the filter's unit 0
+    uint32_t nu;     // units of the filter
+    uint32_t lo, hi; // particles of the unit
+    Rs32Args r;      // the filter's arrays
 };
 
-__device__ __forceinline__ RsChunk rs_chunk_at(const BatchArgs &a, uint32_t v)
+__device__ __forceinline__ RsUnit rs_unit_at(const BatchArgs &a, uint32_t v)
 {
     const uint2 e =
         __ldcg(a.rs_list + static_cast<size_t>(a.rpar) * a.rs_cap + v);
     const BFilter &F = a.flt[e.x];
-    RsChunk c;
+    RsUnit c;
     c.f = e.x;
     c.k = e.y;
     c.base = v - e.y;
-    c.n = F.n;
-    c.off = F.off;
-    c.shift = F.shift;
-    const uint32_t csz = F.rs_chunk;
-    c.nc = (c.n + csz - 1) / csz;
-    c.lo = min(c.n, c.k * csz);
-    c.hi = min(c.n, c.lo + csz);
+    c.nu = (F.n + F.rs_unit - 1) / F.rs_unit;
+    c.lo = min(F.n, c.k * F.rs_unit);
+    c.hi = min(F.n, c.lo + F.rs_unit);
+    c.r = Rs32Args{};
+    c.r.n = F.n;
+    c.r.shift = F.shift;
+    c.r.scheme = a.scheme;
+    c.r.lw = a.lw + F.off;
+    c.r.rep = a.rep + F.off;
+    c.r.idx = a.idx + F.off;
+    c.r.srcs = a.srcs + F.off;
+    c.r.sc = a.st + e.x;
     return c;
 }
 
-// op over the per-chunk totals of the filter: of chunks j < k (before) and
-// of all its chunks (all); every lane of the calling warp gets both
-template <typename T, typename Op>
-__device__ __forceinline__ void chunk_totals(
-    const T *part, const RsChunk &c, Op op, T identity, T &before, T &all)
+// Whether the calling warp's unit is the last of its filter to get here
+// (every lane gets the answer); its writes are ordered before.
+__device__ __forceinline__ bool rs_last_unit(uint32_t *ticket, uint32_t nu)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const T v = lane < c.nc ? __ldcg(part + c.base + lane) : identity;
-    before = warp_reduce(lane < c.k ? v : identity, op);
-    all = warp_reduce(v, op);
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if ((threadIdx.x & 31) == 0) {
+        last = atomicAdd(ticket, 1u) == nu - 1 ? 1 : 0;
+        if (last)
+            *ticket = 0;
+    }
+    last = __shfl_sync(0xFFFFFFFFu, last, 0);
+    if (last)
+        __threadfence();
+    return last != 0;
 }
 
-// pass 1: fixed-point total of each chunk (four tiles in flight per thread).
-// Block 0 also advances the step counter (every step kernel block has read
-// it) and empties the next step's list.
-__global__ void __launch_bounds__(kPfBlock) k_brs_qsum(const BatchArgs a)
+// v[0 .. nu) turned into exclusive prefixes by one warp; the total in every
+// lane.  A filter has at most kMaxRsUnits units.
+constexpr uint32_t kMaxRsUnits = 256;
+
+__device__ __forceinline__ uint64_t rs_prefix(uint64_t *v, uint32_t nu)
+{
+    constexpr uint32_t kK = kMaxRsUnits / 32;
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t x[kK];
+    uint64_t s = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kK; ++k) {
+        const uint32_t j = lane * kK + k;
+        x[k] = j < nu ? __ldcg(v + j) : 0ull;
+        s += x[k];
+    }
+    const uint64_t incl = warp_inclusive_scan(s, OpAdd());
+    uint64_t run = incl - s;
+#pragma unroll
+    for (uint32_t k = 0; k < kK; ++k) {
+        const uint32_t j = lane * kK + k;
+        if (j < nu)
+            v[j] = run;
+        run += x[k];
+    }
+    return __shfl_sync(0xFFFFFFFFu, incl, 31);
+}
+
+// warps of the grid and the calling one's number
+#define RS_UNITS(a, v, count)                                                 \
+    const uint32_t count = __ldcg((a).rs_count + (a).rpar);                   \
+    for (uint32_t v = blockIdx.x * (kPfBlock / 32) + (threadIdx.x >> 5);      \
+         v < count; v += gridDim.x * (kPfBlock / 32))
+
+// pass 1: fixed-point total of each unit; the filter's last one sets the
+// filter's counting constants.  Block 0 also advances the step counter
+// (every step kernel block has read it) and empties the next step's list.
+__global__ void __launch_bounds__(kPfBlock, 4) k_brs_qsum(const BatchArgs a)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(a.step, 1u);
         a.rs_count[a.rpar ^ 1u] = 0;
     }
-    const uint32_t count = __ldcg(a.rs_count + a.rpar);
-    __shared__ uint64_t sh[kPfBlock / 32 + 1];
-    constexpr int kG = 4;
-    for (uint32_t v = blockIdx.x; v < count; v += gridDim.x) {
-        const RsChunk c = rs_chunk_at(a, v);
-        const float M = a.st[c.f].Mf;
-        const float *lw = a.lw + c.off;
-        uint64_t acc = 0;
-        for (uint32_t base = c.lo; base < c.hi; base += kG * kPfTile) {
-            if (base + kG * kPfTile <= c.hi) {
-                float4 x[kG];
-#pragma unroll
-                for (int h = 0; h < kG; ++h)
-                    x[h] = __ldcg(reinterpret_cast<const float4 *>(
-                        lw + base + h * kPfTile + threadIdx.x * 4));
-#pragma unroll
-                for (int h = 0; h < kG; ++h)
-                    acc += fixed_q(x[h].x, M, c.shift) +
-                        fixed_q(x[h].y, M, c.shift) +
-                        fixed_q(x[h].z, M, c.shift) +
-                        fixed_q(x[h].w, M, c.shift);
-            } else {
-                for (int h = 0; h < kG; ++h) {
-                    const uint32_t i0 = base + h * kPfTile + threadIdx.x * 4;
-                    for (uint32_t i = i0; i < c.hi && i < i0 + 4; ++i)
-                        acc += fixed_q(lw[i], M, c.shift);
-                }
-            }
+    RS_UNITS(a, v, count)
+    {
+        const RsUnit c = rs_unit_at(a, v);
+        PfScalars &S = *c.r.sc;
+        const uint64_t q = qsum_range(c.r, c.lo, c.hi, S.Mf);
+        if ((threadIdx.x & 31) == 0)
+            a.rs_q[v] = q;
+        if (rs_last_unit(&S.done3, c.nu)) {
+            const uint64_t Q = rs_prefix(a.rs_q + c.base, c.nu);
+            uint32_t err = 0;
+            cdf_constants(S, Q, c.r.n, a.scheme == VSMC_CUDA_SYSTEMATIC, err);
+            if ((threadIdx.x & 31) == 0 && err)
+                atomicOr(&S.err, err);
         }
-        acc = block_reduce(acc, OpAdd(), uint64_t(0), sh);
-        // the filter's last chunk to finish (a thread-fenced ticket on
-        // done3; nothing waits) sets the filter's counting constants, by
-        // the block's first warp
-        if (threadIdx.x < 32) {
-            PfScalars &S = a.st[c.f];
-            int last = 0;
-            if (threadIdx.x == 0) {
-                a.rs_q[v] = acc;
-                __threadfence();
-                last = atomicAdd(&S.done3, 1u) == c.nc - 1 ? 1 : 0;
-                if (last)
-                    S.done3 = 0;
-                __threadfence();
-            }
-            last = __shfl_sync(0xFFFFFFFFu, last, 0);
-            if (last) {
-                uint64_t Q = 0; // at most 32 chunks
-                for (uint32_t k = threadIdx.x; k < c.nc; k += 32)
-                    Q += __ldcg(a.rs_q + c.base + k);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    Q += __shfl_xor_sync(0xFFFFFFFFu, Q, o);
-                uint32_t err = 0;
-                cdf_constants(S, Q, c.n, a.scheme == VSMC_CUDA_SYSTEMATIC, err);
-                // a zero total: pass 2 says so
-                if (threadIdx.x == 0 && (err & ~DEV_ERR_NONFINITE))
-                    atomicOr(&S.err, err & ~DEV_ERR_NONFINITE);
-            }
-        }
-        __syncthreads(); // the ticket is done before the next chunk
     }
 }
 
-// pass 2: replication counts from the fixed-point CDF; empty and copy
-// counts per chunk.  Each particle's CDF value is its exact 64-bit prefix
-// sum (the chunk's offset, a block scan per tile) and F(C) comes from the
-// filter's fixed-point reciprocal (cdf_floor), set by the filter's last
-// chunk in pass 1.  A thread's first count needs F just before its first
-// particle: lanes 1..31 take it from the lane before, lane 0 evaluates it.
-// Stratified words come from the tile's block of engine words in shared
-// memory.
+// pass 2: replication counts from the fixed-point CDF (count_range).  The
+// filter's last unit records the resample: the empty count, the gather flag
+// and the engine past the words the scheme consumed.  A zero total counts
+// nothing: no resample.
 template <bool Sys>
 __global__ void __launch_bounds__(kPfBlock, 3) k_brs_count(const BatchArgs a)
 {
-    const uint32_t count = __ldcg(a.rs_count + a.rpar);
-    constexpr bool sys = Sys; // the scheme (a.scheme) picked the instance
-    __shared__ uint64_t shs[kPfBlock / 32 + 1];
-    __shared__ uint32_t she[kPfBlock / 32 + 1];
-    __shared__ uint4 wbuf[2 * kPfBlock];        // stratified words of a tile
-    __shared__ uint32_t wsh[2 * (kPfBlock / 32)];
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t v = blockIdx.x; v < count; v += gridDim.x) {
-        const RsChunk c = rs_chunk_at(a, v);
-        PfScalars &S = a.st[c.f];
-        uint64_t offset, Q;
-        chunk_totals(a.rs_q, c, OpAdd(), uint64_t(0), offset, Q);
-        if (Q == 0) { // the same for the whole block
-            if (c.k == 0 && threadIdx.x == 0)
-                atomicOr(&S.err, DEV_ERR_NONFINITE);
-            continue;
-        }
-        // the engine before this resample (pass 3 advances it)
-        const PfScalars &sc = S;
-        const float M = sc.Mf;
-        const uint32_t n = c.n;
-        const float *lw = a.lw + c.off;
-        int32_t *rep = a.rep + c.off;
-        const CdfRcp p = load_cdf_rcp(sc, n);
+    __shared__ uint4 rows[Sys ? 1 : kPfBlock / 32][Sys ? 1 : kStratRow];
+    RS_UNITS(a, v, count)
+    {
+        const RsUnit c = rs_unit_at(a, v);
+        PfScalars &S = *c.r.sc;
+        const CdfRcp p = load_cdf_rcp(S, c.r.n);
         uint32_t empties = 0, copies = 0;
-        // one reciprocal case per chunk (Usual: p.s > 0), chosen once
-        auto run = [&](auto usual) {
-            constexpr bool Usual = decltype(usual)::value;
-            uint64_t carry = offset;
-            // the next tile's log-weights are loaded while this one is counted
-            float4 nxt = make_float4(0, 0, 0, 0);
-            if (c.lo + threadIdx.x * 4 + 3 < c.hi)
-                nxt = __ldcg(reinterpret_cast<const float4 *>(
-                    lw + c.lo + threadIdx.x * 4));
-            for (uint32_t base = c.lo; base < c.hi; base += kPfTile) {
-                const uint32_t i0 = base + threadIdx.x * 4;
-                const float4 x = nxt;
-                if (i0 + kPfTile + 3 < c.hi)
-                    nxt = __ldcg(
-                        reinterpret_cast<const float4 *>(lw + i0 + kPfTile));
-                uint64_t q[4];
-                if (i0 + 3 < c.hi) {
-                    q[0] = fixed_q(x.x, M, c.shift);
-                    q[1] = fixed_q(x.y, M, c.shift);
-                    q[2] = fixed_q(x.z, M, c.shift);
-                    q[3] = fixed_q(x.w, M, c.shift);
-                } else {
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        q[k] = i0 + k < c.hi ? fixed_q(lw[i0 + k], M, c.shift) : 0;
+        if (p.Q != 0) {
+            EnginePos e = {};
+            if (!Sys)
+                e = engine_pos(S);
+            uint4 *row = rows[Sys ? 0 : threadIdx.x >> 5];
+            const uint64_t carry = __ldcg(a.rs_q + v);
+            if (p.s != 0)
+                count_range<Sys, true>(c.r, p, e, row, c.lo, c.hi, carry,
+                    empties, copies);
+            else
+                count_range<Sys, false>(c.r, p, e, row, c.lo, c.hi, carry,
+                    empties, copies);
+            empties = __reduce_add_sync(0xFFFFFFFFu, empties);
+            copies = __reduce_add_sync(0xFFFFFFFFu, copies);
+        }
+        if ((threadIdx.x & 31) == 0)
+            a.rs_ec[v] = (static_cast<uint64_t>(copies) << 32) | empties;
+        if (rs_last_unit(&S.done2, c.nu)) {
+            const uint64_t ec = rs_prefix(a.rs_ec + c.base, c.nu);
+            if ((threadIdx.x & 31) == 0) {
+                S.nempty = static_cast<uint32_t>(ec);
+                if (p.Q != 0) {
+                    S.gather = 1;
+                    if (static_cast<uint32_t>(ec >> 32) != c.r.n)
+                        atomicOr(&S.err, DEV_ERR_INTERNAL);
+                    scheme_words(c.r, S);
                 }
-                uint64_t s[4];
-                s[0] = q[0];
-                s[1] = s[0] + q[1];
-                s[2] = s[1] + q[2];
-                s[3] = s[2] + q[3];
-                uint64_t tile_total;
-                const uint64_t incl =
-                    block_inclusive_scan(s[3], OpAdd(), uint64_t(0), shs, &tile_total);
-                const uint64_t cb = carry + (incl - s[3]);
-                uint32_t Fv[4], Fl = 0;
-                if (sys) {
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        Fv[k] = i0 + k + 1 >= n ? n : sys_F<Usual>(cb + s[k], p);
-                    if (lane == 0 && i0 != 0)
-                        Fl = sys_F<Usual>(cb, p);
-                } else {
-                    uint32_t j[4];
-                    uint64_t r[4];
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        j[k] = strat_j<Usual>(cb + s[k], p, r[k]);
-                    uint32_t jv = 0;
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (j[k] < n)
-                            jv = j[k];
-                    const uint32_t wlo = j[0] < n ? sc.rindex + j[0] : 0xFFFFFFFFu;
-                    const uint32_t whi = j[0] < n ? sc.rindex + jv : 0u;
-                    const WordBuf wv =
-                        fill_words<kPfBlock>(sc, wlo, whi, wbuf, 2 * kPfBlock, wsh);
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        Fv[k] = i0 + k + 1 >= n ? n
-                            : (j[k] >= n ? n
-                                         : j[k] + (ceil_aq(buf_word(sc,
-                                                       sc.rindex + j[k], wv), Q) <=
-                                                           r[k]
-                                                       ? 1u
-                                                       : 0u));
-                    if (lane == 0 && i0 != 0) {
-                        uint64_t r0;
-                        const uint32_t j0 = strat_j<Usual>(cb, p, r0);
-                        Fl = j0 >= n ? n
-                            : j0 + (ceil_aq(buf_word(sc, sc.rindex + j0, wv), Q) <=
-                                           r0
-                                       ? 1u
-                                       : 0u);
-                    }
-                }
-                // F before this thread's first particle (particle 0 has
-                // nothing before it)
-                const uint32_t Fup = __shfl_up_sync(0xFFFFFFFFu, Fv[3], 1);
-                uint32_t Fprev = lane == 0 ? Fl : Fup;
-                int32_t r[4];
-    #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    r[k] = static_cast<int32_t>(Fv[k] - Fprev);
-                    Fprev = Fv[k];
-                }
-                if (i0 + 3 < c.hi) {
-                    *reinterpret_cast<int4 *>(rep + i0) =
-                        make_int4(r[0], r[1], r[2], r[3]);
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        empties += r[k] == 0 ? 1u : 0u;
-                        copies += static_cast<uint32_t>(r[k]);
-                    }
-                } else {
-    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (i0 + k < c.hi) {
-                            rep[i0 + k] = r[k];
-                            empties += r[k] == 0 ? 1u : 0u;
-                            copies += static_cast<uint32_t>(r[k]);
-                        }
-                }
-                carry += tile_total;
             }
-        };
-        if (p.s != 0)
-            run(std::true_type{});
-        else
-            run(std::false_type{});
-        empties = block_reduce(empties, OpAdd(), 0u, she);
-        copies = block_reduce(copies, OpAdd(), 0u, she);
-        if (threadIdx.x == 0) {
-            a.rs_e[v] = empties;
-            a.rs_c[v] = copies;
         }
     }
 }
 
-
-// pass 3: slot assignment.  With c copies and e empty slots before slot i,
-// the first surplus rank of i is c - (i - e); idx[i] = i for a parent,
-// -(e + 1) for the e-th empty slot, and the sources of the surplus ranks of
-// a parent with two or more copies are written by its warp
-// (write_surplus_runs).  Chunk 0 records the filter's resample: Q, the
-// empty count, the gather flag and the engine words the scheme consumed.
-__global__ void __launch_bounds__(kPfBlock) k_brs_assign(const BatchArgs a)
+// pass 3: slot assignment (assign_range)
+__global__ void __launch_bounds__(kPfBlock, 4) k_brs_assign(const BatchArgs a)
 {
-    const uint32_t count = __ldcg(a.rs_count + a.rpar);
-    const bool sys = a.scheme == VSMC_CUDA_SYSTEMATIC;
-    __shared__ uint64_t sh64[kPfBlock / 32 + 1];
     __shared__ __align__(16) uint32_t shm[kPfBlock / 32][kRunChunk];
-    for (uint32_t v = blockIdx.x; v < count; v += gridDim.x) {
-        const RsChunk c = rs_chunk_at(a, v);
-        PfScalars &S = a.st[c.f];
-        uint64_t qb, Q;
-        chunk_totals(a.rs_q, c, OpAdd(), uint64_t(0), qb, Q);
-        if (Q == 0) { // counted nothing: no resample
-            if (c.k == 0 && threadIdx.x == 0)
-                S.nempty = 0;
+    RS_UNITS(a, v, count)
+    {
+        const RsUnit c = rs_unit_at(a, v);
+        const PfScalars &S = *c.r.sc;
+        if (S.Q == 0)
             continue;
-        }
-        uint32_t eoff, etotal, coff, ctotal;
-        chunk_totals(a.rs_e, c, OpAdd(), 0u, eoff, etotal);
-        chunk_totals(a.rs_c, c, OpAdd(), 0u, coff, ctotal);
-        const int32_t *rep = a.rep + c.off;
-        int32_t *idx = a.idx + c.off;
-        uint32_t *srcs = a.srcs + c.off;
-        if (c.k == 0 && threadIdx.x == 0) {
-            S.Q = Q;
-            S.nempty = etotal;
-            S.gather = 1;
-            if (ctotal != c.n)
-                atomicOr(&S.err, DEV_ERR_INTERNAL);
-            // the words U01SequenceSystematic / U01SequenceStratified
-            // consume (rng/u01_sequence.hpp:177-259,
-            // resample/transform.hpp:61-70)
-            if (sys) {
-                engine_advance(S, 1);
-            } else {
-                const uint32_t jf =
-                    c.n - static_cast<uint32_t>(rep[c.n - 1]);
-                engine_advance(S, jf < c.n ? jf + 1 : c.n);
-            }
-        }
-        uint32_t err = 0;
-        int4 nxt = load_rep4(rep, c.lo + threadIdx.x * 4, c.hi);
-        for (uint32_t base = c.lo; base < c.hi; base += kPfTile) {
-            const uint32_t i0 = base + threadIdx.x * 4;
-            const int4 cur = nxt;
-            if (base + kPfTile < c.hi)
-                nxt = load_rep4(rep, i0 + kPfTile, c.hi);
-            const int32_t r[4] = {cur.x, cur.y, cur.z, cur.w};
-            uint32_t tr = 0, te = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (r[k] >= 0) {
-                    tr += static_cast<uint32_t>(r[k]);
-                    te += r[k] == 0 ? 1u : 0u;
-                }
-            const uint64_t w = (static_cast<uint64_t>(tr) << 32) | te;
-            uint64_t tot;
-            const uint64_t incl =
-                block_inclusive_scan(w, OpAdd(), uint64_t(0), sh64, &tot);
-            const uint64_t exv = incl - w;
-            uint32_t cc = coff + static_cast<uint32_t>(exv >> 32);
-            uint32_t e = eoff + static_cast<uint32_t>(exv & 0xFFFFFFFFu);
-            const uint32_t c0 = cc, e0 = e;
-            int32_t out[4];
-            uint32_t rs[4], rl[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t i = i0 + k;
-                rs[k] = 0;
-                rl[k] = 0;
-                if (r[k] == 0) {
-                    out[k] = -static_cast<int32_t>(e) - 1;
-                    ++e;
-                } else {
-                    out[k] = static_cast<int32_t>(i);
-                    if (r[k] >= 2) {
-                        rs[k] = cc - (i - e);
-                        rl[k] = static_cast<uint32_t>(r[k]) - 1;
-                    }
-                }
-                if (r[k] > 0)
-                    cc += static_cast<uint32_t>(r[k]);
-            }
-            // the sources of the warp's surplus ranks
-            {
-                const uint32_t first = c0 - (i0 - e0);
-                const uint32_t W0 = __shfl_sync(0xFFFFFFFFu, first, 0);
-                uint32_t Sw = rl[0] + rl[1] + rl[2] + rl[3];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    Sw += __shfl_xor_sync(0xFFFFFFFFu, Sw, o);
-                if (Sw != 0) {
-                    if (Sw > etotal || W0 > etotal - Sw)
-                        err |= DEV_ERR_INTERNAL;
-                    else
-                        write_surplus_runs(srcs, rs, rl, i0, W0, Sw,
-                            shm[threadIdx.x >> 5], err);
-                }
-            }
-            if (i0 + 3 < c.hi) {
-                *reinterpret_cast<int4 *>(idx + i0) =
-                    make_int4(out[0], out[1], out[2], out[3]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (r[k] >= 0)
-                        idx[i0 + k] = out[k];
-            }
-            coff += static_cast<uint32_t>(tot >> 32);
-            eoff += static_cast<uint32_t>(tot & 0xFFFFFFFFu);
-        }
-        if (err)
-            atomicOr(&S.err, err);
+        const uint64_t ec = __ldcg(a.rs_ec + v);
+        float macc[kMaxMonitorDim];
+        assign_range<false>(c.r, c.lo, c.hi, static_cast<uint32_t>(ec >> 32),
+            static_cast<uint32_t>(ec), S.nempty, shm[threadIdx.x >> 5], macc);
     }
 }
 
@@ -1128,6 +1040,8 @@ __global__ void k_batch_simulate_bearings(
 
 constexpr uint32_t kRsMinChunk = 4 * kPfTile; // resampling chunk: 4096 or more
 constexpr uint32_t kMaxRsChunks = 32;          // chunks of one filter, at most
+constexpr uint32_t kRsUnits = 8;               // warps' units of a chunk
+static_assert(kMaxRsChunks * kRsUnits <= kMaxRsUnits, "units of a filter");
 constexpr int kRsKernels = 3;
 // the scan schedules the autotuner times: the smallest chunk of a filter
 constexpr uint32_t kRsSchedules[] = {4096, 8192, 16384, 32768};
@@ -1251,18 +1165,18 @@ struct vsmc_cuda_batch {
     uint32_t rs_cap = 0;            // resampling chunks of all filters
     int rs_grid[kRsKernels] = {};   // persistent grids of the passes
     std::vector<BFilter> flt;        // internal order
-    std::vector<uint32_t> tile_filter, active;
+    std::vector<uint32_t> active;
+    std::vector<uint4> segs;
     size_t total_particles = 0; // with padding
     size_t max_tiles = 0;
     // device
     BFilter *d_flt = nullptr;
     PfScalars *d_st = nullptr;
-    uint32_t *d_tile_filter = nullptr, *d_active = nullptr,
-             *d_step = nullptr;
+    uint4 *d_segs = nullptr;
+    uint32_t *d_active = nullptr, *d_step = nullptr;
     uint2 *d_rs_list = nullptr;
     uint32_t *d_rs_count = nullptr;
-    uint64_t *d_rs_q = nullptr;
-    uint32_t *d_rs_e = nullptr, *d_rs_c = nullptr;
+    uint64_t *d_rs_q = nullptr, *d_rs_ec = nullptr;
     float *d_state[2] = {nullptr, nullptr};
     float *d_lw = nullptr;
     int32_t *d_rep = nullptr, *d_idx = nullptr;
@@ -1299,9 +1213,9 @@ static void batch_free(vsmc_cuda_batch *b)
 {
     if (b->graph)
         cudaGraphExecDestroy(b->graph);
-    void *ptrs[] = {b->d_flt, b->d_st, b->d_tile_filter, b->d_active,
-        b->d_step, b->d_rs_list, b->d_rs_count, b->d_rs_q, b->d_rs_e,
-        b->d_rs_c, b->d_state[0], b->d_state[1], b->d_lw,
+    void *ptrs[] = {b->d_flt, b->d_st, b->d_segs, b->d_active,
+        b->d_step, b->d_rs_list, b->d_rs_count, b->d_rs_q, b->d_rs_ec,
+        b->d_state[0], b->d_state[1], b->d_lw,
         b->d_rep, b->d_idx, b->d_srcs, b->d_part, b->d_obs, b->d_obsf, b->d_obs_sc,
         b->d_mean, b->d_ess, b->d_logz, b->d_res};
     for (void *p : ptrs)
@@ -1317,15 +1231,25 @@ static int batch_layout(vsmc_cuda_batch *b, Shape s)
     const uint32_t tile = b->kind == kKindLearned
         ? kLearnTile
         : static_cast<uint32_t>(s.ppt * s.block);
-    b->tile_filter.clear();
+    const uint32_t most =
+        b->kind == kKindLearned ? kLearnSeg : seg_tiles(tile);
+    // a segment ends at its filter's last tile and at every `most` tiles
+    b->segs.clear();
+    std::vector<uint32_t> seg_end(b->nf); // segments up to each filter's
+    uint32_t tiles = 0;
     for (uint32_t k = 0; k < b->nf; ++k) {
         BFilter &F = b->flt[k];
-        F.tile0 = static_cast<uint32_t>(b->tile_filter.size());
+        F.tile0 = tiles;
         F.ntiles = (F.n + tile - 1) / tile;
-        for (uint32_t j = 0; j < F.ntiles; ++j)
-            b->tile_filter.push_back(k);
+        tiles += F.ntiles;
+        for (uint32_t j = F.tile0; j < tiles;) {
+            const uint32_t e = std::min(tiles, (j / most + 1) * most);
+            b->segs.push_back(make_uint4(j, e - j, k, 0));
+            j = e;
+        }
+        seg_end[k] = static_cast<uint32_t>(b->segs.size());
     }
-    if (b->tile_filter.size() > b->max_tiles)
+    if (tiles > b->max_tiles)
         return VSMC_CUDA_ERR_INTERNAL;
     // filters are sorted by T descending: those with T >= t are a prefix
     b->active.assign(b->tmax + 1, 0);
@@ -1333,13 +1257,13 @@ static int batch_layout(vsmc_cuda_batch *b, Shape s)
     for (uint32_t t = 0; t <= b->tmax; ++t) {
         while (k > 0 && b->flt[k - 1].T < t)
             --k;
-        b->active[t] = k == 0 ? 0 : b->flt[k - 1].tile0 + b->flt[k - 1].ntiles;
+        b->active[t] = k == 0 ? 0 : seg_end[k - 1];
     }
     cudaStream_t st = b->stream;
     VSMC_CUDA_TRY(cudaMemcpyAsync(b->d_flt, b->flt.data(),
         sizeof(BFilter) * b->nf, cudaMemcpyHostToDevice, st));
-    VSMC_CUDA_TRY(cudaMemcpyAsync(b->d_tile_filter, b->tile_filter.data(),
-        sizeof(uint32_t) * b->tile_filter.size(), cudaMemcpyHostToDevice, st));
+    VSMC_CUDA_TRY(cudaMemcpyAsync(b->d_segs, b->segs.data(),
+        sizeof(uint4) * b->segs.size(), cudaMemcpyHostToDevice, st));
     VSMC_CUDA_TRY(cudaMemcpyAsync(b->d_active, b->active.data(),
         sizeof(uint32_t) * b->active.size(), cudaMemcpyHostToDevice, st));
     VSMC_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1355,7 +1279,7 @@ static BatchArgs batch_args(vsmc_cuda_batch *b, const double *obs, int cur)
     float *B = b->d_state[1 - cur];
     a.flt = b->d_flt;
     a.st = b->d_st;
-    a.tile_filter = b->d_tile_filter;
+    a.segs = b->d_segs;
     a.active = b->d_active;
     a.ax = A;
     a.ay = A + ld;
@@ -1381,8 +1305,7 @@ static BatchArgs batch_args(vsmc_cuda_batch *b, const double *obs, int cur)
     a.rs_count = b->d_rs_count;
     a.work = b->d_rs_count + 2;
     a.rs_q = b->d_rs_q;
-    a.rs_e = b->d_rs_e;
-    a.rs_c = b->d_rs_c;
+    a.rs_ec = b->d_rs_ec;
     a.rs_cap = b->rs_cap;
     a.rpar = static_cast<uint32_t>(cur); // step parity, as the state buffers
     a.packed = b->packed;
@@ -1410,7 +1333,7 @@ static int enqueue_run(
     for (int t = 0; t < nsteps; ++t) {
         const BatchArgs a = batch_args(b, obs, t & 1);
         VSMC_CUDA_TRY(launch_step(b->kind, b->shape, t == 0, grid, a, st));
-        // the filters that resample, in the chunks the step listed
+        // the filters that resample, in the units the step listed
         const dim3 blk(kPfBlock);
         k_brs_qsum<<<b->rs_grid[0], blk, 0, st>>>(a);
         if (a.scheme == VSMC_CUDA_SYSTEMATIC)
@@ -1526,8 +1449,8 @@ static int batch_create(vsmc_cuda_batch **out, int kind, size_t nfilters,
         while ((size_t(1) << lg) < n[f])
             ++lg;
         F.shift = static_cast<uint32_t>(63 - lg);
-        F.rs_chunk = rs_chunk_for(F.n, kRsMinChunk);
-        b->rs_cap += (F.n + F.rs_chunk - 1) / F.rs_chunk;
+        F.rs_unit = rs_chunk_for(F.n, kRsMinChunk) / kRsUnits;
+        b->rs_cap += (F.n + F.rs_unit - 1) / F.rs_unit;
         if (kind == kKindCv)
             F.c = make_cv_const<float>(cv[f]);
         else
@@ -1543,7 +1466,8 @@ static int batch_create(vsmc_cuda_batch **out, int kind, size_t nfilters,
             occupancy_of(k_brs_assign, kPfBlock)};
         for (int k = 0; k < kRsKernels; ++k)
             b->rs_grid[k] = static_cast<int>(std::min<size_t>(
-                static_cast<size_t>(sms) * occ[k], b->rs_cap));
+                static_cast<size_t>(sms) * occ[k],
+                (b->rs_cap + kRsUnits - 1) / kRsUnits));
     }
 
     b->stream = as_stream(stream);
@@ -1567,13 +1491,12 @@ static int batch_create(vsmc_cuda_batch **out, int kind, size_t nfilters,
     } while (0)
     B_TRY(balloc(&b->d_flt, nfilters));
     B_TRY(balloc(&b->d_st, nfilters));
-    B_TRY(balloc(&b->d_tile_filter, tiles));
+    B_TRY(balloc(&b->d_segs, tiles));
     B_TRY(balloc(&b->d_active, tmax + 1));
     B_TRY(balloc(&b->d_rs_list, 2 * static_cast<size_t>(b->rs_cap)));
     B_TRY(balloc(&b->d_rs_count, 4));
     B_TRY(balloc(&b->d_rs_q, b->rs_cap));
-    B_TRY(balloc(&b->d_rs_e, b->rs_cap));
-    B_TRY(balloc(&b->d_rs_c, b->rs_cap));
+    B_TRY(balloc(&b->d_rs_ec, b->rs_cap));
     B_TRY(balloc(&b->d_step, 1));
     B_TRY(balloc(&b->d_state[0], 4 * total));
     B_TRY(balloc(&b->d_state[1], 4 * total));
@@ -1793,7 +1716,7 @@ int vsmc_cuda_batch_set_schedule(vsmc_cuda_batch *b, uint32_t min_chunk)
         return VSMC_CUDA_ERR_ARG;
     for (uint32_t k = 0; k < b->nf; ++k) {
         BFilter &F = b->flt[k];
-        F.rs_chunk = rs_chunk_for(F.n, min_chunk);
+        F.rs_unit = rs_chunk_for(F.n, min_chunk) / kRsUnits;
     }
     b->rs_min_chunk = min_chunk;
     // re-uploads the filter descriptions (their chunks); the list keeps the

@@ -261,12 +261,6 @@ __device__ __forceinline__ void chunk_range(
         hi = n;
 }
 
-__device__ __forceinline__ uint64_t q_at(
-    const Rs32Args &a, uint32_t i, float M)
-{
-    return a.q ? a.q[i] : fixed_q(a.lw[i], M, a.shift);
-}
-
 // Resident blocks per SM of the resampling passes (their grid is SMs times
 // this; 64 registers a thread).
 constexpr int kRsBlocksPerSm = 4;
@@ -393,65 +387,6 @@ __device__ __forceinline__ T scan_blocks_in_place(T *v, uint32_t m, T *sh)
     return tot;
 }
 
-// log-weights i..i+3 (i a multiple of 4) below hi, -inf past it
-__device__ __forceinline__ float4 load_lw4(
-    const float *lw, uint32_t i, uint32_t hi)
-{
-    if (i + 3 < hi)
-        return __ldcg(reinterpret_cast<const float4 *>(lw + i));
-    float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-    if (i < hi)
-        v.x = lw[i];
-    if (i + 1 < hi)
-        v.y = lw[i + 1];
-    if (i + 2 < hi)
-        v.z = lw[i + 2];
-    return v;
-}
-
-// sum of q over [wlo, whi), in every lane of the warp
-__device__ __forceinline__ uint64_t qsum_range(
-    const Rs32Args &a, uint32_t wlo, uint32_t whi, float M)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    uint64_t acc = 0;
-    constexpr int kG = 4;
-    constexpr uint32_t kSpan = kG * 128;
-    if (a.q == nullptr) {
-        // groups of kG float4 per lane; the next group's loads are issued
-        // before this group's weights, and a float4 past the range reads as
-        // -inf (weight 0), so the range's last group needs no other path
-        float4 v[kG], nv[kG];
-#pragma unroll
-        for (int h = 0; h < kG; ++h)
-            v[h] = load_lw4(a.lw, wlo + h * 128 + lane * 4, whi);
-        for (uint32_t base = wlo; base < whi; base += kSpan) {
-#pragma unroll
-            for (int h = 0; h < kG; ++h)
-                nv[h] = load_lw4(a.lw, base + kSpan + h * 128 + lane * 4, whi);
-#pragma unroll
-            for (int h = 0; h < kG; ++h)
-                acc += fixed_q(v[h].x, M, a.shift) +
-                    fixed_q(v[h].y, M, a.shift) +
-                    fixed_q(v[h].z, M, a.shift) + fixed_q(v[h].w, M, a.shift);
-#pragma unroll
-            for (int h = 0; h < kG; ++h)
-                v[h] = nv[h];
-        }
-    } else {
-        for (uint32_t base = wlo; base < whi; base += kSpan)
-            for (int h = 0; h < kG; ++h) {
-                const uint32_t i0 = base + h * 128 + lane * 4;
-                for (uint32_t i = i0; i < whi && i < i0 + 4; ++i)
-                    acc += a.q[i];
-            }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-    return acc;
-}
-
 // Sum of q over each warp range (four groups of four per lane in flight)
 // and over each block, into qpart.  The last block to finish turns the
 // block sums into prefix sums and sets the event's CDF constants: the total
@@ -511,134 +446,7 @@ __device__ __forceinline__ void count_finish(
     }
 }
 
-// Replication counts, one warp per warp range, no block barrier.  Particle
-// i's count is F(C_i) - F(C_{i-1}) for the CDF C_i: exact 64-bit prefix sums
-// (the range's offset from qsum, a warp scan per group of 128 particles).
-// F(C), the uniforms at or below C / Q, comes from the fixed-point
-// reciprocal of Q (cdf_floor): no division and no position carried from
-// particle to particle.  Stratified also reads each particle's word a_{j*}:
-// a group's j* are nondecreasing, so the warp generates the Philox blocks
-// holding them once into its shared-memory row (a word past the row is
-// generated where it is needed).  Per-range empty and copy counts go to
-// epart / cpart.
-constexpr uint32_t kStratRow = 64; // Philox blocks per warp row (256 words)
-
-// One warp's range, carry the CDF before it; Usual picks the reciprocal's
-// case for the whole pass.
-template <bool Sys, bool Usual>
-__device__ __forceinline__ void count_range(const Rs32Args &a,
-    const CdfRcp &p, const EnginePos &e, uint4 *row, uint32_t wlo,
-    uint32_t whi, uint64_t carry, uint32_t &empties, uint32_t &copies)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    const float M = static_cast<float>(a.sc->M);
-    const bool checked = a.q != nullptr;
-    const uint32_t n = a.n;
-    uint32_t Fprev = 0;
-    if (wlo != 0 && wlo < whi) {
-        if (Sys) {
-            Fprev = sys_F<Usual>(carry, p);
-        } else {
-            uint64_t r;
-            const uint32_t j = strat_j<Usual>(carry, p, r);
-            Fprev = strat_F(j, r, p, e, row, 0, 0);
-        }
-    }
-    float4 nxt = make_float4(0, 0, 0, 0);
-    if (!checked && wlo + lane * 4 + 3 < whi)
-        nxt = __ldcg(reinterpret_cast<const float4 *>(a.lw + wlo + lane * 4));
-    for (uint32_t base = wlo; base < whi; base += 128) {
-        const uint32_t i0 = base + lane * 4;
-        const float4 v = nxt;
-        if (!checked && i0 + 128 + 3 < whi)
-            nxt = __ldcg(reinterpret_cast<const float4 *>(a.lw + i0 + 128));
-        uint64_t q[4];
-        if (i0 + 3 < whi && !checked) {
-            q[0] = fixed_q(v.x, M, a.shift);
-            q[1] = fixed_q(v.y, M, a.shift);
-            q[2] = fixed_q(v.z, M, a.shift);
-            q[3] = fixed_q(v.w, M, a.shift);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                q[k] = (i0 + k < whi) ? q_at(a, i0 + k, M) : 0;
-        }
-        uint64_t s[4];
-        s[0] = q[0];
-        s[1] = s[0] + q[1];
-        s[2] = s[1] + q[2];
-        s[3] = s[2] + q[3];
-        const uint64_t incl = warp_inclusive_scan(s[3], OpAdd());
-        const uint64_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        const uint64_t cb = carry + (incl - s[3]);
-        uint32_t F[4];
-        if (Sys) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                F[k] = i0 + k + 1 >= n ? n : sys_F<Usual>(cb + s[k], p);
-        } else {
-            uint32_t j[4];
-            uint64_t r[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                j[k] = strat_j<Usual>(cb + s[k], p, r[k]);
-            // the group's words: j[0] of lane 0 .. j[3] of lane 31 (j = n
-            // needs none)
-            uint32_t jv = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (j[k] < n)
-                    jv = j[k];
-            const uint32_t jl = __reduce_min_sync(0xFFFFFFFFu, j[0]);
-            const uint32_t jh = __reduce_max_sync(0xFFFFFFFFu, jv);
-            uint32_t b0 = 0, nb = 0;
-            if (jl < n) {
-                b0 = (e.index + jl) >> 2;
-                const uint32_t bl = (e.index + (jh > jl ? jh : jl)) >> 2;
-                nb = bl - b0 + 1;
-                if (nb > kStratRow)
-                    nb = kStratRow;
-            }
-            __syncwarp();
-            for (uint32_t d = lane; d < nb; d += 32)
-                row[d] = engine_block(e, b0 + d);
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                F[k] = i0 + k + 1 >= n ? n
-                                       : strat_F(j[k], r[k], p, e, row, b0, nb);
-        }
-        uint32_t Fl = __shfl_up_sync(0xFFFFFFFFu, F[3], 1);
-        if (lane == 0)
-            Fl = Fprev;
-        int32_t r[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            r[k] = static_cast<int32_t>(F[k] - Fl);
-            Fl = F[k];
-        }
-        if (i0 + 3 < whi) {
-            *reinterpret_cast<int4 *>(a.rep + i0) =
-                make_int4(r[0], r[1], r[2], r[3]);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                empties += r[k] == 0 ? 1u : 0u;
-                copies += static_cast<uint32_t>(r[k]);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (i0 + k < whi) {
-                    a.rep[i0 + k] = r[k];
-                    empties += r[k] == 0 ? 1u : 0u;
-                    copies += static_cast<uint32_t>(r[k]);
-                }
-        }
-        carry += tot;
-        Fprev = __shfl_sync(0xFFFFFFFFu, F[3], 31);
-    }
-}
-
+// the counting pass: count_range over each warp's range
 template <bool Sys>
 __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_count(
     const Rs32Args a)
@@ -681,152 +489,7 @@ inline void launch_rs32_count(int grid, cudaStream_t st, const Rs32Args &a)
         k_rs32_count<false><<<grid, kPfBlock, 0, st>>>(a);
 }
 
-// Slot assignment, one warp per warp range (no block barrier).  With
-// c = copies before slot i and e = empty slots before i, the first surplus
-// rank of i is c - (i - e) (every non-empty slot before i keeps one of its
-// copies).  idx[i] = i for a parent (it keeps its slot), idx[i] = -(e + 1)
-// for the e-th empty slot, and srcs[first surplus rank .. + r - 1) = i for a
-// parent with r >= 2 copies: the reference's layout
-// (resample/transform.hpp:116-133) in one pass over the counts.  Each range
-// starts from its offsets (c, e) that the counting pass left in cpart /
-// epart, and a warp scan of (copies, empties) carries them through its
-// 128-particle groups.
-// One warp's range from its offsets (copies and empty slots before it); row:
-// kRunChunk words of the warp's; macc: the monitor's sums when asked for.
-template <bool Mon>
-__device__ __forceinline__ void assign_range(const Rs32Args &a, uint32_t wlo,
-    uint32_t whi, uint32_t coff, uint32_t eoff, uint32_t etotal,
-    uint32_t *row, float (&macc)[kMaxMonitorDim])
-{
-    const uint32_t lane = threadIdx.x & 31;
-    // monitor of the resampled particles, sum_i rep_i x_{d,i}, when the
-    // host asks for it right after resampling (mon_dim > 0); the rows, like
-    // the counts, are loaded one group ahead
-    const uint32_t md = Mon ? a.mon_dim : 0u;
-    float4 mrow[kMaxMonitorDim], mnxt[kMaxMonitorDim];
-#pragma unroll
-    for (int d = 0; d < kMaxMonitorDim; ++d)
-        mnxt[d] = static_cast<uint32_t>(d) < md
-            ? load_row4(a.mon_state + d * a.stride, wlo + lane * 4, whi)
-            : make_float4(0, 0, 0, 0);
-    uint32_t err = 0;
-    int4 nxt = load_rep4(a.rep, wlo + lane * 4, whi);
-    for (uint32_t base = wlo; base < whi; base += 128) {
-        const uint32_t i0 = base + lane * 4;
-        const int4 cur = nxt;
-        if (base + 128 < whi)
-            nxt = load_rep4(a.rep, i0 + 128, whi);
-#pragma unroll
-        for (int d = 0; d < kMaxMonitorDim; ++d) {
-            mrow[d] = mnxt[d];
-            if (static_cast<uint32_t>(d) < md && base + 128 < whi)
-                mnxt[d] = load_row4(a.mon_state + d * a.stride, i0 + 128, whi);
-        }
-        const int32_t r[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-        for (int d = 0; d < kMaxMonitorDim; ++d)
-            if (static_cast<uint32_t>(d) < md)
-                macc[d] += static_cast<float>(max(r[0], 0)) * mrow[d].x +
-                    static_cast<float>(max(r[1], 0)) * mrow[d].y +
-                    static_cast<float>(max(r[2], 0)) * mrow[d].z +
-                    static_cast<float>(max(r[3], 0)) * mrow[d].w;
-
-        uint32_t tr = 0, te = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (r[k] >= 0) {
-                tr += static_cast<uint32_t>(r[k]);
-                te += r[k] == 0 ? 1u : 0u;
-            }
-        // (copies, empties) before each lane: one 32-bit scan of
-        // copies * 256 + empties (a group has at most 128 empties) unless a
-        // lane has 2^16 or more copies
-        uint32_t c, e, tc, tn;
-        if (__any_sync(0xFFFFFFFFu, tr >= (1u << 16))) {
-            const uint64_t v = (static_cast<uint64_t>(tr) << 32) | te;
-            const uint64_t incl = warp_inclusive_scan(v, OpAdd());
-            const uint64_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const uint64_t ex = incl - v;
-            c = coff + static_cast<uint32_t>(ex >> 32);
-            e = eoff + static_cast<uint32_t>(ex & 0xFFFFFFFFu);
-            tc = static_cast<uint32_t>(tot >> 32);
-            tn = static_cast<uint32_t>(tot & 0xFFFFFFFFu);
-        } else {
-            const uint32_t v = (tr << 8) | te;
-            const uint32_t incl = warp_inclusive_scan(v, OpAdd());
-            const uint32_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const uint32_t ex = incl - v;
-            c = coff + (ex >> 8);
-            e = eoff + (ex & 0xFFu);
-            tc = tot >> 8;
-            tn = tot & 0xFFu;
-        }
-        const uint32_t c0 = c, e0 = e;
-        int32_t out[4];
-        uint32_t rs[4], rl[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t i = i0 + k;
-            rs[k] = 0;
-            rl[k] = 0;
-            if (r[k] == 0) {
-                out[k] = -static_cast<int32_t>(e) - 1;
-                ++e;
-            } else {
-                out[k] = static_cast<int32_t>(i);
-                if (r[k] >= 2) {
-                    rs[k] = c - (i - e);
-                    rl[k] = static_cast<uint32_t>(r[k]) - 1;
-                }
-            }
-            if (r[k] > 0)
-                c += static_cast<uint32_t>(r[k]);
-        }
-        // the group's surplus ranks: copies minus kept slots before its
-        // first particle, and the sum of its runs
-        {
-            const uint32_t first = c0 - (i0 - e0);
-            const uint32_t W0 = __shfl_sync(0xFFFFFFFFu, first, 0);
-            const uint32_t Sw =
-                __reduce_add_sync(0xFFFFFFFFu, rl[0] + rl[1] + rl[2] + rl[3]);
-            if (Sw != 0) {
-                if (Sw > etotal || W0 > etotal - Sw) {
-                    err |= DEV_ERR_INTERNAL; // ranks past the empty slots
-                } else {
-                    write_surplus_runs(a.srcs, rs, rl, i0, W0, Sw, row, err);
-                }
-            }
-        }
-        if (i0 + 3 < whi) {
-            *reinterpret_cast<int4 *>(a.idx + i0) =
-                make_int4(out[0], out[1], out[2], out[3]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (r[k] >= 0)
-                    a.idx[i0 + k] = out[k];
-        }
-        coff += tc;
-        eoff += tn;
-    }
-    if (err)
-        atomicOr(&a.sc->err, err);
-}
-
-// The engine past the words the scheme consumed: U01SequenceSystematic draws
-// once in its constructor; U01SequenceStratified draws lazily up to the first
-// uniform above the second-to-last cumulative weight
-// (rng/u01_sequence.hpp:177-259, resample/transform.hpp:61-70)
-__device__ __forceinline__ void scheme_words(const Rs32Args &a, PfScalars &sc)
-{
-    if (a.scheme == VSMC_CUDA_SYSTEMATIC) {
-        engine_advance(sc, 1);
-    } else if (a.n >= 2) {
-        const uint32_t jf = a.n - static_cast<uint32_t>(a.rep[a.n - 1]);
-        engine_advance(sc, jf < a.n ? jf + 1 : a.n);
-    }
-}
-
+// the assign pass: assign_range over each warp's range
 template <bool Mon>
 __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
     const Rs32Args a)

@@ -11,44 +11,28 @@ namespace vsmc_cuda
 
 // ------------------------------------------------------- small utilities
 
+// Both without branches, as LseMon's: the side with the larger max keeps its
+// sums, the other's are scaled by e; what carries no weight adds nothing.
 __device__ __forceinline__ void lse_push(float v, float &m, float &s, float &s2)
 {
-    if (!(v > -INFINITY)) // -inf and NaN carry no weight
-        return;
-    if (v > m) {
-        const float e = __expf(m - v);
-        s = s * e + 1.0f;
-        s2 = s2 * e * e + 1.0f;
-        m = v;
-    } else {
-        const float e = __expf(v - m);
-        s += e;
-        s2 += e * e;
-    }
+    const bool up = v > m;
+    // -inf and NaN carry no weight
+    const float e = v > -INFINITY ? __expf(up ? m - v : v - m) : 0.0f;
+    s = fmaf(up ? s : 1.0f, e, up ? 1.0f : s);
+    s2 = fmaf((up ? s2 : 1.0f) * e, e, up ? 1.0f : s2);
+    m = up ? v : m;
 }
 
 // merge (m2, t, t2) into (m, s, s2): max, sum exp(v - m), sum exp(2(v - m))
 __device__ __forceinline__ void lse_merge_f(
     float &m, float &s, float &s2, float m2, float t, float t2)
 {
-    if (!(m2 > -INFINITY))
-        return;
-    if (!(m > -INFINITY)) {
-        m = m2;
-        s = t;
-        s2 = t2;
-        return;
-    }
-    if (m2 > m) {
-        const float e = __expf(m - m2);
-        s = s * e + t;
-        s2 = s2 * e * e + t2;
-        m = m2;
-    } else {
-        const float e = __expf(m2 - m);
-        s += t * e;
-        s2 += t2 * e * e;
-    }
+    const bool up = m2 > m;
+    const float lo = up ? m : m2, hi = up ? m2 : m;
+    const float e = lo > -INFINITY ? __expf(lo - hi) : 0.0f;
+    s = fmaf(up ? s : t, e, up ? t : s);
+    s2 = fmaf((up ? s2 : t2) * e, e, up ? t2 : s2);
+    m = hi;
 }
 
 // 64 x 64 -> 128 bit product, compared as (hi, lo)
@@ -212,6 +196,19 @@ static __device__ __noinline__ int64_t cdf_floor_near(
     return ok ? k + 1 : k;
 }
 
+// B of the usual case: the truncated high product minus gs (two's
+// complement: -2^s <= B < 2^63)
+__device__ __forceinline__ uint64_t rcp_product(uint64_t C, const CdfRcp &p)
+{
+    const uint32_t c1 = static_cast<uint32_t>(C >> 32);
+    const uint32_t c0 = static_cast<uint32_t>(C);
+    const uint32_t m1 = static_cast<uint32_t>(p.m >> 32);
+    const uint32_t m0 = static_cast<uint32_t>(p.m);
+    const uint64_t H = static_cast<uint64_t>(c1) * m1 + __umulhi(c1, m0) +
+        __umulhi(c0, m1);
+    return H - p.gs;
+}
+
 // floor((C n - G) / Q) for C < Q (at least -1, below n).  Usual: the
 // usual case's reciprocal (p.s > 0) is known to apply, so the loop that
 // calls this holds one path only (the choice is made once per pass).
@@ -219,13 +216,7 @@ template <bool Usual>
 __device__ __forceinline__ int64_t cdf_floor(uint64_t C, const CdfRcp &p)
 {
     if (Usual) {
-        const uint32_t c1 = static_cast<uint32_t>(C >> 32);
-        const uint32_t c0 = static_cast<uint32_t>(C);
-        const uint32_t m1 = static_cast<uint32_t>(p.m >> 32);
-        const uint32_t m0 = static_cast<uint32_t>(p.m);
-        const uint64_t H = static_cast<uint64_t>(c1) * m1 +
-            __umulhi(c1, m0) + __umulhi(c0, m1);
-        const uint64_t B = H - p.gs; // two's complement: -2^s <= B < 2^63
+        const uint64_t B = rcp_product(C, p);
         const uint32_t bl = static_cast<uint32_t>(B);
         // B >> s (20 <= s <= 32): its low 32 bits are the signed answer
         const int32_t k = static_cast<int32_t>(
@@ -286,37 +277,112 @@ static __device__ __noinline__ uint4 engine_block_far(
 
 // Stratified: uniform j lies in [j / n, (j + 1) / n), so the uniforms at or
 // below C / Q are every j < j* = floor(C n / Q), and j* itself when its own
-// word passes, G_{j*} = ceil(a_{j*} Q / 2^32) <= r = C n - j* Q.  r < Q, so
-// 64-bit wrapping arithmetic gives it exactly.  j and r for one CDF value
-// (j = n when C >= Q).
+// word passes: a_{j*} 2^-32 <= V - j*, V = C n / Q.  In the usual case the
+// reciprocal's B gives both: j* = B >> s, and 2^s (V - j*) lies within -1 to
+// 4.5 of B's low s bits, so the word's top s bits decide unless they are
+// within a few units of them (StratPos::near; about 6 words in 2^s).  There,
+// and in the general case, the exact test: G_{j*} = ceil(a_{j*} Q / 2^32) <=
+// r = C n - j* Q (r < Q, so 64-bit wrapping arithmetic gives it exactly).
+// The exact remainder and product took 30 instructions of every particle.
+struct StratPos {
+    uint32_t j;    // j*, n when C >= Q
+    uint32_t frac; // usual case: B's low s bits; all ones when not usable
+    bool near;     // usual case: frac does not decide alone
+};
+
 template <bool Usual>
-__device__ __forceinline__ uint32_t strat_j(
-    uint64_t C, const CdfRcp &p, uint64_t &r)
+__device__ __forceinline__ StratPos strat_pos(uint64_t C, const CdfRcp &p)
 {
-    if (C >= p.Q) {
-        r = 0;
-        return p.n;
+    StratPos q = {p.n, 0, true};
+    if (C >= p.Q)
+        return q;
+    if (Usual) {
+        const uint64_t B = rcp_product(C, p);
+        const uint32_t bl = static_cast<uint32_t>(B);
+        int32_t k = static_cast<int32_t>(
+            __funnelshift_rc(bl, static_cast<uint32_t>(B >> 32), p.s));
+        q.near = ((bl + 6u) & p.fmask) < 8u;
+        if (q.near)
+            k = static_cast<int32_t>(cdf_floor_near(
+                C, k, (bl & p.fmask) < 2u, p.Q, p.G, p.n));
+        q.frac = bl & p.fmask;
+        q.j = static_cast<uint32_t>(k);
+        return q;
     }
-    const uint32_t j = static_cast<uint32_t>(cdf_floor<Usual>(C, p));
-    r = C * static_cast<uint64_t>(p.n) - static_cast<uint64_t>(j) * p.Q;
-    return j;
+    q.j = static_cast<uint32_t>(cdf_floor<false>(C, p));
+    return q;
 }
 
-// F from (j, r), word j taken from the warp's row of Philox blocks
-// [b0, b0 + nb) or generated when past it
-__device__ __forceinline__ uint32_t strat_F(uint32_t j, uint64_t r,
-    const CdfRcp &p, const EnginePos &e, const uint4 *row, uint32_t b0,
-    uint32_t nb)
+// the exact test of word a for j < n (rare: off the common path's registers)
+static __device__ __noinline__ bool strat_exact(
+    uint64_t C, uint32_t j, uint32_t a, uint64_t Q, uint32_t n)
 {
-    if (j >= p.n)
-        return p.n;
+    const uint64_t r =
+        C * static_cast<uint64_t>(n) - static_cast<uint64_t>(j) * Q;
+    return ceil_aq(a, Q) <= r;
+}
+
+// F(C) from its position and word j* (for j < n)
+template <bool Usual>
+__device__ __forceinline__ uint32_t strat_count(
+    uint64_t C, const StratPos &q, uint32_t a, const CdfRcp &p)
+{
+    if (!Usual)
+        return q.j + (strat_exact(C, q.j, a, p.Q, p.n) ? 1u : 0u);
+    const uint32_t as = a >> (32u - p.s); // p.s is 20 to 32
+    bool pass = as <= q.frac - 2u; // frac is 2 or more unless near
+    // frac - as from -4 to 1, or frac itself next to a whole number
+    if (q.near || q.frac - as + 4u <= 5u)
+        pass = strat_exact(C, q.j, a, p.Q, p.n);
+    return q.j + (pass ? 1u : 0u);
+}
+
+// A warp's window of the engine's Philox blocks: blocks [lo, hi) of the
+// stream are at row[b % kStratRow].  Blocks are generated 32 at a time, a
+// lane each, ahead of their use: a group of 128 particles needs 33 or so
+// blocks, and generating each group's own took two rounds of which the
+// second had one or two lanes.
+constexpr uint32_t kStratRow = 64; // blocks of a row (256 words)
+
+struct StratWindow {
+    uint32_t lo, hi;
+};
+
+// Blocks [b0, bl] into the window as far as it reaches (from b0 on).
+__device__ __forceinline__ void strat_fill(const EnginePos &e, uint4 *row,
+    StratWindow &w, uint32_t b0, uint32_t bl)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    if (b0 < w.lo || b0 > w.hi) { // not where the window ends: start anew
+        w.lo = b0;
+        w.hi = b0;
+    }
+    __syncwarp(); // the row's last readers
+    while (w.hi <= bl && w.hi + 32 - b0 <= kStratRow) {
+        const uint32_t b = w.hi + lane;
+        row[b % kStratRow] = engine_block(e, b);
+        w.hi += 32;
+    }
+    if (w.hi - w.lo > kStratRow)
+        w.lo = w.hi - kStratRow;
+    __syncwarp();
+}
+
+// word j of the uniforms, from the window or generated when outside it
+__device__ __forceinline__ uint32_t strat_word(uint32_t j, const EnginePos &e,
+    const uint4 *row, const StratWindow &w)
+{
     const uint32_t pos = e.index + j;
     const uint32_t b = pos >> 2;
-    const uint32_t d = b - b0;
-    const uint4 v = d < nb ? row[d] : engine_block_far(e, b);
-    const uint32_t k = pos & 3u;
-    const uint32_t a = k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
-    return j + (ceil_aq(a, p.Q) <= r ? 1u : 0u);
+    uint32_t a;
+    if (b - w.lo < w.hi - w.lo) {
+        a = reinterpret_cast<const uint32_t *>(row)[pos % (4 * kStratRow)];
+    } else {
+        const uint4 v = engine_block_far(e, b);
+        const uint32_t k = pos & 3u;
+        a = k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
+    }
+    return a;
 }
 
 // The per-event constants above, from the total Q (the same in every lane),
@@ -396,84 +462,6 @@ __device__ __forceinline__ uint64_t fixed_q(float lw, float M, uint32_t shift)
     const uint32_t lo = __float2uint_rz(fmaf(-h, 0x1p32f, x));
     const uint64_t q = (static_cast<uint64_t>(hi) << 32) | lo;
     return lw > -INFINITY ? q : 0ull;
-}
-
-// Stratified counting in the batched filters' block-wide tiles needs, for
-// each CDF value, the engine word of its uniform j* (strat_j).  A tile's CDF
-// values are nondecreasing, so the words it needs lie in one range of the
-// engine stream; the block generates that range's Philox blocks once into
-// shared memory (one or two per thread) instead of each thread generating
-// the blocks its own words fall in.  Block b of the stream is at
-// wb[b - b0] for b0 <= b < b0 + nb; a block beyond the buffer (a tile whose
-// words span more than it) is generated where it is needed.
-struct WordBuf {
-    const uint4 *wb;
-    uint32_t b0, nb;
-};
-
-// block b of the engine stream, for the rare word outside the buffer (not
-// inlined: it stays off the register budget of the common path)
-static __device__ __noinline__ uint4 engine_block_at(
-    const PfScalars &sc, uint32_t b)
-{
-    uint32_t c[4] = {sc.rctr[0], sc.rctr[1], sc.rctr[2], sc.rctr[3]};
-    ctr32_add(c, b);
-    const u32x4 p =
-        philox4x32_10(c[0], c[1], c[2], c[3], sc.rkey[0], sc.rkey[1]);
-    return make_uint4(p.x, p.y, p.z, p.w);
-}
-
-// word `pos` (rindex + j) of the engine stream
-__device__ __forceinline__ uint32_t buf_word(
-    const PfScalars &sc, uint32_t pos, const WordBuf &w)
-{
-    const uint32_t b = pos >> 2;
-    const uint32_t d = b - w.b0;
-    const uint4 v = d < w.nb ? w.wb[d] : engine_block_at(sc, b);
-    const uint32_t r = pos & 3u;
-    return r == 0 ? v.x : (r == 1 ? v.y : (r == 2 ? v.z : v.w));
-}
-
-// Generates the Philox blocks covering every thread's [wlo, whi] into wb
-// (cap blocks) and returns the buffer view.  sh holds 2 * kBlock / 32
-// entries.  Call with the whole block; it has two barriers.
-template <int kBlock>
-__device__ __forceinline__ WordBuf fill_words(const PfScalars &sc,
-    uint32_t wlo, uint32_t whi, uint4 *wb, uint32_t cap, uint32_t *sh)
-{
-    constexpr int kW = kBlock / 32;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, wlo);
-    const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, whi);
-    if (lane == 0) {
-        sh[wid] = lo;
-        sh[kW + wid] = hi;
-    }
-    __syncthreads();
-    uint32_t blo = 0xFFFFFFFFu, bhi = 0;
-#pragma unroll
-    for (int k = 0; k < kW; ++k) {
-        blo = min(blo, sh[k]);
-        bhi = max(bhi, sh[kW + k]);
-    }
-    WordBuf w;
-    w.wb = wb;
-    w.b0 = 0;
-    w.nb = 0;
-    if (blo <= bhi) {
-        w.b0 = blo >> 2;
-        const uint32_t nb = (bhi >> 2) - w.b0 + 1;
-        w.nb = nb < cap ? nb : cap;
-        for (uint32_t d = threadIdx.x; d < w.nb; d += kBlock) {
-            uint32_t c[4] = {sc.rctr[0], sc.rctr[1], sc.rctr[2], sc.rctr[3]};
-            ctr32_add(c, w.b0 + d);
-            const u32x4 p =
-                philox4x32_10(c[0], c[1], c[2], c[3], sc.rkey[0], sc.rkey[1]);
-            wb[d] = make_uint4(p.x, p.y, p.z, p.w);
-        }
-    }
-    __syncthreads();
-    return w;
 }
 
 // counts of slots i0..i0+3 below hi (-1 past hi)
@@ -596,6 +584,343 @@ __device__ __forceinline__ void write_surplus_runs(uint32_t *srcs,
         }
         __syncwarp(); // the row is reused by the next chunk
         p0 += kRunChunk;
+    }
+}
+
+// ------------------------------------------- the passes over one warp range
+
+__device__ __forceinline__ uint64_t q_at(
+    const Rs32Args &a, uint32_t i, float M)
+{
+    return a.q ? a.q[i] : fixed_q(a.lw[i], M, a.shift);
+}
+
+// log-weights i..i+3 (i a multiple of 4) below hi, -inf past it
+__device__ __forceinline__ float4 load_lw4(
+    const float *lw, uint32_t i, uint32_t hi)
+{
+    if (i + 3 < hi)
+        return __ldcg(reinterpret_cast<const float4 *>(lw + i));
+    float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    if (i < hi)
+        v.x = lw[i];
+    if (i + 1 < hi)
+        v.y = lw[i + 1];
+    if (i + 2 < hi)
+        v.z = lw[i + 2];
+    return v;
+}
+
+// sum of q over [wlo, whi), in every lane of the warp
+__device__ __forceinline__ uint64_t qsum_range(
+    const Rs32Args &a, uint32_t wlo, uint32_t whi, float M)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t acc = 0;
+    constexpr int kG = 4;
+    constexpr uint32_t kSpan = kG * 128;
+    if (a.q == nullptr) {
+        // groups of kG float4 per lane; the next group's loads are issued
+        // before this group's weights, and a float4 past the range reads as
+        // -inf (weight 0), so the range's last group needs no other path
+        float4 v[kG], nv[kG];
+#pragma unroll
+        for (int h = 0; h < kG; ++h)
+            v[h] = load_lw4(a.lw, wlo + h * 128 + lane * 4, whi);
+        for (uint32_t base = wlo; base < whi; base += kSpan) {
+#pragma unroll
+            for (int h = 0; h < kG; ++h)
+                nv[h] = load_lw4(a.lw, base + kSpan + h * 128 + lane * 4, whi);
+#pragma unroll
+            for (int h = 0; h < kG; ++h)
+                acc += fixed_q(v[h].x, M, a.shift) +
+                    fixed_q(v[h].y, M, a.shift) +
+                    fixed_q(v[h].z, M, a.shift) + fixed_q(v[h].w, M, a.shift);
+#pragma unroll
+            for (int h = 0; h < kG; ++h)
+                v[h] = nv[h];
+        }
+    } else {
+        for (uint32_t base = wlo; base < whi; base += kSpan)
+            for (int h = 0; h < kG; ++h) {
+                const uint32_t i0 = base + h * 128 + lane * 4;
+                for (uint32_t i = i0; i < whi && i < i0 + 4; ++i)
+                    acc += a.q[i];
+            }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+    return acc;
+}
+
+// Replication counts, one warp per warp range, no block barrier.  Particle
+// i's count is F(C_i) - F(C_{i-1}) for the CDF C_i: exact 64-bit prefix sums
+// (the range's offset from qsum, a warp scan per group of 128 particles).
+// F(C), the uniforms at or below C / Q, comes from the fixed-point
+// reciprocal of Q (cdf_floor): no division and no position carried from
+// particle to particle.  Stratified also reads each particle's word a_{j*}
+// from the warp's window of Philox blocks.  The range's empty slots and
+// copies are added to empties and copies (per lane).
+
+// One warp's range, carry the CDF before it; Usual picks the reciprocal's
+// case for the whole pass.
+template <bool Sys, bool Usual>
+__device__ __forceinline__ void count_range(const Rs32Args &a,
+    const CdfRcp &p, const EnginePos &e, uint4 *row, uint32_t wlo,
+    uint32_t whi, uint64_t carry, uint32_t &empties, uint32_t &copies)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const float M = static_cast<float>(a.sc->M);
+    const bool checked = a.q != nullptr;
+    const uint32_t n = a.n;
+    uint32_t Fprev = 0;
+    StratWindow win = {0, 0};
+    if (wlo != 0 && wlo < whi) {
+        if (Sys) {
+            Fprev = sys_F<Usual>(carry, p);
+        } else {
+            const StratPos q = strat_pos<Usual>(carry, p);
+            const uint32_t b = (e.index + q.j) >> 2;
+            Fprev = n;
+            if (q.j < n) { // the same in every lane
+                strat_fill(e, row, win, b, b);
+                Fprev = strat_count<Usual>(
+                    carry, q, strat_word(q.j, e, row, win), p);
+            }
+        }
+    }
+    float4 nxt = make_float4(0, 0, 0, 0);
+    if (!checked && wlo + lane * 4 + 3 < whi)
+        nxt = __ldcg(reinterpret_cast<const float4 *>(a.lw + wlo + lane * 4));
+    for (uint32_t base = wlo; base < whi; base += 128) {
+        const uint32_t i0 = base + lane * 4;
+        const float4 v = nxt;
+        if (!checked && i0 + 128 + 3 < whi)
+            nxt = __ldcg(reinterpret_cast<const float4 *>(a.lw + i0 + 128));
+        uint64_t q[4];
+        if (i0 + 3 < whi && !checked) {
+            q[0] = fixed_q(v.x, M, a.shift);
+            q[1] = fixed_q(v.y, M, a.shift);
+            q[2] = fixed_q(v.z, M, a.shift);
+            q[3] = fixed_q(v.w, M, a.shift);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                q[k] = (i0 + k < whi) ? q_at(a, i0 + k, M) : 0;
+        }
+        uint64_t s[4];
+        s[0] = q[0];
+        s[1] = s[0] + q[1];
+        s[2] = s[1] + q[2];
+        s[3] = s[2] + q[3];
+        const uint64_t incl = warp_inclusive_scan(s[3], OpAdd());
+        const uint64_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const uint64_t cb = carry + (incl - s[3]);
+        uint32_t F[4];
+        if (Sys) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                F[k] = i0 + k + 1 >= n ? n : sys_F<Usual>(cb + s[k], p);
+        } else {
+            StratPos sp[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                sp[k] = strat_pos<Usual>(cb + s[k], p);
+            // the group's words: j of lane 0's first .. of lane 31's last
+            // (j = n needs none)
+            uint32_t jv = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (sp[k].j < n)
+                    jv = sp[k].j;
+            const uint32_t jl = __reduce_min_sync(0xFFFFFFFFu, sp[0].j);
+            const uint32_t jh = __reduce_max_sync(0xFFFFFFFFu, jv);
+            if (jl < n)
+                strat_fill(e, row, win, (e.index + jl) >> 2,
+                    (e.index + (jh > jl ? jh : jl)) >> 2);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                F[k] = n;
+                if (i0 + k + 1 < n && sp[k].j < n)
+                    F[k] = strat_count<Usual>(cb + s[k], sp[k],
+                        strat_word(sp[k].j, e, row, win), p);
+            }
+        }
+        uint32_t Fl = __shfl_up_sync(0xFFFFFFFFu, F[3], 1);
+        if (lane == 0)
+            Fl = Fprev;
+        int32_t r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = static_cast<int32_t>(F[k] - Fl);
+            Fl = F[k];
+        }
+        if (i0 + 3 < whi) {
+            *reinterpret_cast<int4 *>(a.rep + i0) =
+                make_int4(r[0], r[1], r[2], r[3]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                empties += r[k] == 0 ? 1u : 0u;
+                copies += static_cast<uint32_t>(r[k]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i0 + k < whi) {
+                    a.rep[i0 + k] = r[k];
+                    empties += r[k] == 0 ? 1u : 0u;
+                    copies += static_cast<uint32_t>(r[k]);
+                }
+        }
+        carry += tot;
+        Fprev = __shfl_sync(0xFFFFFFFFu, F[3], 31);
+    }
+}
+
+// Slot assignment, one warp per warp range (no block barrier).  With
+// c = copies before slot i and e = empty slots before i, the first surplus
+// rank of i is c - (i - e) (every non-empty slot before i keeps one of its
+// copies).  idx[i] = i for a parent (it keeps its slot), idx[i] = -(e + 1)
+// for the e-th empty slot, and srcs[first surplus rank .. + r - 1) = i for a
+// parent with r >= 2 copies: the reference's layout
+// (resample/transform.hpp:116-133) in one pass over the counts.  Each range
+// starts from its offsets (c, e) that the counting pass left in cpart /
+// epart, and a warp scan of (copies, empties) carries them through its
+// 128-particle groups.
+// One warp's range from its offsets (copies and empty slots before it); row:
+// kRunChunk words of the warp's; macc: the monitor's sums when asked for.
+template <bool Mon>
+__device__ __forceinline__ void assign_range(const Rs32Args &a, uint32_t wlo,
+    uint32_t whi, uint32_t coff, uint32_t eoff, uint32_t etotal,
+    uint32_t *row, float (&macc)[kMaxMonitorDim])
+{
+    const uint32_t lane = threadIdx.x & 31;
+    // monitor of the resampled particles, sum_i rep_i x_{d,i}, when the
+    // host asks for it right after resampling (mon_dim > 0); the rows, like
+    // the counts, are loaded one group ahead
+    const uint32_t md = Mon ? a.mon_dim : 0u;
+    float4 mrow[kMaxMonitorDim], mnxt[kMaxMonitorDim];
+#pragma unroll
+    for (int d = 0; d < kMaxMonitorDim; ++d)
+        mnxt[d] = static_cast<uint32_t>(d) < md
+            ? load_row4(a.mon_state + d * a.stride, wlo + lane * 4, whi)
+            : make_float4(0, 0, 0, 0);
+    uint32_t err = 0;
+    int4 nxt = load_rep4(a.rep, wlo + lane * 4, whi);
+    for (uint32_t base = wlo; base < whi; base += 128) {
+        const uint32_t i0 = base + lane * 4;
+        const int4 cur = nxt;
+        if (base + 128 < whi)
+            nxt = load_rep4(a.rep, i0 + 128, whi);
+#pragma unroll
+        for (int d = 0; d < kMaxMonitorDim; ++d) {
+            mrow[d] = mnxt[d];
+            if (static_cast<uint32_t>(d) < md && base + 128 < whi)
+                mnxt[d] = load_row4(a.mon_state + d * a.stride, i0 + 128, whi);
+        }
+        const int32_t r[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+        for (int d = 0; d < kMaxMonitorDim; ++d)
+            if (static_cast<uint32_t>(d) < md)
+                macc[d] += static_cast<float>(max(r[0], 0)) * mrow[d].x +
+                    static_cast<float>(max(r[1], 0)) * mrow[d].y +
+                    static_cast<float>(max(r[2], 0)) * mrow[d].z +
+                    static_cast<float>(max(r[3], 0)) * mrow[d].w;
+
+        uint32_t tr = 0, te = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (r[k] >= 0) {
+                tr += static_cast<uint32_t>(r[k]);
+                te += r[k] == 0 ? 1u : 0u;
+            }
+        // (copies, empties) before each lane: one 32-bit scan of
+        // copies * 256 + empties (a group has at most 128 empties) unless a
+        // lane has 2^16 or more copies
+        uint32_t c, e, tc, tn;
+        if (__any_sync(0xFFFFFFFFu, tr >= (1u << 16))) {
+            const uint64_t v = (static_cast<uint64_t>(tr) << 32) | te;
+            const uint64_t incl = warp_inclusive_scan(v, OpAdd());
+            const uint64_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            const uint64_t ex = incl - v;
+            c = coff + static_cast<uint32_t>(ex >> 32);
+            e = eoff + static_cast<uint32_t>(ex & 0xFFFFFFFFu);
+            tc = static_cast<uint32_t>(tot >> 32);
+            tn = static_cast<uint32_t>(tot & 0xFFFFFFFFu);
+        } else {
+            const uint32_t v = (tr << 8) | te;
+            const uint32_t incl = warp_inclusive_scan(v, OpAdd());
+            const uint32_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            const uint32_t ex = incl - v;
+            c = coff + (ex >> 8);
+            e = eoff + (ex & 0xFFu);
+            tc = tot >> 8;
+            tn = tot & 0xFFu;
+        }
+        const uint32_t c0 = c, e0 = e;
+        int32_t out[4];
+        uint32_t rs[4], rl[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = i0 + k;
+            rs[k] = 0;
+            rl[k] = 0;
+            if (r[k] == 0) {
+                out[k] = -static_cast<int32_t>(e) - 1;
+                ++e;
+            } else {
+                out[k] = static_cast<int32_t>(i);
+                if (r[k] >= 2) {
+                    rs[k] = c - (i - e);
+                    rl[k] = static_cast<uint32_t>(r[k]) - 1;
+                }
+            }
+            if (r[k] > 0)
+                c += static_cast<uint32_t>(r[k]);
+        }
+        // the group's surplus ranks: copies minus kept slots before its
+        // first particle, and the sum of its runs
+        {
+            const uint32_t first = c0 - (i0 - e0);
+            const uint32_t W0 = __shfl_sync(0xFFFFFFFFu, first, 0);
+            const uint32_t Sw =
+                __reduce_add_sync(0xFFFFFFFFu, rl[0] + rl[1] + rl[2] + rl[3]);
+            if (Sw != 0) {
+                if (Sw > etotal || W0 > etotal - Sw) {
+                    err |= DEV_ERR_INTERNAL; // ranks past the empty slots
+                } else {
+                    write_surplus_runs(a.srcs, rs, rl, i0, W0, Sw, row, err);
+                }
+            }
+        }
+        if (i0 + 3 < whi) {
+            *reinterpret_cast<int4 *>(a.idx + i0) =
+                make_int4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (r[k] >= 0)
+                    a.idx[i0 + k] = out[k];
+        }
+        coff += tc;
+        eoff += tn;
+    }
+    if (err)
+        atomicOr(&a.sc->err, err);
+}
+
+// The engine past the words the scheme consumed: U01SequenceSystematic draws
+// once in its constructor; U01SequenceStratified draws lazily up to the first
+// uniform above the second-to-last cumulative weight
+// (rng/u01_sequence.hpp:177-259, resample/transform.hpp:61-70)
+__device__ __forceinline__ void scheme_words(const Rs32Args &a, PfScalars &sc)
+{
+    if (a.scheme == VSMC_CUDA_SYSTEMATIC) {
+        engine_advance(sc, 1);
+    } else if (a.n >= 2) {
+        const uint32_t jf = a.n - static_cast<uint32_t>(a.rep[a.n - 1]);
+        engine_advance(sc, jf < a.n ? jf + 1 : a.n);
     }
 }
 
