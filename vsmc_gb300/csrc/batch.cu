@@ -632,19 +632,28 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_batch_step(
     }
 }
 
-constexpr int kLearnBlock = 128;                // 4 warps
-constexpr uint32_t kLearnTile = kLearnBlock;     // 32 particles a warp
+// A learned segment is up to 1024 particles: 8 tiles of 128, 32 particles a
+// warp.  The block's 8 warps evaluate 2 tiles at a time; then 4 warps take
+// the sums, each lane over its particle of tile after tile.
+constexpr int kLearnBlock = 256;
+constexpr uint32_t kLearnTile = 128;
 constexpr uint32_t kLearnSeg = 1024u / kLearnTile; // tiles of a segment
 
-// One global step of the learned-proposal filters.  Each warp evaluates the
+// One global step of the learned-proposal filters.  A tile's evaluation is a
+// chain of about 1560 instructions a warp: with four warps a segment, 64
+// filters of 4096 particles (256 segments) left an SM 8 warps, each with
+// eight evaluations in turn.  Two blocks of 8 warps, four tiles each,
+// take the 50 steps (resampling included) from 3.06 to 2.45 ms; one block of
+// 16 took 2.81, two of 16 (64 registers) 2.56.  Each warp evaluates the
 // proposal network for 32 particles on the tensor cores (two 16-row tiles
 // sharing the weight loads); lane 4g + q then moves particle g + 8q of the
 // warp's 32.
 template <bool First>
-__global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
+__global__ void __launch_bounds__(kLearnBlock, 2) k_batch_step_learned(
     const BatchArgs a)
 {
-    constexpr int kW = kLearnBlock / 32;
+    constexpr int kW = 4; // warps that take the sums
+    constexpr int kLast = kLearnBlock / 32 - 1;
     __shared__ __align__(16) uint32_t sp[kPackedWords];
     const uint32_t t = *a.step;
     const uint32_t nseg = t <= a.tmax ? a.active[t] : 0u;
@@ -654,10 +663,12 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
     const int g = lane >> 2, q = lane & 3;
     __shared__ SegMeta metas[3];
     __shared__ SegSums<kW> sums[2];
+    // a segment's particles: log-weight; previous weight and position
+    __shared__ float s_lw[1024], s_wo[1024], s_x[1024], s_y[1024];
     // the next step's counter was last used by the previous step's launch
     if (blockIdx.x == 0 && threadIdx.x == 0)
         a.work[(t + 1) & 1u] = 0;
-    if (wid == kW - 1) {
+    if (wid == kLast) {
         seg_fetch(a, blockIdx.x, nseg, metas[0]);
         __pipeline_wait_prior(0);
     }
@@ -668,7 +679,7 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
         slot = slot == 2 ? 0 : slot + 1;
         if (meta.count == 0)
             break;
-        if (wid == kW - 1) { // the next segment
+        if (wid == kLast) { // the next segment
             uint32_t next = 0;
             if (lane == 0)
                 next = gridDim.x + atomicAdd(a.work + (t & 1u), 1u);
@@ -682,12 +693,16 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
         const bool gather = First ? false : (meta.gather != 0);
         const float Mprev = First ? 0.0f : meta.Mf;
         const float z = mon ? 0.0f : a.obs[F.obs_off + t];
-        const uint32_t end = meta.tile + meta.count;
-        float m = -INFINITY, s = 0, s2 = 0, sx = 0, sy = 0, sw = 0;
-        for (uint32_t tile = meta.tile; tile < end; ++tile) {
+        const uint32_t i00 = (meta.tile - F.tile0) * kLearnTile;
+        bool written = false;
+        for (uint32_t p = wid / kW; p < meta.count;
+             p += kLearnBlock / 128) {
+            // slot of the segment: tile p, the lane's particle in it
+            const uint32_t slot_i = p * kLearnTile + 32 * (wid % kW) + lane;
             const uint32_t i =
-                (tile - F.tile0) * kLearnTile + 32 * wid + g + 8 * q;
+                i00 + p * kLearnTile + 32 * (wid % kW) + g + 8 * q;
             const bool mine = i < F.n;
+            float wo = 0, x0 = 0, y0 = 0;
             float x = 0, y = 0, vx = 0, vy = 0, lw = 0;
             if (!First && mine) {
                 uint32_t src[1] = {i};
@@ -701,20 +716,17 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
                 vy = a.avy[F.off + src[0]];
                 lw = resampled ? 0.0f : a.lw[F.off + i];
             }
+            x0 = x;
+            y0 = y;
             if (mon) {
-                if (mine) {
-                    const float wo = resampled ? 1.0f : __expf(lw - Mprev);
-                    sx += wo * x;
-                    sy += wo * y;
-                    sw += wo;
-                }
+                if (mine)
+                    wo = resampled ? 1.0f : __expf(lw - Mprev);
             } else if (First) {
                 if (mine) {
                     float e[4];
                     bearings_normals(t, F.seed, i, e);
                     bearings_prior(c, e, x, y, vx, vy);
                     lw = bearings_loglik(c, z, x, y);
-                    lse_push(lw, m, s, s2);
                 }
             } else {
                 const float2 scz = a.obs_sc[F.obs_off + t];
@@ -745,10 +757,7 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
                 out_to_owner2(oa, ob, v);
                 if (mine) {
                     const float lw_old = resampled ? 0.0f : lw - Mprev;
-                    const float wo = resampled ? 1.0f : __expf(lw_old);
-                    sx += wo * x;
-                    sy += wo * y;
-                    sw += wo;
+                    wo = resampled ? 1.0f : __expf(lw_old);
                     float e[4], fr[4], nu[4];
                     bearings_normals(t, F.seed, i, e);
                     float lq = 0;
@@ -761,7 +770,6 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
                     frame_to_axes(sz, cz, fr, nu); // the draw, bearing frame
                     bearings_step(c, nu, x, y, vx, vy);
                     lw = lw_old + bearings_loglik(c, z, x, y) + lq;
-                    lse_push(lw, m, s, s2);
                 }
             }
             if (!mon && mine) {
@@ -772,13 +780,40 @@ __global__ void __launch_bounds__(kLearnBlock) k_batch_step_learned(
                 a.bvy[gi] = vy;
                 a.lw[gi] = lw;
             }
+            if (!written) { // the last segment's sums are taken
+                __syncthreads();
+                written = true;
+            }
+            s_lw[slot_i] = lw;
+            s_wo[slot_i] = wo;
+            s_x[slot_i] = x0;
+            s_y[slot_i] = y0;
         }
-        seg_record_warp(sums[it & 1], m, s, s2, sx, sy, sw);
-        if (wid == kW - 1)
+        if (!written)
+            __syncthreads();
+        if (wid == kLast)
             __pipeline_wait_prior(0);
         __syncthreads();
-        if (static_cast<uint32_t>(wid) == it % kW)
-            seg_finish<kW, First>(a, meta, t, mon, sums[it & 1]);
+        if (wid < kW) {
+            float m = -INFINITY, s = 0, s2 = 0, sx = 0, sy = 0, sw = 0;
+            for (uint32_t p = 0; p < meta.count; ++p) {
+                const uint32_t slot_i = p * kLearnTile + 32 * wid + lane;
+                if (i00 + p * kLearnTile + 32 * wid + g + 8 * q >= F.n)
+                    continue;
+                if (!First) {
+                    const float wo = s_wo[slot_i];
+                    sx += wo * s_x[slot_i];
+                    sy += wo * s_y[slot_i];
+                    sw += wo;
+                }
+                if (!mon)
+                    lse_push(s_lw[slot_i], m, s, s2);
+            }
+            seg_record_warp(sums[it & 1], m, s, s2, sx, sy, sw);
+            asm volatile("bar.sync 1, 128;" : : : "memory");
+            if (static_cast<uint32_t>(wid) == it % kW)
+                seg_finish<kW, First>(a, meta, t, mon, sums[it & 1]);
+        }
     }
 }
 
