@@ -5,6 +5,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "normal64.cuh"
 
 #include <cmath>
 
@@ -63,12 +64,11 @@ __device__ __forceinline__ u32x4 particle_block(
 __device__ __forceinline__ void normal_pair_d(uint32_t w0, uint32_t w1,
     double &z1, double &z2)
 {
-    const double u1 = sqrt(__dmul_rn(-2.0, log(u01_co_d(w0))));
-    const double u2 = __dmul_rn(kPi2, u01_co_d(w1));
-    double sv, cv;
-    sincos(u2, &sv, &cv);
-    z1 = __dmul_rn(u1, cv);
-    z2 = __dmul_rn(u1, sv);
+    double t, sv, cv;
+    n64_polar(static_cast<uint64_t>(w0) << 32, static_cast<uint64_t>(w1) << 32,
+        t, sv, cv);
+    z1 = __dmul_rn(t, cv);
+    z2 = __dmul_rn(t, sv);
 }
 
 // FP32: log1p(qx) + log1p(qy) as one log1p((1 + qx)(1 + qy) - 1)

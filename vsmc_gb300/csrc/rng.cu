@@ -124,16 +124,47 @@ __global__ void __launch_bounds__(256) k_plan_stream(Gen gen, StreamPlan plan,
     }
 }
 
+// the uniform of a word as box_muller_batch takes it: FP32, or (FP64) the
+// 64-bit fraction whose value is the word's [0, 1) uniform
+template <typename R, typename W>
+__device__ __forceinline__ auto normal_uniform(W w)
+{
+    if constexpr (sizeof(R) == 8)
+        return sizeof(W) == 4 ? static_cast<uint64_t>(w) << 32
+                              : static_cast<uint64_t>(w) & ~uint64_t(2047);
+    else if constexpr (sizeof(W) == 4)
+        return u01_co_f(w);
+    else
+        return u01_co_f64(w);
+}
+
+// word p of the stream
+template <typename Gen>
+__device__ typename Gen::word_t stream_word(
+    const Gen &gen, const StreamPlan &plan, uint64_t p)
+{
+    if (p < plan.head)
+        return Gen::word(
+            gen.block_at_start(plan), plan.x + static_cast<uint32_t>(p));
+    const uint64_t j = (p - plan.head) / 4;
+    return Gen::word(
+        gen.block(plan, j), static_cast<uint32_t>((p - plan.head) % 4));
+}
+
 // Box-Muller over the reference's batch layout (normal_distribution.hpp:
 // 222-239: per 1024-value chunk of k values, nu = k / 2 radii then nu
 // angles; out[i] = s sin, out[nu + i] = s cos) in one pass: per chunk, the
 // block generates the chunk's Philox / Threefry blocks once into shared
 // memory (one per thread, the chunk's words in stream order), then turns
 // each (radius, angle) pair into its sine and cosine values, so every value
-// is written once and no word goes through memory.
-template <typename Gen, typename R>
-__global__ void __launch_bounds__(256) k_normal_fused(Gen gen, StreamPlan plan,
-    size_t n, R *r, R mean, R sd)
+// is written once and no word goes through memory.  The last block adds the
+// odd value of an odd n (two more launches and a scratch buffer before: 1001
+// FP32 values took 19 us, 4.6 now).  2^22 + 1 FP64 values: 307 us with the
+// FP64 functions, 50 in integers, of which the five FP64 operations left a
+// pair take 21 and 600 integer instructions a pair the rest.
+template <typename Gen, typename R, bool Odd>
+__global__ void __launch_bounds__(256, 8) k_normal_fused(
+    Gen gen, StreamPlan plan, size_t n, R *r, R mean, R sd)
 {
     using W = typename Gen::word_t;
     __shared__ W words[1024];
@@ -169,39 +200,21 @@ __global__ void __launch_bounds__(256) k_normal_fused(Gen gen, StreamPlan plan,
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < nu; i += blockDim.x) {
-            R u1, u2;
-            if constexpr (sizeof(R) == 8) {
-                if constexpr (sizeof(W) == 4) {
-                    u1 = u01_co_d(words[i]);
-                    u2 = u01_co_d(words[nu + i]);
-                } else {
-                    u1 = u01_co_d64(words[i]);
-                    u2 = u01_co_d64(words[nu + i]);
-                }
-            } else {
-                if constexpr (sizeof(W) == 4) {
-                    u1 = u01_co_f(words[i]);
-                    u2 = u01_co_f(words[nu + i]);
-                } else {
-                    u1 = u01_co_f64(words[i]);
-                    u2 = u01_co_f64(words[nu + i]);
-                }
-            }
             R s, sv, cv;
-            box_muller_batch(u1, u2, sd, s, sv, cv);
+            box_muller_batch(normal_uniform<R>(words[i]),
+                normal_uniform<R>(words[nu + i]), sd, s, sv, cv);
             __stcs(r + base + i, fma_free_add(fma_free_mul(s, sv), mean));
             __stcs(r + base + nu + i, fma_free_add(fma_free_mul(s, cv), mean));
         }
         __syncthreads(); // words[] is reused by the next chunk
     }
-}
-
-template <typename R>
-__global__ void k_normal_odd_tail(size_t n, R *r, const R *extra, R mean, R sd)
-{
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const R u = extra[0], v = extra[1];
-        r[n - 1] = odd_tail_value(u, v, mean, sd);
+    // odd n: the last value takes two scalar words of its own
+    // (normal_distribution.hpp:259-266)
+    if (Odd && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        R s, sv, cv;
+        box_muller_batch(normal_uniform<R>(stream_word(gen, plan, n)),
+            normal_uniform<R>(stream_word(gen, plan, n + 1)), sd, s, sv, cv);
+        r[n - 1] = fma_free_add(mean, fma_free_mul(s, cv));
     }
 }
 
@@ -288,42 +301,26 @@ static int rng_normal_impl(
     const bool odd = (n % 2) != 0;
     // the n u01 words of the chunked calls, then (odd n) two scalar words
     const StreamPlan plan = plan_chunked_calls(*rng, n, odd ? 2 : 0);
-    constexpr Emit E = sizeof(R) == 8 ? Emit::U01D : Emit::U01F;
-    Scratch scratch(st);
-    R *extra = nullptr;
-    if (odd) {
-        extra = scratch.get<R>(2);
-        if (extra == nullptr)
-            return VSMC_CUDA_ERR_ALLOC;
-    }
-    int rc = VSMC_CUDA_OK;
-    // the pairs of every chunk in one pass; the odd value's two words
-    // (positions n, n + 1) through the stream kernel
     const size_t nchunks = (n + 1023) / 1024;
-    const int grid = static_cast<int>(
-        std::min<size_t>(nchunks, static_cast<size_t>(num_sms()) * 8));
-    if (rng->kind == VSMC_CUDA_PHILOX4X32) {
-        PhiloxGen gen(*rng);
-        if (n >= 2)
-            k_normal_fused<PhiloxGen, R><<<grid, 256, 0, st>>>(
-                gen, plan, n, r, mean, sd);
+    // FP64: a block for each chunk up to 64 an SM: 60 us for 2^22 values
+    // against 69 at 8 an SM, whose last round of chunks leaves most SMs idle.
+    // FP32 (bound by its stores): 50 us for 2^24 at 8 an SM, 56 at 64.
+    const int grid = static_cast<int>(std::min<size_t>(
+        nchunks, static_cast<size_t>(num_sms()) * (sizeof(R) == 8 ? 64 : 8)));
+    auto launch = [&](const auto &gen) {
+        using Gen = std::decay_t<decltype(gen)>;
         if (odd)
-            rc = launch_plan<PhiloxGen, E>(gen, plan, n, n + 2, extra, st);
-    } else {
-        ThreefryGen gen(*rng);
-        if (n >= 2)
-            k_normal_fused<ThreefryGen, R><<<grid, 256, 0, st>>>(
+            k_normal_fused<Gen, R, true><<<grid, 256, 0, st>>>(
                 gen, plan, n, r, mean, sd);
-        if (odd)
-            rc = launch_plan<ThreefryGen, E>(gen, plan, n, n + 2, extra, st);
-    }
+        else
+            k_normal_fused<Gen, R, false><<<grid, 256, 0, st>>>(
+                gen, plan, n, r, mean, sd);
+    };
+    if (rng->kind == VSMC_CUDA_PHILOX4X32)
+        launch(PhiloxGen(*rng));
+    else
+        launch(ThreefryGen(*rng));
     VSMC_CUDA_CHECK_LAUNCH();
-    if (rc != VSMC_CUDA_OK)
-        return rc;
-    if (odd) {
-        k_normal_odd_tail<R><<<1, 32, 0, st>>>(n, r, extra, mean, sd);
-        VSMC_CUDA_CHECK_LAUNCH();
-    }
     plan_final_state(*rng, plan);
     return VSMC_CUDA_OK;
 }

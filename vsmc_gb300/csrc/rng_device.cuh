@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "normal64.cuh"
 
 #include <math_constants.h>
 
@@ -316,15 +317,19 @@ __device__ __forceinline__ float fma_free_add(float a, float b)
 
 // Batch Box-Muller step for one (radius, angle) pair
 // (normal_distribution.hpp:229-238): s = sd * sqrt(-2 log u1), angle 2 pi u2.
+// The FP64 one takes its uniforms as 64-bit fractions.
+__device__ __forceinline__ void box_muller_batch(
+    uint64_t u1, uint64_t u2, double sd, double &s, double &sv, double &cv)
+{
+    double t;
+    n64_polar(u1, u2, t, sv, cv);
+    s = __dmul_rn(sd, t);
+}
+
 __device__ __forceinline__ void box_muller_batch(
     double u1, double u2, double sd, double &s, double &sv, double &cv)
 {
-    double t = log(u1);
-    t = __dmul_rn(-2.0, t);
-    t = sqrt(t);
-    const double th = __dmul_rn(kPi2, u2);
-    sincos(th, &sv, &cv);
-    s = __dmul_rn(sd, t);
+    box_muller_batch(n64_fraction(u1), n64_fraction(u2), sd, s, sv, cv);
 }
 
 __device__ __forceinline__ void box_muller_batch(
@@ -342,8 +347,9 @@ __device__ __forceinline__ void box_muller_batch(
 __device__ __forceinline__ double odd_tail_value(
     double u, double v, double mean, double sd)
 {
-    const double a = __dmul_rn(sd, sqrt(__dmul_rn(-2.0, log(u))));
-    return __dadd_rn(mean, __dmul_rn(a, cos(__dmul_rn(kPi2, v))));
+    double a, sv, cv;
+    box_muller_batch(u, v, sd, a, sv, cv);
+    return __dadd_rn(mean, __dmul_rn(a, cv));
 }
 
 __device__ __forceinline__ float odd_tail_value(
@@ -446,12 +452,12 @@ struct NormalScalar {
             z = v;
             saved = false;
         } else {
-            const R u1 = sqrt(__dmul_rn(-2.0, log(eng.u01d())));
-            const R u2 = __dmul_rn(kPi2, eng.u01d());
-            double sv, cv;
-            sincos(u2, &sv, &cv);
-            z = __dmul_rn(u1, cv);
-            v = __dmul_rn(u1, sv);
+            const double u1 = eng.u01d();
+            const double u2 = eng.u01d();
+            double t, sv, cv;
+            n64_polar(n64_fraction(u1), n64_fraction(u2), t, sv, cv);
+            z = __dmul_rn(t, cv);
+            v = __dmul_rn(t, sv);
             saved = true;
         }
         return __dadd_rn(mean, __dmul_rn(sd, z));
