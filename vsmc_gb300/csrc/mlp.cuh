@@ -59,14 +59,16 @@ __device__ __forceinline__ float gelu_f(float x)
     return __fdividef(x, 1.0f + e);
 }
 
-// derivative of gelu_f
-__device__ __forceinline__ float gelu_grad_f(float x)
+// gelu_f(x) and its derivative, from one exponential and one reciprocal
+__device__ __forceinline__ float gelu_with_grad_f(float x, float &grad)
 {
     const float x2 = x * x;
     const float e = __expf(x * fmaf(gelu_k1(), x2, gelu_k0()));
     const float s = __fdividef(1.0f, 1.0f + e); // sigmoid(2u)
+    const float y = x * s;
     // d/dx [x s(2u)] = s + x s (1 - s) 2u'(x), 2u'(x) = -(k0 + 3 k1 x^2)
-    return s - x * s * (1.0f - s) * fmaf(3.0f * gelu_k1(), x2, gelu_k0());
+    grad = s - y * (1.0f - s) * fmaf(3.0f * gelu_k1(), x2, gelu_k0());
+    return y;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
@@ -137,15 +139,18 @@ __device__ __forceinline__ uint2 frag(
 
 // Forward pass of one warp over 16 rows.  a0 holds the input operand
 // fragment (16 x 16, inputs in columns 0..5).  Outputs: out (accumulator
-// fragment of the 16 x 8 result, biases added); if pre1 / pre2 are given,
-// the hidden pre-activations (accumulator fragments of 8 n-tiles) and the
-// BF16 operand fragments of the hidden activations are kept for the
-// backward pass.  packed: the packed parameters (shared memory).
-template <bool Keep, bool Fast = false>
+// fragment of the 16 x 8 result, biases added); Keep: the derivatives of the
+// hidden activations (accumulator fragments of 8 n-tiles) are kept for the
+// backward pass, and the BF16 operand fragments of layer k's activations go to
+// act(k, fragments) as soon as they are there.  packed: the packed parameters (shared memory).
+struct NoActs {
+    __device__ void operator()(int, const uint32_t (&)[4][4]) const {}
+};
+
+template <bool Keep, bool Fast = false, class Acts = NoActs>
 __device__ __forceinline__ void mlp_forward_warp(const uint32_t *packed,
-    const uint32_t (&a0)[4], float (&out)[4], float (*pre1)[4] = nullptr,
-    float (*pre2)[4] = nullptr, uint32_t (*act1)[4] = nullptr,
-    uint32_t (*act2)[4] = nullptr)
+    const uint32_t (&a0)[4], float (&out)[4], float (*der1)[4] = nullptr,
+    float (*der2)[4] = nullptr, const Acts &act = Acts())
 {
     const int lane = threadIdx.x & 31;
     const int tig = lane & 3;
@@ -166,22 +171,21 @@ __device__ __forceinline__ void mlp_forward_warp(const uint32_t *packed,
     uint32_t a[4][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-        if (Keep) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                pre1[nt][r] = h[nt][r];
-        }
         const int kt = nt >> 1, hi = nt & 1;
-        a[kt][0 + 2 * hi] = gelu_pair<Fast>(h[nt][0], h[nt][1]);
-        a[kt][1 + 2 * hi] = gelu_pair<Fast>(h[nt][2], h[nt][3]);
-    }
-    if (Keep) {
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt)
+        if (Keep) {
+            float y[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
-                act1[kt][r] = a[kt][r];
+                y[r] = gelu_with_grad_f(h[nt][r], der1[nt][r]);
+            a[kt][0 + 2 * hi] = pack_bf16(y[0], y[1]);
+            a[kt][1 + 2 * hi] = pack_bf16(y[2], y[3]);
+        } else {
+            a[kt][0 + 2 * hi] = gelu_pair<Fast>(h[nt][0], h[nt][1]);
+            a[kt][1 + 2 * hi] = gelu_pair<Fast>(h[nt][2], h[nt][3]);
+        }
     }
+    if (Keep)
+        act(0, a);
     // ---- layer 2: 4 k-tiles x 8 n-tiles
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
@@ -191,30 +195,33 @@ __device__ __forceinline__ void mlp_forward_warp(const uint32_t *packed,
         h[nt][1] = bh;
         h[nt][2] = bl;
         h[nt][3] = bh;
+    }
+    // k-tiles outside: eight independent products between two of a chain
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
+    for (int kt = 0; kt < 4; ++kt) {
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
             const uint2 b = frag(packed, kF2, kt * 8 + nt, lane);
             mma_bf16(h[nt], a[kt], b.x, b.y);
         }
     }
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
-        if (Keep) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                pre2[nt][r] = h[nt][r];
-        }
         const int kt = nt >> 1, hi = nt & 1;
-        a[kt][0 + 2 * hi] = gelu_pair<Fast>(h[nt][0], h[nt][1]);
-        a[kt][1 + 2 * hi] = gelu_pair<Fast>(h[nt][2], h[nt][3]);
-    }
-    if (Keep) {
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt)
+        if (Keep) {
+            float y[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
-                act2[kt][r] = a[kt][r];
+                y[r] = gelu_with_grad_f(h[nt][r], der2[nt][r]);
+            a[kt][0 + 2 * hi] = pack_bf16(y[0], y[1]);
+            a[kt][1 + 2 * hi] = pack_bf16(y[2], y[3]);
+        } else {
+            a[kt][0 + 2 * hi] = gelu_pair<Fast>(h[nt][0], h[nt][1]);
+            a[kt][1 + 2 * hi] = gelu_pair<Fast>(h[nt][2], h[nt][3]);
+        }
     }
+    if (Keep)
+        act(1, a);
     // ---- layer 3: 4 k-tiles, one n-tile
     {
         const float bl = bias[2 * kHid + 2 * tig];

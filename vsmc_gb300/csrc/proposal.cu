@@ -16,6 +16,7 @@
 #include "tc05.cuh"
 #include "rng_device.cuh"
 
+#include <math_constants.h>
 #include <cmath>
 #include <new>
 #include <vector>
@@ -231,45 +232,59 @@ __global__ void __launch_bounds__(128) k_mlp_forward(
 // pass and the backward data path (deltas through W3 and W2) run per warp
 // on 16 rows with mma.sync, as in the filters.  The weight gradients are
 // contractions over the samples, dW = delta^T a, and run on the Blackwell
-// tensor core: every round of 64 samples the block writes its activations
-// and deltas into shared memory as K-major BF16 operands (K = the samples)
-// and one thread issues tcgen05.mma into FP32 accumulators in tensor memory
-// that live for the whole kernel.  Two products cover every weight:
+// tensor core: every round of 64 samples a group of four warps writes its
+// activations and deltas into shared memory as K-major BF16 operands (K = the
+// samples) and one thread issues tcgen05.mma into FP32 accumulators in tensor
+// memory that live for the whole kernel.  Two products cover every weight:
 //
 //   D1 (128 x 80) = [a1 | a2]^T [dp2 | dout | 0]:
 //       D1[k][j] = dW2[j][k] (k, j < 64), D1[64 + k][64 + d] = dW3[d][k]
 //   D2 (128 x 16) = [dp1 | dp2]^T [a0 | 1 | 0]:
 //       D2[j][c] = dW1[j][c] (c < 6), D2[j][6] = db1[j], D2[64 + j][6] = db2[j]
 //
-// The activations are BF16 already (the forward's operands); each FP32
-// delta is split into BF16 hi + lo parts (v = hi + lo to about 2^-17
-// relative) and both are multiplied, so the sums keep the deltas' FP32
-// precision.  Stage buffers alternate, and an mbarrier per buffer
-// (tcgen05.commit) says when the tensor core has finished reading one, so
-// a round's contraction overlaps the next round's forward and backward
-// passes.  db3 and the loss are register sums.  part: [grid][kNumParams + 1]
-// (the last entry is the block's loss sum); a block whose tensor-core wait
-// ran out writes NaN there and in its gradient entries.
+// [dp1 | dp2 | dout | 0] is one operand of 144 rows: D1 reads its last 80,
+// D2 its first 128.  The activations are BF16 already (the forward's
+// operands); each FP32 delta is split into BF16 hi + lo parts (v = hi + lo to
+// about 2^-17 relative) and both are multiplied, so the sums keep the deltas'
+// FP32 precision.  A register of a fragment is a row of samples by two
+// features, the operands want eight samples of a feature together:
+// stmatrix.trans stores four 8 x 8 blocks at once (24 of them a thread and
+// round; single 16-bit stores were 224).
+//
+// A round is a chain of small products, exponentials and stores, 6 us of one
+// warp a scheduler.  Two groups of four warps, the derivatives kept from the
+// forward pass, operands stored as soon as they are there and the inputs
+// fetched a round ahead take 65536 samples in 22 us; one group took 42.  Three
+// groups (168 registers a thread, a third of the rounds uneven) are no faster.
+// Each group has its own stage buffer and mbarrier (tcgen05.commit), which says
+// when the tensor core has finished reading the buffer, so a round's
+// contraction overlaps the next round's forward and backward passes; the
+// groups add to one accumulator in turn (an mbarrier each, turn).  db3 and the
+// loss are register sums.  part: [grid][kNumParams], part_loss: [grid]; a block
+// whose tensor-core wait ran out writes NaN to both.
 
-constexpr int kGradWarps = 4;
-constexpr int kGradRows = 16 * kGradWarps; // samples per round (the K tile)
+constexpr int kGradGroups = 2;
+constexpr int kGradWarps = 4;                  // warps of a group
+constexpr int kGradRows = 16 * kGradWarps;     // samples per round (the K tile)
+constexpr int kGradGroup = 32 * kGradWarps;    // threads of a group
+constexpr int kGradBlock = kGradGroups * kGradGroup;
+constexpr uint32_t kLossIts = 8;               // rounds of a group between sums
 
 // operands inside one stage buffer: K-major, no swizzle, rows of 64 samples
 // (8 core matrices of 128 B along K, 8-row groups 1024 B apart)
 constexpr uint32_t kTcLbo = 128;
 constexpr uint32_t kTcSbo = 1024;
-constexpr uint32_t kOpA1 = 0;                   // 128 rows: a1, a2
-constexpr uint32_t kOpB1h = kOpA1 + 128 * 128;  // 80 rows: dp2, dout, 0 (hi)
-constexpr uint32_t kOpB1l = kOpB1h + 80 * 128;  // (lo)
-constexpr uint32_t kOpA2h = kOpB1l + 80 * 128;  // 128 rows: dp1, dp2 (hi)
-constexpr uint32_t kOpA2l = kOpA2h + 128 * 128; // (lo)
-constexpr uint32_t kOpB2 = kOpA2l + 128 * 128;  // 16 rows: a0, 1, 0
-constexpr uint32_t kStageBytes = kOpB2 + 16 * 128;
+constexpr uint32_t kOpA = 0;                  // 128 rows: a1, a2
+constexpr uint32_t kOpDh = kOpA + 128 * 128;  // 144 rows: dp1, dp2, dout, 0 (hi)
+constexpr uint32_t kOpDl = kOpDh + 144 * 128; // (lo)
+constexpr uint32_t kOpX = kOpDl + 144 * 128;  // 16 rows: a0, 1, 0
+constexpr uint32_t kStageBytes = kOpX + 16 * 128;
+constexpr uint32_t kOpD2 = 64 * 128;          // D's row 64 within D
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kD1Col = 0, kD2Col = 96;
 constexpr uint32_t kPackedBytes = (sizeof(uint32_t) * kPackedWords + 1023) / 1024 * 1024;
 constexpr size_t kGradSmem = 1024 /* alignment slack */ + kPackedBytes +
-    2 * kStageBytes + 64 /* mbarriers, TMEM address */;
+    kGradGroups * kStageBytes + 64 /* mbarriers, TMEM address */;
 constexpr uint64_t kTcWaitNs = 1000000000ull; // 1 s
 
 // byte offset of (operand row, sample s) in a K-major no-swizzle operand
@@ -304,6 +319,56 @@ __device__ __forceinline__ void st_split(unsigned char *buf, uint32_t oph,
     *reinterpret_cast<__nv_bfloat16 *>(buf + opl + o) = l;
 }
 
+// Four 8 x 8 blocks of fragment registers (row: sample, two features a
+// register) with features as rows: w[0], w[1] the samples' halves of features
+// 16 b .. 16 b + 7, w[2], w[3] of the next eight.  `row`: this lane's row
+// address (lane / 8 the block, lane % 8 the feature in it).
+__device__ __forceinline__ void st_blocks(
+    uint32_t row, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3)
+{
+    asm volatile(
+        "stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], "
+        "{%1, %2, %3, %4};"
+        :
+        : "r"(row), "r"(w0), "r"(w1), "r"(w2), "r"(w3)
+        : "memory");
+}
+
+// the BF16 hi parts of two deltas, and the lo parts
+__device__ __forceinline__ uint32_t split_pair(
+    float v0, float v1, uint32_t &lo)
+{
+    const uint32_t h = pack_bf16(v0, v1);
+    lo = pack_bf16(v0 - __uint_as_float(h << 16),
+        v1 - __uint_as_float(h & 0xFFFF0000u));
+    return h;
+}
+
+// Deltas (accumulator fragments of 8 n-tiles) into the hi and lo operands'
+// rows; h: the hi parts, which are operand fragments.
+__device__ __forceinline__ void st_deltas(
+    uint32_t rowh, uint32_t rowl, const float (&d)[8][4], uint32_t (&h)[4][4])
+{
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+        uint32_t l[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            h[kt][k] = split_pair(d[2 * kt + (k >> 1)][2 * (k & 1)],
+                d[2 * kt + (k >> 1)][2 * (k & 1) + 1], l[k]);
+        const uint32_t o = 2 * kt * kTcSbo;
+        st_blocks(rowh + o, h[kt][0], h[kt][1], h[kt][2], h[kt][3]);
+        st_blocks(rowl + o, l[0], l[1], l[2], l[3]);
+    }
+}
+
+// barrier of one group (named barrier 1 + grp)
+__device__ __forceinline__ void group_sync(int grp)
+{
+    asm volatile("bar.sync %0, %1;" : : "r"(1 + grp), "n"(kGradGroup)
+                 : "memory");
+}
+
 // the round's contraction, issued by one thread on stage buffer `sb`
 __device__ __forceinline__ void grad_mma_round(
     uint32_t sb, uint32_t tmem, bool accumulate)
@@ -314,63 +379,68 @@ __device__ __forceinline__ void grad_mma_round(
     for (uint32_t kk = 0; kk < kGradRows / 16; ++kk) {
         const uint32_t ko = kk * 2 * kTcLbo; // 16 samples = 2 core matrices
         const uint32_t acc = (accumulate || kk > 0) ? 1u : 0u;
-        const uint64_t a1 = tc05::desc_kmajor(sb + kOpA1 + ko, kTcLbo, kTcSbo);
-        tc05::mma_bf16(tmem + kD1Col, a1,
-            tc05::desc_kmajor(sb + kOpB1h + ko, kTcLbo, kTcSbo), id1, acc);
-        tc05::mma_bf16(tmem + kD1Col, a1,
-            tc05::desc_kmajor(sb + kOpB1l + ko, kTcLbo, kTcSbo), id1, 1u);
-        const uint64_t b2 = tc05::desc_kmajor(sb + kOpB2 + ko, kTcLbo, kTcSbo);
+        const uint64_t a = tc05::desc_kmajor(sb + kOpA + ko, kTcLbo, kTcSbo);
+        tc05::mma_bf16(tmem + kD1Col, a,
+            tc05::desc_kmajor(sb + kOpDh + kOpD2 + ko, kTcLbo, kTcSbo), id1,
+            acc);
+        tc05::mma_bf16(tmem + kD1Col, a,
+            tc05::desc_kmajor(sb + kOpDl + kOpD2 + ko, kTcLbo, kTcSbo), id1,
+            1u);
+        const uint64_t x = tc05::desc_kmajor(sb + kOpX + ko, kTcLbo, kTcSbo);
         tc05::mma_bf16(tmem + kD2Col,
-            tc05::desc_kmajor(sb + kOpA2h + ko, kTcLbo, kTcSbo), b2, id2, acc);
+            tc05::desc_kmajor(sb + kOpDh + ko, kTcLbo, kTcSbo), x, id2, acc);
         tc05::mma_bf16(tmem + kD2Col,
-            tc05::desc_kmajor(sb + kOpA2l + ko, kTcLbo, kTcSbo), b2, id2, 1u);
+            tc05::desc_kmajor(sb + kOpDl + ko, kTcLbo, kTcSbo), x, id2, 1u);
     }
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_grad(const uint32_t *packed,
-    uint32_t B, const float *feat, const float *nu_in, float inv_b,
-    double *part)
+__global__ void __launch_bounds__(kGradBlock, 1) k_mlp_grad(
+    const uint32_t *packed, uint32_t B, const float *feat, const float *nu_in,
+    float inv_b, float *part, double *part_loss)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned carve-up (the descriptors need 16)
     const uint32_t raw = tc05::smem_addr(smem_raw);
     unsigned char *smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
     uint32_t *sp = reinterpret_cast<uint32_t *>(smem);
-    unsigned char *stage[2] = {smem + kPackedBytes,
-        smem + kPackedBytes + kStageBytes};
     uint64_t *mbar = reinterpret_cast<uint64_t *>(
-        smem + kPackedBytes + 2 * kStageBytes);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 2);
-    __shared__ double shl[128 / 32 + 1];
-    __shared__ float shb3[kGradWarps][kOut];
+        smem + kPackedBytes + kGradGroups * kStageBytes);
+    uint64_t *turn = mbar + kGradGroups;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(turn + kGradGroups);
+    __shared__ double shl[kGradBlock / 32 + 1];
+    __shared__ float shb3[kGradGroups * kGradWarps][kOut];
+    __shared__ float terms[kLossIts][kGradGroups][4][kGradRows];
 
     const int tid = threadIdx.x;
-    const int lane = tid & 31, wid = tid >> 5;
+    const int lane = tid & 31;
+    const int grp = tid / kGradGroup, wid = (tid / 32) % kGradWarps;
     const int g = lane >> 2, q = lane & 3;
+    unsigned char *buf = smem + kPackedBytes + grp * kStageBytes;
 
-    // constant operand rows: dout padding (B1 rows 72..79), the ones row
-    // and padding of B2 (rows 6..15), in both buffers
-    for (int b = 0; b < 2; ++b) {
-        for (uint32_t w = tid; w < 8 * 64; w += 128) {
-            const uint32_t row = 72 + w / 64, s = w % 64;
-            st16(stage[b], kOpB1h + op_off(row, s), 0);
-            st16(stage[b], kOpB1l + op_off(row, s), 0);
-        }
-        for (uint32_t w = tid; w < 10 * 64; w += 128) {
-            const uint32_t row = 6 + w / 64, s = w % 64;
-            st16(stage[b], kOpB2 + op_off(row, s), row == 6 ? 0x3F80u : 0u);
-        }
+    // constant operand rows: D's padding (rows 136..143), the ones row and
+    // padding of X (rows 6..15)
+    for (uint32_t w = tid % kGradGroup; w < 8 * 64; w += kGradGroup) {
+        const uint32_t row = 136 + w / 64, s = w % 64;
+        st16(buf, kOpDh + op_off(row, s), 0);
+        st16(buf, kOpDl + op_off(row, s), 0);
     }
-    if (tid == 0) {
-        tc05::mbar_init(&mbar[0], 1);
-        tc05::mbar_init(&mbar[1], 1);
+    for (uint32_t w = tid % kGradGroup; w < 10 * 64; w += kGradGroup) {
+        const uint32_t row = 6 + w / 64, s = w % 64;
+        st16(buf, kOpX + op_off(row, s), row == 6 ? 0x3F80u : 0u);
     }
-    if (wid == 0)
+    if (tid == 0)
+        for (int k = 0; k < 2 * kGradGroups; ++k)
+            tc05::mbar_init(&mbar[k], 1); // and turn
+    if (tid < 32)
         tc05::tmem_alloc(tmem_slot, kTmemCols);
     tc05::fence_before_sync();
     load_packed(sp, packed); // ends with __syncthreads
     tc05::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    // st_blocks' row of this lane at feature 0
+    const uint32_t row0 = tc05::smem_addr(buf) +
+        static_cast<uint32_t>((lane >> 4) * kTcSbo +
+            (2 * wid + ((lane >> 3) & 1)) * kTcLbo + (lane & 7) * 16);
 
     float gb3[kOut];
 #pragma unroll
@@ -379,34 +449,83 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const uint32_t *packed,
     float loss = 0;
     bool timed_out = false;
     const uint32_t rounds = (B + kGradRows - 1) / kGradRows;
-    uint32_t it = 0;
-    for (uint32_t rd = blockIdx.x; rd < rounds; rd += gridDim.x, ++it) {
-        const uint32_t p0 = rd * kGradRows + 16 * wid;
-        const uint32_t i = p0 + g + (q == 1 ? 8u : 0u);
-        const bool mine = q < 2 && i < B;
-        float f[6];
+    const uint32_t slot = 16 * wid + g + (q == 1 ? 8u : 0u); // lane's sample
+    // its features and targets in round rd
+    float f[6], target[4];
+    auto fetch = [&](uint32_t rd) {
+        const uint32_t i = rd * kGradRows + slot;
+        const bool mine = q < 2 && rd < rounds && i < B;
 #pragma unroll
         for (int k = 0; k < 6; ++k)
-            f[k] = mine ? feat[6 * i + k] : 0.0f;
+            f[k] = mine ? feat[6 * static_cast<size_t>(i) + k] : 0.0f;
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+            target[d] = mine ? nu_in[4 * static_cast<size_t>(i) + d] : 0.0f;
+    };
+    // The loss is summed per lane over the block's rounds in their order,
+    // whichever group they fall to: the terms wait in shared memory, and the
+    // first group adds those of up to kLossIts rounds a group at a time.
+    const uint32_t stride = kGradGroups * gridDim.x;
+    uint32_t done = 0; // rounds of a group already added
+    auto add_terms = [&](uint32_t upto) {
+        __syncthreads();
+        if (grp == 0 && q < 2)
+            for (uint32_t k = done; k < upto; ++k)
+                for (int j = 0; j < kGradGroups; ++j) {
+                    const uint32_t r = blockIdx.x + j * gridDim.x + k * stride;
+                    if (r < rounds && r * kGradRows + slot < B)
+#pragma unroll
+                        for (int d = 0; d < 4; ++d)
+                            loss += terms[k % kLossIts][j][d][slot];
+                }
+        done = upto;
+        __syncthreads();
+    };
+    const uint32_t its = (rounds - blockIdx.x + stride - 1) / stride;
+    const uint32_t rd0 = blockIdx.x + grp * gridDim.x;
+    fetch(rd0);
+    uint32_t it = 0; // rounds of this group
+    for (uint32_t k = 0; k < its; ++k) {
+        if (k > 0 && k % kLossIts == 0)
+            add_terms(k);
+        const uint32_t rd = rd0 + k * stride;
+        if (rd >= rounds) // the last one, of a later group
+            continue;
+        const bool mine = q < 2 && rd * kGradRows + slot < B;
         uint32_t a0[4];
         features_to_a(f, a0);
+        float tg[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+            tg[d] = target[d];
+        fetch(rd + stride); // the next round's
+        // The stage buffer is free once the last round's contraction has
+        // finished.  A wait that ran out is not repeated: the round's values
+        // are of no use then, but every barrier is reached.
+        if (it > 0 && !timed_out)
+            timed_out = !tc05::mbar_wait(&mbar[grp], (it - 1) & 1, kTcWaitNs);
         float o[4];
-        float pre1[8][4], pre2[8][4];
-        uint32_t act1[4][4], act2[4][4];
-        mlp_forward_warp<true>(sp, a0, o, pre1, pre2, act1, act2);
+        float der1[8][4], der2[8][4];
+        mlp_forward_warp<true>(sp, a0, o, der1, der2,
+            [&](int layer, const uint32_t (&act)[4][4]) {
+#pragma unroll
+                for (int kt = 0; kt < 4; ++kt)
+                    st_blocks(row0 + kOpA + layer * kOpD2 + 2 * kt * kTcSbo,
+                        act[kt][0], act[kt][1], act[kt][2], act[kt][3]);
+            });
         float v[8];
         out_to_owner(o, v);
         // d loss / d output of the owner's row (rows past B contribute 0)
         float dv[8];
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
-            float target = mine ? nu_in[4 * i + d] : 0.0f;
-            const float r = target - v[d];
+            const float r = tg[d] - v[d];
             const float el = __expf(-v[4 + d]);
             dv[d] = mine ? -r * el * inv_b : 0.0f;
             dv[4 + d] = mine ? 0.5f * (1.0f - r * r * el) * inv_b : 0.0f;
             if (mine)
-                loss += 0.5f * (r * r * el + v[4 + d]);
+                terms[k % kLossIts][grp][d][slot] =
+                    0.5f * (r * r * el + v[4 + d]);
         }
 #pragma unroll
         for (int d = 0; d < kOut; ++d)
@@ -422,135 +541,109 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const uint32_t *packed,
             mma_bf16(dp2[nt], ad, b.x, b.y);
 #pragma unroll
             for (int r = 0; r < 4; ++r)
-                dp2[nt][r] *= gelu_grad_f(pre2[nt][r]);
+                dp2[nt][r] *= der2[nt][r];
         }
         // dh1 = dpre2 W2, dpre1 = dh1 * gelu'(pre1)
         uint32_t a2[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            const int kt = nt >> 1, hi = nt & 1;
-            a2[kt][0 + 2 * hi] = pack_bf16(dp2[nt][0], dp2[nt][1]);
-            a2[kt][1 + 2 * hi] = pack_bf16(dp2[nt][2], dp2[nt][3]);
-        }
+        st_deltas(row0 + kOpDh + kOpD2, row0 + kOpDl + kOpD2, dp2, a2);
         float dp1[8][4];
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             dp1[nt][0] = dp1[nt][1] = dp1[nt][2] = dp1[nt][3] = 0;
+        }
 #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
+        for (int kt = 0; kt < 4; ++kt)
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) {
                 const uint2 b = frag(sp, kF2b, kt * 8 + nt, lane);
                 mma_bf16(dp1[nt], a2[kt], b.x, b.y);
             }
 #pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
             for (int r = 0; r < 4; ++r)
-                dp1[nt][r] *= gelu_grad_f(pre1[nt][r]);
-        }
-        // ---- the stage buffer is free once the contraction that last
-        // read it (two rounds ago) has finished
-        const int sbi = static_cast<int>(it & 1);
-        bool ok = true;
-        if (it >= 2)
-            ok = tc05::mbar_wait(&mbar[sbi], ((it >> 1) - 1) & 1, kTcWaitNs);
-        if (__syncthreads_or(!ok)) {
-            timed_out = true;
-            break;
-        }
-        unsigned char *buf = stage[sbi];
+                dp1[nt][r] *= der1[nt][r];
+        uint32_t h1[4][4];
+        st_deltas(row0 + kOpDh, row0 + kOpDl, dp1, h1);
         const uint32_t s0 = 16 * wid + g, s1 = s0 + 8;
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-            const uint32_t c = 16 * kt + 2 * q;
-            st_pair(buf, kOpA1, c, s0, act1[kt][0]);
-            st_pair(buf, kOpA1, c, s1, act1[kt][1]);
-            st_pair(buf, kOpA1, c + 8, s0, act1[kt][2]);
-            st_pair(buf, kOpA1, c + 8, s1, act1[kt][3]);
-            st_pair(buf, kOpA1, 64 + c, s0, act2[kt][0]);
-            st_pair(buf, kOpA1, 64 + c, s1, act2[kt][1]);
-            st_pair(buf, kOpA1, 64 + c + 8, s0, act2[kt][2]);
-            st_pair(buf, kOpA1, 64 + c + 8, s1, act2[kt][3]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            const uint32_t c = 8 * nt + 2 * q;
-            st_split(buf, kOpB1h, kOpB1l, c, s0, dp2[nt][0]);
-            st_split(buf, kOpB1h, kOpB1l, c + 1, s0, dp2[nt][1]);
-            st_split(buf, kOpB1h, kOpB1l, c, s1, dp2[nt][2]);
-            st_split(buf, kOpB1h, kOpB1l, c + 1, s1, dp2[nt][3]);
-            st_split(buf, kOpA2h, kOpA2l, 64 + c, s0, dp2[nt][0]);
-            st_split(buf, kOpA2h, kOpA2l, 64 + c + 1, s0, dp2[nt][1]);
-            st_split(buf, kOpA2h, kOpA2l, 64 + c, s1, dp2[nt][2]);
-            st_split(buf, kOpA2h, kOpA2l, 64 + c + 1, s1, dp2[nt][3]);
-            st_split(buf, kOpA2h, kOpA2l, c, s0, dp1[nt][0]);
-            st_split(buf, kOpA2h, kOpA2l, c + 1, s0, dp1[nt][1]);
-            st_split(buf, kOpA2h, kOpA2l, c, s1, dp1[nt][2]);
-            st_split(buf, kOpA2h, kOpA2l, c + 1, s1, dp1[nt][3]);
-        }
         if (q < 2) {
             const uint32_t s = q == 0 ? s0 : s1;
 #pragma unroll
             for (int d = 0; d < kOut; ++d)
-                st_split(buf, kOpB1h, kOpB1l, 64 + d, s, dv[d]);
+                st_split(buf, kOpDh, kOpDl, 128 + d, s, dv[d]);
         }
         if (q < 3) { // inputs 2q, 2q + 1 of rows s0 (a0[0]) and s1 (a0[1])
-            st_pair(buf, kOpB2, 2 * q, s0, a0[0]);
-            st_pair(buf, kOpB2, 2 * q, s1, a0[1]);
+            st_pair(buf, kOpX, 2 * q, s0, a0[0]);
+            st_pair(buf, kOpX, 2 * q, s1, a0[1]);
         }
         tc05::fence_async_shared();
-        __syncthreads();
-        if (tid == 0) {
+        group_sync(grp);
+        // One accumulator, so the groups' rounds take turns; another warp
+        // issues each time.
+        if (wid == static_cast<int>(it % kGradWarps) && lane == 0) {
+            const uint32_t seq = it * kGradGroups + grp;
+            if (seq > 0 && !timed_out)
+                timed_out = !tc05::mbar_wait(&turn[grp],
+                    (grp == 0 ? it - 1 : it) & 1, kTcWaitNs);
             tc05::fence_after_sync();
-            grad_mma_round(tc05::smem_addr(buf), tmem, it > 0);
-            tc05::commit(&mbar[sbi]);
+            if (!timed_out)
+                grad_mma_round(tc05::smem_addr(buf), tmem, seq > 0);
+            tc05::commit(&mbar[grp]);
+            tc05::fence_before_sync();
+            tc05::mbar_arrive(&turn[(grp + 1) % kGradGroups]);
         }
+        __syncwarp();
+        ++it;
     }
-    // ---- every contraction finished: the last commit covers the earlier
-    if (it > 0) {
-        const uint32_t last = it - 1;
-        const bool ok = tc05::mbar_wait(
-            &mbar[last & 1], (last >> 1) & 1, kTcWaitNs);
-        if (__syncthreads_or(!ok))
-            timed_out = true;
-    }
+    add_terms(its);
+    // ---- every contraction finished (a group's last commit covers its
+    // earlier ones)
+    if (it > 0 && !timed_out)
+        timed_out = !tc05::mbar_wait(&mbar[grp], (it - 1) & 1, kTcWaitNs);
+    tc05::fence_before_sync();
+    const bool gave_up = __syncthreads_or(timed_out);
     tc05::fence_after_sync();
-    double *out = part + static_cast<size_t>(blockIdx.x) * (kNumParams + 1);
-    if (timed_out) {
+    float *out = part + static_cast<size_t>(blockIdx.x) * kNumParams;
+    if (gave_up) {
         // record it; give the tensor core one more bounded wait before the
         // accumulators are released
-        if (it > 0)
-            tc05::mbar_wait(&mbar[(it - 1) & 1], ((it - 1) >> 1) & 1,
-                kTcWaitNs);
-        for (int k = tid; k <= kNumParams; k += 128)
-            out[k] = __longlong_as_double(0x7FF8000000000000ll);
-    } else if (it == 0) {
-        for (int k = tid; k <= kNumParams; k += 128)
-            out[k] = 0.0;
+        if (timed_out && it > 0)
+            tc05::mbar_wait(&mbar[grp], (it - 1) & 1, kTcWaitNs);
+        for (int k = tid; k < kNumParams; k += kGradBlock)
+            out[k] = CUDART_NAN_F;
+        if (tid == 0)
+            part_loss[blockIdx.x] = CUDART_NAN;
     } else {
-        // ---- accumulators -> block partials (warp w reads TMEM lanes
-        // 32w .. 32w + 31: row m = 32w + lane)
+        // ---- accumulators -> block partials (every block has a round).
+        // Warp w of a group reads TMEM lanes 32w .. 32w + 31: row
+        // m = 32w + lane.  D1's 64 columns are shared out in sixteens; the
+        // first group takes dW3, the last D2.
         const uint32_t m = 32 * wid + lane;
         const uint32_t tw = tmem + ((32u * wid) << 16);
         float vv[16];
         if (wid < 2) {
-#pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 16) {
+            for (int c0 = 16 * grp; c0 < 64; c0 += 16 * kGradGroups) {
                 tc05::ld16(tw + kD1Col + c0, vv);
 #pragma unroll
                 for (int c = 0; c < 16; ++c) // dW2[j = c0 + c][k = m]
                     out[kW2 + (c0 + c) * kHid + m] = vv[c];
             }
-            tc05::ld16(tw + kD2Col, vv);
-#pragma unroll
-            for (int c = 0; c < kIn; ++c)
-                out[kW1 + m * kIn + c] = vv[c];
-            out[kB1 + m] = vv[kIn];
-        } else {
-            const uint32_t k = m - 64;
+        } else if (grp == 0) {
             tc05::ld16(tw + kD1Col + 64, vv);
 #pragma unroll
             for (int d = 0; d < kOut; ++d) // dW3[d][k]
-                out[kW3 + d * kHid + k] = vv[d];
+                out[kW3 + d * kHid + m - 64] = vv[d];
+        }
+        if (grp == kGradGroups - 1) {
             tc05::ld16(tw + kD2Col, vv);
-            out[kB2 + k] = vv[kIn];
+            if (wid < 2) {
+#pragma unroll
+                for (int c = 0; c < kIn; ++c)
+                    out[kW1 + m * kIn + c] = vv[c];
+                out[kB1 + m] = vv[kIn];
+            } else {
+                out[kB2 + m - 64] = vv[kIn];
+            }
         }
         // db3 and the loss: register sums over the block
 #pragma unroll
@@ -560,24 +653,24 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const uint32_t *packed,
             for (int o2 = 16; o2 > 0; o2 >>= 1)
                 s += __shfl_xor_sync(0xFFFFFFFFu, s, o2);
             if (lane == 0)
-                shb3[wid][d] = s;
+                shb3[tid / 32][d] = s;
         }
         __syncthreads();
         if (tid < kOut) {
             float s = 0;
-            for (int w = 0; w < kGradWarps; ++w)
+            for (int w = 0; w < kGradGroups * kGradWarps; ++w)
                 s += shb3[w][tid];
             out[kB3 + tid] = s;
         }
         const double lb = block_reduce(static_cast<double>(loss), OpAdd(),
             0.0, shl);
         if (tid == 0)
-            out[kNumParams] = lb;
+            part_loss[blockIdx.x] = lb;
     }
     // ---- release the tensor memory (after every warp's reads)
     tc05::fence_before_sync();
     __syncthreads();
-    if (wid == 0) {
+    if (tid < 32) {
         tc05::fence_after_sync();
         tc05::tmem_free(tmem, kTmemCols);
     }
@@ -782,20 +875,92 @@ __global__ void __launch_bounds__(128, 4) k_mlp_forward_tc(
     }
 }
 
-// sum of the block partials (fixed order); grad = mean gradient
-__global__ void k_mlp_grad_reduce(const double *part, int nblocks,
-    float inv_b, float *grad, double *loss)
+// Sum of the block partials; grad = mean gradient.  A warp's lanes take 32
+// entries, its block's warps the partials b = w, w + 8, ... (one block more
+// sums the losses).  An entry's partials are added as integers aligned to the
+// largest of them: 31 bits below its last, so the error is below 2^-54 of it a
+// term, no more than an FP64 sum's, and exact in any order.  Per entry read by
+// one thread, 152 FP64 partials one after another took 15 us; eight warps
+// adding FP64 10 us (an FP64 addition of a warp holds its SM for 19 clocks);
+// 4.4 us now.
+constexpr int kRedWarps = 8;
+constexpr int kRedBatch = 20; // partials of a thread: 160 blocks
+constexpr int kRedBlocks = (kNumParams + 31) / 32;
+__global__ void __launch_bounds__(32 * kRedWarps) k_mlp_grad_reduce(
+    const float *part, const double *part_loss, int nblocks, float inv_b,
+    float *grad, double *loss)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > kNumParams)
+    __shared__ double sums[kRedWarps][32];
+    __shared__ uint32_t tops[kRedWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    if (blockIdx.x == kRedBlocks) {
+        double s = 0;
+        for (int b = threadIdx.x; b < nblocks; b += 32 * kRedWarps)
+            s += part_loss[b];
+        s = block_reduce(s, OpAdd(), 0.0, &sums[0][0]);
+        if (threadIdx.x == 0 && loss)
+            *loss = s * inv_b;
         return;
-    double s = 0;
-    for (int b = 0; b < nblocks; ++b)
-        s += part[static_cast<size_t>(b) * (kNumParams + 1) + i];
-    if (i < kNumParams)
-        grad[i] = static_cast<float>(s);
-    else if (loss)
-        *loss = s * inv_b;
+    }
+    double total = 0;
+    for (int b0 = 0; b0 < nblocks; b0 += kRedWarps * kRedBatch) {
+        uint32_t v[kRedBatch];
+        uint32_t top = 0;
+#pragma unroll
+        for (int k = 0; k < kRedBatch; ++k) {
+            const int b = b0 + w + kRedWarps * k;
+            v[k] = b < nblocks && i < kNumParams
+                ? __float_as_uint(part[static_cast<size_t>(b) * kNumParams + i])
+                : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kRedBatch; ++k)
+            top = max(top, v[k] & 0x7F800000u);
+        tops[w][lane] = top;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kRedWarps; ++k)
+            top = max(top, tops[k][lane]);
+        const uint32_t E = max(top >> 23, 1u);
+        int64_t sum = 0;
+        double special = 0; // an infinity or a NaN among them
+        if (E == 255u) {
+#pragma unroll
+            for (int k = 0; k < kRedBatch; ++k)
+                special += __uint_as_float(v[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kRedBatch; ++k) {
+                const uint32_t e = (v[k] >> 23) & 255u;
+                const uint64_t m =
+                    (v[k] & 0x7FFFFFu) | (e != 0 ? 0x800000u : 0u);
+                const int64_t a = static_cast<int64_t>(
+                    (m << 31) >> min(E - max(e, 1u), 63u));
+                sum += v[k] >> 31 ? -a : a;
+            }
+        }
+        // sum 2^(E - 127 - 23 - 31)
+        sums[w][lane] =
+            E == 255u ? special : __longlong_as_double(sum);
+        __syncthreads();
+        if (w == 0) {
+            if (E == 255u) {
+                for (int k = 0; k < kRedWarps; ++k)
+                    total += sums[k][lane];
+            } else {
+                int64_t t = 0;
+#pragma unroll
+                for (int k = 0; k < kRedWarps; ++k)
+                    t += __double_as_longlong(sums[k][lane]);
+                total += __ll2double_rn(t) *
+                    __hiloint2double(static_cast<int>((E + 842u) << 20), 0);
+            }
+        }
+        __syncthreads();
+    }
+    if (w == 0 && i < kNumParams)
+        grad[i] = static_cast<float>(total);
 }
 
 // Adam on the master parameters, then the packed copy is rebuilt
@@ -1032,6 +1197,13 @@ static int grad_blocks(uint32_t B)
     return rounds < cap ? rounds : cap;
 }
 
+// the partials of `grid` blocks: their losses, then their gradients
+static double *grad_part(Scratch &scratch, int grid)
+{
+    return scratch.get<double>(static_cast<size_t>(grid) +
+        (static_cast<size_t>(grid) * kNumParams + 1) / 2);
+}
+
 static bool grad_smem_ready()
 {
     static bool ok = cudaFuncSetAttribute(k_mlp_grad,
@@ -1040,7 +1212,7 @@ static bool grad_smem_ready()
     return ok;
 }
 
-// enqueue loss + gradient of B samples (part: [grid][kNumParams + 1])
+// enqueue loss + gradient of B samples (part: grad_part)
 static int enqueue_grad(const uint32_t *packed, uint32_t B, const float *feat,
     const float *nu, double *part, float *grad, double *loss,
     cudaStream_t st)
@@ -1049,9 +1221,11 @@ static int enqueue_grad(const uint32_t *packed, uint32_t B, const float *feat,
         return VSMC_CUDA_ERR_CUDA;
     const int grid = grad_blocks(B);
     const float inv_b = 1.0f / static_cast<float>(B);
-    k_mlp_grad<<<grid, 128, kGradSmem, st>>>(packed, B, feat, nu, inv_b, part);
-    k_mlp_grad_reduce<<<(kNumParams + 1 + 255) / 256, 256, 0, st>>>(
-        part, grid, inv_b, grad, loss);
+    float *part_grad = reinterpret_cast<float *>(part + grid);
+    k_mlp_grad<<<grid, kGradBlock, kGradSmem, st>>>(
+        packed, B, feat, nu, inv_b, part_grad, part);
+    k_mlp_grad_reduce<<<kRedBlocks + 1, 32 * kRedWarps, 0, st>>>(
+        part_grad, part, grid, inv_b, grad, loss);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1145,9 +1319,8 @@ int vsmc_cuda_mlp_loss_grad(const uint32_t *packed, size_t B,
         return VSMC_CUDA_ERR_SIZE;
     cudaStream_t st = as_stream(stream);
     Scratch scratch(st);
-    double *part = scratch.get<double>(
-        static_cast<size_t>(grad_blocks(static_cast<uint32_t>(B))) *
-        (kNumParams + 1));
+    double *part =
+        grad_part(scratch, grad_blocks(static_cast<uint32_t>(B)));
     if (part == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
     return enqueue_grad(packed, static_cast<uint32_t>(B), feat, nu, part,
@@ -1270,9 +1443,8 @@ int vsmc_cuda_mlp_train_rows(const vsmc_cuda_bearings_model *model,
     float *m2 = scratch.get<float>(kNumParams);
     uint32_t *packed = scratch.get<uint32_t>(kPackedWords);
     double *losses = scratch.get<double>(steps);
-    double *part = scratch.get<double>(
-        static_cast<size_t>(grad_blocks(static_cast<uint32_t>(batch))) *
-        (kNumParams + 1));
+    double *part =
+        grad_part(scratch, grad_blocks(static_cast<uint32_t>(batch)));
     if (!tx || !ty || !tvx || !tvy || !feat || !nu || !mf || !mn || !grad ||
         !m1 || !m2 || !packed || !losses || !part)
         return VSMC_CUDA_ERR_ALLOC;

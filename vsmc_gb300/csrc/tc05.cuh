@@ -154,26 +154,43 @@ __device__ __forceinline__ uint64_t global_ns()
     return t;
 }
 
+// whether the phase of the given parity has completed
+__device__ __forceinline__ bool mbar_try(uint64_t *mbar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(done)
+                 : "r"(smem_addr(mbar)), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
+
 // Wait until the phase of the given parity has completed; false after
-// `limit_ns` of wall time without it.
+// `limit_ns` of wall time without it (the clock is read only if the first
+// try fails).
 __device__ __forceinline__ bool mbar_wait(
     uint64_t *mbar, uint32_t parity, uint64_t limit_ns)
 {
-    const uint32_t a = smem_addr(mbar);
+    if (mbar_try(mbar, parity))
+        return true;
     const uint64_t t0 = global_ns();
     for (;;) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(done)
-                     : "r"(a), "r"(parity)
-                     : "memory");
-        if (done)
+        if (mbar_try(mbar, parity))
             return true;
         if (global_ns() - t0 > limit_ns)
             return false;
     }
+}
+
+// one arrival of this thread
+__device__ __forceinline__ void mbar_arrive(uint64_t *mbar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
+                 :
+                 : "r"(smem_addr(mbar))
+                 : "memory");
 }
 
 } // namespace tc05
