@@ -240,15 +240,15 @@ VSMC_N64 double n64_double(uint64_t m53, int e)
 #endif
 }
 
-// sqrt(-2 ln(u 2^-64)), u > 0
-VSMC_N64 double n64_radius(uint64_t u)
+// -ln(v 2^-(64 + k)) = m 2^(e - 64), v and m with the top bit set, not for
+// v = 2^64 - 1 rounded up to 1 (the logarithm of 1); 0 <= k <= 63, Wide: 1100
+template <bool Wide>
+VSMC_N64 uint64_t n64_neg_log(uint64_t v, int k, int &e)
 {
-    const int lz = n64_clz(u);
-    const uint64_t v = u << lz;
     const uint32_t i = static_cast<uint32_t>(v >> 56) & 127u;
     const N64Log tab = n64_log_entry(i);
     // t = 1 - v c / 2^15 as a 70-bit fraction: (2^79 - v c) / 2^9, rounded up
-    // and exact for the last interval (c = 2^15), where u near 1 needs all of it
+    // and exact for the last interval (c = 2^15), where v near 1 needs all of it
     const uint64_t p0 = n64_mul(static_cast<uint32_t>(v), tab.c);
     const uint64_t p1 =
         n64_mul(static_cast<uint32_t>(v >> 32), tab.c) + (p0 >> 32);
@@ -261,21 +261,35 @@ VSMC_N64 double n64_radius(uint64_t u)
     q = 0x015555555555f16full + n64_mulhi(t, q);
     q = 0x7ffffffffffffee7ull + n64_mulhi(t, q);
     const uint64_t w = n64_mulhi(t, q) >> 6;
-    // R = lz ln2 + ln c + t + t w: 2^-64 units below 1 (lz = 0), else 2^-58
+    // k ln2 + ln c + t + t w: 2^-64 units below 1 (k = 0), else 2^-58 (Wide:
+    // 2^-53 from k = 64 on)
     const uint64_t y = t + n64_mulhi(t, w);
-    const int sh = lz != 0 ? 6 : 0;
-    uint64_t m = ((tab.L + (y >> 6)) >> sh) +
-        static_cast<uint64_t>(lz) * 0x02c5c85fdf473de7ull;
-    int e = sh + 1; // 2 R = m 2^(e - 64)
-    if (lz == 0 && i == 127) { // R = t + t w: keep the bits of a small t
+    const int sh = k == 0 ? 0 : (Wide && k > 63 ? 11 : 6);
+    uint64_t m = (tab.L + (y >> 6)) >> sh;
+    if (Wide) // ln2 in two 32-bit halves
+        m += (n64_mul(static_cast<uint32_t>(k), 0xb17217f7u) << (32 - sh)) +
+            (n64_mul(static_cast<uint32_t>(k), 0xd1cf79acu) >> sh);
+    else
+        m += static_cast<uint64_t>(k) * 0x02c5c85fdf473de7ull;
+    e = sh;
+    if (k == 0 && i == 127) { // t + t w alone: keep the bits of a small t
         const int s = n64_clz(t) - 1;
         const uint64_t tn = t << s;
         m = tn + n64_mulhi(tn, w);
-        e = -5 - s;
+        e = -6 - s;
     }
     const int z = n64_clz(m);
-    m <<= z;
     e -= z;
+    return m << z;
+}
+
+// sqrt(-2 ln(u 2^-64)), u > 0
+VSMC_N64 double n64_radius(uint64_t u)
+{
+    const int lz = n64_clz(u);
+    int e;
+    uint64_t m = n64_neg_log<false>(u << lz, lz, e);
+    ++e; // 2 R
     // -2 ln u as the FP64 logarithm would give it, 53 bits (as 2^-63 units)
     m = ((m >> 1) + 512) & ~1023ull;
     // e even, m in [1/4, 1]

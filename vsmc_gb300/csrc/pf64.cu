@@ -21,6 +21,7 @@
 // warp), so they run in 64-thread blocks over all SMs: at 2^14 particles a
 // step took 320 us with 256-thread blocks on 16 to 64 SMs, about 60 launches
 // and four waits.
+#include "explog64.cuh"
 #include "pf_internal.cuh"
 #include "pf_model.cuh"
 #include "resample_internal.cuh"
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
         s[3 * ld + i] = VY;
         double lw = cv_loglik(c, ox, oy, X, Y);
         if (t != 0)
-            lw = __dadd_rn(logeq ? *logeq : log(W[i]), lw);
+            lw = __dadd_rn(logeq ? *logeq : log_of_fraction(W[i]), lw);
         W[i] = lw;
         m = max(m, max_key(lw));
     }
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kB64) k_exp64(
     const double m = from_max_key(*key);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
-        W[i] = exp(W[i] - m);
+        W[i] = exp_of_negative(W[i] - m);
 }
 
 // where a step's results go

@@ -8,6 +8,7 @@
 // prefix maximum pm_j of the uniforms, F(cdf_i) = #{j : pm_j <= cdf_i} and
 // rep_i = F(cdf_i) - F(cdf_{i-1}); the last particle takes the rest.
 #include "common.cuh"
+#include "explog64.cuh"
 #include "rng_device.cuh"
 #include "scan.cuh"
 #include "seqsum.cuh"
@@ -515,13 +516,34 @@ __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
 }
 
 // U01SequenceSorted terms: -log(U_j) / (n - j), summed left to right below
-__global__ void __launch_bounds__(kB64) k_sorted_terms(
-    EngineState e, size_t n, double *t)
+// (a Philox block's four words, as in k_stratified_seq).
+__global__ void k_sorted_terms(EngineState e, size_t n, double *t)
 {
-    GRID_LOOP(j, n)
+    const uint64_t first = e.index;
+    const uint64_t nblk = (first + n + 3) / 4;
+    GRID_LOOP(b, nblk)
     {
-        const double U = u01_co_d(stream_word(e, j));
-        t[j] = -(log(U) / static_cast<double>(n - j));
+        uint32_t c[4] = {e.c[0], e.c[1], e.c[2], e.c[3]};
+        ctr32_add(c, b);
+        const u32x4 w = philox4x32_10(c[0], c[1], c[2], c[3], e.k0, e.k1);
+        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+        const uint64_t p0 = 4 * static_cast<uint64_t>(b);
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            // (past either end: not stored)
+            const uint64_t j = p0 + k - first;
+            const uint32_t d = j < n ? static_cast<uint32_t>(n - j) : 1u;
+            v[k] = ws[k] == 0 ? CUDART_INF : n64_neg_log_over(ws[k], d);
+        }
+        if (p0 >= first && p0 + 4 - first <= n) {
+            store4(t + (p0 - first), v);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (p0 + k >= first && p0 + k - first < n)
+                    t[p0 + k - first] = v[k];
+        }
     }
 }
 
@@ -535,15 +557,15 @@ __global__ void __launch_bounds__(kB64) k_sorted_terms_arr(
 // sums s.  They are non-decreasing up to exp's last bit: *unsorted is set
 // where two sums are within 2^-50 (exp is within an ulp, so a larger step
 // cannot be reversed).
-__global__ void __launch_bounds__(kB64) k_sorted_finish(
+__global__ void k_sorted_finish(
     size_t n, const double *s, double *u, uint32_t *unsorted)
 {
     GRID_LOOP(j, n)
     {
         const double sj = s[j];
-        if (unsorted && j > 0 && !(sj - s[j - 1] >= 0x1p-50))
+        if (unsorted && j > 0 && !n64_apart(n64_bits(sj), n64_bits(s[j - 1])))
             *unsorted = 1;
-        u[j] = 1.0 - exp(-sj);
+        u[j] = 1.0 - exp_of_negative(-sj);
     }
 }
 
@@ -995,8 +1017,8 @@ struct OpMaxD {
 };
 
 // The largest log-weight into *key (zero before).  Add: the log-weights are
-// log(W) + l first (add_log, weight.hpp:168-173), stored in W.  FP64 log is
-// the cost: 64-thread blocks, one integer atomic each.
+// log(W) + l first (add_log, weight.hpp:168-173), stored in W.  64-thread
+// blocks, one integer atomic each.
 template <bool Add>
 __global__ void __launch_bounds__(kB64) k_lw_max(
     size_t n, const double *l, double *W, unsigned long long *key)
@@ -1006,7 +1028,7 @@ __global__ void __launch_bounds__(kB64) k_lw_max(
     {
         double v = l[i];
         if (Add) {
-            v = __dadd_rn(log(W[i]), v);
+            v = __dadd_rn(log_of_fraction(W[i]), v);
             W[i] = v;
         }
         m = max(m, max_key(v));
@@ -1022,7 +1044,7 @@ __global__ void __launch_bounds__(kB64) k_exp_shift(
     size_t n, const double *lw, const unsigned long long *key, double *W)
 {
     const double m = from_max_key(*key);
-    GRID_LOOP(i, n) W[i] = exp(lw[i] - m);
+    GRID_LOOP(i, n) W[i] = exp_of_negative(lw[i] - m);
 }
 
 // the normalized weights, stored, and their squares as the terms to sum
@@ -1360,14 +1382,15 @@ int scheme_enqueue(size_t m, size_t n, const vsmc_cuda_rng &rng,
             k_systematic_seq<<<grid1(N), kB, 0, st>>>(es, N, log2n, u);
         } else {
             order = UniformOrder::Sorted;
-            double *t = scratch.get<double>(N);
+            double *t = scratch.get<double>(N + 4);
             if (t == nullptr)
                 return VSMC_CUDA_ERR_ALLOC;
-            k_sorted_terms<<<grid64(N), kB64, 0, st>>>(es, N, t);
+            t += es.index % 4; // as u
+            k_sorted_terms<<<grid1(N), kB, 0, st>>>(es, N, t);
             rc = seqsum_device(N, t, t, nullptr, err, scratch, st, true);
             if (rc != VSMC_CUDA_OK)
                 return rc;
-            k_sorted_finish<<<grid64(N), kB64, 0, st>>>(
+            k_sorted_finish<<<grid1(N), kB, 0, st>>>(
                 N, t, u, err + kErrUnsorted);
             k_running_max<<<1, 1024, 0, st>>>(N, u, err + kErrUnsorted);
         }
@@ -1559,7 +1582,7 @@ int vsmc_cuda_u01_sorted(size_t n, const double *u01, double *u01seq,
         int rc = seqsum_device(n, t, t, nullptr, err, sc, st, true);
         if (rc != VSMC_CUDA_OK)
             return rc;
-        k_sorted_finish<<<grid64(n), kB64, 0, st>>>(n, t, u01seq, nullptr);
+        k_sorted_finish<<<grid1(n), kB, 0, st>>>(n, t, u01seq, nullptr);
         VSMC_CUDA_CHECK_LAUNCH();
         return static_cast<int>(VSMC_CUDA_OK);
     });
