@@ -6,6 +6,7 @@
 // the reference (rng/philox.hpp:76-101, rng/threefry.hpp:71-146).
 #pragma once
 
+#include <type_traits>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -33,6 +34,39 @@ void set_last_cuda_error(cudaError_t e);
     } while (0)
 
 #define VSMC_CUDA_CHECK_LAUNCH() VSMC_CUDA_TRY(cudaGetLastError())
+
+// A kernel that may be set up while the one before it in the stream still runs
+// (programmatic dependent launch): it begins with pdl_begin(), which lets the
+// next one be set up and then waits until everything before has completed and
+// its writes are visible.  For chains of short kernels: set_log of 2^20 weights
+// (8 kernels) takes 110 us instead of 121, the FP64 filter's step (7) 62
+// instead of 67.  The batched filters' captured steps are slower with it (the
+// next kernel's waiting blocks take places of the running one's: 2.57 ms
+// instead of 2.49 for 64 learned filters) and are launched plainly.
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid,
+    dim3 block, size_t smem, cudaStream_t st, const Args &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel,
+        static_cast<std::remove_cv_t<std::remove_reference_t<Params>>>(
+            args)...);
+}
+
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
     uint32_t t, uint32_t seed, CvConst<double> c, const double *obs,
     double *s, double *W, const double *logeq, unsigned long long *key)
 {
+    pdl_begin();
     const double ox = obs[2 * t + 0], oy = obs[2 * t + 1];
     unsigned long long m = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
 __global__ void __launch_bounds__(kB64) k_exp64(
     uint32_t n, double *W, const unsigned long long *key)
 {
+    pdl_begin();
     const double m = from_max_key(*key);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x)
@@ -154,6 +156,7 @@ __device__ __forceinline__ void step64_record(
 
 __global__ void k_record64(const Step64 a)
 {
+    pdl_begin();
     if (threadIdx.x == 0 && blockIdx.x == 0)
         step64_record(a, a.scal[4], a.scal[5]);
 }
@@ -163,6 +166,7 @@ __global__ void k_record64(const Step64 a)
 __global__ void __launch_bounds__(kSeqBlock) k_weigh64(
     SeqArgs q, const Step64 a)
 {
+    pdl_begin();
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     SeqClusterSmem &S = seq_cluster_smem(q);
@@ -225,6 +229,7 @@ __global__ void __launch_bounds__(kSeqBlock) k_weigh64(
 __global__ void __launch_bounds__(kSelB) k_select64(
     const Step64 a, double *state, const int *idx, double *part)
 {
+    pdl_begin();
     __shared__ double sh[kSelB / 32 + 1];
     __shared__ bool last;
     const double w = a.scal[2];
@@ -361,7 +366,7 @@ static int weigh_large(vsmc_cuda_pf *pf, const Step64 &a)
     int rc = weight_sums(q, a.W, a.W, p->scal + 5, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    k_record64<<<1, 32, 0, st>>>(a);
+    launch_after(k_record64, 1, 32, 0, st, a);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -403,9 +408,10 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
             cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
     }
     const CvConst<double> c = make_cv_const<double>(pf->model);
-    k_move64<<<grid64(n), kB64, 0, st>>>(a.n, static_cast<uint32_t>(a.ld), t,
+    launch_after(k_move64, grid64(n), kB64, 0, st, a.n,
+        static_cast<uint32_t>(a.ld), t,
         pf->seed, c, pf->obs, S, a.W, p->equal ? p->scal + 3 : nullptr, a.key);
-    k_exp64<<<grid64(n), kB64, 0, st>>>(a.n, a.W, a.key);
+    launch_after(k_exp64, grid64(n), kB64, 0, st, a.n, a.W, a.key);
     VSMC_CUDA_CHECK_LAUNCH();
     int rc = small ? seq_cluster_launch(k_weigh64, p->seq, st, a)
                    : weigh_large(pf, a);
@@ -430,7 +436,8 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
         rc = rep_index_device(n, n, p->rep, p->idx, p->err, scratch, st);
         if (rc != VSMC_CUDA_OK)
             return rc;
-        k_select64<<<select_grid(n), kSelB, 0, st>>>(a, S, p->idx, p->part);
+        launch_after(k_select64, select_grid(n), kSelB, 0, st, a, S,
+            p->idx, p->part);
         VSMC_CUDA_CHECK_LAUNCH();
         p->equal = true;
         p->pending = true;

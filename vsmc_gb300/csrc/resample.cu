@@ -456,6 +456,7 @@ __device__ __forceinline__ double mul_u32(
 // u - first is 32-byte aligned, so a block's four uniforms are one store.
 __global__ void k_stratified_seq(EngineState e, size_t n, int log2n, double *u)
 {
+    pdl_begin();
     const double delta = 1.0 / static_cast<double>(n);
     const double d32 = delta * 0x1p-32;
     const double m52 = -0x1p52 * delta, m20 = -0x1p20 * delta;
@@ -502,6 +503,7 @@ __global__ void k_stratified_seq(EngineState e, size_t n, int log2n, double *u)
 // every operation is monotone in j
 __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
 {
+    pdl_begin();
     const uint32_t w0 = stream_word(e, 0);
     if (log2n >= 0) {
         GRID_LOOP(j, n)
@@ -519,6 +521,7 @@ __global__ void k_systematic_seq(EngineState e, size_t n, int log2n, double *u)
 // (a Philox block's four words, as in k_stratified_seq).
 __global__ void k_sorted_terms(EngineState e, size_t n, double *t)
 {
+    pdl_begin();
     const uint64_t first = e.index;
     const uint64_t nblk = (first + n + 3) / 4;
     GRID_LOOP(b, nblk)
@@ -560,6 +563,7 @@ __global__ void __launch_bounds__(kB64) k_sorted_terms_arr(
 __global__ void k_sorted_finish(
     size_t n, const double *s, double *u, uint32_t *unsorted)
 {
+    pdl_begin();
     GRID_LOOP(j, n)
     {
         const double sj = s[j];
@@ -574,6 +578,7 @@ __global__ void k_sorted_finish(
 __global__ void __launch_bounds__(1024) k_running_max(
     size_t n, double *u, uint32_t *unsorted)
 {
+    pdl_begin();
     if (*unsorted == 0)
         return;
     long long carry = 0;
@@ -837,6 +842,7 @@ __device__ __forceinline__ void slot_range(
 
 __global__ void __launch_bounds__(kSeqBlock) k_slots_count(const SlotArgs a)
 {
+    pdl_begin();
     uint32_t t0, t1;
     slot_range(a, t0, t1);
     ES acc = {0, 0, 0};
@@ -884,6 +890,7 @@ __global__ void __launch_bounds__(kSeqBlock) k_slots_count(const SlotArgs a)
 
 __global__ void __launch_bounds__(kSeqBlock) k_slots_assign(const SlotArgs a)
 {
+    pdl_begin();
     if (*a.err & DEV_ERR_COUNTS)
         return;
     uint32_t t0, t1;
@@ -902,6 +909,7 @@ __global__ void __launch_bounds__(kSeqBlock) k_slots_assign(const SlotArgs a)
 
 __global__ void __launch_bounds__(kB) k_slots_decode(const SlotArgs a)
 {
+    pdl_begin();
     if (*a.err & DEV_ERR_COUNTS)
         return;
     GRID_LOOP(i, a.n)
@@ -916,6 +924,7 @@ __global__ void __launch_bounds__(kB) k_slots_decode(const SlotArgs a)
 __global__ void __launch_bounds__(kSeqBlock) k_slots_small(
     SeqArgs, const SlotArgs a)
 {
+    pdl_begin();
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     __shared__ ES s_tot;
@@ -972,6 +981,7 @@ __global__ void k_hist(size_t m, size_t n, const int *idx, int *rep,
 
 __global__ void k_check_fixed_points(size_t n, const int *idx, uint32_t *err)
 {
+    pdl_begin();
     GRID_LOOP(d, n)
     {
         const int s = idx[d];
@@ -984,6 +994,7 @@ template <typename T>
 __global__ void k_copy_state(size_t n, size_t dim, size_t ld, const int *idx,
     T *state, const uint32_t *err)
 {
+    pdl_begin();
     if (*err)
         return;
     GRID_LOOP(d, n)
@@ -1023,6 +1034,7 @@ template <bool Add>
 __global__ void __launch_bounds__(kB64) k_lw_max(
     size_t n, const double *l, double *W, unsigned long long *key)
 {
+    pdl_begin();
     unsigned long long m = 0;
     GRID_LOOP(i, n)
     {
@@ -1043,6 +1055,7 @@ __global__ void __launch_bounds__(kB64) k_lw_max(
 __global__ void __launch_bounds__(kB64) k_exp_shift(
     size_t n, const double *lw, const unsigned long long *key, double *W)
 {
+    pdl_begin();
     const double m = from_max_key(*key);
     GRID_LOOP(i, n) W[i] = exp_of_negative(lw[i] - m);
 }
@@ -1073,6 +1086,7 @@ struct SquareLoad {
 __global__ void __launch_bounds__(kSeqBlock) k_normalize_small(
     SeqArgs a, const double *v, double *W, double *ess)
 {
+    pdl_begin();
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     SeqClusterSmem &S = seq_cluster_smem(a);
@@ -1112,6 +1126,7 @@ template <typename T>
 __global__ void __launch_bounds__(kB) k_wsum(size_t n, size_t dim, size_t ld,
     const T *state, const double *W, double *part)
 {
+    pdl_begin();
     constexpr int kD = 4;
     __shared__ double sh[kB / 32 + 1];
     for (size_t d0 = 0; d0 < dim; d0 += kD) {
@@ -1138,6 +1153,7 @@ __global__ void __launch_bounds__(kB) k_wsum(size_t n, size_t dim, size_t ld,
 __global__ void __launch_bounds__(kB) k_wsum_final(
     int nb, const double *part, double *out)
 {
+    pdl_begin();
     __shared__ double sh[kB / 32 + 1];
     double s = 0;
     for (int b = threadIdx.x; b < nb; b += kB)
@@ -1247,9 +1263,9 @@ static int rep_index_square(size_t n, const int *rep, int *idx, uint32_t *err,
     a.E = scratch.get<uint32_t>(a.blocks + 1);
     if (!a.S || !a.E)
         return VSMC_CUDA_ERR_ALLOC;
-    k_slots_count<<<a.blocks, kSeqBlock, 0, st>>>(a);
-    k_slots_assign<<<a.blocks, kSeqBlock, 0, st>>>(a);
-    k_slots_decode<<<grid1(n), kB, 0, st>>>(a);
+    launch_after(k_slots_count, a.blocks, kSeqBlock, 0, st, a);
+    launch_after(k_slots_assign, a.blocks, kSeqBlock, 0, st, a);
+    launch_after(k_slots_decode, grid1(n), kB, 0, st, a);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1377,22 +1393,25 @@ int scheme_enqueue(size_t m, size_t n, const vsmc_cuda_rng &rng,
     UniformOrder order = UniformOrder::Near;
     if (N > 0) {
         if (base == VSMC_CUDA_STRATIFIED) {
-            k_stratified_seq<<<grid1(N), kB, 0, st>>>(es, N, log2n, u);
+            launch_after(k_stratified_seq, grid1(N), kB, 0, st, es, N, log2n,
+                u);
         } else if (base == VSMC_CUDA_SYSTEMATIC) {
-            k_systematic_seq<<<grid1(N), kB, 0, st>>>(es, N, log2n, u);
+            launch_after(k_systematic_seq, grid1(N), kB, 0, st, es, N, log2n,
+                u);
         } else {
             order = UniformOrder::Sorted;
             double *t = scratch.get<double>(N + 4);
             if (t == nullptr)
                 return VSMC_CUDA_ERR_ALLOC;
             t += es.index % 4; // as u
-            k_sorted_terms<<<grid1(N), kB, 0, st>>>(es, N, t);
+            launch_after(k_sorted_terms, grid1(N), kB, 0, st, es, N, t);
             rc = seqsum_device(N, t, t, nullptr, err, scratch, st, true);
             if (rc != VSMC_CUDA_OK)
                 return rc;
-            k_sorted_finish<<<grid1(N), kB, 0, st>>>(
-                N, t, u, err + kErrUnsorted);
-            k_running_max<<<1, 1024, 0, st>>>(N, u, err + kErrUnsorted);
+            launch_after(k_sorted_finish, grid1(N), kB, 0, st, N, t, u,
+                err + kErrUnsorted);
+            launch_after(k_running_max, 1, 1024, 0, st, N, u,
+                err + kErrUnsorted);
         }
         VSMC_CUDA_CHECK_LAUNCH();
     }
@@ -1471,8 +1490,9 @@ unsigned long long *max_word(uint32_t *err)
 int weight_set_log_device(size_t n, const double *lw, double *W,
     double *ess_dev, uint32_t *err, Scratch &scratch, cudaStream_t st)
 {
-    k_lw_max<false><<<grid64(n), kB64, 0, st>>>(n, lw, nullptr, max_word(err));
-    k_exp_shift<<<grid64(n), kB64, 0, st>>>(n, lw, max_word(err), W);
+    launch_after(k_lw_max<false>, grid64(n), kB64, 0, st, n, lw, nullptr,
+        max_word(err));
+    launch_after(k_exp_shift, grid64(n), kB64, 0, st, n, lw, max_word(err), W);
     VSMC_CUDA_CHECK_LAUNCH();
     return weight_normalize_device(n, W, W, ess_dev, err, scratch, st);
 }
@@ -1488,8 +1508,9 @@ int weight_set_equal_device(size_t n, double *W, double *ess_dev,
 int weight_add_log_device(size_t n, const double *l, double *W,
     double *ess_dev, uint32_t *err, Scratch &scratch, cudaStream_t st)
 {
-    k_lw_max<true><<<grid64(n), kB64, 0, st>>>(n, l, W, max_word(err));
-    k_exp_shift<<<grid64(n), kB64, 0, st>>>(n, W, max_word(err), W);
+    launch_after(k_lw_max<true>, grid64(n), kB64, 0, st, n, l, W,
+        max_word(err));
+    launch_after(k_exp_shift, grid64(n), kB64, 0, st, n, W, max_word(err), W);
     VSMC_CUDA_CHECK_LAUNCH();
     return weight_normalize_device(n, W, W, ess_dev, err, scratch, st);
 }
@@ -1502,10 +1523,10 @@ int monitor_mean_device(size_t n, size_t dim, size_t ld, const T *state,
     double *part = scratch.get<double>(dim * nb);
     if (part == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
-    k_wsum<T><<<nb, kB, 0, st>>>(n, dim, ld, state, W, part);
+    launch_after(k_wsum<T>, nb, kB, 0, st, n, dim, ld, state, W, part);
     if (dim)
-        k_wsum_final<<<static_cast<unsigned>(dim), kB, 0, st>>>(
-            nb, part, out);
+        launch_after(k_wsum_final, static_cast<unsigned>(dim), kB, 0, st, nb,
+            part, out);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1519,8 +1540,9 @@ template <typename T>
 int state_copy_device(size_t n, size_t dim, size_t ld, const int *idx,
     T *state, uint32_t *err, cudaStream_t st)
 {
-    k_check_fixed_points<<<grid1(n), kB, 0, st>>>(n, idx, err);
-    k_copy_state<T><<<grid1(n), kB, 0, st>>>(n, dim, ld, idx, state, err);
+    launch_after(k_check_fixed_points, grid1(n), kB, 0, st, n, idx, err);
+    launch_after(k_copy_state<T>, grid1(n), kB, 0, st, n, dim, ld, idx, state,
+        err);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1582,7 +1604,8 @@ int vsmc_cuda_u01_sorted(size_t n, const double *u01, double *u01seq,
         int rc = seqsum_device(n, t, t, nullptr, err, sc, st, true);
         if (rc != VSMC_CUDA_OK)
             return rc;
-        k_sorted_finish<<<grid1(n), kB, 0, st>>>(n, t, u01seq, nullptr);
+        launch_after(k_sorted_finish, grid1(n), kB, 0, st, n, t, u01seq,
+            nullptr);
         VSMC_CUDA_CHECK_LAUNCH();
         return static_cast<int>(VSMC_CUDA_OK);
     });

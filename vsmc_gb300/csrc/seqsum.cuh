@@ -821,6 +821,7 @@ template <class Load>
 __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_sums(
     const SeqArgs a, const Load load)
 {
+    pdl_begin();
     __shared__ SeqSmem sh;
     uint32_t t0, t1;
     seq_range(a, t0, t1);
@@ -853,6 +854,7 @@ template <class Load>
 __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_classify(
     const SeqArgs a, const Load load)
 {
+    pdl_begin();
     __shared__ SeqSmem sh;
     uint32_t t0, t1;
     seq_range(a, t0, t1);
@@ -905,6 +907,7 @@ template <class Load, class Out>
 __global__ void __launch_bounds__(kSeqBlock, kSeqOcc) k_seq_out(
     const SeqArgs a, const Load load, const Out out)
 {
+    pdl_begin();
     __shared__ SeqSmem sh;
     uint32_t t0, t1;
     seq_range(a, t0, t1);
@@ -1083,6 +1086,7 @@ template <class Load, class Out>
 __global__ void __launch_bounds__(kSeqBlock) k_seq_small(
     SeqArgs a, const Load load, const Out out)
 {
+    pdl_begin();
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     SeqClusterSmem &S = seq_cluster_smem(a);
@@ -1163,13 +1167,15 @@ int seq_cluster_launch(void (*kernel)(SeqArgs, Params...), const SeqArgs &a,
     cfg.blockDim = dim3(kSeqBlock);
     cfg.dynamicSmemBytes = sizeof(SeqClusterSmem);
     cfg.stream = st;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = c;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1; // as launch_after
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     VSMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a,
         static_cast<std::remove_cv_t<std::remove_reference_t<Params>>>(
             args)...));
@@ -1189,8 +1195,8 @@ template <class Sums, class Load>
 int seq_total_large(const SeqArgs &a, const Sums &sums, const Load &load,
     cudaStream_t st)
 {
-    k_seq_sums<Sums><<<a.blocks, kSeqBlock, 0, st>>>(a, sums);
-    k_seq_classify<Load><<<a.blocks, kSeqBlock, 0, st>>>(a, load);
+    launch_after(k_seq_sums<Sums>, a.blocks, kSeqBlock, 0, st, a, sums);
+    launch_after(k_seq_classify<Load>, a.blocks, kSeqBlock, 0, st, a, load);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -1214,7 +1220,8 @@ int seq_scan(const SeqArgs &a, const Load &load, const Out &out,
     const int rc = seq_total(a, load, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    k_seq_out<Load, Out><<<a.blocks, kSeqBlock, 0, st>>>(a, load, out);
+    launch_after(k_seq_out<Load, Out>, a.blocks, kSeqBlock, 0, st, a, load,
+        out);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
