@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "explog64.cuh"
 #include "normal64.cuh"
 
 #include <math_constants.h>
@@ -508,13 +509,13 @@ struct StudentTScalar {
         if (alg == 0) {
             for (; tries < kGammaMaxTries; ++tries) {
                 double u = eng.u01d();
-                double e = -log(eng.u01d());
+                double e = -log_of_fraction(eng.u01d());
                 if (u > d) {
                     u = -log(__dmul_rn(c, 1 - u));
                     e = __dadd_rn(e, u);
                     u = __dadd_rn(d, __dmul_rn(alpha, u));
                 }
-                const double x = exp(__dmul_rn(c, log(u)));
+                const double x = exp_of_negative(__dmul_rn(c, log(u)));
                 if (fabs(x) < e) {
                     r = x;
                     break;
@@ -522,9 +523,9 @@ struct StudentTScalar {
             }
         } else if (alg == 1) {
             for (; tries < kGammaMaxTries; ++tries) {
-                const double u = -log(eng.u01d());
-                const double e = -log(eng.u01d());
-                const double x = exp(__dmul_rn(c, log(u)));
+                const double u = -log_of_fraction(eng.u01d());
+                const double e = -log_of_fraction(eng.u01d());
+                const double x = exp_of_negative(__dmul_rn(c, log(u)));
                 if (!(__dadd_rn(u, e) < __dadd_rn(d, x))) {
                     r = x;
                     break;
@@ -555,13 +556,13 @@ struct StudentTScalar {
                 }
                 e = __dadd_rn(w2 / 2,
                     __dmul_rn(d, __dadd_rn(__dadd_rn(1.0, -v), log(v))));
-                if (log(u) < e) {
+                if (log_of_fraction(u) < e) {
                     r = __dmul_rn(d, v);
                     break;
                 }
             }
         } else {
-            r = -log(eng.u01d());
+            r = -log_of_fraction(eng.u01d());
         }
         if (tries >= kGammaMaxTries)
             err |= DEV_ERR_BOUND;
