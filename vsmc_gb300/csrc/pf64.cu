@@ -150,8 +150,9 @@ __device__ __forceinline__ void step64_record(
     a.h_res[a.t] = res ? 1 : 0;
     *a.key = 0; // for the next step's maximum
     a.host->err = atomicOr(a.err, 0u);
+    // (the host reads these after waiting for the stream: no fence, which took
+    // a microsecond of the step)
     a.host->resample = res ? 1 : 0;
-    __threadfence_system();
 }
 
 __global__ void k_record64(const Step64 a)
@@ -280,7 +281,6 @@ __global__ void __launch_bounds__(kSelB) k_select64(
         a.err[kErrTicket] = 0;
         a.host->tail = a.err[kErrTail];
         a.host->err = atomicOr(a.err, 0u);
-        __threadfence_system();
     }
 }
 
