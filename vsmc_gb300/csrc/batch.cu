@@ -633,9 +633,8 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_batch_step(
 }
 
 // A learned segment is up to 1024 particles: 8 tiles of 128, 32 particles a
-// warp.  The block's 8 warps evaluate 2 tiles at a time; then 4 warps take
-// the sums, each lane over its particle of tile after tile.
-constexpr int kLearnBlock = 256;
+// warp.  A block of 8 warps evaluates 2 tiles at a time, one of 4 warps one;
+// then 4 warps take the sums, each lane over its particle of tile after tile.
 constexpr uint32_t kLearnTile = 128;
 constexpr uint32_t kLearnSeg = 1024u / kLearnTile; // tiles of a segment
 
@@ -644,16 +643,20 @@ constexpr uint32_t kLearnSeg = 1024u / kLearnTile; // tiles of a segment
 // filters of 4096 particles (256 segments) left an SM 8 warps, each with
 // eight evaluations in turn.  Two blocks of 8 warps, four tiles each,
 // take the 50 steps (resampling included) from 3.06 to 2.45 ms; one block of
-// 16 took 2.81, two of 16 (64 registers) 2.56.  Each warp evaluates the
+// 16 took 2.81, two of 16 (64 registers) 2.56.  With more segments than those
+// blocks (two an SM) hold at once the SMs are full either way and four blocks
+// of 4 warps lose less at the segments' ends: 20 steps of 128 filters of 4096
+// take 1.43 ms against 1.56, of 1024 7.36 against 7.77; of 64 1.27 against
+// 1.00 (step_shape).  Each warp evaluates the
 // proposal network for 32 particles on the tensor cores (two 16-row tiles
 // sharing the weight loads); lane 4g + q then moves particle g + 8q of the
 // warp's 32.
-template <bool First>
-__global__ void __launch_bounds__(kLearnBlock, 2) k_batch_step_learned(
+template <bool First, int kBlock>
+__global__ void __launch_bounds__(kBlock, 512 / kBlock) k_batch_step_learned(
     const BatchArgs a)
 {
     constexpr int kW = 4; // warps that take the sums
-    constexpr int kLast = kLearnBlock / 32 - 1;
+    constexpr int kLast = kBlock / 32 - 1;
     __shared__ __align__(16) uint32_t sp[kPackedWords];
     const uint32_t t = *a.step;
     const uint32_t nseg = t <= a.tmax ? a.active[t] : 0u;
@@ -696,7 +699,7 @@ __global__ void __launch_bounds__(kLearnBlock, 2) k_batch_step_learned(
         const uint32_t i00 = (meta.tile - F.tile0) * kLearnTile;
         bool written = false;
         for (uint32_t p = wid / kW; p < meta.count;
-             p += kLearnBlock / 128) {
+             p += kBlock / 128) {
             // slot of the segment: tile p, the lane's particle in it
             const uint32_t slot_i = p * kLearnTile + 32 * (wid % kW) + lane;
             const uint32_t i =
@@ -1120,16 +1123,23 @@ static cudaError_t launch_step_t(int kind, bool first, int grid,
         : launch_step_k<kBlock, kPPT, kKindBearings>(first, grid, a, st);
 }
 
+template <int kBlock>
+static cudaError_t launch_learned(
+    bool first, int grid, const BatchArgs &a, cudaStream_t st)
+{
+    if (first)
+        k_batch_step_learned<true, kBlock><<<grid, kBlock, 0, st>>>(a);
+    else
+        k_batch_step_learned<false, kBlock><<<grid, kBlock, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
 static cudaError_t launch_step(int kind, Shape s, bool first, int grid,
     const BatchArgs &a, cudaStream_t st)
 {
-    if (kind == kKindLearned) {
-        if (first)
-            k_batch_step_learned<true><<<grid, kLearnBlock, 0, st>>>(a);
-        else
-            k_batch_step_learned<false><<<grid, kLearnBlock, 0, st>>>(a);
-        return cudaGetLastError();
-    }
+    if (kind == kKindLearned)
+        return s.block == 128 ? launch_learned<128>(first, grid, a, st)
+                              : launch_learned<256>(first, grid, a, st);
     if (s.block == 128) {
         if (s.ppt == 1)
             return launch_step_t<128, 1>(kind, first, grid, a, st);
@@ -1167,7 +1177,9 @@ static int occupancy_t(int kind)
 static int occupancy(int kind, Shape s)
 {
     if (kind == kKindLearned)
-        return occupancy_of(k_batch_step_learned<false>, kLearnBlock);
+        return s.block == 128
+            ? occupancy_of(k_batch_step_learned<false, 128>, 128)
+            : occupancy_of(k_batch_step_learned<false, 256>, 256);
     if (s.block == 128)
         return s.ppt == 1 ? occupancy_t<128, 1>(kind)
                           : (s.ppt == 2 ? occupancy_t<128, 2>(kind)
@@ -1306,6 +1318,17 @@ static int batch_layout(vsmc_cuda_batch *b, Shape s)
     return VSMC_CUDA_OK;
 }
 
+// The step kernel's shape: the tiles', and for learned filters the block that
+// suits their number of segments (see k_batch_step_learned).
+static Shape step_shape(const vsmc_cuda_batch *b)
+{
+    Shape s = b->shape;
+    if (b->kind == kKindLearned)
+        s.block = b->segs.size() <= 2 * static_cast<size_t>(num_sms()) ? 256
+                                                                       : 128;
+    return s;
+}
+
 static BatchArgs batch_args(vsmc_cuda_batch *b, const double *obs, int cur)
 {
     BatchArgs a = {};
@@ -1367,7 +1390,7 @@ static int enqueue_run(
     VSMC_CUDA_CHECK_LAUNCH();
     for (int t = 0; t < nsteps; ++t) {
         const BatchArgs a = batch_args(b, obs, t & 1);
-        VSMC_CUDA_TRY(launch_step(b->kind, b->shape, t == 0, grid, a, st));
+        VSMC_CUDA_TRY(launch_step(b->kind, step_shape(b), t == 0, grid, a, st));
         // the filters that resample, in the units the step listed
         const dim3 blk(kPfBlock);
         k_brs_qsum<<<b->rs_grid[0], blk, 0, st>>>(a);
@@ -1655,7 +1678,7 @@ int vsmc_cuda_batch_run_device(vsmc_cuda_batch *b, const double *obs_dev)
             cudaGraphExecDestroy(b->graph);
             b->graph = nullptr;
         }
-        const int grid = num_sms() * occupancy(b->kind, b->shape);
+        const int grid = num_sms() * occupancy(b->kind, step_shape(b));
         VSMC_CUDA_TRY(cudaStreamBeginCapture(
             b->stream, cudaStreamCaptureModeThreadLocal));
         const int rc = enqueue_run(b, obs_dev, nsteps, grid);
@@ -1771,7 +1794,7 @@ int vsmc_cuda_batch_get_schedule(vsmc_cuda_batch *b, uint32_t *min_chunk)
 static int time_steps(vsmc_cuda_batch *b, const double *obs_dev, int nsteps,
     cudaEvent_t e0, cudaEvent_t e1, float *ms)
 {
-    const int grid = num_sms() * occupancy(b->kind, b->shape);
+    const int grid = num_sms() * occupancy(b->kind, step_shape(b));
     int rc = enqueue_run(b, obs_dev, nsteps, grid); // warm-up
     if (rc != VSMC_CUDA_OK)
         return rc;
@@ -1844,7 +1867,7 @@ int vsmc_cuda_batch_autotune(vsmc_cuda_batch *b, const double *obs_dev,
         rc = batch_layout(b, kShapes[k]);
         if (rc != VSMC_CUDA_OK)
             break;
-        const int grid = num_sms() * occupancy(b->kind, b->shape);
+        const int grid = num_sms() * occupancy(b->kind, step_shape(b));
         rc = enqueue_run(b, obs_dev, nsteps, grid); // warm-up
         if (rc != VSMC_CUDA_OK)
             break;
