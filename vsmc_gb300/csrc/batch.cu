@@ -473,6 +473,7 @@ template <int kBlock, int kPPT, bool First, int Kind>
 __global__ void __launch_bounds__(kBlock, 1024 / kBlock) k_batch_step(
     const BatchArgs a)
 {
+    pdl_wait();
     constexpr uint32_t kTile = kBlock * kPPT;
     constexpr int kW = kBlock / 32;
     const uint32_t t = *a.step;
@@ -655,6 +656,7 @@ template <bool First, int kBlock>
 __global__ void __launch_bounds__(kBlock, 512 / kBlock) k_batch_step_learned(
     const BatchArgs a)
 {
+    pdl_wait();
     constexpr int kW = 4; // warps that take the sums
     constexpr int kLast = kBlock / 32 - 1;
     __shared__ __align__(16) uint32_t sp[kPackedWords];
@@ -929,6 +931,7 @@ __device__ __forceinline__ uint64_t rs_prefix(uint64_t *v, uint32_t nu)
 // (every step kernel block has read it) and empties the next step's list.
 __global__ void __launch_bounds__(kPfBlock, 4) k_brs_qsum(const BatchArgs a)
 {
+    pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(a.step, 1u);
         a.rs_count[a.rpar ^ 1u] = 0;
@@ -957,6 +960,7 @@ __global__ void __launch_bounds__(kPfBlock, 4) k_brs_qsum(const BatchArgs a)
 template <bool Sys>
 __global__ void __launch_bounds__(kPfBlock, 3) k_brs_count(const BatchArgs a)
 {
+    pdl_wait();
     __shared__ uint4 rows[Sys ? 1 : kPfBlock / 32][Sys ? 1 : kStratRow];
     RS_UNITS(a, v, count)
     {
@@ -999,6 +1003,7 @@ __global__ void __launch_bounds__(kPfBlock, 3) k_brs_count(const BatchArgs a)
 // pass 3: slot assignment (assign_range)
 __global__ void __launch_bounds__(kPfBlock, 4) k_brs_assign(const BatchArgs a)
 {
+    pdl_wait();
     __shared__ __align__(16) uint32_t shm[kPfBlock / 32][kRunChunk];
     RS_UNITS(a, v, count)
     {
@@ -1108,9 +1113,11 @@ static cudaError_t launch_step_k(bool first, int grid, const BatchArgs &a,
     cudaStream_t st)
 {
     if (first)
-        k_batch_step<kBlock, kPPT, true, Kind><<<grid, kBlock, 0, st>>>(a);
+        launch_after(k_batch_step<kBlock, kPPT, true, Kind>, grid, kBlock, 0,
+            st, a);
     else
-        k_batch_step<kBlock, kPPT, false, Kind><<<grid, kBlock, 0, st>>>(a);
+        launch_after(k_batch_step<kBlock, kPPT, false, Kind>, grid, kBlock, 0,
+            st, a);
     return cudaGetLastError();
 }
 
@@ -1128,9 +1135,11 @@ static cudaError_t launch_learned(
     bool first, int grid, const BatchArgs &a, cudaStream_t st)
 {
     if (first)
-        k_batch_step_learned<true, kBlock><<<grid, kBlock, 0, st>>>(a);
+        launch_after(k_batch_step_learned<true, kBlock>, grid, kBlock, 0, st,
+            a);
     else
-        k_batch_step_learned<false, kBlock><<<grid, kBlock, 0, st>>>(a);
+        launch_after(k_batch_step_learned<false, kBlock>, grid, kBlock, 0, st,
+            a);
     return cudaGetLastError();
 }
 
@@ -1393,12 +1402,12 @@ static int enqueue_run(
         VSMC_CUDA_TRY(launch_step(b->kind, step_shape(b), t == 0, grid, a, st));
         // the filters that resample, in the units the step listed
         const dim3 blk(kPfBlock);
-        k_brs_qsum<<<b->rs_grid[0], blk, 0, st>>>(a);
+        launch_after(k_brs_qsum, b->rs_grid[0], blk, 0, st, a);
         if (a.scheme == VSMC_CUDA_SYSTEMATIC)
-            k_brs_count<true><<<b->rs_grid[1], blk, 0, st>>>(a);
+            launch_after(k_brs_count<true>, b->rs_grid[1], blk, 0, st, a);
         else
-            k_brs_count<false><<<b->rs_grid[1], blk, 0, st>>>(a);
-        k_brs_assign<<<b->rs_grid[2], blk, 0, st>>>(a);
+            launch_after(k_brs_count<false>, b->rs_grid[1], blk, 0, st, a);
+        launch_after(k_brs_assign, b->rs_grid[2], blk, 0, st, a);
         VSMC_CUDA_CHECK_LAUNCH();
     }
     return VSMC_CUDA_OK;

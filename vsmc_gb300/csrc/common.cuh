@@ -36,13 +36,16 @@ void set_last_cuda_error(cudaError_t e);
 #define VSMC_CUDA_CHECK_LAUNCH() VSMC_CUDA_TRY(cudaGetLastError())
 
 // A kernel that may be set up while the one before it in the stream still runs
-// (programmatic dependent launch): it begins with pdl_begin(), which lets the
-// next one be set up and then waits until everything before has completed and
-// its writes are visible.  For chains of short kernels: set_log of 2^20 weights
-// (8 kernels) takes 110 us instead of 121, the FP64 filter's step (7) 62
-// instead of 67.  The batched filters' captured steps are slower with it (the
-// next kernel's waiting blocks take places of the running one's: 2.57 ms
-// instead of 2.49 for 64 learned filters) and are launched plainly.
+// (programmatic dependent launch).  It begins with pdl_wait(), which waits
+// until everything before has completed and its writes are visible, or with
+// pdl_begin(), which also lets the next one be set up from the start on.
+// For chains of short kernels from the start on: set_log of 2^20 weights (8
+// kernels) takes 110 us instead of 121, the FP64 filter's step (7) 62 instead
+// of 67.  In the batched filters' captured steps the next kernel's waiting
+// blocks would take places of the running one's (64 learned filters of 4096,
+// 20 steps: 1043 us, 1007 with plain launches); set up as the blocks of the one
+// before leave, they take 990, and 512 filters of 512 to 1024 particles 1238
+// instead of 1265.
 template <class... Params, class... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid,
     dim3 block, size_t smem, cudaStream_t st, const Args &...args)
@@ -62,10 +65,15 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid,
             args)...);
 }
 
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void pdl_begin()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
 }
 
 inline cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
