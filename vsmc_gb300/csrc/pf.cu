@@ -125,7 +125,7 @@ static void launch_resample32(
 {
     const Rs32Args r = make_rs_args32(pf, mon_state, force, with_mon);
     cudaStream_t st = pf->stream;
-    k_rs32_qsum<<<pf->grid_rs, kPfBlock, 0, st>>>(r);
+    launch_after(k_rs32_qsum, pf->grid_rs, kPfBlock, 0, st, r);
     launch_rs32_count(pf->grid_rs, st, r);
     launch_rs32_assign(pf->grid_rs, st, r);
 }
@@ -896,7 +896,7 @@ int vsmc_cuda_resample_fixed(size_t n, const uint64_t *q, int scheme,
         static_cast<uint32_t>(rng->key[1]), static_cast<uint32_t>(rng->ctr[0]),
         static_cast<uint32_t>(rng->ctr[1]), static_cast<uint32_t>(rng->ctr[2]),
         static_cast<uint32_t>(rng->ctr[3]), rng->index);
-    k_rs32_qsum<<<grid, kPfBlock, 0, st>>>(r);
+    launch_after(k_rs32_qsum, grid, kPfBlock, 0, st, r);
     launch_rs32_count(grid, st, r);
     launch_rs32_assign(grid, st, r);
     VSMC_CUDA_CHECK_LAUNCH();
@@ -1318,7 +1318,7 @@ extern "C" int vsmc_cuda_resample_fixed_noalloc(size_t n, const uint64_t *q,
         static_cast<uint32_t>(rng->ctr[1]), static_cast<uint32_t>(rng->ctr[2]),
         static_cast<uint32_t>(rng->ctr[3]), rng->index);
     const int g = static_cast<int>(grid);
-    k_rs32_qsum<<<g, kPfBlock, 0, st>>>(r);
+    launch_after(k_rs32_qsum, g, kPfBlock, 0, st, r);
     launch_rs32_count(g, st, r);
     launch_rs32_assign(g, st, r);
     VSMC_CUDA_CHECK_LAUNCH();

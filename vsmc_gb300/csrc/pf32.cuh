@@ -394,6 +394,7 @@ __device__ __forceinline__ T scan_blocks_in_place(T *v, uint32_t m, T *sh)
 __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_qsum(
     const Rs32Args a)
 {
+    pdl_begin();
     if (!(a.force || a.sc->resampled))
         return;
     if (a.force && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -451,6 +452,7 @@ template <bool Sys>
 __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_count(
     const Rs32Args a)
 {
+    pdl_begin();
     if (!a.sc->resampled)
         return;
     uint32_t lo, hi;
@@ -484,9 +486,9 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_count(
 inline void launch_rs32_count(int grid, cudaStream_t st, const Rs32Args &a)
 {
     if (a.scheme == VSMC_CUDA_SYSTEMATIC)
-        k_rs32_count<true><<<grid, kPfBlock, 0, st>>>(a);
+        launch_after(k_rs32_count<true>, grid, kPfBlock, 0, st, a);
     else
-        k_rs32_count<false><<<grid, kPfBlock, 0, st>>>(a);
+        launch_after(k_rs32_count<false>, grid, kPfBlock, 0, st, a);
 }
 
 // the assign pass: assign_range over each warp's range
@@ -494,6 +496,7 @@ template <bool Mon>
 __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
     const Rs32Args a)
 {
+    pdl_begin();
     if (!a.sc->resampled)
         return;
     uint32_t lo, hi;
@@ -519,9 +522,9 @@ __global__ void __launch_bounds__(kPfBlock, kRsBlocksPerSm) k_rs32_assign(
 inline void launch_rs32_assign(int grid, cudaStream_t st, const Rs32Args &a)
 {
     if (a.mon_dim > 0)
-        k_rs32_assign<true><<<grid, kPfBlock, 0, st>>>(a);
+        launch_after(k_rs32_assign<true>, grid, kPfBlock, 0, st, a);
     else
-        k_rs32_assign<false><<<grid, kPfBlock, 0, st>>>(a);
+        launch_after(k_rs32_assign<false>, grid, kPfBlock, 0, st, a);
 }
 
 // Genealogy row of the step just finished (t = step - 1): each particle's
