@@ -353,13 +353,6 @@ __device__ __forceinline__ double odd_tail_value(
     return __dadd_rn(mean, __dmul_rn(a, cv));
 }
 
-__device__ __forceinline__ float odd_tail_value(
-    float u, float v, float mean, float sd)
-{
-    const float a = __fmul_rn(sd, sqrtf(__fmul_rn(-2.0f, logf(u))));
-    return __fadd_rn(mean, __fmul_rn(a, cosf(__fmul_rn(kPi2f, v))));
-}
-
 // ------------------------------------------------- scalar-path engines
 
 // CounterEngine scalar operator() (counter.hpp:347-355) for one stream placed
