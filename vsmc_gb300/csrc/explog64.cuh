@@ -216,9 +216,8 @@ VSMC_N64 bool n64_apart(uint64_t a, uint64_t b)
     return ea <= 10 && static_cast<int64_t>(fa - fb) >= 9;
 }
 
-#ifdef __CUDACC__
 // exp(x) for x <= 0 and anything else exp takes
-__device__ __forceinline__ double exp_of_negative(double x)
+VSMC_N64 double exp_of_negative(double x)
 {
     const uint64_t b = n64_bits(x);
     if ((b >> 63 || b == 0) && n64_exp_ok(b))
@@ -226,6 +225,36 @@ __device__ __forceinline__ double exp_of_negative(double x)
     return exp(x);
 }
 
+// uniform of a sum s >= 0 of the sorted sequence
+struct SortedUniform {
+    VSMC_N64 double operator()(double s) const
+    {
+        return 1.0 - exp_of_negative(-s);
+    }
+};
+
+// The running maximum up to j of the sorted uniforms u_i = form(s_i), for
+// non-decreasing sums s_i >= 0.  form is 1 - exp(-s) with an exp within an
+// ulp, so u_j can only be below a u_i whose sum is within 2^-50 of s_j: the
+// few predecessors that near (a look at one neighbour nearly always) are
+// formed again.  Nothing is above u_j = 1, which an infinite sum and every
+// one from 38 on gives.
+template <class Sums, class Form>
+VSMC_N64 double n64_sorted_max(const Sums &s, size_t j, const Form &form)
+{
+    const double sj = s[j];
+    double u = form(sj);
+    for (size_t i = j; i > 0 && u < 1.0; --i) {
+        const double si = s[i - 1];
+        if (n64_apart(n64_bits(sj), n64_bits(si)))
+            break;
+        const double v = form(si);
+        u = v > u ? v : u;
+    }
+    return u;
+}
+
+#ifdef __CUDACC__
 // log(x) for x in (0, 1) and anything else log takes
 __device__ __forceinline__ double log_of_fraction(double x)
 {

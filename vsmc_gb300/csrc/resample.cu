@@ -557,44 +557,21 @@ __global__ void __launch_bounds__(kB64) k_sorted_terms_arr(
 }
 
 // The sorted uniforms u_j = 1 - exp(lmax_j), lmax_j = -s_j, from the running
-// sums s.  They are non-decreasing up to exp's last bit: *unsorted is set
-// where two sums are within 2^-50 (exp is within an ulp, so a larger step
-// cannot be reversed).
-__global__ void k_sorted_finish(
-    size_t n, const double *s, double *u, uint32_t *unsorted)
+// sums s; Max: their running maximum, which the counts compare (exp's last bit
+// could turn two neighbours around).  The maximum is found where it is needed,
+// by the predecessors within 2^-50 (n64_sorted_max): the expected number of
+// such pairs is 4.5 n^2 2^-53, 0.1 at n = 2^24 and 2 at 2^26.  A flag and one
+// block that then walked all of u took 17 ms of a call's 18 at 2^24 whenever
+// one pair was that near.
+template <bool Max>
+__global__ void k_sorted_finish(size_t n, const double *s, double *u)
 {
     pdl_begin();
     GRID_LOOP(j, n)
     {
-        const double sj = s[j];
-        if (unsorted && j > 0 && !n64_apart(n64_bits(sj), n64_bits(s[j - 1])))
-            *unsorted = 1;
-        u[j] = 1.0 - exp_of_negative(-sj);
+        const SortedUniform form;
+        u[j] = Max ? n64_sorted_max(s, j, form) : form(s[j]);
     }
-}
-
-// The running maximum of u in place by one block, if *unsorted (rare, so one
-// block is enough): non-negative doubles order as their bits.
-__global__ void __launch_bounds__(1024) k_running_max(
-    size_t n, double *u, uint32_t *unsorted)
-{
-    pdl_begin();
-    if (*unsorted == 0)
-        return;
-    long long carry = 0;
-    for (size_t base = 0; base < n; base += 1024) {
-        const size_t i = base + threadIdx.x;
-        const long long v = i < n ? __double_as_longlong(u[i]) : 0;
-        long long tot;
-        const long long ex =
-            block_excl_any<long long, OpMaxK, 1024>(v, OpMaxK(), 0, &tot);
-        const long long r = OpMaxK()(carry, OpMaxK()(ex, v));
-        if (i < n)
-            u[i] = __longlong_as_double(r);
-        carry = OpMaxK()(carry, tot);
-    }
-    if (threadIdx.x == 0)
-        *unsorted = 0;
 }
 
 __global__ void k_stratified_arr(size_t n, const double *u01, double *out)
@@ -1408,10 +1385,7 @@ int scheme_enqueue(size_t m, size_t n, const vsmc_cuda_rng &rng,
             rc = seqsum_device(N, t, t, nullptr, err, scratch, st, true);
             if (rc != VSMC_CUDA_OK)
                 return rc;
-            launch_after(k_sorted_finish, grid1(N), kB, 0, st, N, t, u,
-                err + kErrUnsorted);
-            launch_after(k_running_max, 1, 1024, 0, st, N, u,
-                err + kErrUnsorted);
+            launch_after(k_sorted_finish<true>, grid1(N), kB, 0, st, N, t, u);
         }
         VSMC_CUDA_CHECK_LAUNCH();
     }
@@ -1604,8 +1578,8 @@ int vsmc_cuda_u01_sorted(size_t n, const double *u01, double *u01seq,
         int rc = seqsum_device(n, t, t, nullptr, err, sc, st, true);
         if (rc != VSMC_CUDA_OK)
             return rc;
-        launch_after(k_sorted_finish, grid1(n), kB, 0, st, n, t, u01seq,
-            nullptr);
+        launch_after(
+            k_sorted_finish<false>, grid1(n), kB, 0, st, n, t, u01seq);
         VSMC_CUDA_CHECK_LAUNCH();
         return static_cast<int>(VSMC_CUDA_OK);
     });

@@ -9,7 +9,6 @@ namespace vsmc_cuda
 {
 
 // the words of new_err past the sums' tickets
-constexpr int kErrUnsorted = 3; // sorted uniforms that step back
 constexpr int kErrTail = 4;     // uniforms left to the last particle
 constexpr int kErrTicket = 5;   // ticket of another last-block reduction
 constexpr int kErrMax = 6;      // key of the largest log-weight (two words)
