@@ -43,15 +43,14 @@ struct Pf64Host {
 struct Pf64State {
     int *rep = nullptr;
     int *idx = nullptr;
-    double *scal = nullptr; // [0] ess, [1] log-evidence, [2] 1 / n normalized
-                            // and [3] its log, [4], [5] sums
+    double *scal = nullptr; // [0] ess, [1] log-evidence, [2] 1 / n normalized,
+                            // [4], [5] sums
     double *part = nullptr; // weighted sums of blocks
     uint32_t *err = nullptr; // kErrWords words (resample_internal.cuh)
     Pf64Host *host = nullptr, *host_dev = nullptr;
     Scratch *work = nullptr; // the sums' buffers
     SeqArgs seq = {};
     vsmc_cuda_rng reng = {};
-    bool equal = false;   // every weight is 1 / n normalized
     bool pending = false; // the engine has yet to pass the last resample
     size_t pending_n = 0; // its uniforms
 };
@@ -62,11 +61,11 @@ namespace
 constexpr int kSelB = 128;
 
 // Move, log-likelihood and log-weight of every particle; the largest
-// log-weight into *key.  logeq: the logarithm of the common weight when all
-// are equal (null otherwise).
+// log-weight into *key.  The weights are read after a resample too: a caller
+// may have written them (vsmc_cuda_pf_state).
 __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
     uint32_t t, uint32_t seed, CvConst<double> c, const double *obs,
-    double *s, double *W, const double *logeq, unsigned long long *key)
+    double *s, double *W, unsigned long long *key)
 {
     pdl_begin();
     const double ox = obs[2 * t + 0], oy = obs[2 * t + 1];
@@ -98,7 +97,7 @@ __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
         s[3 * ld + i] = VY;
         double lw = cv_loglik(c, ox, oy, X, Y);
         if (t != 0)
-            lw = __dadd_rn(logeq ? *logeq : log_of_fraction(W[i]), lw);
+            lw = __dadd_rn(log_of_fraction(W[i]), lw);
         W[i] = lw;
         m = max(m, max_key(lw));
     }
@@ -286,10 +285,8 @@ __global__ void __launch_bounds__(kSelB) k_select64(
 
 __global__ void k_equal64(const double *W, double *scal)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
+    if (threadIdx.x == 0 && blockIdx.x == 0)
         scal[2] = W[0];
-        scal[3] = log(W[0]);
-    }
 }
 
 int select_grid(size_t n) { return grid_for(n, kSelB, 1, 4); }
@@ -326,7 +323,7 @@ int pf64_create(vsmc_cuda_pf *pf)
     int rc = seq_args(n, p->err, false, *p->work, &p->seq);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    // the weight that Weight::set_equal leaves in every slot, and its log
+    // the weight that Weight::set_equal leaves in every slot
     double *W = static_cast<double *>(pf->weight);
     {
         Scratch scratch(st);
@@ -402,7 +399,6 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
         vsmc_cuda_rng_set_key(&p->reng, 2, key);
         const uint64_t ctr[4] = {0, 0, 1, 0};
         vsmc_cuda_rng_set_ctr(&p->reng, 4, ctr);
-        p->equal = false;
         p->pending = false;
         VSMC_CUDA_TRY(
             cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
@@ -410,7 +406,7 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     const CvConst<double> c = make_cv_const<double>(pf->model);
     launch_after(k_move64, grid64(n), kB64, 0, st, a.n,
         static_cast<uint32_t>(a.ld), t,
-        pf->seed, c, pf->obs, S, a.W, p->equal ? p->scal + 3 : nullptr, a.key);
+        pf->seed, c, pf->obs, S, a.W, a.key);
     launch_after(k_exp64, grid64(n), kB64, 0, st, a.n, a.W, a.key);
     VSMC_CUDA_CHECK_LAUNCH();
     int rc = small ? seq_cluster_launch(k_weigh64, p->seq, st, a)
@@ -418,7 +414,6 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     if (rc != VSMC_CUDA_OK)
         return rc;
     VSMC_CUDA_TRY(cudaStreamSynchronize(st));
-    p->equal = false;
     rc = err_status(p->host->err);
     if (rc != VSMC_CUDA_OK)
         return rc;
@@ -439,7 +434,6 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
         launch_after(k_select64, select_grid(n), kSelB, 0, st, a, S,
             p->idx, p->part);
         VSMC_CUDA_CHECK_LAUNCH();
-        p->equal = true;
         p->pending = true;
         p->pending_n = N;
     } else if (!small) {
