@@ -8,25 +8,26 @@
 // reads the ESS back to decide on resampling, as Particle::resample does.
 //
 // A step is three launches and one host wait:
-//   move   every particle moves, its log-weight log(W) + l is stored in W and
-//          the largest found (an integer atomic);
-//   exp    W = exp(lw - max);
+//   move   every particle moves; the largest log-weight lw = log(W) + l and
+//          the largest l are found (integer atomics);
+//   exp    W = exp(lw - max), and block sums of the evidence's terms
+//          W exp(l - max l);
 //   weigh  both left-to-right sums, the normalized weights, ESS, evidence,
 //          the decision and, without a resample, the weighted mean: one
 //          cluster up to 16384 particles, the passes of seqsum.cuh above.
 // The decision and the error word go to mapped host memory.  A resample adds
 // the uniforms, the counts, the slots and one pass that copies particles,
 // sets the weights and takes the mean.  move and exp are bound by the FP64
-// pipe (about 200 and 17 instructions a particle at 19 cycles of an SM per
-// warp), so they run in 64-thread blocks over all SMs: at 2^14 particles a
-// step took 320 us with 256-thread blocks on 16 to 64 SMs, about 60 launches
-// and four waits.
+// pipe (19 cycles of an SM per warp's instruction), so they run in 64-thread
+// blocks over all SMs: at 2^14 particles a step took 320 us with 256-thread
+// blocks on 16 to 64 SMs, about 60 launches and four waits.
 #include "explog64.cuh"
 #include "pf_internal.cuh"
 #include "pf_model.cuh"
 #include "resample_internal.cuh"
 #include "seqsum.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <new>
 
@@ -45,10 +46,11 @@ struct Pf64State {
     int *idx = nullptr;
     double *scal = nullptr; // [0] ess, [1] log-evidence, [2] 1 / n normalized,
                             // [4], [5] sums
-    double *part = nullptr; // weighted sums of blocks
+    double *ll = nullptr; // the step's log-likelihoods, then its log-weights
+    double *part = nullptr; // sums of blocks
     uint32_t *err = nullptr; // kErrWords words (resample_internal.cuh)
     Pf64Host *host = nullptr, *host_dev = nullptr;
-    Scratch *work = nullptr; // the sums' buffers
+    Scratch *work = nullptr; // the sums' buffers, ll
     SeqArgs seq = {};
     vsmc_cuda_rng reng = {};
     bool pending = false; // the engine has yet to pass the last resample
@@ -60,16 +62,17 @@ namespace
 
 constexpr int kSelB = 128;
 
-// Move, log-likelihood and log-weight of every particle; the largest
-// log-weight into *key.  The weights are read after a resample too: a caller
-// may have written them (vsmc_cuda_pf_state).
+// Move, log-likelihood and log-weight of every particle (into ll[0 .. n) and
+// ll[n .. 2 n)); the largest log-weight into key[0], the largest
+// log-likelihood into key[1].  The weights are read after a resample too: a
+// caller may have written them (vsmc_cuda_pf_state).
 __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
     uint32_t t, uint32_t seed, CvConst<double> c, const double *obs,
-    double *s, double *W, unsigned long long *key)
+    double *s, double *ll, const double *W, unsigned long long *key)
 {
     pdl_begin();
     const double ox = obs[2 * t + 0], oy = obs[2 * t + 1];
-    unsigned long long m = 0;
+    unsigned long long m = 0, ml = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         const u32x4 w = particle_block(t, seed, i);
@@ -95,27 +98,52 @@ __global__ void __launch_bounds__(kB64) k_move64(uint32_t n, uint32_t ld,
         s[ld + i] = Y;
         s[2 * ld + i] = VX;
         s[3 * ld + i] = VY;
-        double lw = cv_loglik(c, ox, oy, X, Y);
-        if (t != 0)
-            lw = __dadd_rn(log_of_fraction(W[i]), lw);
-        W[i] = lw;
+        const double l = cv_loglik(c, ox, oy, X, Y);
+        const double lw =
+            t == 0 ? l : __dadd_rn(log_of_fraction(W[i]), l);
+        ll[i] = l;
+        ll[static_cast<size_t>(n) + i] = lw;
         m = max(m, max_key(lw));
+        ml = max(ml, max_key(l));
     }
-    __shared__ unsigned long long sh[kB64 / 32 + 1];
-    m = block_reduce(m, OpMax(), 0ull, sh);
-    if (threadIdx.x == 0)
-        atomicMax(key, m);
+    __shared__ unsigned long long sh[2];
+    m = warp_reduce(m, OpMax());
+    ml = warp_reduce(ml, OpMax());
+    if (threadIdx.x == 32) {
+        sh[0] = m;
+        sh[1] = ml;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(key, max(m, sh[0]));
+        atomicMax(key + 1, max(ml, sh[1]));
+    }
 }
 
-// W = exp(lw - max)
-__global__ void __launch_bounds__(kB64) k_exp64(
-    uint32_t n, double *W, const unsigned long long *key)
+// W = exp(lw - max), and the block's sum of W exp(l - max l) over the weights
+// before the step (1 each at t == 0) into part.  The evidence is the log of
+// these sums' tree sum, not of the left-to-right sum of the new weights: its
+// n roundings in a row, and that of log(W) + l, made an increment's error
+// 3e-15 at 2^14 and 2.4e-14 at 2^20 particles, against 1.5e-16.
+__global__ void __launch_bounds__(kB64) k_exp64(uint32_t n, uint32_t t,
+    const double *ll, double *W, const unsigned long long *key, double *part)
 {
     pdl_begin();
-    const double m = from_max_key(*key);
+    const double m = from_max_key(key[0]), ml = from_max_key(key[1]);
+    double ev = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += gridDim.x * blockDim.x)
-        W[i] = exp_of_negative(W[i] - m);
+         i += gridDim.x * blockDim.x) {
+        const double e = exp_of_negative(ll[i] - ml);
+        ev += t == 0 ? e : W[i] * e;
+        W[i] = exp_of_negative(ll[static_cast<size_t>(n) + i] - m);
+    }
+    __shared__ double sh;
+    ev = warp_reduce(ev, OpAdd());
+    if (threadIdx.x == 32)
+        sh = ev;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        part[blockIdx.x] = ev + sh;
 }
 
 // where a step's results go
@@ -129,36 +157,43 @@ struct Step64 {
     int *h_res;
     uint32_t *err;
     unsigned long long *key;
+    const double *part; // the evidence's block sums
+    uint32_t nb;
     Pf64Host *host;
 };
 
 // The step's records, by one thread: the evidence increment is
-// log sum_i W_{t-1,i} exp(l_i) = max + log(sum), the sum being that of the
-// weights before they are normalized (over n equal ones at t = 0).
+// log sum_i W_{t-1,i} exp(l_i) = max l + log(sum) with the sum of k_exp64's
+// terms (over n equal weights at t = 0).
 __device__ __forceinline__ void step64_record(
     const Step64 &a, double sum, double ess)
 {
     const bool res = ess < a.threshold * static_cast<double>(a.n);
     const double mass = a.t == 0 ? sum / static_cast<double>(a.n) : sum;
     const double logz = (a.t == 0 ? 0.0 : a.scal[1]) +
-        (from_max_key(*a.key) + log(mass));
+        (from_max_key(a.key[1]) + log(mass));
     a.scal[0] = ess;
     a.scal[1] = logz;
     a.h_ess[a.t] = ess;
     a.h_logz[a.t] = logz;
     a.h_res[a.t] = res ? 1 : 0;
-    *a.key = 0; // for the next step's maximum
+    a.key[0] = a.key[1] = 0; // for the next step's maxima
     a.host->err = atomicOr(a.err, 0u);
     // (the host reads these after waiting for the stream: no fence, which took
     // a microsecond of the step)
     a.host->resample = res ? 1 : 0;
 }
 
-__global__ void k_record64(const Step64 a)
+__global__ void __launch_bounds__(kSeqBlock) k_record64(const Step64 a)
 {
     pdl_begin();
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        step64_record(a, a.scal[4], a.scal[5]);
+    __shared__ double sh[kSeqBlock / 32 + 1];
+    double sum = 0;
+    for (uint32_t b = threadIdx.x; b < a.nb; b += kSeqBlock)
+        sum += a.part[b];
+    sum = block_reduce(sum, OpAdd(), 0.0, sh);
+    if (threadIdx.x == 0)
+        step64_record(a, sum, a.scal[5]);
 }
 
 // Normalization, ESS, records and (without a resample) the weighted mean of
@@ -170,14 +205,34 @@ __global__ void __launch_bounds__(kSeqBlock) k_weigh64(
     namespace cg = cooperative_groups;
     const cg::cluster_group cl = cg::this_cluster();
     SeqClusterSmem &S = seq_cluster_smem(q);
-    __shared__ double s_inv, s_mean[2], sh[kSeqBlock / 32 + 1];
+    __shared__ double s_inv, s_mass, s_mean[2], sh[kSeqBlock / 32 + 1];
     __shared__ bool s_res;
     const uint32_t tile = cl.block_rank();
     double w[kSeqItems], sq[kSeqItems];
     seq_load(SeqLoad{a.W}, tile, q.n, w);
+    // the evidence's block sums (at most 256), by a warp of the first block
+    // while another thread divides
+    constexpr int kP = static_cast<int>(kSeqSmall) / kB64 / 32;
+    const bool adds = tile == 0 && threadIdx.x >= 32 && threadIdx.x < 64;
+    double part[kP];
+#pragma unroll
+    for (int k = 0; k < kP; ++k) {
+        const uint32_t b = threadIdx.x % 32 + 32 * k;
+        part[k] = adds && b < a.nb ? a.part[b] : 0.0;
+    }
     const double total = seq_cluster_total(cl, q, w, S);
     if (threadIdx.x == 0)
         s_inv = 1.0 / total;
+    if (adds) {
+#pragma unroll
+        for (int d = kP / 2; d > 0; d /= 2)
+#pragma unroll
+            for (int k = 0; k < d; ++k)
+                part[k] += part[k + d];
+        const double s = warp_reduce(part[0], OpAdd());
+        if (threadIdx.x == 32)
+            s_mass = s;
+    }
     __syncthreads();
     const double inv = s_inv;
 #pragma unroll
@@ -193,7 +248,7 @@ __global__ void __launch_bounds__(kSeqBlock) k_weigh64(
         const double ess = 1.0 / tsq;
         s_res = ess < a.threshold * static_cast<double>(a.n);
         if (tile == 0)
-            step64_record(a, total, ess);
+            step64_record(a, s_mass, ess);
     }
     __syncthreads();
     if (s_res) // the same in every block
@@ -307,9 +362,10 @@ int pf64_create(vsmc_cuda_pf *pf)
         *q = static_cast<std::remove_pointer_t<decltype(q)>>(v);
         return e == cudaSuccess;
     };
+    const size_t blocks = std::max(2 * select_grid(n), grid64(n));
     if (!get(&p->rep, sizeof(int) * n) || !get(&p->idx, sizeof(int) * n) ||
         !get(&p->scal, sizeof(double) * 8) ||
-        !get(&p->part, sizeof(double) * 2 * select_grid(n)) ||
+        !get(&p->part, sizeof(double) * blocks) ||
         !get(&p->err, sizeof(uint32_t) * kErrWords) ||
         cudaHostAlloc(reinterpret_cast<void **>(&p->host), sizeof(Pf64Host),
             cudaHostAllocMapped) != cudaSuccess ||
@@ -318,6 +374,9 @@ int pf64_create(vsmc_cuda_pf *pf)
         return VSMC_CUDA_ERR_ALLOC;
     p->work = new (std::nothrow) Scratch(st);
     if (p->work == nullptr)
+        return VSMC_CUDA_ERR_ALLOC;
+    p->ll = p->work->get<double>(2 * n);
+    if (p->ll == nullptr)
         return VSMC_CUDA_ERR_ALLOC;
     VSMC_CUDA_TRY(cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
     int rc = seq_args(n, p->err, false, *p->work, &p->seq);
@@ -363,7 +422,7 @@ static int weigh_large(vsmc_cuda_pf *pf, const Step64 &a)
     int rc = weight_sums(q, a.W, a.W, p->scal + 5, st);
     if (rc != VSMC_CUDA_OK)
         return rc;
-    launch_after(k_record64, 1, 32, 0, st, a);
+    launch_after(k_record64, 1, kSeqBlock, 0, st, a);
     VSMC_CUDA_CHECK_LAUNCH();
     return VSMC_CUDA_OK;
 }
@@ -389,6 +448,8 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     a.h_res = pf->h_res;
     a.err = p->err;
     a.key = reinterpret_cast<unsigned long long *>(p->err + kErrMax);
+    a.part = p->part;
+    a.nb = static_cast<uint32_t>(grid64(n));
     a.host = p->host_dev;
     double *S = static_cast<double *>(pf->state);
     if (first) {
@@ -404,10 +465,11 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
             cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
     }
     const CvConst<double> c = make_cv_const<double>(pf->model);
-    launch_after(k_move64, grid64(n), kB64, 0, st, a.n,
-        static_cast<uint32_t>(a.ld), t,
-        pf->seed, c, pf->obs, S, a.W, a.key);
-    launch_after(k_exp64, grid64(n), kB64, 0, st, a.n, a.W, a.key);
+    launch_after(k_move64, a.nb, kB64, 0, st, a.n,
+        static_cast<uint32_t>(a.ld), t, pf->seed, c, pf->obs, S, p->ll, a.W,
+        a.key);
+    launch_after(k_exp64, a.nb, kB64, 0, st, a.n, t, p->ll, a.W, a.key,
+        p->part);
     VSMC_CUDA_CHECK_LAUNCH();
     int rc = small ? seq_cluster_launch(k_weigh64, p->seq, st, a)
                    : weigh_large(pf, a);
