@@ -337,7 +337,8 @@ int vsmc_cuda_pf_create(vsmc_cuda_pf **pf, size_t n, int precision,
     const vsmc_cuda_cv_model *model, size_t max_steps, void *stream);
 int vsmc_cuda_pf_destroy(vsmc_cuda_pf *pf);
 /* Sampler::initialize (core/sampler.hpp:443-455) with observation obs_dev[0..1]
- * (device, 2 doubles). */
+ * (device, 2 doubles).  Precision 64: this call and pf_iterate return with the
+ * step finished on the filter's stream, and its status. */
 int vsmc_cuda_pf_initialize(vsmc_cuda_pf *pf, const double *obs_dev);
 /* Sampler::iterate() (core/sampler.hpp:464-476) with observation obs_dev[0..1]. */
 int vsmc_cuda_pf_iterate(vsmc_cuda_pf *pf, const double *obs_dev);

@@ -103,3 +103,29 @@ def test_evidence_increments_are_accurate(vc, n):
         pf.close()
     assert np.mean(e0) < 3e-15, e0
     assert np.mean(e1) < 3e-15 + np.mean(ulp), e1
+
+
+@pytest.mark.parametrize("n", [16384, 1 << 20])
+def test_a_single_step_returns_finished(vc, n):
+    """initialize and iterate leave nothing running on the filter's stream,
+    also after a resample (1.1: at every step), so its pointers can be read
+    from any stream."""
+    import ctypes
+
+    import torch
+    d = dev(np.array([[0.3, -0.2]] * 6))
+    pf = vc.ParticleFilter(n, 64, vc.MULTINOMIAL, 1.1, seed=1, max_steps=6)
+    st = ctypes.c_void_p()
+    vc.call("vsmc_cuda_pf_stream", pf.handle, ctypes.byref(st))
+    stream = torch.cuda.ExternalStream(st.value)
+    vc.call("vsmc_cuda_pf_initialize", pf.handle, d[0].data_ptr())
+    assert stream.query()
+    for t in range(1, 6):
+        vc.call("vsmc_cuda_pf_iterate", pf.handle, d[t].data_ptr())
+        assert stream.query()
+    state, weight = (v.cpu().numpy() for v in _views(pf, n))
+    h = pf.history(6)
+    assert (h["resampled"] == 1).all()
+    assert (weight == weight[0]).all()
+    np.testing.assert_allclose(state[0].mean(), h["mean"][5][0], rtol=1e-10)
+    pf.close()

@@ -952,7 +952,16 @@ int vsmc_cuda_pf_state(vsmc_cuda_pf *pf, void **state_dev, void **weight_dev)
     return VSMC_CUDA_OK;
 }
 
-static int pf_begin(vsmc_cuda_pf *pf)
+// A step of the FP64 filter; alone: its caller gets it finished, with its
+// status.  (A run's steps overlap: a resample's kernels run on while the host
+// queues the next step, whose wait sees their errors.)
+static int step64(vsmc_cuda_pf *pf, bool first, bool alone)
+{
+    const int rc = pf64_step(pf, first);
+    return rc == VSMC_CUDA_OK && alone ? pf64_finish(pf) : rc;
+}
+
+static int pf_begin(vsmc_cuda_pf *pf, bool alone)
 {
     int rc = reset_scalars(pf);
     if (rc != VSMC_CUDA_OK)
@@ -962,7 +971,7 @@ static int pf_begin(vsmc_cuda_pf *pf)
             sizeof(uint32_t) * pf->max_steps, pf->stream));
     pf->t = 0;
     pf->mean_pending = false;
-    rc = pf->precision == 32 ? launch_first32(pf) : pf64_step(pf, true);
+    rc = pf->precision == 32 ? launch_first32(pf) : step64(pf, true, alone);
     if (rc != VSMC_CUDA_OK)
         return rc;
     pf->t = 1;
@@ -970,9 +979,10 @@ static int pf_begin(vsmc_cuda_pf *pf)
     return VSMC_CUDA_OK;
 }
 
-static int pf_next(vsmc_cuda_pf *pf)
+static int pf_next(vsmc_cuda_pf *pf, bool alone)
 {
-    const int rc = pf->precision == 32 ? step32(pf) : pf64_step(pf, false);
+    const int rc =
+        pf->precision == 32 ? step32(pf) : step64(pf, false, alone);
     if (rc != VSMC_CUDA_OK)
         return rc;
     ++pf->t;
@@ -1001,7 +1011,7 @@ static int pf_flush_mean(vsmc_cuda_pf *pf)
             VSMC_CUDA_CHECK_LAUNCH();
         }
     } else {
-        rc = pf64_final_mean(pf);
+        rc = pf64_finish(pf);
     }
     if (rc == VSMC_CUDA_OK)
         pf->mean_pending = false;
@@ -1014,7 +1024,7 @@ int vsmc_cuda_pf_initialize(vsmc_cuda_pf *pf, const double *obs_dev)
         return VSMC_CUDA_ERR_ARG;
     VSMC_CUDA_TRY(cudaMemcpyAsync(pf->obs, obs_dev, 2 * sizeof(double),
         cudaMemcpyDeviceToDevice, pf->stream));
-    return pf_begin(pf);
+    return pf_begin(pf, true);
 }
 
 int vsmc_cuda_pf_iterate(vsmc_cuda_pf *pf, const double *obs_dev)
@@ -1027,7 +1037,7 @@ int vsmc_cuda_pf_iterate(vsmc_cuda_pf *pf, const double *obs_dev)
         return VSMC_CUDA_ERR_SIZE;
     VSMC_CUDA_TRY(cudaMemcpyAsync(pf->obs + 2 * pf->t, obs_dev,
         2 * sizeof(double), cudaMemcpyDeviceToDevice, pf->stream));
-    return pf_next(pf);
+    return pf_next(pf, true);
 }
 
 int vsmc_cuda_pf_run_device(vsmc_cuda_pf *pf, size_t T, const double *obs_dev)
@@ -1047,9 +1057,9 @@ int vsmc_cuda_pf_run_device(vsmc_cuda_pf *pf, size_t T, const double *obs_dev)
         if (rc == VSMC_CUDA_OK)
             rc = run32(pf, T);
     } else {
-        rc = pf_begin(pf);
+        rc = pf_begin(pf, false);
         for (size_t t = 1; rc == VSMC_CUDA_OK && t < T; ++t)
-            rc = pf_next(pf);
+            rc = pf_next(pf, false);
     }
     if (rc == VSMC_CUDA_OK)
         rc = pf_flush_mean(pf);

@@ -505,8 +505,9 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     return rc;
 }
 
-// errors of the last step's resample, which its own wait did not see
-int pf64_final_mean(vsmc_cuda_pf *pf)
+// Waits for the last step's resample and returns its errors, which the step's
+// own wait did not see.
+int pf64_finish(vsmc_cuda_pf *pf)
 {
     VSMC_CUDA_TRY(cudaStreamSynchronize(pf->stream));
     return err_status(pf->p64->host->err);

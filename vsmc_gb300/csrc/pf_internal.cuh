@@ -75,6 +75,6 @@ namespace vsmc_cuda
 int pf64_create(vsmc_cuda_pf *pf);
 void pf64_destroy(vsmc_cuda_pf *pf);
 int pf64_step(vsmc_cuda_pf *pf, bool first);
-int pf64_final_mean(vsmc_cuda_pf *pf);
+int pf64_finish(vsmc_cuda_pf *pf);
 
 } // namespace vsmc_cuda
