@@ -281,6 +281,9 @@ __global__ void __launch_bounds__(kSeqBlock) k_weigh64(
 // After a resample: particles copied to the empty slots (parents keep
 // theirs, so in place), every weight 1 / n normalized, and the mean of the
 // result: block sums, added by the last block (its ticket; nothing waits).
+// After an error of the counts or slots nothing is copied: idx may be an
+// earlier resample's then, whose copies from slots that are not parents would
+// overlap.
 __global__ void __launch_bounds__(kSelB) k_select64(
     const Step64 a, double *state, const int *idx, double *part)
 {
@@ -288,10 +291,11 @@ __global__ void __launch_bounds__(kSelB) k_select64(
     __shared__ double sh[kSelB / 32 + 1];
     __shared__ bool last;
     const double w = a.scal[2];
+    const bool copy = __ldcg(a.err) == 0;
     double m[2] = {0.0, 0.0};
     for (uint32_t i = blockIdx.x * kSelB + threadIdx.x; i < a.n;
          i += gridDim.x * kSelB) {
-        const uint32_t j = static_cast<uint32_t>(idx[i]);
+        const uint32_t j = copy ? static_cast<uint32_t>(idx[i]) : i;
         if (j >= a.n) {
             atomicOr(a.err, DEV_ERR_INTERNAL);
             continue;
