@@ -571,7 +571,8 @@ __device__ __forceinline__ void pf_step_combine(const PfStepArgs &a,
     float M = -INFINITY;
     double tot = 0; // lane k of the finishing warps: value k
     if (nblk == 1) {
-        // one record: the sums are its own (every factor is exp(0) = 1)
+        // one record: the sums are its own (every factor is exp(M - M) = 1,
+        // or not a number for an infinite M)
         M = static_cast<float>(ld(&part->m));
         if (lane < NV)
             tot = lane == 0 ? ld(&part->s)
@@ -579,6 +580,8 @@ __device__ __forceinline__ void pf_step_combine(const PfStepArgs &a,
                 : lane < 2 + AMD ? ld(&part->mon[lane - 2])
                 : lane < NV - 1  ? ld(&part->prev[lane - 2 - AMD])
                                  : ld(&part->prev_w);
+        if (M == INFINITY && lane < 2 + AMD)
+            tot += M - M;
         __syncthreads(); // sc.S is read
     } else {
         for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x)
