@@ -271,7 +271,7 @@ static size_t run_tiles_most(int scheme)
         return kRunCluster;
     return std::max(kRunCluster,
         static_cast<size_t>(num_sms()) *
-            static_cast<size_t>(std::min(occ, kRunOcc)));
+            static_cast<size_t>(std::min(occ, kRunShare)));
 }
 
 // Whether a run of this filter is one kernel: the plain step

@@ -2,7 +2,7 @@
 // one tile each.
 //
 // A step of the graph path is four dependent launches, three of which return
-// at once when the step does not resample; at 1000 to 600000 particles their
+// at once when the step does not resample; at 1000 to 150000 particles their
 // latencies are most of the step (20 to 25 us, against 2 to 8 us of work).
 // Here the blocks stay resident for all steps and meet at a grid barrier:
 // once a step (the records are there), and three times more in a resampling
@@ -15,12 +15,17 @@
 //
 // Measured per step, launches against this kernel: n = 1000 19.6 -> 6.6 us
 // (one block), 8192 20.7 -> 8.7 (one cluster of 8 blocks), 100003 22.0 -> 12.4
-// and 300000 24.9 -> 17.8 (cooperative grid).  What is left is a chain: the
-// tile 3.8k cycles, its warp and block sums 1.5k, the FP64 quotient and
-// logarithm 2k, a grid barrier 2k.  Every block combines all records, so more
-// blocks per SM share its FP64 pipe: level with the launches at 450000
-// particles (3 blocks per SM) and slower at 600000 (4), so it is taken up to
-// kRunOcc blocks per SM.
+// (cooperative grid).  What is left is a chain: the tile, its warp and block
+// sums, the FP64 quotient and logarithm, a grid barrier.
+//
+// It is taken up to a block an SM (155648 particles), where two runs are
+// resident at once (kRunOcc): filters on streams of their own overlap then.
+// 50 steps of 1, 2, 4, 8 and 16 filters of 155000 take 0.49, 0.59, 1.1, 2.2
+// and 4.5 ms, 1.5, 1.6, 1.9, 2.4 and 4.3 by launches that returned at once
+// without a resample.  A run of more blocks holds the chip while it waits at
+// its barriers: filters of 300000 took 0.78, 1.5, 3.0, 6.1 and 12.1 ms, by
+// the launches 1.6, 1.8, 2.1, 2.9 and 5.5 then, 1.1, 1.3, 1.7, 2.5 and 4.7
+// now (figures at 320000).
 #pragma once
 
 #include "pf32.cuh"
@@ -48,8 +53,10 @@ __device__ __forceinline__ uint64_t run_clock()
 // cluster barrier); a cooperative grid (a counter in memory, about 1.5 us).
 enum class RunKind { Block, Cluster, Grid };
 
-// Blocks per SM that a run's grid may take (see the file comment).
+// Blocks an SM holds (registers), and those of them that one run may take
+// (see the file comment).
 constexpr int kRunOcc = 2;
+constexpr int kRunShare = 1;
 
 // Every block waits for every other; writes before it are visible after it.
 // false, in every thread of the block, if the wait ran out (two seconds):
