@@ -99,6 +99,15 @@ def test_paths_and_bits(child):
         assert resampled > 0 or n < 32, n
 
 
+def test_a_refused_launch_goes_by_launches(child):
+    """The runtime refuses cooperative launches (and this watch cluster ones):
+    the run is the same by launches, and the kernel is not tried again."""
+    for n, _, graph, _, same, _ in child([[n, 1] for n in
+                                          (1000, 3000, 8193, 100003, -1)]):
+        assert graph == [1, 0], n
+        assert same, n
+
+
 def _time_runs(vc, n, k, T=50):
     import torch
     rng = np.random.default_rng(3)

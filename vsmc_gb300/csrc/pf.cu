@@ -285,6 +285,9 @@ static bool run_is_one_kernel(const vsmc_cuda_pf *pf)
 // Steps of one launch: a bound on a kernel's time, not on the run.
 constexpr size_t kRunSteps = 1024;
 
+// Steps 0 .. T - 1, or as many (pf->t) as the whole-run kernel takes: where
+// its launch is refused (a stream that has a part of the SMs only, where the
+// blocks cannot all be resident), the filter goes by launches from then on.
 static int run32(vsmc_cuda_pf *pf, size_t T)
 {
     for (size_t t0 = 0; t0 < T; t0 += kRunSteps) {
@@ -327,12 +330,16 @@ static int run32(vsmc_cuda_pf *pf, size_t T)
         }
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        VSMC_CUDA_TRY(cudaLaunchKernelExC(&cfg, f, args));
+        if (cudaLaunchKernelExC(&cfg, f, args) != cudaSuccess) {
+            cudaGetLastError();
+            pf->run_blocks = 0;
+            return VSMC_CUDA_OK;
+        }
         if (run.steps % 2)
             pf->cur = 1 - pf->cur;
         pf->t = t0 + run.steps;
+        pf->mean_pending = true;
     }
-    pf->mean_pending = true;
     return VSMC_CUDA_OK;
 }
 
@@ -1049,18 +1056,18 @@ int vsmc_cuda_pf_run_device(vsmc_cuda_pf *pf, size_t T, const double *obs_dev)
     if (obs_dev != pf->obs)
         VSMC_CUDA_TRY(cudaMemcpyAsync(pf->obs, obs_dev, 2 * T * sizeof(double),
             cudaMemcpyDeviceToDevice, pf->stream));
-    int rc;
+    int rc = VSMC_CUDA_OK;
+    pf->t = 0;
     if (run_is_one_kernel(pf)) {
         rc = reset_scalars(pf);
-        pf->t = 0;
         pf->mean_pending = false;
         if (rc == VSMC_CUDA_OK)
             rc = run32(pf, T);
-    } else {
-        rc = pf_begin(pf, false);
-        for (size_t t = 1; rc == VSMC_CUDA_OK && t < T; ++t)
-            rc = pf_next(pf, false);
     }
+    if (rc == VSMC_CUDA_OK && pf->t == 0)
+        rc = pf_begin(pf, false);
+    while (rc == VSMC_CUDA_OK && pf->t < T)
+        rc = pf_next(pf, false);
     if (rc == VSMC_CUDA_OK)
         rc = pf_flush_mean(pf);
     return rc;
