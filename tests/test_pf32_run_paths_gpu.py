@@ -3,6 +3,7 @@ the sizes of the whole-run kernel: one block, clusters of every number of tiles
 (padded to a power of two), grids up to a block an SM, and one tile more, which
 goes by launches.  In a child process with launch_watch.c in front of the CUDA
 runtime."""
+import ctypes
 import json
 import os
 import subprocess
@@ -133,3 +134,36 @@ def test_two_filters_overlap(vc, n):
     to 1.25 where the chip has room for both; 2 where one holds it all)."""
     one, two = _time_runs(vc, n, 1), _time_runs(vc, n, 2)
     assert two < 1.6 * one, (one, two)
+
+
+@pytest.mark.parametrize("n", [500, 5000, 50000, 400000])
+def test_a_run_under_capture_is_refused(vc, n):
+    """A run of several steps replays graphs of its own, so it cannot be
+    captured; whichever path the size takes, it is refused, and the filter runs
+    as before once the capture has ended."""
+    import torch
+    T = 4
+    obs = np.random.default_rng(1).normal(0, 0.5, (T, 2))
+    d = dev(obs)
+    rt = ctypes.CDLL("libcudart.so.13")
+    stream = torch.cuda.Stream()
+    s = ctypes.c_void_p(stream.cuda_stream)
+    pf = vc.ParticleFilter(n, 32, vc.SYSTEMATIC, 0.5, seed=1, max_steps=T,
+                           stream=stream.cuda_stream)
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(s, 1) == 0
+    status = vc.lib().vsmc_cuda_pf_run_device(
+        pf.handle, ctypes.c_size_t(T), ctypes.c_void_p(d.data_ptr()))
+    graph = ctypes.c_void_p()
+    rt.cudaStreamEndCapture(s, ctypes.byref(graph))
+    if graph.value:
+        rt.cudaGraphDestroy(graph)
+    rt.cudaGetLastError()
+    assert status == vc.ERR_CUDA
+    got = pf.run(obs)
+    pf.close()
+    pf = vc.ParticleFilter(n, 32, vc.SYSTEMATIC, 0.5, seed=1, max_steps=T)
+    want = pf.run(obs)
+    pf.close()
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k

@@ -276,10 +276,15 @@ static size_t run_tiles_most(int scheme)
 
 // Whether a run of this filter is one kernel: the plain step
 // (its kernels follow nothing else), a tile per block, all blocks resident.
+// Under capture (of a stream of the caller's) the steps' graphs refuse the
+// run, at every size.
 static bool run_is_one_kernel(const vsmc_cuda_pf *pf)
 {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return pf->precision == 32 && !pf->custom && pf->use_graph &&
-        pf->run_blocks > 0 && !pf->record_gen && pf->mcmc_sweeps == 0;
+        pf->run_blocks > 0 && !pf->record_gen && pf->mcmc_sweeps == 0 &&
+        cudaStreamIsCapturing(pf->stream, &cap) == cudaSuccess &&
+        cap == cudaStreamCaptureStatusNone;
 }
 
 // Steps of one launch: a bound on a kernel's time, not on the run.
