@@ -122,6 +122,7 @@ PROTOTYPES = {
     "vsmc_cuda_status_string": (ctypes.c_char_p, [I32]),
     "vsmc_cuda_last_cuda_error": (I32, []),
     "vsmc_cuda_version": (I32, []),
+    "vsmc_cuda_trim_scratch": (I32, []),
     "vsmc_cuda_rng_init": (I32, [_RNGP, I32, U64]),
     "vsmc_cuda_rng_set_key": (I32, [_RNGP, I32, VP]),
     "vsmc_cuda_rng_set_ctr": (I32, [_RNGP, I32, VP]),

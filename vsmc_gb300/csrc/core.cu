@@ -53,7 +53,8 @@ int grid_for(
 // and 3.3 ms at 2^24; 70 us and 0.35 ms from this pool).  It keeps at most
 // kScratchKeep of what no call uses (a resampling call takes about 24 bytes
 // per particle, 0.4 GB at 2^24); anything above goes back at the next
-// synchronization, and all of it when a device allocation fails.
+// synchronization, and all of it when a device allocation of the library's
+// fails or vsmc_cuda_trim_scratch is called.
 // Allocations and frees are stream-ordered, from any thread.
 constexpr uint64_t kScratchKeep = 1ull << 30;
 constexpr int kMaxDevices = 64;
@@ -84,12 +85,16 @@ static cudaMemPool_t scratch_pool(int dev)
     return g_pool[dev];
 }
 
-static void scratch_trim()
+static cudaError_t scratch_trim()
 {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    for (cudaMemPool_t pool : g_pool)
-        if (pool)
-            cudaMemPoolTrimTo(pool, 0);
+    for (cudaMemPool_t pool : g_pool) {
+        const cudaError_t e =
+            pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t device_malloc(void **p, size_t bytes)
@@ -126,6 +131,11 @@ void *Scratch::alloc(size_t bytes)
     cudaError_t e = pool
         ? cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, stream_)
         : cudaMallocAsync(&p, bytes ? bytes : 1, stream_);
+    if (pool && e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_trim();
+        e = cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, stream_);
+    }
     if (e != cudaSuccess) {
         set_last_cuda_error(e);
         return nullptr;
@@ -160,5 +170,11 @@ int vsmc_cuda_last_cuda_error(void)
 }
 
 int vsmc_cuda_version(void) { return 100; }
+
+int vsmc_cuda_trim_scratch(void)
+{
+    VSMC_CUDA_TRY(vsmc_cuda::scratch_trim());
+    return VSMC_CUDA_OK;
+}
 
 } // extern "C"
