@@ -45,8 +45,8 @@ int vsmc_cuda_version(void); /* major * 10000 + minor * 100 + patch */
 /* Calls take their scratch memory from a pool of the library's on each device,
  * which keeps up to 1 GiB between calls (mapping it anew cost 0.2 to 2.4 ms a
  * call) that no other allocator of the process can use meanwhile.  This call
- * gives back what no queued work uses: all of it once the streams in use have
- * been synchronized.  The library does the same itself when an allocation of
+ * gives back what no queued work uses on the current device: all of it once
+ * the streams in use have been synchronized.  The library does the same itself when an allocation of
  * its own fails. */
 int vsmc_cuda_trim_scratch(void);
 

@@ -306,6 +306,9 @@ class Scratch
 
     private:
     cudaStream_t stream_;
+    // the pool that the first allocation found (null: the default pool)
+    cudaMemPool_t pool_ = nullptr;
+    bool found_ = false;
     std::vector<void *> ptrs_;
 };
 

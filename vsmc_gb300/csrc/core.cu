@@ -2,7 +2,9 @@
 #include "common.cuh"
 
 #include <atomic>
+#include <cuda.h>
 #include <mutex>
+#include <vector>
 
 namespace vsmc_cuda
 {
@@ -55,42 +57,85 @@ int grid_for(
 // per particle, 0.4 GB at 2^24); anything above goes back at the next
 // synchronization, and all of it when a device allocation of the library's
 // fails or vsmc_cuda_trim_scratch is called.
-// Allocations and frees are stream-ordered, from any thread.
+// Allocations and frees are stream-ordered, from any thread.  A device reset
+// (cudaDeviceReset) ends the pool with the context, so a pool belongs to the
+// context that made it: its id is never used again, where the handle is.
 constexpr uint64_t kScratchKeep = 1ull << 30;
-constexpr int kMaxDevices = 64;
-static std::mutex g_pool_mutex;
-static cudaMemPool_t g_pool[kMaxDevices] = {};
 
-static cudaMemPool_t scratch_pool(int dev)
+struct ScratchPool {
+    int dev;
+    unsigned long long context;
+    cudaMemPool_t pool;
+};
+
+static std::mutex g_pool_mutex;
+static std::vector<ScratchPool> g_pools;
+
+// id of a stream's context (0: none, or no driver call that tells)
+static unsigned long long context_id(cudaStream_t st)
 {
-    if (dev < 0 || dev >= kMaxDevices)
-        return nullptr;
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (g_pool[dev] == nullptr) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError(); // the caller takes the default pool
-            return nullptr;
+    using StreamCtx = CUresult (*)(CUstream, CUcontext *);
+    using CtxId = CUresult (*)(CUcontext, unsigned long long *);
+    static const auto entry = [](const char *name) {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion(name, &f, 12000,
+                cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
         }
-        uint64_t keep = kScratchKeep;
-        cudaMemPoolSetAttribute(
-            pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        g_pool[dev] = pool;
-    }
-    return g_pool[dev];
+        return f;
+    };
+    static const auto stream_ctx =
+        reinterpret_cast<StreamCtx>(entry("cuStreamGetCtx"));
+    static const auto ctx_id = reinterpret_cast<CtxId>(entry("cuCtxGetId"));
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (!stream_ctx || !ctx_id || stream_ctx(st, &ctx) != CUDA_SUCCESS ||
+        ctx_id(ctx, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
 }
 
+// the pool of a stream's device in its context; null: the default pool
+static cudaMemPool_t scratch_pool(cudaStream_t st)
+{
+    int dev = -1;
+    const unsigned long long id = context_id(st);
+    if (id == 0 || cudaStreamGetDevice(st, &dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (const ScratchPool &p : g_pools)
+        if (p.dev == dev && p.context == id)
+            return p.pool;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    uint64_t keep = kScratchKeep;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pools.push_back({dev, id, pool});
+    return pool;
+}
+
+// the pools of the current context
 static cudaError_t scratch_trim()
 {
+    const unsigned long long id = context_id(nullptr);
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    for (cudaMemPool_t pool : g_pool) {
-        const cudaError_t e =
-            pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+    for (const ScratchPool &p : g_pools) {
+        const cudaError_t e = id != 0 && p.context == id
+            ? cudaMemPoolTrimTo(p.pool, 0)
+            : cudaSuccess;
         if (e != cudaSuccess)
             return e;
     }
@@ -118,23 +163,23 @@ Scratch::~Scratch()
 void *Scratch::alloc(size_t bytes)
 {
     void *p = nullptr;
-    // a stream under capture gets the graph's own allocation nodes
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-    int dev = -1;
-    cudaMemPool_t pool = nullptr;
-    if (cudaStreamIsCapturing(stream_, &cap) == cudaSuccess &&
-        cap == cudaStreamCaptureStatusNone &&
-        cudaStreamGetDevice(stream_, &dev) == cudaSuccess)
-        pool = scratch_pool(dev);
-    else
-        cudaGetLastError();
-    cudaError_t e = pool
-        ? cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, stream_)
+    if (!found_) {
+        // a stream under capture gets the graph's own allocation nodes
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(stream_, &cap) == cudaSuccess &&
+            cap == cudaStreamCaptureStatusNone)
+            pool_ = scratch_pool(stream_);
+        else
+            cudaGetLastError();
+        found_ = true;
+    }
+    cudaError_t e = pool_
+        ? cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool_, stream_)
         : cudaMallocAsync(&p, bytes ? bytes : 1, stream_);
-    if (pool && e == cudaErrorMemoryAllocation) {
+    if (pool_ && e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         scratch_trim();
-        e = cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool, stream_);
+        e = cudaMallocFromPoolAsync(&p, bytes ? bytes : 1, pool_, stream_);
     }
     if (e != cudaSuccess) {
         set_last_cuda_error(e);
