@@ -43,7 +43,7 @@ def test_copy_only_without_an_error(lib, n, err):
     parent = rng.random(n) < 0.4
     parent[0] = True
     idx = np.where(parent, np.arange(n), rng.choice(np.flatnonzero(parent), n))
-    words = np.zeros(10, np.uint32)
+    words = np.zeros(8, np.uint32)
     words[0] = err
     words[4] = 17  # the uniforms left, handed on to the host
     state, W = dev(s0), dev(np.zeros(n))

@@ -45,7 +45,7 @@ struct Pf64State {
     int *rep = nullptr;
     int *idx = nullptr;
     double *scal = nullptr; // [0] ess, [1] log-evidence, [2] 1 / n normalized,
-                            // [4], [5] sums
+                            // [4], [5] sums, [6], [7] the maxima's keys
     double *ll = nullptr; // the step's log-likelihoods, then its log-weights
     double *part = nullptr; // sums of blocks
     uint32_t *err = nullptr; // kErrWords words (resample_internal.cuh)
@@ -451,7 +451,7 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
     a.h_logz = pf->h_logz;
     a.h_res = pf->h_res;
     a.err = p->err;
-    a.key = reinterpret_cast<unsigned long long *>(p->err + kErrMax);
+    a.key = reinterpret_cast<unsigned long long *>(p->scal + 6);
     a.part = p->part;
     a.nb = static_cast<uint32_t>(grid64(n));
     a.host = p->host_dev;
@@ -467,6 +467,7 @@ int pf64_step(vsmc_cuda_pf *pf, bool first)
         p->pending = false;
         VSMC_CUDA_TRY(
             cudaMemsetAsync(p->err, 0, sizeof(uint32_t) * kErrWords, st));
+        VSMC_CUDA_TRY(cudaMemsetAsync(a.key, 0, 2 * sizeof(*a.key), st));
     }
     const CvConst<double> c = make_cv_const<double>(pf->model);
     launch_after(k_move64, a.nb, kB64, 0, st, a.n,

@@ -11,8 +11,7 @@ namespace vsmc_cuda
 // the words of new_err past the sums' tickets
 constexpr int kErrTail = 4;     // uniforms left to the last particle
 constexpr int kErrTicket = 5;   // ticket of another last-block reduction
-constexpr int kErrMax = 6;      // key of the largest log-weight (two words;
-                                // the FP64 filter's log-likelihood: two more)
+constexpr int kErrMax = 6;      // key of the largest log-weight (two words)
 
 // Threads of a block where each element takes many FP64 instructions (19
 // cycles of an SM each): small blocks spread a short vector over all SMs.

@@ -1142,7 +1142,7 @@ struct SeqStore {
 
 // A zeroed error word followed by the sums' two tickets (which every pass
 // leaves zero) and words of the caller's, kErrWords in all; null on failure.
-constexpr int kErrWords = 10;
+constexpr int kErrWords = 8;
 uint32_t *new_err(Scratch &scratch, cudaStream_t st);
 
 // The buffers for sums of n (1 <= n < 2^31) terms from one scratch
