@@ -580,8 +580,8 @@ __device__ __forceinline__ void pf_step_combine(const PfStepArgs &a,
                 : lane < 2 + AMD ? ld(&part->mon[lane - 2])
                 : lane < NV - 1  ? ld(&part->prev[lane - 2 - AMD])
                                  : ld(&part->prev_w);
-        if (M == INFINITY && lane < 2 + AMD)
-            tot += M - M;
+        if (M == INFINITY && lane < 2 + AMD) // (no FP64 operation)
+            tot = __longlong_as_double(0x7FF8000000000000ll);
         __syncthreads(); // sc.S is read
     } else {
         for (uint32_t b = threadIdx.x; b < nblk; b += blockDim.x)
