@@ -148,7 +148,8 @@ int vsmc_cuda_student_t_streams(int kind, const uint64_t key[4],
 /* u01 sequence array forms (rng/u01_sequence.hpp:53-89).  Replace
  * vsmc_rng_u01_sorted / _stratified / _systematic (vsmc.h:76-83).  The
  * sorted form's running log sum is the reference's left-to-right sum
- * bit for bit; log/exp come from CUDA's libm. */
+ * bit for bit; the logarithm is CUDA's, the exponential the
+ * library's own, both within an ulp. */
 int vsmc_cuda_u01_sorted(size_t n, const double *u01, double *u01seq,
     void *stream);
 int vsmc_cuda_u01_stratified(size_t n, const double *u01, double *u01seq,
@@ -212,8 +213,9 @@ int vsmc_cuda_resample_trans_residual(size_t m, size_t n,
 /* Resampling schemes with an engine: counts identical to the reference
  * functors for the same weights and engine state, and the engine advanced by
  * exactly the words the reference consumes.  Multinomial / Residual build
- * their sorted uniforms with CUDA's log/exp, so a uniform can differ from the
- * reference's in the last bit; every other scheme is bit-exact end to end.
+ * their sorted uniforms with a logarithm and an exponential of the library's
+ * own (within 0.55 ulp), so a uniform can differ from the reference's in the
+ * last bit; every other scheme is bit-exact end to end.
  * `rng` (host) is advanced; the call synchronizes the stream.  Philox4x32
  * engines only.  Replaces vsmc_resample_<scheme> and vsmc_resample
  * (vsmc.h:277-310, lib/src/vsmc_resample.cpp:84-116) and
@@ -290,7 +292,8 @@ int vsmc_cuda_state_copy_f64(size_t n, size_t dim, const int *index,
 /* The Weight class on device (core/weight.hpp:67-230).  W holds normalized
  * weights (n doubles); *ess_dev (device, 1 double) receives 1 / sum W^2.
  * Sums run left to right in the reference's order, so set() is bit-exact;
- * set_log / add_log use CUDA's exp / log.
+ * set_log / add_log take their exponentials and logarithms within an ulp (the
+ * library's own integer functions; CUDA's for arguments outside their range).
  *   set:       Weight::set (weight.hpp:115-120)     W = w / sum(w)
  *   set_log:   Weight::set_log (weight.hpp:145-149) W = exp(lw - max) normalized
  *   add_log:   Weight::add_log (weight.hpp:168-173) W = W * exp(l) normalized

@@ -36,7 +36,7 @@ def test_schemes_at_tile_edges(vc, port, scheme, m, n):
     vc.call("vsmc_cuda_rng_rand", ctypes.byref(r), 4, nxt.data_ptr(), None)
     got = host(rep)
     assert got.sum() == n
-    # multinomial and residual take CUDA's log and exp: a uniform may differ
+    # multinomial and residual take a log and an exp: a uniform may differ
     # in its last bit, which at these sizes moves no count
     assert np.array_equal(got, rep_ref)
     assert np.array_equal(host(nxt).view(np.uint32), next_ref)

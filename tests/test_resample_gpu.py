@@ -220,7 +220,7 @@ def test_schemes_counts_and_engine(vc, port, scheme, m, n):
     if scheme in EXACT:
         assert np.array_equal(got, rep_ref)
     else:
-        # sorted uniforms use CUDA's log / exp: a uniform may differ from the
+        # sorted uniforms take a log and an exp: a uniform may differ from the
         # reference's in its last bit, which can move one copy across a CDF
         # boundary; such moves must be rare and local
         diff = np.abs(got - rep_ref)

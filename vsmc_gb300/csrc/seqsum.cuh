@@ -41,8 +41,9 @@
 // add mantissas aligned to the warp's largest exponent (error below 2^-52 of
 // that element each), and increments are shifts.
 //
-// At n = 2^24: sums 27 us (x read at 4.9 TB/s), classify 53 us (bound by the
-// integer pipe, 40 us, and the serial walk), out 52 us (5.1 TB/s), against
+// At n = 2^24: sums 27 us (x read at 4.9 TB/s), classify 55 us (36 with the
+// ALU pipe 60 % busy, then the last block's serial walk), out 52 us (5.1 TB/s),
+// against
 // 0.46 ms for two generic scans (FP64 prefixes, then 16-byte increment
 // records) that moved 104 bytes per element.
 #pragma once
